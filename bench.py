@@ -489,10 +489,11 @@ def run_gpu(args, cfg, peaks, peak_kind):
         first, second = (rp, cp) if stage_raw["update.fused"][0] >= stage_raw["update.upsilon"][0] else (cp, rp)
         roof = dict(first)
         roof["other_kernel"] = second
-    elif rbf:
-        roof = tc_roof("sgemm_kernel (T = K_w Psi~^T, FP32 SIMT)", "update.psi", 2 * m_local * n * s, 74.4,
-                       "nominal FP32 SIMT (148 SMs x 128 FMA/clk x 2 x 1.965 GHz)", bound="fp32-simt")
-    elif a.precision:
+    elif not a.precision:
+        # the FP32 [Y|T] product: six BF16 tensor-core products per FP32 one
+        roof = tc_roof("gemm_x3_kernel (six BF16 products per FP32 product)", "update.fused",
+                       6 * 2 * m_local * n * (k + s), tc_peak, peak_kind)
+    else:
         # the two large kernels per window: [Y|T] on the tensor pipe and the X^T
         # product that streams the FP32 window (4 B read + 2 B BF16 copy written
         # per element); the one with more measured time is the roofline kernel
@@ -509,9 +510,6 @@ def run_gpu(args, cfg, peaks, peak_kind):
         first, second = (yt, xa) if stage_raw["update.fused"][0] >= stage_raw["update.upsilon"][0] else (xa, yt)
         roof = dict(first)
         roof["other_kernel"] = second
-    else:
-        roof = tc_roof("sgemm_kernel", "update.psi", 2 * m_local * n * s, 74.4,
-                       "nominal FP32 SIMT (148 SMs x 128 FMA/clk x 2 x 1.965 GHz)", bound="fp32-simt")
     if not sparse:
         roof["step_flops"] = step_flops
         roof["step_tflops"] = step_flops / (ms / 1e3) / 1e12

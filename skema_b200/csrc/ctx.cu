@@ -44,6 +44,9 @@ static void set_wait_limit(skema_ctx* c, int64_t ns) {
 
 void check_device_error(skema_ctx* c) {
   if (!c->dev_err_armed || !c->dev_err) return;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  SKEMA_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return;  // left for the next call outside the capture
   int h = 0;
   SKEMA_CUDA(cudaMemcpyAsync(&h, c->dev_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   SKEMA_CUDA(cudaStreamSynchronize(c->stream));
@@ -79,6 +82,16 @@ void* workspace(skema_ctx* c, size_t bytes) {
   SKEMA_CUDA(cudaMalloc(&c->ws, b));
   c->ws_bytes = b;
   return c->ws;
+}
+
+void* try_workspace(skema_ctx* c, size_t bytes) {
+  if (bytes <= c->ws_bytes) return c->ws;
+  try {
+    return workspace(c, bytes);
+  } catch (const Error& e) {
+    if (e.status != SKEMA_ENOMEM) throw;
+    return nullptr;
+  }
 }
 
 // A pitched copy whose rows lie back to back on both sides goes as one

@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "x3.h"
 
 namespace skema {
 
@@ -112,6 +113,9 @@ void dense_update(skema_ctx* c, Mat A, int64_t row0, int64_t nrows) {
     tc_dense_update(c, A, row0, nrows);
     return;
   }
+  if (c->p.precision == SKEMA_PREC_FP32 && c->p.dim_redux == SKEMA_MAP_GAUSS &&
+      x3_update(c, X3Input{A, nullptr}, row0, nrows))
+    return;
   const int64_t W = c->w;
   float* T = (float*)workspace(c, dense_scratch_bytes(c, std::min(W, nrows)));
   for (int64_t r = 0; r < nrows; r += W) {

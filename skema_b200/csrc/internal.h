@@ -47,6 +47,9 @@ struct Map {
   // Gauss: FP32 values; logical (r, c) at f32[r*rs + c*cs].
   float* f32 = nullptr;
   int64_t rs = 0, cs = 0;
+  // Imported values of 2^100 or more, or infinite: the products of this map
+  // stay on the SIMT kernels.
+  bool big = false;
   // Gauss, tensor-core forms: logical rows in row-major BF16 / FP8 copies.
   void* lowp = nullptr;
   // SparseSign: stored rows, zeta packed entries each: column | sign << 31.
@@ -219,6 +222,9 @@ class StageScope {
 };
 
 void* workspace(skema_ctx* c, size_t bytes);
+// The same, or nullptr when the limit or the device does not allow it (what
+// the context holds may have been given back by then).
+void* try_workspace(skema_ctx* c, size_t bytes);
 void* staging(skema_ctx* c, size_t bytes);
 bool y_rows_clean(const skema_ctx* c, int64_t a, int64_t b);
 void y_rows_mark(skema_ctx* c, int64_t a, int64_t b);

@@ -236,6 +236,7 @@ void map_import(skema_ctx* c, Map& mp, const double* values, const int32_t* indi
     gauss_import_kernel<<<grid_for(total, threads, c->sm_count), threads, 0, c->stream>>>(
         mp.f32, d, mp.lrows, mp.lcols, mp.rs, mp.cs, mp.nrow, mp.transposed ? 1 : 0);
     SKEMA_LAUNCHED(c);
+    mp.big = std::any_of(values, values + total, [](double v) { return std::fabs(v) >= 0x1p100; });
     SKEMA_CUDA(cudaStreamSynchronize(c->stream));
     return;
   }

@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "x3.h"
 
 namespace skema {
 
@@ -130,6 +131,75 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Kernel rows as the row-blocked BF16 planes of the tensor-core FP32 form
+// (x3.h): K is split where it is made, so it is written once (6 bytes) and
+// never as FP32. 64 rows x 128 points per CTA, 4 x 8 per thread: a thread's
+// four rows are adjacent, so 16 lanes write one 128-byte line of a plane, and
+// three 16-byte shared loads feed 32 differences. FCONTIG: a point's features
+// are contiguous (pcs = 1).
+template <bool FCONTIG>
+__global__ void __launch_bounds__(256, 2)
+    rbf_planes_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N, int64_t d, float gamma,
+                      int64_t R0, int64_t wr, __nv_bfloat16* __restrict__ out, int64_t pstride) {
+  constexpr int TI = 64, TJ = 128, F = 16;
+  __shared__ __align__(16) float xi[F][TI + 4];
+  __shared__ __align__(16) float xj[F][TJ + 4];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int64_t tiles_j = (N + TJ - 1) / TJ, tiles_i = (wr + TI - 1) / TI;
+  for (int64_t tile = blockIdx.x; tile < tiles_i * tiles_j; tile += gridDim.x) {
+    const int64_t ib = tile / tiles_j, i0 = ib * TI, j0 = (tile - ib * tiles_j) * TJ;
+    float acc[4][8];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
+    for (int64_t f0 = 0; f0 < d; f0 += F) {
+#pragma unroll
+      for (int q = 0; q < F * (TI + TJ) / 256; ++q) {
+        const int e = threadIdx.x + 256 * q;
+        const int ff = FCONTIG ? e % F : e / (TI + TJ), rr = FCONTIG ? e / F : e % (TI + TJ);
+        const int64_t f = f0 + ff;
+        if (rr < TI)
+          xi[ff][rr] = (f < d && i0 + rr < wr) ? P[(R0 + i0 + rr) * prs + f * pcs] : 0.f;
+        else
+          xj[ff][rr - TI] = (f < d && j0 + rr - TI < N) ? P[(j0 + rr - TI) * prs + f * pcs] : 0.f;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int ff = 0; ff < F; ++ff) {
+        const float4 a4 = *reinterpret_cast<const float4*>(&xi[ff][4 * tx]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&xj[ff][8 * ty]);
+        const float4 c4 = *reinterpret_cast<const float4*>(&xj[ff][8 * ty + 4]);
+        const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+        const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            const float df = a[u] - b[v];
+            acc[u][v] = fmaf(df, df, acc[u][v]);
+          }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const int64_t gj = j0 + 8 * ty + v;
+      if (gj >= N) break;
+      __nv_bfloat16 q[3][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t li = i0 + 4 * tx + u;
+        const float kv = li >= wr ? 0.f : (gj == R0 + li) ? 1.f : expf(-gamma * acc[u][v]);
+        tc::split3(kv, q[0][u], q[1][u], q[2][u]);
+      }
+      __nv_bfloat16* dp = out + (ib * N + gj) * 64 + 4 * tx;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dp + p * pstride) = *reinterpret_cast<const uint2*>(q[p]);
+    }
+  }
+}
+
 // dX = -2 gamma * (r o X - S), r = rsum + csum (N), S = S1 + S2 (N x d).
 __global__ void rbf_dx_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N,
                               int64_t d, float gamma, const float* __restrict__ rsum,
@@ -187,6 +257,16 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
   const int64_t W = c->w;
   const int64_t N = npts;
   const float gamma = (float)c->p.kernel_gamma;
+  if (c->p.precision == SKEMA_PREC_FP32 && c->p.dim_redux == SKEMA_MAP_GAUSS && gamma >= 0.f) {
+    X3Input in{Mat{nullptr, 0, 0}, [&](int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride) {
+                 const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
+                 auto kern = P.cs == 1 ? rbf_planes_kernel<true> : rbf_planes_kernel<false>;
+                 kern<<<grid_cap(c, tiles, 8), 256, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr, planes,
+                                                                    pstride);
+                 SKEMA_LAUNCHED(c);
+               }};
+    if (x3_update(c, in, row0, nrows)) return;
+  }
   const int64_t wmax = std::min(W, nrows);
   const size_t kbytes = (sizeof(float) * (size_t)(wmax * N) + 255) / 256 * 256;
   char* ws = (char*)workspace(c, kbytes + dense_scratch_bytes(c, wmax));

@@ -1,0 +1,384 @@
+// x3.cu -- the FP32 form of the dense and kernel sketch on the tensor cores
+// (update(dense, Gauss), src/Skema_SketchySVD.cpp:256-268, and the Gauss-RBF
+// window), by three BF16 planes per FP32 operand (tc_x3.cuh).
+//
+// Per block of rows [R0, R0 + wr) of the input:
+//   planes of A_w        row-blocked (64-row blocks, a 128-byte line of 64
+//                        rows per column), written once, read by both products
+//   [Y_w | T] = A_w [Omega~; Psi~]^T   M = wr, N = k + s, K = n
+//   X^T += eta A_w^T Upsilon~_w^T      M = n,  N = k,     K = wr
+//   Z^T += eta T^T Phi~_w^T            M = s,  N = s,     K = wr
+// T stays in planes. Blocks need not follow the windows: with
+// X = nu X + eta x_w after each of G windows, X = nu^G X + eta sum_w
+// nu^(G-1-w) x_w, so the weights go into the converted columns of Upsilon~
+// and Phi~, and a call of many short windows is one block.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "internal.h"
+#include "tc_host.h"
+#include "tc_x3.cuh"
+#include "x3.h"
+
+namespace skema {
+
+namespace {
+
+// |x| at or above this (2^100) leaves the range in which planes and sums are
+// certain to stay finite (infinities included; a NaN is a NaN in its planes
+// too and passes): the block is then formed by x3_plain_kernel instead.
+constexpr uint32_t kBigBits = 0x71800000u;  // 2^100
+__device__ __forceinline__ bool too_big(float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+  return b >= kBigBits && b <= 0x7f800000u;
+}
+
+__device__ __forceinline__ void store_planes8(const float* v, __nv_bfloat16* d, int64_t pstride) {
+  __nv_bfloat16 q[3][8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) tc::split3(v[t], q[0][t], q[1][t], q[2][t]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(d + p * pstride) = *reinterpret_cast<const uint4*>(q[p]);
+}
+
+// A window block into row-blocked planes; rows past `rows` in the last 64 are
+// zeros. VEC: rows contiguous and 16-byte aligned (a thread: 8 rows of one
+// column, two 16-byte loads, three 16-byte stores). 10 bytes per element, HBM
+// bound.
+__global__ void __launch_bounds__(256)
+    x3_block_vec_kernel(const float* __restrict__ S, int64_t scs, int64_t rows, int64_t cols,
+                        __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t* __restrict__ flag) {
+  const int64_t total = nrb * 8 * cols;
+  bool big = false;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+    // 64-row block outermost, then columns, then the 8 groups of a line: a
+    // warp's stores are 512 contiguous bytes per plane
+    const int64_t rb = q / (8 * cols), w = q - rb * 8 * cols, j = w >> 3, i = rb * 64 + (w & 7) * 8;
+    const float* sp = S + i + j * scs;
+    float v[8];
+    if (i + 8 <= rows) {
+      const float4 a = __ldcs(reinterpret_cast<const float4*>(sp));
+      const float4 b = __ldcs(reinterpret_cast<const float4*>(sp + 4));
+      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; ++t) v[t] = (i + t < rows) ? sp[t] : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) big |= too_big(v[t]);
+    store_planes8(v, D + (rb * cols + j) * 64 + (w & 7) * 8, pstride);
+  }
+  if (big) atomicOr(flag, 1u);
+}
+
+// The same from any strides, by 64 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256)
+    x3_block_tiled_kernel(const float* __restrict__ S, int64_t srs, int64_t scs, int64_t rows, int64_t cols,
+                          __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t* __restrict__ flag) {
+  __shared__ float tile[32][65];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t tj = (cols + 31) / 32;
+  const bool rowfast = srs <= scs;
+  bool big = false;
+  for (int64_t t = blockIdx.x; t < nrb * tj; t += gridDim.x) {
+    const int64_t rb = t / tj, j0 = (t - rb * tj) * 32;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = ty + 8 * q;  // 0 .. 63: (32-row half, column) or row
+      const int r = rowfast ? tx + 32 * (e >> 5) : e, j = rowfast ? (e & 31) : tx;
+      const int64_t gi = rb * 64 + r, gj = j0 + j;
+      const float v = (gi < rows && gj < cols) ? S[gi * srs + gj * scs] : 0.f;
+      big |= too_big(v);
+      tile[j][r] = v;
+    }
+    __syncthreads();
+    const int j = threadIdx.x >> 3, g8 = (threadIdx.x & 7) * 8;
+    if (j0 + j < cols) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = tile[j][g8 + e];
+      store_planes8(v, D + (rb * cols + j0 + j) * 64 + g8, pstride);
+    }
+    __syncthreads();
+  }
+  if (big) atomicOr(flag, 1u);
+}
+
+// Map columns [0, cols) of up to two row-contiguous FP32 sources into one
+// stack of K-major planes, row r of plane q at D[q * pstride + r * ld]. Column
+// j is scaled by nu^(nwin - 1 - (j0 + j) / W) (nu = 1: unscaled).
+struct X3Src {
+  const float* p;
+  int64_t rs, rows;
+};
+__global__ void __launch_bounds__(256)
+    x3_maps_kernel(X3Src a, X3Src b, int64_t cols, __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu,
+                   int64_t W, int64_t nwin, int64_t j0) {
+  const int64_t c8 = ld / 8, total = (a.rows + b.rows) * c8;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = q / c8, j = (q - r * c8) * 8;
+    const float* sp = (r < a.rows ? a.p + r * a.rs : b.p + (r - a.rows) * b.rs) + j;
+    float v[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) v[t] = (j + t < cols) ? sp[t] : 0.f;
+    if (nu != 1.f) {
+      int64_t w = -1;
+      float s = 1.f;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const int64_t wt = (j0 + j + t) / W;
+        if (wt != w) w = wt, s = (float)pow((double)nu, (double)max((int64_t)0, nwin - 1 - wt));
+        v[t] *= s;
+      }
+    }
+    store_planes8(v, D + r * ld + j, pstride);
+  }
+}
+
+// C = alpha op + beta C in plain FP32 for the rare block that too_big()
+// refuses (returns at once otherwise): 64 x 64 tiles, up to three products
+// per launch. A(i, kk) is scaled by the window weight of kk when nu != 1.
+struct X3Plain {
+  const float* A;
+  int64_t ars, acs;
+  const float* B;
+  int64_t brs, bcs;
+  float* C;
+  int64_t crs, ccs;
+  int64_t M, N, K;
+  float alpha, beta, nu;
+  int64_t W, nwin, j0;
+};
+struct X3Plain3 {
+  X3Plain g[3];
+  int n;
+};
+__global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_t* __restrict__ flag) {
+  if (*flag == 0) return;
+  __shared__ float As[16][65], Bs[16][65];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  for (int w = 0; w < a.n; ++w) {
+    const X3Plain& g = a.g[w];
+    const int64_t tm = (g.M + 63) / 64, tn = (g.N + 63) / 64;
+    for (int64_t t = blockIdx.x; t < tm * tn; t += gridDim.x) {
+      const int64_t m0 = (t / tn) * 64, n0 = (t % tn) * 64;
+      float acc[4][4] = {};
+      for (int64_t k0 = 0; k0 < g.K; k0 += 16) {
+        for (int q = threadIdx.x; q < 1024; q += 256) {
+          const int r = q & 63, kk = q >> 6;
+          const int64_t k = k0 + kk;
+          float av = (m0 + r < g.M && k < g.K) ? g.A[(m0 + r) * g.ars + k * g.acs] : 0.f;
+          if (g.nu != 1.f && k < g.K)
+            av *= (float)pow((double)g.nu, (double)(g.nwin - 1 - (g.j0 + k) / g.W));
+          As[kk][r] = av;
+          Bs[kk][r] = (n0 + r < g.N && k < g.K) ? g.B[k * g.brs + (n0 + r) * g.bcs] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < 16; ++kk)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(As[kk][ty + 16 * i], Bs[kk][tx + 16 * j], acc[i][j]);
+        __syncthreads();
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int64_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+          if (m >= g.M || n >= g.N) continue;
+          float* p = g.C + m * g.crs + n * g.ccs;
+          *p = g.beta == 0.f ? g.alpha * acc[i][j] : fmaf(g.beta, *p, g.alpha * acc[i][j]);
+        }
+    }
+  }
+}
+
+int grid_1d(const skema_ctx* c, int64_t items, int per_sm) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, (int64_t)c->sm_count * per_sm));
+}
+
+size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+CUtensorMap tmap_planes_k(const __nv_bfloat16* p, int64_t K, int64_t rows, int64_t ld, int64_t pstride, uint32_t brows,
+                          uint32_t bplanes) {
+  return tmap_3d(CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, p, (uint64_t)K, (uint64_t)rows, 3, (uint64_t)ld * 2,
+                 (uint64_t)pstride * 2, tc::kX3BK, brows, bplanes, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+constexpr size_t kX3Smem = 226 * 1024;
+
+}  // namespace
+
+size_t x3_part_bytes(const skema_ctx* c) {
+  return (size_t)2 * c->sm_count * 256 * tc::BM * sizeof(float);
+}
+
+void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int64_t K, const tc::X3Out& o, float* part,
+             const uint32_t* flag) {
+  if (M <= 0 || N <= 0 || K <= 0) return;
+  tc::X3Grid g;
+  g.mtiles = (int)((M + tc::BM - 1) / tc::BM);
+  g.ntiles = (int)((N + 255) / 256);
+  g.nt = (int)((N + (int64_t)g.ntiles * 16 - 1) / ((int64_t)g.ntiles * 16) * 16);
+  g.ksteps = (int)((K + tc::kX3BK - 1) / tc::kX3BK);
+  const size_t stage = tc::kX3ABytes + (size_t)3 * g.nt * tc::kX3BK * 2;
+  g.stages = (int)std::min<size_t>(tc::kX3MaxStages, (kX3Smem - 2048) / stage);
+  const int64_t tiles = (int64_t)g.mtiles * g.ntiles;
+  // a run of at least four K steps per CTA
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>(c->sm_count, tiles * g.ksteps / 4));
+  g.full = (int)(tiles / G * G);
+  CUtensorMap ta;
+  if (a.blocked)
+    ta = tmap_3d(CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.p, 64, (uint64_t)a.cols, (uint64_t)(3 * a.nrb), 128,
+                 (uint64_t)a.cols * 128, a.mn ? 64 : tc::kX3BK, a.mn ? tc::kX3BK : tc::BM, 1,
+                 a.mn ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+  else
+    ta = tmap_planes_k(a.p, K, M, a.ld, a.pstride, tc::BM, 1);
+  const CUtensorMap tb = tmap_planes_k(b.p, K, N, b.ld, b.pstride, (uint32_t)g.nt, 3);
+  auto kern = a.mn ? tc::gemm_x3_kernel<true> : tc::gemm_x3_kernel<false>;
+  SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kX3Smem));
+  kern<<<G, tc::kX3Threads, kX3Smem, c->stream>>>(ta, tb, g, o, a.blocked ? 1 : 0, (int)a.nrb, part, flag, c->dev_err);
+  SKEMA_LAUNCHED(c);
+  c->dev_err_armed = true;
+  const int rem = (int)(tiles - g.full);
+  if (rem > 0) {
+    tc::x3_reduce_kernel<<<dim3(rem, g.nt / 16), 256, 0, c->stream>>>(g, o, G, part, flag);
+    SKEMA_LAUNCHED(c);
+  }
+}
+
+void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
+                     uint32_t* flag) {
+  const int64_t nrb = (rows + 63) / 64;
+  if (src.rs == 1 && src.cs % 4 == 0 && reinterpret_cast<uintptr_t>(src.p) % 16 == 0)
+    x3_block_vec_kernel<<<grid_1d(c, nrb * 8 * cols, 16), 256, 0, c->stream>>>(src.p, src.cs, rows, cols, D, nrb,
+                                                                               pstride, flag);
+  else
+    x3_block_tiled_kernel<<<grid_1d(c, nrb * ((cols + 31) / 32) * 256, 16), 256, 0, c->stream>>>(
+        src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, flag);
+  SKEMA_LAUNCHED(c);
+}
+
+bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
+  const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w;
+  const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
+  if (nrows <= 0 || !(nu > 0.f)) return false;
+  for (const Map* mp : {&c->ups, &c->omg, &c->phi, &c->psi})
+    if (mp->big) return false;
+  // below this the launches and conversions cost more than the products
+  if ((double)nrows * (double)n * (double)(2 * k + s) < 2e7) return false;
+  const int64_t ldn = pad8(n);
+  const size_t b_op = up256(sizeof(__nv_bfloat16) * (size_t)(3 * (k + s) * ldn));
+  const size_t b_part = up256(x3_part_bytes(c));
+  // rows per block: all of them, or equal blocks whose planes fit the budget
+  int64_t rb = 0;
+  char* ws = nullptr;
+  size_t b_a = 0, b_uf = 0, b_t = 0, b_t32 = 0, b_flag = 0;
+  for (size_t budget = (size_t)2 << 30; budget >= ((size_t)64 << 20) && !ws; budget >>= 2) {
+    const int64_t cap = std::max<int64_t>(64, (int64_t)(budget / (size_t)(6 * n)) / 64 * 64);
+    const int64_t nb = (nrows + cap - 1) / cap;
+    rb = ((nrows + nb - 1) / nb + 63) / 64 * 64;
+    b_a = up256(sizeof(__nv_bfloat16) * (size_t)(3 * rb * n));
+    b_uf = up256(sizeof(__nv_bfloat16) * (size_t)(3 * (k + s) * rb));
+    b_t = up256(sizeof(__nv_bfloat16) * (size_t)(3 * s * rb));
+    b_t32 = in.A.p ? up256(sizeof(float) * (size_t)(s * rb)) : 0;
+    b_flag = up256(sizeof(uint32_t) * (size_t)((nrows + rb - 1) / rb));
+    ws = static_cast<char*>(try_workspace(c, b_op + b_part + b_a + b_uf + b_t + b_t32 + b_flag));
+    if (cap == 64) break;
+  }
+  if (!ws) return false;
+  auto take = [&](size_t bytes) {
+    char* p = ws;
+    ws += bytes;
+    return p;
+  };
+  __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(take(b_op));
+  float* part = reinterpret_cast<float*>(take(b_part));
+  __nv_bfloat16* Ap = reinterpret_cast<__nv_bfloat16*>(take(b_a));
+  __nv_bfloat16* uf = reinterpret_cast<__nv_bfloat16*>(take(b_uf));
+  __nv_bfloat16* Tp = reinterpret_cast<__nv_bfloat16*>(take(b_t));
+  float* T32 = reinterpret_cast<float*>(take(b_t32));
+  uint32_t* flags = in.A.p ? reinterpret_cast<uint32_t*>(take(b_flag)) : nullptr;
+
+  const int64_t nwin = (nrows + W - 1) / W;
+  const float ybeta = y_beta(c, row0, row0 + nrows, nu);
+  const float xbeta = (float)std::pow((double)nu, (double)nwin);
+  if (flags) SKEMA_CUDA(cudaMemsetAsync(flags, 0, b_flag, c->stream));
+  {
+    StageScope st(c, ST_WINDOW);
+    const X3Src so{c->omg.f32, c->omg.rs, k}, sp{c->psi.f32, c->psi.rs, s};
+    x3_maps_kernel<<<grid_1d(c, (k + s) * ldn / 8, 16), 256, 0, c->stream>>>(so, sp, n, op, ldn, (k + s) * ldn, 1.f, 1,
+                                                                            1, 0);
+    SKEMA_LAUNCHED(c);
+  }
+  for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
+    const int64_t wr = std::min(rb, nrows - r), R0 = row0 + r;
+    const int64_t nrb = (wr + 63) / 64, ldw = pad8(wr), ps = nrb * 64 * n;
+    uint32_t* flag = flags ? flags + i : nullptr;
+    const Mat Aw{in.A.p ? in.A.p + r * in.A.rs : nullptr, in.A.rs, in.A.cs};
+    {
+      StageScope st(c, ST_WINDOW);
+      if (in.A.p)
+        x3_block_planes(c, Aw, wr, n, Ap, ps, flag);
+      else
+        in.fill(R0, wr, Ap, ps);
+      if (s > 0) {
+        const X3Src su{c->ups.f32 + R0, c->ups.rs, k}, sf{c->phi.f32 + R0, c->phi.rs, s};  // cs = 1
+        x3_maps_kernel<<<grid_1d(c, (k + s) * ldw / 8, 16), 256, 0, c->stream>>>(su, sf, wr, uf, ldw, (k + s) * ldw, nu,
+                                                                                W, nwin, r);
+        SKEMA_LAUNCHED(c);
+      }
+    }
+    const X3A an{Ap, true, true, n, nrb, 0, 0}, at{Ap, true, false, n, nrb, 0, 0};
+    {
+      StageScope st(c, s > 0 ? ST_FUSED : ST_OMEGA);
+      x3_gemm(c, an, X3B{op, ldn, (k + s) * ldn}, wr, k + s, n,
+              tc::X3Out{c->Y + R0, 1, c->m, eta, ybeta, Tp, ldw, s * ldw, wr, k, k + s}, part, flag);
+    }
+    if (s > 0) {
+      const float xb = i == 0 ? xbeta : 1.f;
+      {
+        StageScope st(c, ST_UPSILON);
+        x3_gemm(c, at, X3B{uf, ldw, (k + s) * ldw}, n, k, wr, tc::X3Out{c->X, 1, n, eta, xb, nullptr, 0, 0, n, k, k},
+                part, flag);
+      }
+      StageScope st(c, ST_PHI);
+      x3_gemm(c, X3A{Tp, false, false, 0, 0, ldw, s * ldw}, X3B{uf + k * ldw, ldw, (k + s) * ldw}, s, s, wr,
+              tc::X3Out{c->Z, 1, s, eta, xb, nullptr, 0, 0, s, s, s}, part, flag);
+    }
+    if (flag) {
+      const int64_t j0 = r;
+      const float xb = i == 0 ? xbeta : 1.f;
+      X3Plain3 p;
+      p.g[0] = X3Plain{Aw.p, Aw.rs, Aw.cs, c->omg.f32, c->omg.cs, c->omg.rs, c->Y + R0, 1, c->m,
+                       wr, k, n, eta, ybeta, 1.f, 1, 1, 0};
+      p.n = 1;
+      if (s > 0) {
+        p.g[1] = X3Plain{Aw.p, Aw.rs, Aw.cs, c->psi.f32, c->psi.cs, c->psi.rs, T32, 1, wr,
+                         wr, s, n, 1.f, 0.f, 1.f, 1, 1, 0};
+        p.g[2] = X3Plain{c->ups.f32 + R0, c->ups.rs, 1, Aw.p, Aw.rs, Aw.cs, c->X, n, 1,
+                         k, n, wr, eta, xb, nu, W, nwin, j0};
+        p.n = 3;
+      }
+      x3_plain_kernel<<<2 * c->sm_count, 256, 0, c->stream>>>(p, flag);
+      SKEMA_LAUNCHED(c);
+      if (s > 0) {
+        X3Plain3 z;
+        z.g[0] = X3Plain{c->phi.f32 + R0, c->phi.rs, 1, T32, 1, wr, c->Z, s, 1,
+                         s, s, wr, eta, xb, nu, W, nwin, j0};
+        z.n = 1;
+        x3_plain_kernel<<<c->sm_count, 256, 0, c->stream>>>(z, flag);
+        SKEMA_LAUNCHED(c);
+      }
+    }
+  }
+  y_rows_mark(c, row0, row0 + nrows);
+  return true;
+}
+
+}  // namespace skema

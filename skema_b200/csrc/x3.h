@@ -1,0 +1,60 @@
+// x3.h -- FP32 products on the tensor cores through three BF16 planes per
+// operand (x3.cu, tc_x3.cuh).
+#pragma once
+#include <cuda_bf16.h>
+
+#include <functional>
+
+#include "internal.h"
+
+namespace skema {
+
+namespace tc {
+struct X3Out;
+
+// x as the sum of three BF16 values
+__device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
+  h = __float2bfloat16(x);
+  const float r = x - __bfloat162float(h);
+  m = __float2bfloat16(r);
+  l = __float2bfloat16(r - __bfloat162float(m));
+}
+}  // namespace tc
+
+// The M-side operand. blocked: the row-blocked window planes (element (i, j)
+// of plane q at p[((q nrb + i / 64) cols + j) 64 + i % 64]), with the output's
+// rows along i (mn) or along j; else K-major rows of ld elements, pstride
+// between planes.
+struct X3A {
+  const __nv_bfloat16* p;
+  bool blocked, mn;
+  int64_t cols, nrb, ld, pstride;
+};
+// The N-side operand: K-major rows.
+struct X3B {
+  const __nv_bfloat16* p;
+  int64_t ld, pstride;
+};
+// Room for the parts of cut tiles.
+size_t x3_part_bytes(const skema_ctx* c);
+// acc(i, j) = sum_kk A(i, kk) B(j, kk) into o; nothing when *flag (may be
+// null) is set.
+void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int64_t K, const tc::X3Out& o, float* part,
+             const uint32_t* flag);
+// A strided FP32 block into row-blocked planes (zero rows up to a multiple of
+// 64); sets *flag when a value is out of the planes' range.
+void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
+                     uint32_t* flag);
+
+// One call's input: a dense matrix, or a filler of window planes (A.p null)
+// whose values are at most 1 in magnitude or NaN.
+struct X3Input {
+  Mat A;
+  std::function<void(int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride)> fill;
+};
+// All windows of one call of a Gauss-map FP32 context. False (and nothing
+// done) when the call is small, its workspace is not to be had, or nu or the
+// maps are outside the form's range: the caller then takes the SIMT form.
+bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows);
+
+}  // namespace skema
