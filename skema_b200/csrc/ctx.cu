@@ -841,6 +841,9 @@ int skema_get_sketch(skema_ctx* c, int32_t which, float* buf, int64_t ld, int32_
     if (want_row == irow) {
       SKEMA_CUDA(copy2d(buf, sizeof(float) * ld, src, sizeof(float) * inner,
                                    sizeof(float) * inner, outer, kind, c->stream));
+    } else if (mem == SKEMA_MEM_DEVICE && (want_row ? cols : rows) <= 256 && ld == (want_row ? cols : rows)) {
+      // a dense fetch of a tall sketch (Y by rows, X by columns)
+      transpose_narrow(c, src, inner, outer, inner, buf, c->stream);
     } else if (mem == SKEMA_MEM_DEVICE) {
       copy_block(c, sm, want_row ? MatOut{buf, ld, 1} : MatOut{buf, 1, ld}, rows, cols);
     } else {
