@@ -20,6 +20,8 @@
 #include <cmath>
 
 #include "internal.h"
+#include "tc_x3.cuh"
+#include "x3.h"
 
 namespace skema {
 
@@ -340,6 +342,191 @@ __global__ void csr_gauss_scatter_kernel(const int64_t* __restrict__ rowptr,
   }
 }
 
+// CSR x Gauss for all windows of a call: rows of [Y | T] = A [Omega Psi], 32
+// rows per CTA. A warp takes a row of the tile at a time (from a counter, so
+// a long row holds up one warp only) and its lanes hold up to 192 output
+// columns, six each. The tile is turned in shared memory, so that Y (column
+// major) and T leave as lines of 32 rows. T goes out as the three BF16 planes
+// of the tensor-core product Z += Phi^T T (T32 null), or as FP32 columns of
+// ldt when a value left the planes' range (run again under *cond).
+// Bound by the gathered bytes, 4 (k + s) per nonzero out of L2: 100,000 x
+// 20,000 with 1e6 nonzeros at k = 81, s = 163 takes 178 us, 5.4 TB/s. With all
+// 244 columns in one pass of eight slots it took 338 (the loads of a group not
+// all in flight) and 588 us (144 registers, one CTA per SM); 64 registers and
+// four CTAs per SM are what pays.
+struct GaussGather {
+  const int64_t* rowptr;
+  const int32_t* col;
+  const float* val;
+  int64_t col_offset, nrows, ncol;
+  const float* omg;  // ncol x k
+  const float* psi;  // ncol x s
+  int64_t k, s;
+  float* Y;  // column-major; null: T only
+  int64_t ldy;
+  float alpha, beta;
+  __nv_bfloat16* T;
+  float* T32;
+  int64_t ldt, pstride;
+  uint32_t* big;  // set when |T| >= 2^100 or infinite
+};
+// One row against NU x 32 columns of a map: acc[u] = sum_p a_p map(j_p, c0 +
+// lane + 32 u), cols columns left from c0 on. 32 entries are loaded at once,
+// one per lane, and go through four at a time: 4 NU loads per lane in flight,
+// at one address and constant offsets per entry.
+template <int NU>
+__device__ __forceinline__ void gauss_row(const GaussGather& g, int64_t b, int64_t e, const float* __restrict__ map,
+                                          int64_t stride, int cols, int lane, float* acc) {
+  constexpr int Q = NU > 4 ? 2 : 4;
+  const bool last = lane + 32 * (NU - 1) < cols;
+#pragma unroll
+  for (int u = 0; u < NU; ++u) acc[u] = 0.f;
+  for (int64_t p0 = b; p0 < e; p0 += 32) {
+    const int cnt = (int)min((int64_t)32, e - p0);
+    int32_t jl = -1;
+    float al = 0.f;
+    if (lane < cnt) jl = __ldg(g.col + p0 + lane), al = __ldg(g.val + p0 + lane);
+    if ((uint64_t)(int64_t)jl >= (uint64_t)g.ncol) jl = -1;
+    for (int p = 0; p < cnt; p += Q) {
+      float m[Q][NU], a[Q];
+      int32_t j[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        j[q] = __shfl_sync(0xffffffffu, jl, p + q);
+        a[q] = __shfl_sync(0xffffffffu, al, p + q);
+        const float* mp = map + (int64_t)max(j[q], 0) * stride + lane;
+#pragma unroll
+        for (int u = 0; u < NU; ++u) m[q][u] = (u < NU - 1 || last) ? __ldg(mp + 32 * u) : 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (j[q] >= 0) {  // an entry outside the matrix adds nothing
+#pragma unroll
+          for (int u = 0; u < NU; ++u) acc[u] = fmaf(a[q], m[q][u], acc[u]);
+        }
+    }
+  }
+}
+
+template <int NU>
+__device__ __forceinline__ void gauss_tile(const GaussGather& g, int64_t r0, int nr, const float* map, int64_t stride,
+                                           int cols, int lane, int* next, float* tile) {
+  while (true) {
+    int i = 0;
+    if (lane == 0) i = atomicAdd(next, 1);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= nr) return;
+    float acc[NU];
+    gauss_row<NU>(g, g.rowptr[r0 + i] - g.col_offset, g.rowptr[r0 + i + 1] - g.col_offset, map, stride, cols, lane, acc);
+#pragma unroll
+    for (int u = 0; u < NU; ++u) tile[(lane + 32 * u) * 33 + i] = acc[u];
+  }
+}
+
+__global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g, const uint32_t* __restrict__ cond) {
+  if (cond && *cond == 0) return;
+  constexpr int CH = 192;  // columns per pass
+  extern __shared__ float gg_tile[];  // CH x 33
+  __shared__ int next;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * 32;
+  const int nr = (int)min((int64_t)32, g.nrows - r0);
+  bool big = false;
+  // the columns of Omega, then those of Psi
+  for (int64_t c = g.Y ? 0 : g.k; c < g.k + g.s;) {
+    const bool om = c < g.k;
+    const int64_t c0 = om ? c : c - g.k, width = om ? g.k : g.s;
+    const int cols = (int)min((int64_t)CH, width - c0);
+    const float* map = (om ? g.omg : g.psi) + c0;
+    if (threadIdx.x == 0) next = 0;
+    __syncthreads();
+    switch ((cols + 31) / 32) {
+      case 1: gauss_tile<1>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+      case 2: gauss_tile<2>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+      case 3: gauss_tile<3>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+      case 4: gauss_tile<4>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+      case 5: gauss_tile<5>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+      default: gauss_tile<6>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
+    }
+    __syncthreads();
+    for (int cl = warp; cl < cols; cl += 8) {
+      const float v = gg_tile[cl * 33 + lane];
+      if (lane >= nr) continue;
+      if (om) {
+        float* yp = g.Y + r0 + lane + (c0 + cl) * g.ldy;
+        *yp = (g.beta == 0.f) ? g.alpha * v : fmaf(g.beta, *yp, g.alpha * v);
+      } else if (g.T32) {
+        g.T32[(c0 + cl) * g.ldt + r0 + lane] = v;
+      } else {
+        const uint32_t bits = __float_as_uint(v) & 0x7fffffffu;
+        big |= bits >= 0x71800000u && bits <= 0x7f800000u;
+        __nv_bfloat16 h, m, l;
+        tc::split3(v, h, m, l);
+        __nv_bfloat16* tp = g.T + (c0 + cl) * g.ldt + r0 + lane;
+        tp[0] = h, tp[g.pstride] = m, tp[2 * g.pstride] = l;
+      }
+    }
+    __syncthreads();
+    c += cols;
+  }
+  if (big) atomicOr(g.big, 1u);
+}
+
+// X^T(j, :) += w_i a_ij Upsilon(i, :) into a zeroed n x kp scratch (kp a
+// multiple of 4), w_i = nu^(windows after row i): a warp per row, one 16-byte
+// reduction per four columns and nonzero. The rows of X itself are n apart, so
+// its columns would take one 4-byte reduction in a sector of its own each
+// (that form, with the same for Phi, took 174 us per 10,000 rows; this one
+// takes 83 us for 100,000).
+__global__ void __launch_bounds__(256)
+    csr_gauss_xt_kernel(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                        const float* __restrict__ val, int64_t col_offset, int64_t nrows, int64_t ncol,
+                        const float* __restrict__ ups, int64_t k, int64_t kp, float* __restrict__ XT, float nu,
+                        int64_t W, int64_t nwin) {
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = gw; i < nrows; i += nwarps) {
+    const int64_t b = rowptr[i] - col_offset, e = rowptr[i + 1] - col_offset;
+    if (b >= e) continue;
+    float w = 1.f;
+    if (nu != 1.f) w = (float)pow((double)nu, (double)(nwin - 1 - i / W));
+    for (int64_t c = 4 * lane; c < kp; c += 128) {
+      float u[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) u[q] = c + q < k ? w * __ldg(ups + i * k + c + q) : 0.f;
+      for (int64_t p = b; p < e; ++p) {
+        const int32_t j = __ldg(col + p);
+        if ((uint64_t)(int64_t)j >= (uint64_t)ncol) continue;
+        const float a = __ldg(val + p);
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(XT + (int64_t)j * kp + c), "f"(a * u[0]),
+                     "f"(a * u[1]), "f"(a * u[2]), "f"(a * u[3])
+                     : "memory");
+      }
+    }
+  }
+}
+
+// X(r, j) = beta X + alpha XT(j, r), by 32 x 32 tiles.
+__global__ void __launch_bounds__(256) xt_add_kernel(const float* __restrict__ XT, int64_t kp, int64_t k, int64_t n,
+                                                     float* __restrict__ X, float alpha, float beta) {
+  __shared__ float t[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t tk = (k + 31) / 32, tn = (n + 31) / 32;
+  for (int64_t q = blockIdx.x; q < tk * tn; q += gridDim.x) {
+    const int64_t r0 = (q % tk) * 32, j0 = (q / tk) * 32;
+    for (int y = ty; y < 32; y += 8)
+      if (j0 + y < n && r0 + tx < k) t[y][tx] = XT[(j0 + y) * kp + r0 + tx];
+    __syncthreads();
+    for (int y = ty; y < 32; y += 8)
+      if (r0 + y < k && j0 + tx < n) {
+        float* p = X + (r0 + y) * n + j0 + tx;
+        *p = beta == 0.f ? alpha * t[tx][y] : fmaf(beta, *p, alpha * t[tx][y]);
+      }
+    __syncthreads();
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Dense window x SparseSign (three-sketch, dense input, update(dense,
 // SparseSign) src/Skema_SketchySVD.cpp:271-293).
@@ -517,6 +704,81 @@ static void launch_csr_ssign_y(skema_ctx* c, const int64_t* rowptr, const int32_
   launch_csr_ssign_y_variant<4>(c, wpb, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta);
 }
 
+// CSR x Gauss over all windows of a call (src/Skema_SketchySVD.cpp:296-316):
+// Z = nu^G Z + eta sum_i w_i Phi(i, :)^T T(i, :) with T = A Psi, the
+// association of the dense form, instead of an n x s scatter and an n-deep
+// product per window: 3.64 -> 0.52 ms for 100,000 x 20,000, 1e6 nonzeros, ten
+// windows, k = 81, s = 163. False when the workspace is not to be had.
+static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const float* val,
+                             int64_t col_offset, int64_t row0, int64_t nrows, float ybeta) {
+  const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
+  const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w, nwin = (nrows + W - 1) / W;
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  GaussGather g{rowptr, col, val, col_offset, nrows, n, c->omg.f32, c->psi.f32, k, s, c->Y + row0, c->m,
+                eta, ybeta, nullptr, nullptr, 0, 0, nullptr};
+  const size_t smem = sizeof(float) * 192 * 33;
+  auto gather = [&](const GaussGather& q, const uint32_t* cond) {
+    csr_gauss_gather_kernel<<<(unsigned)((q.nrows + 31) / 32), 256, smem, c->stream>>>(q, cond);
+    SKEMA_LAUNCHED(c);
+  };
+  if (c->spd) {
+    StageScope st(c, ST_OMEGA);
+    gather(g, nullptr);
+    y_rows_mark(c, row0, row0 + nrows);
+    return true;
+  }
+  if (c->phi.big) return false;  // an imported map beyond the planes' range
+  const int64_t kp = (k + 3) / 4 * 4;
+  // rows per block: T, its FP32 form and Phi's planes within 512 MB
+  const int64_t rb = std::min<int64_t>(nrows, std::max<int64_t>(32, ((int64_t)512 << 20) / (16 * s) / 32 * 32));
+  const int64_t ldt = (rb + 7) / 8 * 8, nblk = (nrows + rb - 1) / rb;
+  const size_t b_xt = up(sizeof(float) * (size_t)(n * kp)), b_pl = up(sizeof(__nv_bfloat16) * (size_t)(3 * s * ldt)),
+               b_t32 = up(sizeof(float) * (size_t)(s * ldt)), b_flag = up(sizeof(uint32_t) * (size_t)nblk);
+  char* ws = static_cast<char*>(try_workspace(c, b_xt + 2 * b_pl + b_t32 + x3_part_bytes(c) + b_flag));
+  if (!ws) return false;
+  float* XT = reinterpret_cast<float*>(ws);
+  __nv_bfloat16* Tp = reinterpret_cast<__nv_bfloat16*>(ws + b_xt);
+  __nv_bfloat16* Fp = reinterpret_cast<__nv_bfloat16*>(ws + b_xt + b_pl);
+  float* T32 = reinterpret_cast<float*>(ws + b_xt + 2 * b_pl);
+  float* part = reinterpret_cast<float*>(ws + b_xt + 2 * b_pl + b_t32);
+  uint32_t* flags = reinterpret_cast<uint32_t*>(ws + b_xt + 2 * b_pl + b_t32 + x3_part_bytes(c));
+  const float wn = (float)std::pow((double)nu, (double)nwin);
+  {
+    StageScope st(c, ST_UPSILON);
+    SKEMA_CUDA(cudaMemsetAsync(XT, 0, b_xt, c->stream));
+    SKEMA_CUDA(cudaMemsetAsync(flags, 0, b_flag, c->stream));
+    csr_gauss_xt_kernel<<<grid_cap(c, (nrows + 7) / 8, 16), 256, 0, c->stream>>>(
+        rowptr, col, val, col_offset, nrows, n, c->ups.f32 + row0 * k, k, kp, XT, nu, W, nwin);
+    SKEMA_LAUNCHED(c);
+    xt_add_kernel<<<grid_cap(c, ((k + 31) / 32) * ((n + 31) / 32), 16), 256, 0, c->stream>>>(XT, kp, k, n, c->X, eta,
+                                                                                            wn);
+    SKEMA_LAUNCHED(c);
+  }
+  for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
+    const int64_t wr = std::min(rb, nrows - r), ps = s * ldt;
+    GaussGather q = g;
+    q.rowptr += r, q.nrows = wr, q.Y += r, q.T = Tp, q.ldt = ldt, q.pstride = ps, q.big = flags + i;
+    {
+      StageScope st(c, ST_OMEGA);
+      gather(q, nullptr);
+    }
+    StageScope st(c, ST_PHI);
+    const float* F = c->phi.f32 + (row0 + r) * s;
+    const float zb = i == 0 ? wn : 1.f;
+    x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r);
+    x3_gemm(c, X3A{Tp, false, false, 0, 0, ldt, ps}, X3B{Fp, ldt, ps}, s, s, wr,
+            tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, flags + i);
+    q.Y = nullptr, q.T32 = T32;
+    gather(q, flags + i);
+    X3Plain3 z;
+    z.n = 1;
+    z.g[0] = X3Plain{F, 1, s, T32, 1, ldt, c->Z, s, 1, s, s, wr, eta, zb, nu, W, nwin, r};
+    x3_plain(c, z, flags + i);
+  }
+  y_rows_mark(c, row0, row0 + nrows);
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 void csr_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const float* val,
                 int64_t col_offset, int64_t row0, int64_t nrows) {
@@ -573,6 +835,9 @@ void csr_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const f
   }
 
   xz_materialize(c, c->stream);
+  if (csr_gauss_update(c, rowptr, col, val, col_offset, row0, nrows, ybeta)) return;
+  // The same window by window, for a workspace limit that has no room for
+  // the call's T and X^T.
   // Gauss maps, all stored transposed (src/Skema_SketchySVD.cpp:296-316):
   // stored rows contiguous, logical (r, j) at f32[r + j*lrows].
   const int threads = 256;

@@ -302,8 +302,10 @@ __global__ void __launch_bounds__(kX3Threads, 1)
 }
 
 // Adds the parts of the tiles that were cut, in K order, and stores them.
-// blockIdx.x: tile, blockIdx.y: 16 columns; G: the product's grid. Half a CTA
-// per 8 columns, a thread per row.
+// blockIdx.x: tile, blockIdx.y: two columns; G: the product's grid; a thread
+// per row and column. A product of few tiles cuts each into as many as G
+// parts, so eight parts are loaded at a time (one after another took 79
+// us, this way 22, for two tiles of 74 parts).
 static __global__ void __launch_bounds__(256) x3_reduce_kernel(X3Grid g, X3Out o, int G, const float* __restrict__ part,
                                                         const uint32_t* __restrict__ flag) {
   if (flag && *flag) return;
@@ -314,24 +316,26 @@ static __global__ void __launch_bounds__(256) x3_reduce_kernel(X3Grid g, X3Out o
   while (b > 0 && x3_run(g, b, G) > kb) --b;
   while (x3_run(g, b + 1, G) <= kb) ++b;
   if (x3_run(g, b, G) <= kb && x3_run(g, b + 1, G) >= ke) return;  // one run: stored by the product
+  int64_t e = (ke - 1) * G / T;  // the run that holds the tile's last step
+  while (x3_run(g, e, G) > ke - 1) --e;
+  while (x3_run(g, e + 1, G) <= ke - 1) ++e;
   const int tile = g.full + (int)q;
-  const int r = threadIdx.x & 127, cl = blockIdx.y * 16 + (threadIdx.x >> 7) * 8;
+  const int r = threadIdx.x & 127, cl = blockIdx.y * 2 + (threadIdx.x >> 7);
   const int64_t row = (int64_t)(tile / g.ntiles) * BM + r;
-  float sum[8];
+  const float* pp = part + (int64_t)cl * BM + r;
+  const int64_t slot = (int64_t)g.nt * BM;
+  // the first run may begin in the tile before: its part of this tile is its
+  // second; every other run begins inside the tile (runs are never empty)
+  float sum = pp[(2 * b + (x3_run(g, b, G) < kb ? 1 : 0)) * slot];
+  pp += 2 * slot;
+  for (int64_t i = b; i < e; i += 8) {
+    float v[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) sum[e] = 0.f;
-  for (; b < G && x3_run(g, b, G) < ke; ++b) {
-    const int64_t p = x3_run(g, b, G);
-    if (x3_run(g, b + 1, G) <= p) continue;  // an empty run
-    const int64_t seg = q - p / g.ksteps;
-    const float* pp = part + ((2 * b + seg) * g.nt + cl) * BM + r;
+    for (int u = 0; u < 8; ++u) v[u] = i + u < e ? pp[2 * (i + u) * slot] : 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) sum[e] += pp[e * BM];
+    for (int u = 0; u < 8; ++u) sum += v[u];
   }
-  if (row >= o.rows) return;
-  const int64_t col = (int64_t)(tile % g.ntiles) * g.nt + cl;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) x3_store(o, row, col + e, sum[e]);
+  if (row < o.rows) x3_store(o, row, (int64_t)(tile % g.ntiles) * g.nt + cl, sum);
 }
 
 }  // namespace tc

@@ -138,24 +138,8 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// C = alpha op + beta C in plain FP32 for the rare block that too_big()
-// refuses (returns at once otherwise): 64 x 64 tiles, up to three products
-// per launch. A(i, kk) is scaled by the window weight of kk when nu != 1.
-struct X3Plain {
-  const float* A;
-  int64_t ars, acs;
-  const float* B;
-  int64_t brs, bcs;
-  float* C;
-  int64_t crs, ccs;
-  int64_t M, N, K;
-  float alpha, beta, nu;
-  int64_t W, nwin, j0;
-};
-struct X3Plain3 {
-  X3Plain g[3];
-  int n;
-};
+// The products of X3Plain3 for the rare block that too_big() refuses (returns
+// at once otherwise), by 64 x 64 tiles.
 __global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_t* __restrict__ flag) {
   if (*flag == 0) return;
   __shared__ float As[16][65], Bs[16][65];
@@ -198,6 +182,37 @@ __global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_
   }
 }
 
+// K-major planes D[q * pstride + c * ld + i] of a row-major source (rows i of
+// `cols` values, rs apart), turned by 64 x 32 tiles; columns i past `rows` up
+// to ld are zeros. Row i is scaled by nu^(nwin - 1 - (j0 + i) / W).
+__global__ void __launch_bounds__(256)
+    x3_transposed_kernel(const float* __restrict__ S, int64_t rs, int64_t rows, int64_t cols,
+                         __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin,
+                         int64_t j0) {
+  __shared__ float tile[32][65];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t ti = (ld + 63) / 64, tj = (cols + 31) / 32;
+  for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
+    const int64_t i0 = (t / tj) * 64, c0 = (t % tj) * 32;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = ty + 8 * q;
+      float v = (i0 + r < rows && c0 + tx < cols) ? S[(i0 + r) * rs + c0 + tx] : 0.f;
+      if (nu != 1.f && i0 + r < rows) v *= (float)pow((double)nu, (double)(nwin - 1 - (j0 + i0 + r) / W));
+      tile[tx][r] = v;
+    }
+    __syncthreads();
+    const int j = threadIdx.x >> 3, g8 = (threadIdx.x & 7) * 8;
+    if (c0 + j < cols && i0 + g8 < ld) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = tile[j][g8 + e];
+      store_planes8(v, D + (c0 + j) * ld + i0 + g8, pstride);
+    }
+    __syncthreads();
+  }
+}
+
 int grid_1d(const skema_ctx* c, int64_t items, int per_sm) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, (int64_t)c->sm_count * per_sm));
 }
@@ -229,7 +244,7 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   const size_t stage = tc::kX3ABytes + (size_t)3 * g.nt * tc::kX3BK * 2;
   g.stages = (int)std::min<size_t>(tc::kX3MaxStages, (kX3Smem - 2048) / stage);
   const int64_t tiles = (int64_t)g.mtiles * g.ntiles;
-  // a run of at least four K steps per CTA
+  // a run of at least four K steps per CTA (so that none is empty)
   const int G = (int)std::max<int64_t>(1, std::min<int64_t>(c->sm_count, tiles * g.ksteps / 4));
   g.full = (int)(tiles / G * G);
   CUtensorMap ta;
@@ -247,7 +262,7 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   c->dev_err_armed = true;
   const int rem = (int)(tiles - g.full);
   if (rem > 0) {
-    tc::x3_reduce_kernel<<<dim3(rem, g.nt / 16), 256, 0, c->stream>>>(g, o, G, part, flag);
+    tc::x3_reduce_kernel<<<dim3(rem, g.nt / 2), 256, 0, c->stream>>>(g, o, G, part, flag);
     SKEMA_LAUNCHED(c);
   }
 }
@@ -261,6 +276,19 @@ void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfl
   else
     x3_block_tiled_kernel<<<grid_1d(c, nrb * ((cols + 31) / 32) * 256, 16), 256, 0, c->stream>>>(
         src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, flag);
+  SKEMA_LAUNCHED(c);
+}
+
+void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0) {
+  const int64_t tiles = ((ld + 63) / 64) * ((cols + 31) / 32);
+  x3_transposed_kernel<<<grid_1d(c, tiles * 256, 16), 256, 0, c->stream>>>(S, rs, rows, cols, D, ld, pstride, nu, W,
+                                                                          nwin, j0);
+  SKEMA_LAUNCHED(c);
+}
+
+void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag) {
+  x3_plain_kernel<<<2 * c->sm_count, 256, 0, c->stream>>>(p, flag);
   SKEMA_LAUNCHED(c);
 }
 
@@ -365,15 +393,13 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
                          k, n, wr, eta, xb, nu, W, nwin, j0};
         p.n = 3;
       }
-      x3_plain_kernel<<<2 * c->sm_count, 256, 0, c->stream>>>(p, flag);
-      SKEMA_LAUNCHED(c);
+      x3_plain(c, p, flag);
       if (s > 0) {
         X3Plain3 z;
         z.g[0] = X3Plain{c->phi.f32 + R0, c->phi.rs, 1, T32, 1, wr, c->Z, s, 1,
                          s, s, wr, eta, xb, nu, W, nwin, j0};
         z.n = 1;
-        x3_plain_kernel<<<c->sm_count, 256, 0, c->stream>>>(z, flag);
-        SKEMA_LAUNCHED(c);
+        x3_plain(c, z, flag);
       }
     }
   }

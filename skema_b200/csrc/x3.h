@@ -46,6 +46,32 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
 void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
                      uint32_t* flag);
 
+// K-major planes of a row-major source's transpose: row i of S (rows x cols,
+// rs apart), scaled by nu^(nwin - 1 - (j0 + i) / W), is K index i; D holds
+// cols rows of ld (a multiple of 8) per plane.
+void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0);
+
+// Up to three FP32 products C = alpha A B + beta C by plain FMA, run when
+// *flag is set: the form of a block whose values the planes cannot carry.
+// A(i, kk) is scaled by nu^(nwin - 1 - (j0 + kk) / W).
+struct X3Plain {
+  const float* A;
+  int64_t ars, acs;
+  const float* B;
+  int64_t brs, bcs;
+  float* C;
+  int64_t crs, ccs;
+  int64_t M, N, K;
+  float alpha, beta, nu;
+  int64_t W, nwin, j0;
+};
+struct X3Plain3 {
+  X3Plain g[3];
+  int n;
+};
+void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag);
+
 // One call's input: a dense matrix, or a filler of window planes (A.p null)
 // whose values are at most 1 in magnitude or NaN.
 struct X3Input {
