@@ -34,80 +34,129 @@ namespace skema {
 namespace {
 
 // ---------------------------------------------------------------- DGEMM ----
-// C(i,j) = alpha * sum A(i,kk) B(kk,j) + beta*C(i,j); A, B may be float or
-// double; FP64 accumulation. 64x64 tile, 4x4 per thread, split-K atomic.
-template <typename TA, typename TB, bool ATOMIC>
-__global__ void __launch_bounds__(256)
-    dgemm_kernel(int64_t M, int64_t N, int64_t K, double alpha, const TA* __restrict__ A,
-                 int64_t ars, int64_t acs, const TB* __restrict__ B, int64_t brs, int64_t bcs,
-                 double beta, double* __restrict__ C, int64_t crs, int64_t ccs, int64_t kchunk) {
-  __shared__ double As[8][64 + 1];
-  __shared__ double Bs[8][64 + 1];
-  const int tid = threadIdx.x;
-  const int64_t m0 = (int64_t)blockIdx.x * 64, n0 = (int64_t)blockIdx.y * 64;
-  const int64_t kb = (int64_t)blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  if (kb >= ke) return;
-  const bool am = (ars == 1);
-  const bool bn = (bcs == 1);
-  // 512 elements per operand tile: 2 per thread
-  int la_m[2], la_k[2], lb_n[2], lb_k[2];
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int e = tid + 256 * q;
-    if (am) { la_m[q] = e & 63; la_k[q] = e >> 6; } else { la_k[q] = e & 7; la_m[q] = e >> 3; }
-    if (bn) { lb_n[q] = e & 63; lb_k[q] = e >> 6; } else { lb_k[q] = e & 7; lb_n[q] = e >> 3; }
-  }
-  const int tx = tid & 15, ty = tid >> 4;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-  for (int64_t k0 = kb; k0 < ke; k0 += 8) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int64_t gm = m0 + la_m[q], gk = k0 + la_k[q];
-      As[la_k[q]][la_m[q]] = (gm < M && gk < ke) ? (double)A[gm * ars + gk * acs] : 0.0;
-      const int64_t gn = n0 + lb_n[q], gk2 = k0 + lb_k[q];
-      Bs[lb_k[q]][lb_n[q]] = (gn < N && gk2 < ke) ? (double)B[gk2 * brs + gn * bcs] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a[u] = As[kk][ty + 16 * u];
-        b[u] = Bs[kk][tx + 16 * u];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t gm = m0 + ty + 16 * i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t gn = n0 + tx + 16 * j;
-      if (gn >= N) continue;
-      double* cp = C + gm * crs + gn * ccs;
-      if (ATOMIC)
-        atomicAdd(cp, alpha * acc[i][j]);
-      else
-        *cp = (beta == 0.0) ? alpha * acc[i][j] : fma(beta, *cp, alpha * acc[i][j]);
-    }
-  }
+// FP64 tensor cores: mma.sync m8n8k4 (D = A B + C, 8 x 4 by 4 x 8). Per lane:
+// A holds element (lane / 4, lane % 4), B element (lane % 4, lane / 4), C / D
+// elements (lane / 4, 2 (lane % 4) + i), i < 2.
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 
-template <typename TA, typename TB>
-void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA* A, int64_t ars,
-           int64_t acs, const TB* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs,
-           int64_t ccs, bool allow_split = true);
+// The sm_90 shape m16n8k16: A element (lane / 4 + 8 (i % 2), lane % 4 + 4 (i / 2)),
+// i < 8; B (lane % 4 + 4 i, lane / 4), i < 4; D (lane / 4 + 8 (i / 2),
+// 2 (lane % 4) + i % 2), i < 4.
+__device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7, %8, %9, %10, %11}, "
+      "{%12, %13, %14, %15}, {%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
+        "d"(b[2]), "d"(b[3]));
+}
+
+// C(i,j) = alpha * sum A(i,kk) B(kk,j) + beta*C(i,j); A, B may be float or
+// double (widened when they are staged); FP64 accumulation. WM x WN warps of
+// MB x NB blocks of 16 x 8 each; K steps of 16 through double-buffered shared memory
+// whose rows are 4 (mod 16) doubles long, so that a fragment's 4 x 8 reads hit
+// distinct banks. atomic: the K range is split over grid.z and the parts are
+// added to C. Two shapes: 128 x 8 NB for a tall C (eight warps along M, so each
+// A value is staged and widened once for all columns) and 32 x 32, four warps,
+// for the k-sized products, which would fill a few SMs only with larger tiles.
+// The residual pass on 50,000 x 10,000 at r = 50 (1e11 FP64 flop) takes 4.5 ms
+// in these products (22 TFLOP/s; the tensor and the FMA pipe both peak at 66 FMA
+// per cycle and SM, 37 TFLOP/s), the 64 x 64 SIMT form took 11.1.
+template <typename TA, typename TB, int WM, int WN, int MB, int NB>
+__global__ void __launch_bounds__(32 * WM * WN)
+    dgemm_mma_kernel(int64_t M, int64_t N, int64_t K, double alpha, const TA* __restrict__ A, int64_t ars, int64_t acs,
+                     const TB* __restrict__ B, int64_t brs, int64_t bcs, double beta, double* __restrict__ C,
+                     int64_t crs, int64_t ccs, int64_t kchunk, int atomic) {
+  constexpr int NT = 32 * WM * WN, BM = 16 * MB * WM, BN = 8 * NB * WN, KS = 16;
+  constexpr int lda = (BM + 15) / 16 * 16 + 4, ldb = (BN + 15) / 16 * 16 + 4;
+  constexpr int QA = BM * KS / NT, QB = (BN * KS + NT - 1) / NT;
+  extern __shared__ __align__(16) double dg_smem[];
+  double* As = dg_smem;                   // 2 x KS x lda
+  double* Bs = dg_smem + 2 * KS * lda;    // 2 x KS x ldb
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane & 3, lc = lane >> 2;
+  const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
+  const int64_t kb = (int64_t)blockIdx.z * kchunk, ke = min(K, kb + kchunk);
+  if (kb >= ke) return;
+  const bool am = ars == 1, bn = bcs == 1;
+  TA ra[QA];
+  TB rb[QB];
+  auto load = [&](int64_t k0) {
+#pragma unroll
+    for (int q = 0; q < QA; ++q) {
+      const int e = tid + NT * q;
+      const int m = am ? e % BM : e / KS, k = am ? e / BM : e % KS;
+      ra[q] = (m0 + m < M && k0 + k < ke) ? A[(m0 + m) * ars + (k0 + k) * acs] : TA(0);
+    }
+#pragma unroll
+    for (int q = 0; q < QB; ++q) {
+      const int e = tid + NT * q;
+      const int n = bn ? e % BN : e / KS, k = bn ? e / BN : e % KS;
+      rb[q] = (e < BN * KS && n0 + n < N && k0 + k < ke) ? B[(k0 + k) * brs + (n0 + n) * bcs] : TB(0);
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int q = 0; q < QA; ++q) {
+      const int e = tid + NT * q;
+      As[(buf * KS + (am ? e / BM : e % KS)) * lda + (am ? e % BM : e / KS)] = (double)ra[q];
+    }
+#pragma unroll
+    for (int q = 0; q < QB; ++q) {
+      const int e = tid + NT * q;
+      if (e < BN * KS) Bs[(buf * KS + (bn ? e / BN : e % KS)) * ldb + (bn ? e % BN : e / KS)] = (double)rb[q];
+    }
+  };
+  const int wm = (warp % WM) * 16 * MB, wn = (warp / WM) * 8 * NB;
+  double acc[MB][NB][4];
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0;
+  load(kb);
+  store(0);
+  __syncthreads();
+  int buf = 0;
+  for (int64_t k0 = kb; k0 < ke; k0 += KS, buf ^= 1) {
+    const bool more = k0 + KS < ke;
+    if (more) load(k0 + KS);
+    const double* as = As + (buf * KS + lr) * lda + wm + lc;
+    const double* bs = Bs + (buf * KS + lr) * ldb + wn + lc;
+    double a[MB][8];
+#pragma unroll
+    for (int i = 0; i < MB; ++i)
+#pragma unroll
+      for (int h = 0; h < 8; ++h) a[i][h] = as[(h >> 1) * 4 * lda + 16 * i + 8 * (h & 1)];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      double b[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) b[h] = bs[4 * h * ldb + 8 * j];
+#pragma unroll
+      for (int i = 0; i < MB; ++i) dmma16(acc[i][j], a[i], b);
+    }
+    if (more) store(buf ^ 1);  // read last one step ago, before the barrier
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int64_t gm = m0 + wm + 16 * i + lc + 8 * (h >> 1), gn = n0 + wn + 8 * j + 2 * lr + (h & 1);
+        if (gm >= M || gn >= N) continue;
+        double* cp = C + gm * crs + gn * ccs;
+        const double v = alpha * acc[i][j][h];
+        if (atomic)
+          atomicAdd(cp, v);
+        else
+          *cp = (beta == 0.0) ? v : fma(beta, *cp, v);
+      }
+}
 
 __global__ void dscale_kernel(double* C, int64_t crs, int64_t ccs, int64_t M, int64_t N, double b) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < M * N;
@@ -118,44 +167,65 @@ __global__ void dscale_kernel(double* C, int64_t crs, int64_t ccs, int64_t M, in
   }
 }
 
-template <typename TA, typename TB>
-void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA* A, int64_t ars,
-           int64_t acs, const TB* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs,
-           int64_t ccs, bool allow_split) {
-  if (M <= 0 || N <= 0) return;
-  const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64);
+template <typename TA, typename TB, int WM, int WN, int MB, int NB>
+void launch_dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA* A, int64_t ars, int64_t acs,
+                  const TB* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs, int64_t ccs,
+                  bool allow_split) {
+  constexpr int64_t BM = 16 * MB * WM, BN = 8 * NB * WN;
+  constexpr size_t smem = sizeof(double) * 2 * 16 * ((BM + 15) / 16 * 16 + 4 + (BN + 15) / 16 * 16 + 4);
+  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
+  if (gy > 65535) fail(SKEMA_EUNSUPPORTED, "dgemm: N too large");
+  // K ranges of 256 or more, about four CTAs per SM in all; with tiles for
+  // two to eight per SM, ranges of 1024 or more and sixteen per SM, so that
+  // no SM is left with one tile more than the others
   int64_t split = 1;
-  if (allow_split && tiles < 2 * c->sm_count && K >= 512)
-    split = std::min<int64_t>((2 * c->sm_count + tiles - 1) / tiles, K / 256);
+  if (allow_split && gx * gy < 2 * c->sm_count && K >= 512)
+    split = std::min<int64_t>((4 * c->sm_count + gx * gy - 1) / (gx * gy), K / 256);
+  if (allow_split && gx * gy < 8 * c->sm_count)
+    split = std::max(split, std::min<int64_t>((16 * c->sm_count + gx * gy - 1) / (gx * gy), K / 1024));
   if (split > 1) {
-    dscale_kernel<<<(int)std::min<int64_t>((M * N + 255) / 256, 4096), 256, 0, c->stream>>>(
-        C, crs, ccs, M, N, beta);
+    dscale_kernel<<<(int)std::min<int64_t>((M * N + 255) / 256, 4096), 256, 0, c->stream>>>(C, crs, ccs, M, N, beta);
     SKEMA_LAUNCHED(c);
   }
-  int64_t kchunk = (K + split - 1) / split;
-  kchunk = (kchunk + 7) / 8 * 8;
+  const int64_t kchunk = ((K + split - 1) / split + 15) / 16 * 16;
   const int64_t gz = std::max<int64_t>(1, (K + kchunk - 1) / kchunk);
-  if ((N + 63) / 64 > 65535) fail(SKEMA_EUNSUPPORTED, "dgemm: N too large");
-  dim3 grid((unsigned)((M + 63) / 64), (unsigned)((N + 63) / 64), (unsigned)gz);
-  if (split > 1)
-    dgemm_kernel<TA, TB, true><<<grid, 256, 0, c->stream>>>(M, N, K, alpha, A, ars, acs, B, brs,
-                                                            bcs, beta, C, crs, ccs, kchunk);
-  else
-    dgemm_kernel<TA, TB, false><<<grid, 256, 0, c->stream>>>(M, N, K, alpha, A, ars, acs, B, brs,
-                                                             bcs, beta, C, crs, ccs, kchunk);
+  auto kern = dgemm_mma_kernel<TA, TB, WM, WN, MB, NB>;
+  SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), 32 * WM * WN, smem, c->stream>>>(
+      M, N, K, alpha, A, ars, acs, B, brs, bcs, beta, C, crs, ccs, kchunk, split > 1 ? 1 : 0);
   SKEMA_LAUNCHED(c);
 }
 
-// ----------------------------------------- tall-skinny FP64 products -------
-// Both run on the FP64 tensor cores: mma.sync m8n8k4 (D = A B + C, 8 x 4 by
-// 4 x 8). Per lane: A holds element (lane / 4, lane % 4), B element
-// (lane % 4, lane / 4), C / D elements (lane / 4, 2 (lane % 4) + i), i < 2.
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
+template <typename TA, typename TB>
+void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA* A, int64_t ars,
+           int64_t acs, const TB* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs,
+           int64_t ccs, bool allow_split = true) {
+  if (M <= 0 || N <= 0) return;
+  if (K <= 0) {
+    dscale_kernel<<<(int)std::min<int64_t>((M * N + 255) / 256, 4096), 256, 0, c->stream>>>(C, crs, ccs, M, N, beta);
+    SKEMA_LAUNCHED(c);
+    return;
+  }
+  auto go = [&](auto launch) {
+    launch(c, M, N, K, alpha, A, ars, acs, B, brs, bcs, beta, C, crs, ccs, allow_split);
+  };
+  if (M < 1024) {
+    go(launch_dgemm<TA, TB, 2, 2, 1, 2>);
+    return;
+  }
+  switch (std::min<int64_t>(8, (N + 7) / 8)) {
+    case 1: go(launch_dgemm<TA, TB, 8, 1, 1, 1>); break;
+    case 2: go(launch_dgemm<TA, TB, 8, 1, 1, 2>); break;
+    case 3: go(launch_dgemm<TA, TB, 8, 1, 1, 3>); break;
+    case 4: go(launch_dgemm<TA, TB, 8, 1, 1, 4>); break;
+    case 5: go(launch_dgemm<TA, TB, 8, 1, 1, 5>); break;
+    case 6: go(launch_dgemm<TA, TB, 8, 1, 1, 6>); break;
+    case 7: go(launch_dgemm<TA, TB, 8, 1, 1, 7>); break;
+    default: go(launch_dgemm<TA, TB, 8, 1, 1, 8>); break;
+  }
 }
 
+// ----------------------------------------- tall-skinny FP64 products -------
 // G += A^T A for a tall column-major A (rows x k, ld lda, k <= 256; T float
 // or double, widened to FP64 exactly). The k x k product is cut into 32 x 32
 // tiles and only the tiles on or above the diagonal are formed (6 of 9 at

@@ -38,21 +38,33 @@ __global__ void cm_to_rm_kernel(const double* __restrict__ S, int64_t ld, int64_
 }
 
 // sq[j] += sum_i (M[i*r + j] - B[i*r + j] * S[j])^2 over rows i < rows.
-// Threads: 32 lanes over columns (chunks of 32), 8 rows per block step.
+// Threads: 32 lanes over columns (chunks of 32), 8 rows per block step. The
+// block's sums meet in shared memory, so a column takes one atomic per block:
+// with one per warp the r addresses were the kernel's time (89 us for 8192 x
+// 50; 15 us for 50,000 x 50 now).
 __global__ void __launch_bounds__(256)
     colsumsq_diff_kernel(const double* __restrict__ M, const double* __restrict__ B, const double* __restrict__ S,
                          int64_t rows, int64_t r, double* __restrict__ sq) {
+  __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int64_t c0 = 0; c0 < r; c0 += 32) {
     const int64_t j = c0 + lane;
-    if (j >= r) continue;
-    const double s = S[j];
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * 8 + ty; i < rows; i += (int64_t)gridDim.x * 8) {
-      const double d = M[i * r + j] - B[i * r + j] * s;
-      acc = fma(d, d, acc);
+    if (j < r) {
+      const double s = S[j];
+      for (int64_t i = (int64_t)blockIdx.x * 8 + ty; i < rows; i += (int64_t)gridDim.x * 8) {
+        const double d = M[i * r + j] - B[i * r + j] * s;
+        acc = fma(d, d, acc);
+      }
     }
-    atomicAdd(sq + j, acc);
+    red[ty][lane] = acc;
+    __syncthreads();
+    if (ty == 0 && j < r) {
+#pragma unroll
+      for (int q = 1; q < 8; ++q) acc += red[q][lane];
+      atomicAdd(sq + j, acc);
+    }
+    __syncthreads();
   }
 }
 
@@ -158,19 +170,26 @@ void residual_begin_kept(skema_ctx* c) {
   residual_open(c);
 }
 
-// Rows [row0, row0 + nrows) of a dense A, in windows of params.window rows
-// (map_A_by_window): A_w V -> (A_w V - U_w S)^2 into the sums; A^T U += A_w^T U_w.
+// Rows [row0, row0 + nrows) of a dense A, in blocks (map_A_by_window's sums do
+// not depend on where the windows end): A_w V -> (A_w V - U_w S)^2 into the
+// sums; A^T U += A_w^T U_w. Blocks of up to 65,536 rows, or params.window rows
+// where the workspace has no room for that.
 void residual_dense(skema_ctx* c, Mat A, int64_t row0, int64_t nrows) {
   need_ready(c);
-  const int64_t n = c->n, r = c->p.rank, W = c->w;
+  const int64_t n = c->n, r = c->p.rank;
   const double* Urows = c->spd ? c->res_V : c->res_U;  // SPD: A V - V S
-  double* AVw = static_cast<double*>(workspace(c, sizeof(double) * (size_t)(std::min(W, nrows) * r)));
+  int64_t W = std::min<int64_t>(nrows, std::max<int64_t>(c->w, 65536));
+  double* AVw = static_cast<double*>(try_workspace(c, sizeof(double) * (size_t)(W * r)));
+  if (!AVw) {
+    W = std::min<int64_t>(nrows, c->w);
+    AVw = static_cast<double*>(workspace(c, sizeof(double) * (size_t)(W * r)));
+  }
   for (int64_t q = 0; q < nrows; q += W) {
     const int64_t wr = std::min(W, nrows - q), R0 = row0 + q;
     const float* Ap = A.p + q * A.rs;
     // AV_w (wr x r, row-major) = A_w V
     dgemm_f32_f64(c, wr, r, n, 1.0, Ap, A.rs, A.cs, c->res_V, r, 1, 0.0, AVw, r, 1);
-    colsumsq_diff_kernel<<<grid_of(c, (wr + 7) / 8, 8), 256, 0, c->stream>>>(AVw, Urows + R0 * r, c->res_S, wr, r,
+    colsumsq_diff_kernel<<<grid_of(c, (wr + 7) / 8, 2), 256, 0, c->stream>>>(AVw, Urows + R0 * r, c->res_S, wr, r,
                                                                              c->res_sq);
     SKEMA_LAUNCHED(c);
     // A^T U (n x r, row-major) += A_w^T U_w
@@ -217,7 +236,7 @@ void residual_finish(skema_ctx* c, double* rnorms) {
   const int64_t n = c->n, r = c->p.rank;
   if (!c->spd) {
     // (A^T U - V S)^2 column sums join those of A V - U S
-    colsumsq_diff_kernel<<<grid_of(c, (n + 7) / 8, 8), 256, 0, c->stream>>>(c->res_AtU, c->res_V, c->res_S, n, r,
+    colsumsq_diff_kernel<<<grid_of(c, (n + 7) / 8, 2), 256, 0, c->stream>>>(c->res_AtU, c->res_V, c->res_S, n, r,
                                                                             c->res_sq);
     SKEMA_LAUNCHED(c);
   }
