@@ -569,105 +569,215 @@ __global__ void trsm_upper_kernel(const double* __restrict__ R, int64_t k, doubl
 __device__ __forceinline__ int up_off(int j) { return j * (j + 1) / 2; }
 __device__ __forceinline__ int lo_off(int j, int k) { return j * k - j * (j - 1) / 2; }
 
-// Largest k for which one packed triangle plus k doubles fits the 200 KB
-// that the single-CTA kernels below use.
+// Largest k for which a packed triangle and one warp's right-hand sides fit
+// shared memory (217,800 bytes at 225).
 constexpr int kPackedMaxK = 225;
-size_t packed_smem_bytes(int64_t k) { return sizeof(double) * (size_t)(k * (k + 1) / 2 + k); }
+size_t packed_smem_bytes(int64_t k) { return sizeof(double) * (size_t)(k * (k + 1) / 2); }
+// Row stride of a warp's right-hand sides: k rounded up to 16, plus 4, so that
+// the 4 x 8 fragment reads hit distinct banks.
+__host__ __device__ __forceinline__ int tri_ld(int k) { return (k + 15) / 16 * 16 + 4; }
 
-// Value v of the register array b (v known only at run time) without a
-// local-memory copy: a chain of selects the compiler keeps in registers.
-template <int VMAX>
-__device__ __forceinline__ double pick(const double (&b)[VMAX], int v) {
-  double r = 0.0;
+// Solve R X = B, R upper triangular (column-major k x k), B k x nrhs (column
+// stride ldb) in place, or with B the identity (its columns are not read: X =
+// R^{-1}). R packed in shared memory with its 8 x 8 diagonal blocks inverted in
+// place; a warp (nw of them) takes eight right-hand sides and goes up by block rows,
+//   X_I = inv(R_II) (B_I - sum_{K > I} R_IK X_K),
+// every product on the FP64 tensor cores (m8n8k4), so a step is a few MMAs
+// instead of eight dependent eliminations. The right-hand sides are spread over
+// the grid, so the inverse of a Cholesky factor no longer runs in one CTA.
+// k = 201, nrhs = 201: 44 us, 35 for the identity (a column at a time in
+// registers took 75; 114 when only the solving warps filled shared memory).
+// Returns at once when *status (may be null) is not 0.
+constexpr int kTriThreads = 512;
+__global__ void __launch_bounds__(kTriThreads)
+    tri_solve_kernel(const double* __restrict__ R, int k, double* B, int64_t ldb, int nrhs, int nw, int identity,
+                     const int* __restrict__ status) {
+  if (status && *status != 0) return;
+  extern __shared__ __align__(16) double ts_smem[];
+  double* Rp = ts_smem;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane & 3, lc = lane >> 2;
+  const int ld = tri_ld(k), nblk = (k + 7) >> 3;
+  double* X = Rp + k * (k + 1) / 2 + (size_t)warp * 8 * ld;  // column c, row i at X[c * ld + i]
+  const int nall = blockDim.x >> 5;  // all warps fill shared memory, nw solve
+#pragma unroll 4
+  for (int j = warp; j < k; j += nall)
 #pragma unroll
-  for (int q = 0; q < VMAX; ++q)
-    if (q == v) r = b[q];
-  return r;
-}
-
-// Solve R X = B in place, R upper triangular (column-major k x k, k <=
-// min(32 VMAX, kPackedMaxK)) and B k x nrhs (column stride ldb). R is held
-// packed in shared memory with the reciprocals of its diagonal; one warp
-// per right-hand side keeps its column in registers (entry i in lane i % 32,
-// slot i / 32) and eliminates column by column: x_i = b_i / R(i, i), then
-// b_l -= R(l, i) x_i for l < i.
-template <int VMAX>
-__global__ void __launch_bounds__(256) trsm_upper_packed_kernel(const double* __restrict__ R, int k, double* B,
-                                                                int64_t ldb, int nrhs) {
-  extern __shared__ double tp_smem[];
-  double* Rp = tp_smem;
-  double* inv = Rp + k * (k + 1) / 2;
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
-    const int i = q % k, j = q / k;
-    if (i <= j) Rp[up_off(j) + i] = R[q];
-  }
-  for (int i = threadIdx.x; i < k; i += blockDim.x) inv[i] = 1.0 / R[i + (int64_t)i * k];
+    for (int v = 0; v < 8; ++v) {  // k <= 225 rows
+      const int i = lane + 32 * v;
+      if (i <= j) Rp[up_off(j) + i] = R[i + j * k];
+    }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (col >= nrhs) return;
-  double* x = B + (int64_t)col * ldb;
-  double b[VMAX];
+  for (int t = warp; t < nblk; t += nall) {
+    const int o = 8 * t, nb = min(8, k - o);
+    double x[8];
+    if (lane < nb) {  // column `lane` of the block's inverse
 #pragma unroll
-  for (int v = 0; v < VMAX; ++v) {
-    const int i = lane + 32 * v;
-    b[v] = i < k ? x[i] : 0.0;
-  }
-  for (int i = k - 1; i >= 0; --i) {
-    const double xi = __shfl_sync(0xffffffffu, pick(b, i >> 5) * inv[i], i & 31);
-    const double* rc = Rp + up_off(i);
+      for (int i = 7; i >= 0; --i) {
+        x[i] = 0.0;
+        if (i >= nb || i > lane) continue;
+        double v = i == lane ? 1.0 : 0.0;
 #pragma unroll
-    for (int v = 0; v < VMAX; ++v) {
-      const int l = lane + 32 * v;
-      if (l < i)
-        b[v] = fma(-rc[l], xi, b[v]);
-      else if (l == i)
-        b[v] = xi;
+        for (int l = i + 1; l < 8; ++l)
+          if (l <= lane && l < nb) v = fma(-Rp[up_off(o + l) + o + i], x[l], v);
+        x[i] = v / Rp[up_off(o + i) + o + i];
+      }
+    }
+    __syncwarp();
+    if (lane < nb) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i <= lane) Rp[up_off(o + lane) + o + i] = x[i];
     }
   }
-#pragma unroll
-  for (int v = 0; v < VMAX; ++v) {
-    const int i = lane + 32 * v;
-    if (i < k) x[i] = b[v];
+  __syncthreads();
+  const int c0 = ((int)blockIdx.x * nw + warp) * 8;
+  if (warp >= nw || c0 >= nrhs) return;
+  const int nc = min(8, nrhs - c0);
+  for (int q = lane; q < 8 * ld; q += 32) {
+    const int c = q / ld, i = q - c * ld;
+    X[q] = (c >= nc || i >= k) ? 0.0 : identity ? (i == c0 + c ? 1.0 : 0.0) : B[(int64_t)(c0 + c) * ldb + i];
   }
+  __syncwarp();
+  // columns of the identity start at their own block row
+  for (int I = identity ? min(nblk - 1, c0 >> 3) : nblk - 1; I >= 0; --I) {
+    const int row = 8 * I + lc;
+    double s0[2] = {0.0, 0.0}, s1[2] = {0.0, 0.0};
+    const int Kend = identity ? min(nblk - 1, c0 >> 3) : nblk - 1;
+#pragma unroll 4
+    for (int K = I + 1; K <= Kend; ++K) {
+      const int ca = 8 * K + lr, cb = ca + 4;
+      const double a0 = ca < k ? Rp[up_off(ca) + row] : 0.0, a1 = cb < k ? Rp[up_off(cb) + row] : 0.0;
+      dmma(s0, a0, X[lc * ld + ca]);
+      dmma(s1, a1, X[lc * ld + cb]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) X[(2 * lr + h) * ld + row] -= s0[h] + s1[h];
+    __syncwarp();
+    const int ca = 8 * I + lr, cb = ca + 4;
+    const double a0 = (ca < k && row <= ca) ? Rp[up_off(ca) + row] : 0.0;
+    const double a1 = (cb < k && row <= cb) ? Rp[up_off(cb) + row] : 0.0;
+    double y[2] = {0.0, 0.0};
+    dmma(y, a0, X[lc * ld + ca]);
+    dmma(y, a1, X[lc * ld + cb]);
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) X[(2 * lr + h) * ld + row] = y[h];
+    __syncwarp();
+  }
+  for (int c = 0; c < nc; ++c)
+    for (int i = lane; i < k; i += 32) B[(int64_t)(c0 + c) * ldb + i] = X[c * ld + i];
 }
 
-// Cholesky of the symmetric positive definite G (column-major k x k, lower
-// triangle read) with its factor and inverse: R = L^T and Rinv = R^{-1}
-// (both upper, column-major k x k, zeros below the diagonal). One CTA of
-// 1024 threads, the lower triangle packed in shared memory. Right-looking:
-// step j subtracts L(a, j) L(b, j) / d_j from the trailing triangle using
-// the unscaled column, so one barrier per column suffices; the columns are
-// scaled by sqrt(d_j) afterwards. L^{-1} comes from forward substitution of
-// the unit vectors (one warp per column, the column in registers), and
-// Rinv(j, i) = L^{-1}(i, j). G is read completely before anything is
-// written, so Rinv may alias G. status[0] = 0, or j + 1 when the j-th pivot
-// is not positive (R and Rinv are then not written).
-template <int VMAX>
-__global__ void __launch_bounds__(1024) chol_factor_kernel(const double* G, int k, double* R, double* Rinv,
-                                                           int* status) {
+// Cholesky G = L L^T of the symmetric positive definite G (column-major k x k,
+// lower triangle read), R = L^T (upper, column-major, zeros below the
+// diagonal). One CTA, the lower triangle packed in shared memory, in panels of
+// eight columns: every thread that owns a row factors the panel's 8 x 8
+// diagonal block in registers for itself (no barrier per column), solves its
+// row against it, and then all warps subtract the panel's rank-8 product from
+// the trailing triangle, four columns at a time with their 32 panel values in
+// registers. Two barriers per panel; bound by the chain of 8 reciprocal square
+// roots per panel and the FP64 FMAs of the update (k = 201: 128 us, and
+// 35 us for the inverse by tri_solve_kernel; one column at a time with a barrier
+// each, and the inverse column by column in the same CTA, took 690). status[0] = 0, or j + 1 when the j-th pivot is not positive
+// (R is then not written).
+constexpr int kCholThreads = 512;
+__global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double* __restrict__ G, int k, double* R,
+                                                                   int* status) {
   extern __shared__ double cf_smem[];
   double* L = cf_smem;
-  double* aux = L + k * (k + 1) / 2;  // pivots, then their reciprocals
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
-    const int i = q % k, j = q / k;
-    if (i >= j) L[lo_off(j, k) + i - j] = G[q];
-  }
-  __syncthreads();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  int bad = 0;
-  for (int j = 0; j < k; ++j) {
-    const double d = L[lo_off(j, k)];
-    if (!(d > 0.0)) {  // every thread reads the same pivot: a uniform exit
-      bad = j + 1;
-      break;
+  __shared__ int bad;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) bad = 0;
+#pragma unroll 4
+  for (int j = warp; j < k; j += kCholThreads / 32)
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {  // k <= 225 rows
+      const int i = lane + 32 * v;
+      if (i >= j && i < k) L[lo_off(j, k) + i - j] = G[i + j * k];
     }
-    const double dinv = 1.0 / d;
-    const double* colj = L + lo_off(j, k) - j;  // colj[a] = L(a, j)
-    for (int b = j + 1 + ty; b < k; b += 32) {
-      const double lbj = colj[b] * dinv;
-      double* colb = L + lo_off(b, k) - b;
-      for (int a = b + tx; a < k; a += 32) colb[a] = fma(-colj[a], lbj, colb[a]);
+  __syncthreads();
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    const int nb = min(8, k - j0);
+    const int i = j0 + threadIdx.x;  // this thread's row
+    double x[8];
+    if (i < k) {
+      // the diagonal block, a pad of the identity past k
+      double d[8][8], inv[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int e = c; e < 8; ++e)
+          d[e][c] = (e < nb && c < nb) ? L[lo_off(j0 + c, k) + e - c] : (e == c ? 1.0 : 0.0);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) x[c] = (c < nb && i >= j0 + c) ? L[lo_off(j0 + c, k) + i - j0 - c] : 0.0;
+      int wrong = 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        double p = d[c][c];
+        if (!(p > 0.0)) {
+          if (!wrong) wrong = j0 + c + 1;
+          p = 1.0;
+        }
+        inv[c] = rsqrt(p);
+        d[c][c] = p * inv[c];
+#pragma unroll
+        for (int e = c + 1; e < 8; ++e) d[e][c] *= inv[c];
+#pragma unroll
+        for (int f = c + 1; f < 8; ++f)
+#pragma unroll
+          for (int e = f; e < 8; ++e) d[e][f] = fma(-d[e][c], d[f][c], d[e][f]);
+      }
+      if (wrong && threadIdx.x == 0) bad = wrong;
+      if (threadIdx.x < 8) {
+        // a row of the diagonal block
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (e == (int)threadIdx.x) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) x[c] = c <= e ? d[e][c] : 0.0;
+          }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+#pragma unroll
+          for (int e = 0; e < c; ++e) x[c] = fma(-x[e], d[c][e], x[c]);
+          x[c] *= inv[c];
+        }
+      }
+    }
+    __syncthreads();  // every thread has read the panel
+    if (bad) break;
+    if (i < k) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c < nb && i >= j0 + c) L[lo_off(j0 + c, k) + i - j0 - c] = x[c];
+    }
+    __syncthreads();
+    const double* pc[8];  // pc[c][a] = L(a, j0 + c)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) pc[c] = L + lo_off(j0 + c, k) - (j0 + c);
+    // nb < 8 only in the last panel, which has no trailing columns
+    for (int b0 = j0 + 8 + 4 * warp; b0 < k; b0 += 4 * (kCholThreads / 32)) {
+      double lb[4][8];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) lb[q][c] = b0 + q < k ? pc[c][b0 + q] : 0.0;
+      for (int a = b0 + lane; a < k; a += 32) {
+        double la[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) la[c] = pc[c][a];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (b0 + q >= k || a < b0 + q) continue;
+          double* g = L + lo_off(b0 + q, k) + a - b0 - q;
+          double v = *g;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) v = fma(-la[c], lb[q][c], v);
+          *g = v;
+        }
+      }
     }
     __syncthreads();
   }
@@ -675,42 +785,12 @@ __global__ void __launch_bounds__(1024) chol_factor_kernel(const double* G, int 
     if (threadIdx.x == 0) status[0] = bad;
     return;
   }
-  for (int j = threadIdx.x; j < k; j += blockDim.x) aux[j] = sqrt(L[lo_off(j, k)]);
-  __syncthreads();
-  for (int j = ty; j < k; j += 32) {
-    const double p = aux[j];
-    double* colj = L + lo_off(j, k) - j;
-    for (int i = j + tx; i < k; i += 32) colj[i] = (i == j) ? p : colj[i] / p;
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
-    const int i = q % k, j = q / k;
-    R[q] = (i <= j) ? L[lo_off(i, k) + j - i] : 0.0;
-  }
-  for (int j = threadIdx.x; j < k; j += blockDim.x) aux[j] = 1.0 / aux[j];
-  __syncthreads();
-  for (int j = ty; j < k; j += 32) {
-    double b[VMAX];
+  for (int j = warp; j < k; j += kCholThreads / 32)
 #pragma unroll
-    for (int v = 0; v < VMAX; ++v) b[v] = (tx + 32 * v == j) ? 1.0 : 0.0;
-    for (int l = j; l < k; ++l) {
-      const double yl = __shfl_sync(0xffffffffu, pick(b, l >> 5) * aux[l], l & 31);
-      const double* coll = L + lo_off(l, k) - l;
-#pragma unroll
-      for (int v = 0; v < VMAX; ++v) {
-        const int i = tx + 32 * v;
-        if (i > l && i < k)
-          b[v] = fma(-coll[i], yl, b[v]);
-        else if (i == l)
-          b[v] = yl;
-      }
+    for (int v = 0; v < 8; ++v) {
+      const int i = lane + 32 * v;
+      if (i < k) R[i + j * k] = (i <= j) ? L[lo_off(i, k) + j - i] : 0.0;
     }
-#pragma unroll
-    for (int v = 0; v < VMAX; ++v) {
-      const int i = tx + 32 * v;
-      if (i < k) Rinv[j + (int64_t)i * k] = (i >= j) ? b[v] : 0.0;
-    }
-  }
   if (threadIdx.x == 0) status[0] = 0;
 }
 
@@ -1118,29 +1198,29 @@ int g1(const skema_ctx* c, int64_t total) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)c->sm_count * 16));
 }
 
-// R X = B in place for upper-triangular R (k x k) and B (k x nrhs, ld ldb):
-// the packed shared-memory kernel when R fits, else one warp per right-hand
-// side reading R from global memory.
+// R X = B in place (identity: X = R^{-1}) for upper-triangular R (k x k) and
+// B (k x nrhs, ld ldb): the packed shared-memory kernel when R fits, else one
+// warp per right-hand side reading R from global memory.
+void tri_solve(skema_ctx* c, const double* R, int64_t k, double* B, int64_t ldb, int64_t nrhs, bool identity,
+               const int* status) {
+  // up to four warps a CTA, as many as have room for their right-hand sides
+  const size_t warp_bytes = sizeof(double) * 8 * (size_t)tri_ld((int)k);
+  const int warps =
+      (int)std::max<size_t>(1, std::min<size_t>({4, (size_t)(nrhs + 7) / 8, (226 * 1024 - packed_smem_bytes(k)) / warp_bytes}));
+  const size_t smem = packed_smem_bytes(k) + warps * warp_bytes;
+  SKEMA_CUDA(cudaFuncSetAttribute(tri_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = (int)((nrhs + 8 * warps - 1) / (8 * warps));
+  tri_solve_kernel<<<grid, kTriThreads, smem, c->stream>>>(R, (int)k, B, ldb, (int)nrhs, warps, identity ? 1 : 0,
+                                                          status);
+  SKEMA_LAUNCHED(c);
+}
 void trsm_upper(skema_ctx* c, const double* R, int64_t k, double* B, int64_t ldb, int64_t nrhs) {
   if (nrhs <= 0 || k <= 0) return;
   if (k <= kPackedMaxK) {
-    const size_t smem = packed_smem_bytes(k);
-    const int grid = (int)((nrhs + 7) / 8);
-    auto launch = [&](auto kern) {
-      SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      kern<<<grid, 256, smem, c->stream>>>(R, (int)k, B, ldb, (int)nrhs);
-    };
-    if (k <= 32)
-      launch(trsm_upper_packed_kernel<1>);
-    else if (k <= 64)
-      launch(trsm_upper_packed_kernel<2>);
-    else if (k <= 128)
-      launch(trsm_upper_packed_kernel<4>);
-    else
-      launch(trsm_upper_packed_kernel<8>);
-  } else {
-    trsm_upper_kernel<<<(int)((nrhs * 32 + 255) / 256), 256, 0, c->stream>>>(R, k, B, ldb, nrhs);
+    tri_solve(c, R, k, B, ldb, nrhs, false, nullptr);
+    return;
   }
+  trsm_upper_kernel<<<(int)((nrhs * 32 + 255) / 256), 256, 0, c->stream>>>(R, k, B, ldb, nrhs);
   SKEMA_LAUNCHED(c);
 }
 
@@ -1150,19 +1230,10 @@ void trsm_upper(skema_ctx* c, const double* R, int64_t k, double* B, int64_t ldb
 void chol_inverse(skema_ctx* c, double* G, int64_t k, double* R, double* Rinv, int* st) {
   if (k <= kPackedMaxK) {
     const size_t smem = packed_smem_bytes(k);
-    auto launch = [&](auto kern) {
-      SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      kern<<<1, 1024, smem, c->stream>>>(G, (int)k, R, Rinv, st);
-    };
-    if (k <= 32)
-      launch(chol_factor_kernel<1>);
-    else if (k <= 64)
-      launch(chol_factor_kernel<2>);
-    else if (k <= 128)
-      launch(chol_factor_kernel<4>);
-    else
-      launch(chol_factor_kernel<8>);
+    SKEMA_CUDA(cudaFuncSetAttribute(chol_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    chol_factor_kernel<<<1, kCholThreads, smem, c->stream>>>(G, (int)k, R, st);
     SKEMA_LAUNCHED(c);
+    tri_solve(c, R, k, Rinv, k, k, true, st);
     return;
   }
   cholesky_kernel<<<1, 1024, 0, c->stream>>>(G, k, st);
