@@ -17,7 +17,8 @@
 // when the Gram matrix is not numerically positive definite. The Q factor
 // equals Householder's up to column signs, so S is unchanged and U, V match
 // LAPACK's up to sign. The SVD of the k x k core is a one-sided (Hestenes)
-// Jacobi SVD with round-robin pair ordering in one CTA.
+// Jacobi SVD with round-robin pair ordering in one cluster of CTAs.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -897,106 +898,365 @@ __global__ void colsparse_apply_smem_kernel(const uint32_t* __restrict__ mp, int
 }
 
 // ------------------------------------------------------ Jacobi SVD ---------
-// One-sided Jacobi on the column-major k x k A (overwritten by A V = U S),
-// V accumulated (column-major k x k). One CTA; each half-warp rotates one
-// pair of a round-robin round, and a sweep ends the loop when it made no
-// rotation (every pair within tol of orthogonal).
-// A and V are worked on in shared memory (2 k^2 doubles, k <= 114), copied
-// in at the start and out at the end; every rotation reads and writes two
-// columns of each, so global memory would put an L2 round trip on every
-// step.
-__global__ void __launch_bounds__(1024) jacobi_svd_kernel(double* Ag, double* Vg, int64_t k64, int max_sweeps,
-                                                            double tol, int* sweeps_out) {
-  __shared__ int rotated;
-  extern __shared__ double jac_smem[];
-  const int k = (int)k64;
-  double* A = jac_smem;
-  double* V = jac_smem + (size_t)k * k;
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
-    A[q] = Ag[q];
-    V[q] = (q % k == q / k) ? 1.0 : 0.0;
+// The rotation of a pair of columns with squared norms al, be and product ga:
+// tan of the angle is the smaller root of t^2 + 2 zeta t - 1 with zeta = d / h,
+// d = beta - alpha, h = 2 gamma, t = sign(d) h / (|d| + sqrt(d^2 + h^2)). It is
+// on the chain that every round waits for, and a dependent FP64 operation takes
+// about 30 cycles, so (c0, s0) comes from FP32 (d and h scaled by a power of
+// two) and one Newton step corrects it in FP64: the rotated product is
+//   F = (c0^2 - s0^2) h / 2 - c0 s0 d,  delta = F / (sign(d) sqrt(d^2 + h^2)),
+// the angle moves by delta (1e-7, so its square is FP64 rounding) and the pair
+// is normalised by 1 - e / 2 + 3 e^2 / 8 - delta^2 / 2, e = c0^2 + s0^2 - 1, which
+// needs neither the corrected values nor a square root. False: the pair is
+// orthogonal to tol and stays.
+__device__ __forceinline__ bool jacobi_angle(double al, double be, double ga, double tol2, double& cs, double& sn) {
+  cs = 1.0, sn = 0.0;
+  if (ga == 0.0 || ga * ga <= tol2 * (al * be)) return false;
+  double d = be - al, h = ga + ga;
+  const int e = max(__double2hiint(d) & 0x7ff00000, __double2hiint(h) & 0x7ff00000);
+  const double sc = __hiloint2double(0x7fe00000 - e, 0);  // 2^-exponent, a normal number
+  d *= sc;
+  h *= sc;
+  const float df = (float)d, hf = (float)h;
+  const float w2 = fmaf(df, df, hf * hf), rw = rsqrtf(w2);  // w2 is at least 1
+  const float sg = df < 0.f ? -1.f : 1.f;
+  const float t = sg * __fdividef(hf, fabsf(df) + w2 * rw);
+  const float cf = rsqrtf(fmaf(t, t, 1.f));
+  const double c0 = (double)cf, s0 = (double)(cf * t), rwd = (double)(sg * rw);
+  const double cc = c0 * c0, ss = s0 * s0;
+  const double delta = fma(0.5 * h, cc - ss, -(d * (c0 * s0))) * rwd;
+  const double eps = (cc - 1.0) + ss;
+  const double f0 = fma(fma(0.375, eps, -0.5), eps, 1.0), c1 = c0 * f0, s1 = s0 * f0;
+  const double hd = -0.5 * delta;
+  cs = fma(delta, fma(hd, c1, -s1), c1);
+  sn = fma(delta, fma(hd, s1, c1), s1);
+  return true;
+}
+
+// Players p < q of pair pr in a round of a round-robin among np (even) players:
+// the last stays, the others rotate.
+__device__ __forceinline__ void robin_pair(int np, int round, int pr, int& p, int& q) {
+  if (pr == 0) {
+    p = round;
+    q = np - 1;
+    return;
   }
-  // a pair per half-warp: 64 pairs at a time, all of them for k <= 128
-  const int hl = threadIdx.x & 15, slot = threadIdx.x >> 4, nslot = blockDim.x >> 4;
+  p = round + pr;
+  if (p >= np - 1) p -= np - 1;
+  q = round - pr;
+  if (q < 0) q += np - 1;
+}
+
+// One-sided Jacobi on the column-major k x k A (overwritten by A V = U S),
+// V accumulated (column-major k x k), k <= 114. A cluster of two CTAs: CTA 0
+// holds A in shared memory and rotates the pairs of each round of a round-robin,
+// a half-warp per pair with the pair's columns in registers (EPL values of each
+// per lane), writing every (cs, sn) of the sweep to rot; CTA 1 holds V and
+// applies the sweep before, rows along the threads and the round's pairs over
+// groups of threads. So a round is one read and one write of A, its dot products
+// and one angle; V's traffic and FP64 work (as much again) are off that chain. A sweep without a rotation
+// (every pair within tol of orthogonal) ends the loop.
+// rot: two buffers of (kp - 1) (kp / 2) double2, kp = k rounded up to even, and
+// two flags after them. k = 81, 11 sweeps: 1.18 ms (2,500 cycles a round: the chain of
+// dependent FP64 operations and 1,000 cycles of shared memory); one CTA with A
+// and V took 1.80.
+constexpr int kJacMaxK = 114;
+constexpr size_t kJacRotBytes = sizeof(double2) * 2 * (kJacMaxK - 1) * (kJacMaxK / 2) + 16;
+
+template <int EPL>
+__global__ void __launch_bounds__(EPL == 8 ? 960 : 128 * EPL) jacobi_svd_kernel(double* __restrict__ Ag, double* __restrict__ Vg, int k,
+                                                            int max_sweeps, double tol, double2* rot,
+                                                            int* sweeps_out) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ __align__(16) double jac_smem[];
+  __shared__ int any;
+  const int kp = (k + 1) & ~1, npair = kp / 2, nrot = (kp - 1) * npair;
+  volatile int* flags = reinterpret_cast<int*>(rot + 2 * nrot);
+  const bool is_v = cl.block_rank() == 1;
+  double* M = jac_smem;  // A or V
+  for (int q = threadIdx.x; q < k * k; q += blockDim.x) M[q] = is_v ? ((q % k == q / k) ? 1.0 : 0.0) : Ag[q];
+  double2* rs = reinterpret_cast<double2*>(jac_smem + ((size_t)k * k + 1) / 2 * 2);  // CTA 1: a sweep's rotations
+  __syncthreads();
+  const int hl = threadIdx.x & 15, pr = threadIdx.x >> 4;
   const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
-  const int kp = (k + 1) & ~1;  // even number of players
-  int sweep = 0;
-  for (; sweep < max_sweeps; ++sweep) {
-    if (threadIdx.x == 0) rotated = 0;
+  const double tol2 = tol * tol;
+  // rows of V along the threads, the pairs of a round over the groups of rows
+  const int rk = (k + 31) & ~31, grp = threadIdx.x / rk, ngrp = blockDim.x / rk, row = threadIdx.x - grp * rk;
+  auto apply_v = [&](const double2* src) {
+    for (int q = threadIdx.x; q < nrot; q += blockDim.x) rs[q] = __ldcg(src + q);
     __syncthreads();
     for (int round = 0; round < kp - 1; ++round) {
-      for (int pr = slot; pr < kp / 2; pr += nslot) {
-        // round-robin pairing: player kp-1 stays, the others rotate
-        int p, q;
-        if (pr == 0) {
-          p = round;
-          q = kp - 1;
-        } else {
-          p = round + pr;
-          if (p >= kp - 1) p -= kp - 1;
-          q = round - pr;
-          if (q < 0) q += kp - 1;
+      if (grp < ngrp && row < k)
+        for (int g = grp; g < npair; g += 2 * ngrp) {
+          int p[2], q[2];
+          double x[2], y[2];
+          double2 r[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int pp = min(g + u * ngrp, npair - 1);
+            robin_pair(kp, round, pp, p[u], q[u]);
+            if (p[u] > q[u]) {
+              const int t = p[u];
+              p[u] = q[u];
+              q[u] = t;
+            }
+            if (g + u * ngrp >= npair || q[u] >= k) p[u] = -1;
+            if (p[u] >= 0) x[u] = M[p[u] * k + row], y[u] = M[q[u] * k + row], r[u] = rs[round * npair + pp];
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            if (p[u] >= 0) {
+              M[p[u] * k + row] = r[u].x * x[u] - r[u].y * y[u];
+              M[q[u] * k + row] = r[u].y * x[u] + r[u].x * y[u];
+            }
         }
+      __syncthreads();
+    }
+  };
+  int sweep = 0;
+  bool more = true;
+  for (; sweep < max_sweeps; ++sweep) {
+    if (!is_v) {
+      if (threadIdx.x == 0) any = 0;
+      __syncthreads();
+      double2* out = rot + (sweep & 1) * nrot;
+      for (int round = 0; round < kp - 1; ++round) {
+        int p, q;
+        robin_pair(kp, round, min(pr, npair - 1), p, q);
         if (p > q) {
           const int t = p;
           p = q;
           q = t;
         }
-        if (q >= k) continue;  // bye
-        double* ap = A + (size_t)p * k;
-        double* aq = A + (size_t)q * k;
-        double al = 0.0, be = 0.0, ga = 0.0;
-        for (int i = hl; i < k; i += 16) {
-          const double x = ap[i], y = aq[i];
-          al = fma(x, x, al);
-          be = fma(y, y, be);
-          ga = fma(x, y, ga);
+        if (pr < npair && q < k) {  // q == k: a bye
+          double* ap = M + p * k;
+          double* aq = M + q * k;
+          // two sums of each product: the chains of dependent FMAs are half as long
+          double x[EPL], y[EPL], sa[2] = {0.0, 0.0}, sb[2] = {0.0, 0.0}, sg[2] = {0.0, 0.0};
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) {
+            const int i = hl + 16 * e;
+            x[e] = i < k ? ap[i] : 0.0;
+            y[e] = i < k ? aq[i] : 0.0;
+          }
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) {
+            sa[e & 1] = fma(x[e], x[e], sa[e & 1]);
+            sb[e & 1] = fma(y[e], y[e], sb[e & 1]);
+            sg[e & 1] = fma(x[e], y[e], sg[e & 1]);
+          }
+          // lanes 0-7 of the half-warp go on with al and ga, lanes 8-15 with be:
+          // fewer FP64 additions than three full butterflies
+          double al = sa[0] + sa[1], be = sb[0] + sb[1], ga = sg[0] + sg[1];
+          const bool up = hl & 8;
+          double n1 = (up ? be : al) + __shfl_xor_sync(hmask, up ? al : be, 8);
+          ga += __shfl_xor_sync(hmask, ga, 8);
+          // then lanes 4-7 (mod 8) take ga, the others the norm
+          const bool up2 = hl & 4;
+          double n2 = (up2 ? ga : n1) + __shfl_xor_sync(hmask, up2 ? n1 : ga, 4);
+#pragma unroll
+          for (int o = 2; o > 0; o >>= 1) n2 += __shfl_xor_sync(hmask, n2, o);
+          const int l0 = threadIdx.x & 16;
+          al = __shfl_sync(hmask, n2, l0);
+          ga = __shfl_sync(hmask, n2, l0 + 4);
+          be = __shfl_sync(hmask, n2, l0 + 8);
+          double cs, sn;
+          if (jacobi_angle(al, be, ga, tol2, cs, sn)) {
+            if (hl == 0) any = 1;
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) {
+              const int i = hl + 16 * e;
+              if (i < k) {
+                ap[i] = cs * x[e] - sn * y[e];
+                aq[i] = sn * x[e] + cs * y[e];
+              }
+            }
+          }
+          if (hl == 0) __stcg(out + round * npair + pr, make_double2(cs, sn));
+        }
+        __syncthreads();
+      }
+      if (threadIdx.x == 0) flags[sweep & 1] = any;
+    } else if (sweep > 0) {
+      apply_v(rot + ((sweep - 1) & 1) * nrot);
+    }
+    cl.sync();  // releases the sweep's rotations and flag to CTA 1
+    more = flags[sweep & 1] != 0;
+    if (!more) break;
+  }
+  // CTA 1 is one sweep behind; a sweep without rotations leaves nothing to do
+  if (is_v && more && sweep > 0) apply_v(rot + ((sweep - 1) & 1) * nrot);
+  if (!is_v && threadIdx.x == 0) sweeps_out[0] = sweep;
+  __syncthreads();
+  double* out = is_v ? Vg : Ag;
+  for (int q = threadIdx.x; q < k * k; q += blockDim.x) out[q] = M[q];
+}
+
+// Block one-sided Jacobi, 114 < k <= 256: the columns are cut into nb blocks of
+// eight, an outer round pairs the blocks round-robin and a CTA takes a pair of
+// blocks (16 columns); nb / 2 CTAs form one cluster and meet at its barrier
+// after every round, so all sweeps are one launch. Per round a CTA forms the
+// Gram matrix of its 16 columns (FP64 tensor cores), runs one inner sweep of
+// rotations on it (the two-sided update of 16 x 16 values, one barrier per inner
+// round, no pass over the columns), and multiplies its columns of A and V by the
+// accumulated 16 x 16 rotation. The Gram matrix is formed afresh in every
+// round, so what its updates lose early is corrected later, and a round without
+// rotations leaves the columns as they are; sweeps go on until one makes none.
+// k = 201, 13 sweeps: 4.0 ms, four fifths of it the chain of angles (about 1,000
+// cycles per inner round). With every rotation passing over the columns and a
+// launch per round it took 10.
+constexpr int kJacClusterMaxK = 256;
+__global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(double* Ag, double* Vg, int k, int nb, int max_sweeps,
+                                                             double tol, int* sweeps_out) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  constexpr int P = 16, LG = 17;
+  extern __shared__ __align__(16) double jc_smem[];
+  __shared__ double G[2][P * LG], J[2][P * LG], part[8][3][64];
+  __shared__ int any_round, any_sweep;
+  const int ld = tri_ld(k);
+  double* Ac = jc_smem;           // column c at Ac + c * ld, rows past k zero
+  double* Vc = jc_smem + P * ld;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane & 3, lc = lane >> 2;
+  const int kr = (k + 7) & ~7;  // rows in whole MMA blocks
+  const double tol2 = tol * tol;
+  int sweep = 0;
+  for (; sweep < max_sweeps; ++sweep) {
+    if (tid == 0) any_sweep = 0;
+    for (int round = 0; round < nb - 1; ++round) {
+      int bi, bj;
+      robin_pair(nb, round, (int)blockIdx.x, bi, bj);
+      auto gcol = [&](int c) { return c < 8 ? bi * 8 + c : bj * 8 + (c - 8); };
+      for (int c = warp; c < P; c += 8) {
+        const int g = gcol(c);
+        double x[8], y[8];  // k <= 256: a column of each in flight
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const int i = lane + 32 * v;
+          const bool in = g < k && i < k;
+          x[v] = in ? __ldcg(Ag + (size_t)g * k + i) : 0.0;
+          y[v] = in ? __ldcg(Vg + (size_t)g * k + i) : 0.0;
         }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-          al += __shfl_xor_sync(hmask, al, o);
-          be += __shfl_xor_sync(hmask, be, o);
-          ga += __shfl_xor_sync(hmask, ga, o);
+        for (int v = 0; v < 8; ++v) {
+          const int i = lane + 32 * v;
+          if (i < kr) Ac[c * ld + i] = x[v], Vc[c * ld + i] = y[v];
         }
-        // converged pair: |gamma| <= tol sqrt(alpha beta), compared squared
-        if (ga == 0.0 || ga * ga <= (tol * tol) * (al * be)) continue;
-        if (hl == 0) rotated = 1;
-        // tan of the rotation angle, the smaller root of t^2 + 2 zeta t - 1
-        // with zeta = d / h, d = beta - alpha, h = 2 gamma, written as
-        // t = sign(d) h / (|d| + sqrt(d^2 + h^2)): one square root and one
-        // division on the chain that every round waits for
-        const double d = be - al, h = 2.0 * ga;
-        const double t = (d >= 0.0 ? h : -h) / (fabs(d) + sqrt(fma(d, d, h * h)));
-        const double cs = rsqrt(fma(t, t, 1.0)), sn = cs * t;
-        for (int i = hl; i < k; i += 16) {
-          const double x = ap[i], y = aq[i];
-          ap[i] = cs * x - sn * y;
-          aq[i] = sn * x + cs * y;
+      }
+      if (tid == 0) any_round = 0;
+      __syncthreads();
+      {  // Gram matrix: a warp per K steps of four rows, then a sum in warp order
+        double s00[2] = {0.0, 0.0}, s01[2] = {0.0, 0.0}, s11[2] = {0.0, 0.0};
+        for (int r = 4 * warp; r < kr; r += 32) {
+          const double a0 = Ac[lc * ld + r + lr], a1 = Ac[(8 + lc) * ld + r + lr];
+          dmma(s00, a0, a0);
+          dmma(s01, a0, a1);
+          dmma(s11, a1, a1);
         }
-        double* vp = V + (size_t)p * k;
-        double* vq = V + (size_t)q * k;
-        for (int i = hl; i < k; i += 16) {
-          const double x = vp[i], y = vq[i];
-          vp[i] = cs * x - sn * y;
-          vq[i] = sn * x + cs * y;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int e = lc * 8 + 2 * lr + h;
+          part[warp][0][e] = s00[h];
+          part[warp][1][e] = s01[h];
+          part[warp][2][e] = s11[h];
         }
       }
       __syncthreads();
+      if (tid < 192) {
+        const int blk = tid >> 6, e = tid & 63, i = e >> 3, j = e & 7;
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += part[w][blk][e];
+        if (blk == 0) {
+          G[0][i * LG + j] = v;
+        } else if (blk == 1) {
+          G[0][i * LG + 8 + j] = v;
+          G[0][(8 + j) * LG + i] = v;
+        } else {
+          G[0][(8 + i) * LG + 8 + j] = v;
+        }
+      }
+      J[0][(tid >> 4) * LG + (tid & 15)] = (tid >> 4) == (tid & 15) ? 1.0 : 0.0;
+      __syncthreads();
+      int cur = 0;
+      for (int r = 0; r < P - 1; ++r, cur ^= 1) {
+        // threads 0-63: the 2 x 2 block of pairs (a, b); 64-191: row i of J in
+        // pair b. Each works out the angles that it needs.
+        const double* Gc = G[cur];
+        if (tid < 192) {
+          const int b = tid & 7;
+          int p2, q2;
+          robin_pair(P, r, b, p2, q2);
+          double c2, s2;
+          const bool rot =
+              jacobi_angle(Gc[p2 * LG + p2], Gc[q2 * LG + q2], Gc[p2 * LG + q2], tol2, c2, s2);
+          if (tid < 64) {
+            int p1, q1;
+            robin_pair(P, r, tid >> 3, p1, q1);
+            double c1, s1;
+            jacobi_angle(Gc[p1 * LG + p1], Gc[q1 * LG + q1], Gc[p1 * LG + q1], tol2, c1, s1);
+            const double pp = Gc[p1 * LG + p2], pq = Gc[p1 * LG + q2], qp = Gc[q1 * LG + p2], qq = Gc[q1 * LG + q2];
+            const double rp = c1 * pp - s1 * qp, rq = c1 * pq - s1 * qq;
+            const double tp = s1 * pp + c1 * qp, tq = s1 * pq + c1 * qq;
+            double* Gn = G[cur ^ 1];
+            Gn[p1 * LG + p2] = c2 * rp - s2 * rq;
+            Gn[p1 * LG + q2] = s2 * rp + c2 * rq;
+            Gn[q1 * LG + p2] = c2 * tp - s2 * tq;
+            Gn[q1 * LG + q2] = s2 * tp + c2 * tq;
+            if (rot) any_round = 1;
+          } else {
+            const int i = (tid - 64) >> 3;
+            const double x = J[cur][i * LG + p2], y = J[cur][i * LG + q2];
+            J[cur ^ 1][i * LG + p2] = c2 * x - s2 * y;
+            J[cur ^ 1][i * LG + q2] = s2 * x + c2 * y;
+          }
+        }
+        __syncthreads();
+      }
+      if (any_round) {
+        if (tid == 0) any_sweep = 1;
+        const double* Jc = J[cur];
+        double jb[4][2];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int n = 0; n < 2; ++n) jb[t][n] = Jc[(4 * t + lr) * LG + 8 * n + lc];
+        for (int w = warp; w < kr / 4; w += 8) {  // row blocks of A, then of V
+          const bool v = w >= kr / 8;
+          const int row = 8 * (v ? w - kr / 8 : w) + lc;
+          const double* S = v ? Vc : Ac;
+          double* D = v ? Vg : Ag;
+          double o[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const double a = S[(4 * t + lr) * ld + row];
+            dmma(o[0], a, jb[t][0]);
+            dmma(o[1], a, jb[t][1]);
+          }
+          if (row < k) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int g = gcol(8 * n + 2 * lr + h);
+                if (g < k) __stcg(D + (size_t)g * k + row, o[n][h]);
+              }
+          }
+        }
+      }
+      cl.sync();  // the round's columns are in place for the next round's CTAs
     }
-    const bool more = rotated != 0;
-    __syncthreads();
+    bool more = false;
+    for (unsigned b = 0; b < cl.num_blocks(); ++b) more |= *cl.map_shared_rank(&any_sweep, b) != 0;
+    cl.sync();  // every CTA has read every flag
     if (!more) break;
   }
-  if (threadIdx.x == 0) sweeps_out[0] = sweep;
-  __syncthreads();
-  for (int q = threadIdx.x; q < k * k; q += blockDim.x) {
-    Ag[q] = A[q];
-    Vg[q] = V[q];
-  }
+  if (blockIdx.x == 0 && tid == 0) sweeps_out[0] = sweep;
 }
 
-// Block one-sided Jacobi for a k x k problem too large for one CTA's shared
-// memory. The columns are cut into nb blocks of bs (the last ones short or
+// Block one-sided Jacobi for k above the cluster form, or where the device has
+// no room for its cluster: one launch per outer round. The columns are cut into nb blocks of bs (the last ones short or
 // empty). An outer round pairs the blocks round-robin; each CTA takes one
 // pair (I, J), copies the up to 2 bs columns of A and V into shared memory,
 // runs one inner sweep of the one-sided Jacobi rotations over all pairs of
@@ -1130,41 +1390,79 @@ void jacobi_svd_blocked(skema_ctx* c, double* A, double* V, int64_t k, int max_s
   SKEMA_LAUNCHED(c);
 }
 
-// The SVD kernel for a k x k problem: shared memory when A and V fit.
-void jacobi_svd(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, double tol, int* sweeps_out) {
-  const size_t smem = sizeof(double) * (size_t)(2 * k * k);
-  // a half-warp per pair of a round: (k + 1) / 2 pairs, at most 64 at a time
-  const int threads = (int)std::min<int64_t>(1024, ((k + 1) / 2 * 16 + 31) / 32 * 32);
-  if (smem <= 200 * 1024) {
-    SKEMA_CUDA(cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    jacobi_svd_kernel<<<1, threads, smem, c->stream>>>(A, V, k, max_sweeps, tol, sweeps_out);
-    SKEMA_LAUNCHED(c);
-    return;
+// One cluster of `ctas` CTAs; false when the device cannot place it.
+template <typename Kern, typename... Args>
+bool launch_one_cluster(skema_ctx* c, Kern kern, int ctas, int threads, size_t smem, Args... args) {
+  SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (ctas > 8) SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    return false;
   }
-  // larger k: block sweeps in shared memory (a single CTA working on A and
-  // V in global memory took 51 ms at k = 201, with every rotation waiting
-  // on L2)
+  SKEMA_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  SKEMA_LAUNCHED(c);
+  return true;
+}
+
+// The SVD kernel for a k x k problem: one pair of CTAs while A and V fit their
+// shared memory, block sweeps in one cluster up to k = 256, else block sweeps
+// driven from the host.
+void jacobi_svd(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, double tol, int* sweeps_out) {
+  if (k <= kJacMaxK) {
+    const int kp = (int)((k + 1) & ~1);
+    const size_t smem = sizeof(double) * ((size_t)(k * k + 1) / 2 * 2) + sizeof(double2) * (size_t)(kp - 1) * (kp / 2);
+    const int threads = std::max(128, (kp / 2 * 16 + 31) / 32 * 32);
+    double2* rot = static_cast<double2*>(c->jac_rot);
+    auto go = [&](auto kern) {
+      return launch_one_cluster(c, kern, 2, threads, smem, A, V, (int)k, max_sweeps, tol, rot, sweeps_out);
+    };
+    if (k <= 32 ? go(jacobi_svd_kernel<2>) : k <= 64 ? go(jacobi_svd_kernel<4>) : k <= 96 ? go(jacobi_svd_kernel<6>) : go(jacobi_svd_kernel<8>)) return;
+  } else if (k <= kJacClusterMaxK) {
+    const int nb = (int)((k + 15) / 16 * 2);
+    const size_t smem = sizeof(double) * 2 * 16 * (size_t)tri_ld((int)k);
+    identity_kernel<<<(unsigned)std::min<int64_t>((k * k + 255) / 256, 4096), 256, 0, c->stream>>>(V, k);
+    SKEMA_LAUNCHED(c);
+    if (launch_one_cluster(c, jacobi_cluster_kernel, nb / 2, 256, smem, A, V, (int)k, nb, max_sweeps, tol, sweeps_out))
+      return;
+  }
   jacobi_svd_blocked(c, A, V, k, max_sweeps, tol, sweeps_out);
 }
 
 // sigma_j = ||a_j||, ranks by descending sigma (ties by index), then
 // U(:, rank) = a_j / sigma_j, Vout(:, rank) = v_j, S(rank) = sigma_j.
-__global__ void svd_finish_kernel(const double* A, const double* V, int64_t k, double* U,
-                                  double* Vout, double* S, double* sig) {
-  for (int64_t j = threadIdx.x; j < k; j += blockDim.x) {
+// One CTA, a warp per column (a thread per column walked k^2 values 8 k bytes
+// apart: 108 us at k = 201).
+constexpr int kFinishThreads = 1024;
+__global__ void __launch_bounds__(kFinishThreads) svd_finish_kernel(const double* A, const double* V, int64_t k,
+                                                                    double* U, double* Vout, double* S, double* sig) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t j = warp; j < k; j += kFinishThreads / 32) {
     double s = 0.0;
-    for (int64_t i = 0; i < k; ++i) s += A[i + j * k] * A[i + j * k];
-    sig[j] = sqrt(s);
+    for (int64_t i = lane; i < k; i += 32) s = fma(A[i + j * k], A[i + j * k], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) sig[j] = sqrt(s);
   }
   __syncthreads();
-  for (int64_t j = threadIdx.x; j < k; j += blockDim.x) {
-    int64_t rank = 0;
+  for (int64_t j = warp; j < k; j += kFinishThreads / 32) {
     const double sj = sig[j];
-    for (int64_t l = 0; l < k; ++l)
-      if (sig[l] > sj || (sig[l] == sj && l < j)) ++rank;
-    S[rank] = sj;
+    int rank = 0;
+    for (int64_t l = lane; l < k; l += 32) rank += (sig[l] > sj || (sig[l] == sj && l < j)) ? 1 : 0;
+    rank = __reduce_add_sync(0xffffffffu, rank);
     const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-    for (int64_t i = 0; i < k; ++i) {
+    if (lane == 0) S[rank] = sj;
+    for (int64_t i = lane; i < k; i += 32) {
       U[i + rank * k] = A[i + j * k] * inv;
       Vout[i + rank * k] = V[i + j * k];
     }
@@ -1357,7 +1655,7 @@ void orth(skema_ctx* c, double* Qm, int64_t rows, int64_t k, double* Rscratch, d
   dgemm<double, double>(c, k, k, rows, 1.0, Qm, rows, 1, Qm, 1, rows, 0.0, G, 1, k);
   jacobi_svd(c, G, V, k, 60, 1e-15, dstatus + 1);
   // G V = U diag(lambda) with U = V for the symmetric positive semidefinite G
-  svd_finish_kernel<<<1, 256, 0, c->stream>>>(G, V, k, Rscratch /*U, unused*/, Vs, Sv, sig);
+  svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(G, V, k, Rscratch /*U, unused*/, Vs, Sv, sig);
   SKEMA_LAUNCHED(c);
   std::vector<double> lam(k), vs((size_t)(k * k));
   SKEMA_CUDA(cudaMemcpyAsync(lam.data(), Sv, sizeof(double) * (size_t)k, cudaMemcpyDeviceToHost, c->stream));
@@ -1603,7 +1901,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   // nu = ||Y||_2 = sqrt(lambda_max(Y^T Y))
   dgemm<double, double>(c, k, k, m, 1.0, Yd, m, 1, Yd, 1, m, 0.0, G, 1, k);
   jacobi_svd(c, G, Vc, k, 60, 1e-15, st + 1);
-  svd_finish_kernel<<<1, 256, 0, c->stream>>>(G, Vc, k, Uc, Vt, Sv, sig);
+  svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(G, Vc, k, Uc, Vt, Sv, sig);
   SKEMA_LAUNCHED(c);
   double lmax = 0.0;
   SKEMA_CUDA(cudaMemcpyAsync(&lmax, Sv, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1639,7 +1937,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   cholqr(c, E, m, k, RE, W, st);
   SKEMA_CUDA(cudaMemcpyAsync(Cw, RE, sizeof(double) * (size_t)(k * k), cudaMemcpyDeviceToDevice, c->stream));
   jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st + 1);
-  svd_finish_kernel<<<1, 256, 0, c->stream>>>(Cw, Vc, k, Uc, Vt, Sv, sig);
+  svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(Cw, Vc, k, Uc, Vt, Sv, sig);
   SKEMA_LAUNCHED(c);
   if (Uout) dgemm<double, double>(c, m, r, k, 1.0, E, 1, m, Uc, 1, k, 0.0, Uout, 1, m, false);
   if (Sout) {
@@ -1648,6 +1946,8 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   }
   SKEMA_CUDA(cudaStreamSynchronize(c->stream));
 }
+
+size_t jacobi_rot_bytes() { return kJacRotBytes; }
 
 void dgemm_f32_f64(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const float* A, int64_t ars,
                    int64_t acs, const double* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs,
@@ -1724,7 +2024,7 @@ void low_rank_approx_rows(skema_ctx* c, int64_t row0, int64_t nrows, const RankS
     dtranspose_kernel<<<g1(c, k * k), 256, 0, c->stream>>>(Z2t, Cw, k);
     SKEMA_LAUNCHED(c);
     jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st + 1);
-    svd_finish_kernel<<<1, 256, 0, c->stream>>>(Cw, Vc, k, C, Z2 /*Vout*/, Sv, sig);
+    svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(Cw, Vc, k, C, Z2 /*Vout*/, Sv, sig);
     SKEMA_LAUNCHED(c);
   }
   {

@@ -192,6 +192,9 @@ struct skema_ctx {
   // dev_err[0] non-zero when a wait timed out (checked at the next
   // synchronising call); dev_err[2..3] the wait limit in ns (64-bit).
   int* dev_err = nullptr;
+  // The rotations that the Jacobi SVD's two CTAs exchange (approx.cu), in the
+  // allocation of dev_err.
+  void* jac_rot = nullptr;
   bool dev_err_armed = false;
   // stage timers
   bool timing = false;
@@ -324,6 +327,7 @@ void rbf_vjp(skema_ctx* c, const float* pts, int64_t N, int64_t d,
              float* dpts, double* dgamma);
 
 // ---- FP64 approximation (approx.cu) ----
+size_t jacobi_rot_bytes();
 void low_rank_approx(skema_ctx* c, double* U, double* S, double* V);
 // Rows [row0, row0 + nrows) of a row-block sharded sketch, sums over the
 // ranks through fn (skema_low_rank_approx_rows).
