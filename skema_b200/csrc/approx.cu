@@ -228,41 +228,119 @@ void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA
 
 // ----------------------------------------- tall-skinny FP64 products -------
 // G += A^T A for a tall column-major A (rows x k, ld lda, k <= 256; T float
-// or double, widened to FP64 exactly). The k x k product is cut into 32 x 32
-// tiles and only the tiles on or above the diagonal are formed (6 of 9 at
-// k <= 96), each by P warps of the CTA that split the CTA's rows four at a
-// time; a warp holds its tile as 4 x 4 MMA blocks. For a step of four rows
-// the A fragment of column block c is A(r + lane % 4, c + lane / 4) and
-// the B fragment of the same block is the same value, so a tile reads its
-// two column ranges once per step. The partial tiles go to G (column-major
-// k x k, zeroed beforehand) with atomics, mirrored below the diagonal.
-//
-// The same kernel forms C = A^T B for two tall matrices with the same rows
-// (SYM = false: A rows x ka, B rows x kb, every 32 x 32 tile of the ka x kb
-// product; C column-major with ld ka), which is how a dense map meets a
-// tall basis (Phi~ Q = (Phi~^T)^T Q).
-template <typename TA, typename TB, bool SYM>
+// or double, widened to FP64 exactly). A CTA stages 32 rows of all k columns in
+// shared memory (128- or 256-byte runs of a column, widened once; a column's
+// 32 rows are 36 doubles apart, so fragment reads hit distinct banks) and its
+// warps form the 16 x 8 blocks on or above the diagonal with m16n8k16, up to
+// NT each, in registers over all of the CTA's rows; blockIdx.y takes a group of
+// blocks when they do not all fit. Up to three blocks a warp, two CTAs per SM
+// run, one staging while the other multiplies. The parts go to G (column-major k x k, zeroed
+// beforehand) with atomics, mirrored below the diagonal. Bound by the FP64
+// pipe: 1e6 x 81 takes 502 us from FP32 and 490 from FP64 (793 and 734 with
+// fragments read from global memory by every warp that needs them).
+constexpr int kGramTiles = 6, kGramLd = 36;
+template <typename T, int NT>
+__global__ void __launch_bounds__(512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T* __restrict__ A, int64_t lda, int k, int64_t rows,
+                                                          double* __restrict__ G, int64_t rows_per_cta) {
+  extern __shared__ __align__(16) double gr_smem[];  // (k up to 16) x kGramLd
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, lr = lane & 3, lc = lane >> 2;
+  const int nm = (k + 15) >> 4, nn = (k + 7) >> 3;
+  // this warp's blocks (mi, ni), ni >= 2 mi, m-major, consecutive
+  int mi[NT], ni[NT], cnt = 0;
+  {
+    const int per = NT * nw;
+    int total = 0;
+    for (int m = 0; m < nm; ++m) total += nn - 2 * m;
+    const int first = (int)blockIdx.y * per, last = min(total, first + per), n = last - first;
+    int t = first + (int)((int64_t)n * warp / nw);
+    const int te = first + (int)((int64_t)n * (warp + 1) / nw);
+    int m = 0, base = 0;
+    while (m < nm - 1 && t >= base + nn - 2 * m) base += nn - 2 * m, ++m;
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+      mi[q] = ni[q] = 0;
+      if (t < te) {
+        while (t >= base + nn - 2 * m) base += nn - 2 * m, ++m;
+        mi[q] = m;
+        ni[q] = 2 * m + t - base;
+        ++cnt;
+        ++t;
+      }
+    }
+  }
+  double acc[NT][4];
+#pragma unroll
+  for (int q = 0; q < NT; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0;
+  const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
+  const int kpad = nm * 16;
+  for (int64_t r = r0; r < r1; r += 32) {
+    const bool rv = r + lane < r1;
+    for (int c = warp; c < kpad; c += 4 * nw) {
+      T v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int cc = c + u * nw;
+        v[u] = (rv && cc < k) ? A[(int64_t)cc * lda + r + lane] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c + u * nw < kpad) gr_smem[(c + u * nw) * kGramLd + lane] = (double)v[u];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+      double a[8];
+      int held = -1;
+#pragma unroll
+      for (int q = 0; q < NT; ++q) {
+        if (q >= cnt) continue;
+        if (mi[q] != held) {
+          held = mi[q];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            a[i] = gr_smem[(16 * held + lc + 8 * (i & 1)) * kGramLd + h + lr + 4 * (i >> 1)];
+        }
+        double b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) b[i] = gr_smem[(8 * ni[q] + lc) * kGramLd + h + lr + 4 * i];
+        dmma16(acc[q], a, b);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < NT; ++q) {
+    if (q >= cnt) continue;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int gi = 16 * mi[q] + lc + 8 * (h >> 1), gj = 8 * ni[q] + 2 * lr + (h & 1);
+      if (gi >= k || gj >= k || gi > gj) continue;
+      atomicAdd(G + gi + (int64_t)gj * k, acc[q][h]);
+      if (gi != gj) atomicAdd(G + gj + (int64_t)gi * k, acc[q][h]);
+    }
+  }
+}
+
+// C += A^T B for two tall column-major matrices with the same rows (A rows x
+// ka, B rows x kb, kb <= 256; T float or double; C column-major with ld ka,
+// zeroed beforehand), which is how a dense map meets a tall basis (Phi~ Q =
+// (Phi~^T)^T Q). The product is cut into 32 x 32 tiles, each formed by P warps
+// of the CTA that split the CTA's rows four at a time; a warp holds its tile as
+// 4 x 4 MMA blocks (m8n8k4). For a step of four rows the fragment of column
+// block c is (r + lane % 4, c + lane / 4), for A and B alike. The partial tiles
+// go to C with atomics.
+template <typename TA, typename TB>
 __global__ void __launch_bounds__(512) atb_mma_kernel(const TA* __restrict__ A, int64_t lda, int ka,
                                                       const TB* __restrict__ B, int64_t ldb, int kb, int64_t rows,
                                                       double* __restrict__ G, int64_t rows_per_cta, int P) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nia = (ka + 31) >> 5, njb = (kb + 31) >> 5;
-  const int ntiles = SYM ? nia * (nia + 1) / 2 : nia * njb;
+  const int ntiles = nia * njb;
   // blockIdx.y takes a group of tiles when they do not all fit one CTA
   const int per_cta = (int)(blockDim.x >> 5) / P;
   const int tile = (int)blockIdx.y * per_cta + warp / P, part = warp % P;
   if (tile >= ntiles) return;
-  int ti, tj;
-  if (SYM) {  // tile -> (ti, tj), ti <= tj, row-major over the upper triangle
-    ti = 0, tj = tile;
-    while (tj >= nia - ti) {
-      tj -= nia - ti;
-      ++ti;
-    }
-    tj += ti;
-  } else {
-    ti = tile / njb, tj = tile - (tile / njb) * njb;
-  }
+  const int ti = tile / njb, tj = tile - (tile / njb) * njb;
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
   const int lr = lane & 3, lc = lane >> 2;
   const TA* ci[4];
@@ -283,7 +361,6 @@ __global__ void __launch_bounds__(512) atb_mma_kernel(const TA* __restrict__ A, 
     for (int n = 0; n < 4; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
   // two steps of four rows per iteration: their 16 loads are in flight
   // together before the 32 MMAs that use them
-  const bool diag = SYM && ti == tj;
   for (int64_t r = r0 + 4 * part; r < r1; r += 8 * P) {
     double a[2][4], b[2][4];
 #pragma unroll
@@ -293,7 +370,7 @@ __global__ void __launch_bounds__(512) atb_mma_kernel(const TA* __restrict__ A, 
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
         a[u][m] = (rv && vi[m]) ? (double)ci[m][row] : 0.0;
-        b[u][m] = (!diag && rv && vj[m]) ? (double)cj[m][row] : 0.0;
+        b[u][m] = (rv && vj[m]) ? (double)cj[m][row] : 0.0;
       }
     }
 #pragma unroll
@@ -301,7 +378,7 @@ __global__ void __launch_bounds__(512) atb_mma_kernel(const TA* __restrict__ A, 
 #pragma unroll
       for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) dmma(acc[m][n], a[u][m], diag ? a[u][n] : b[u][n]);
+        for (int n = 0; n < 4; ++n) dmma(acc[m][n], a[u][m], b[u][n]);
   }
 #pragma unroll
   for (int m = 0; m < 4; ++m)
@@ -312,18 +389,22 @@ __global__ void __launch_bounds__(512) atb_mma_kernel(const TA* __restrict__ A, 
         const int gi = 32 * ti + 8 * m + lc, gj = 32 * tj + 8 * n + 2 * lr + i;
         if (gi >= ka || gj >= kb) continue;
         atomicAdd(G + gi + (int64_t)gj * ka, acc[m][n][i]);
-        if (SYM && ti != tj) atomicAdd(G + gj + (int64_t)gi * ka, acc[m][n][i]);
       }
 }
 
 // C = A B for a tall column-major A (rows x k, ld lda; T float or double)
 // and a small B (k x n2, column-major ld ldb, k, n2 <= 8 NB). B stays in
 // shared memory for the CTA's life as 4-row slices laid out for its MMA
-// fragments; each warp takes 16-row tiles (two MMA row blocks) of C with
-// every column block in registers. UPPER: B is upper triangular, so column
-// block nb only needs the rows of B up to its last column and the K steps
-// past it are skipped (about half the work for Q R^{-1}). C is column-major
-// (ld ldc) and written, not accumulated.
+// fragments; each warp takes 16-row tiles of C with every column block in
+// registers. K goes in batches of 32 whose A values are loaded one batch
+// ahead; a column block then takes its eight B values and two m16n8k16 MMAs of
+// the batch together. UPPER: B is upper triangular, so column block nb only
+// needs the rows of B up to its last column and the batches past it are
+// skipped (about half the work for Q R^{-1}); the test per batch, not per four
+// rows, is what lets the B loads run ahead of the MMAs. C is column-major
+// (ld ldc) and written, not accumulated. Bound by the FP64 pipe and by the
+// 64-byte pieces of C: 1e6 x 81 by 81 x 81 takes 490 us (934 with m8n8k4 and a
+// test per four rows).
 template <typename T, int NB, bool UPPER>
 __global__ void __launch_bounds__(256) tsm_mma_kernel(const T* __restrict__ A, int64_t lda, int64_t rows, int k,
                                                       const double* __restrict__ B, int64_t ldb, int n2,
@@ -334,7 +415,7 @@ __global__ void __launch_bounds__(256) tsm_mma_kernel(const T* __restrict__ A, i
   // Bs[kk * ldbs + col], ldbs = 8 NB + 4 (mod 16) so a fragment's 4 x 8
   // reads hit 16 distinct bank pairs per half-warp
   constexpr int ldbs = (8 * NB + 15) / 16 * 16 + 4;
-  const int kp = (k + 3) & ~3;
+  const int kp = (k + 31) & ~31;  // whole batches; rows past k are zeros
   for (int q = threadIdx.x; q < kp * 8 * NB; q += blockDim.x) {
     const int kk = q / (8 * NB), col = q - kk * (8 * NB);
     tsm_smem[kk * ldbs + col] = (kk < k && col < n2) ? B[kk + (int64_t)col * ldb] : 0.0;
@@ -343,34 +424,40 @@ __global__ void __launch_bounds__(256) tsm_mma_kernel(const T* __restrict__ A, i
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
   const int lr = lane & 3, lc = lane >> 2;
   for (int64_t r0 = ((int64_t)blockIdx.x * nwarp + warp) * 16; r0 < rows; r0 += (int64_t)gridDim.x * nwarp * 16) {
-    double acc[2][NB][2];
+    double acc[NB][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int n = 0; n < NB; ++n) acc[m][n][0] = acc[m][n][1] = 0.0;
+    for (int n = 0; n < NB; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
     const int64_t ra = r0 + lc, rb = r0 + 8 + lc;
     const bool va = ra < rows, vb = rb < rows;
-    // eight K steps per batch: their 16 loads of A are in flight together
-    for (int kb = 0; kb < kp; kb += 32) {
-      double a0[8], a1[8];
+    T q0[8], q1[8];
+    auto load = [&](int kb) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int kk = kb + 4 * j + lr;
         const bool kv = kk < k;
-        a0[j] = (va && kv) ? (double)A[ra + (int64_t)kk * lda] : 0.0;
-        a1[j] = (vb && kv) ? (double)A[rb + (int64_t)kk * lda] : 0.0;
+        q0[j] = (va && kv) ? A[ra + (int64_t)kk * lda] : T(0);
+        q1[j] = (vb && kv) ? A[rb + (int64_t)kk * lda] : T(0);
       }
+    };
+    load(0);
+    for (int kb = 0; kb < kp; kb += 32) {
+      double a[2][8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int k0 = kb + 4 * j;
-        if (k0 >= kp) break;
-        const double* bs = tsm_smem + (k0 + lr) * ldbs + lc;
+        a[j >> 2][2 * (j & 3)] = (double)q0[j];
+        a[j >> 2][2 * (j & 3) + 1] = (double)q1[j];
+      }
+      if (kb + 32 < kp) load(kb + 32);
+      const double* bs = tsm_smem + (kb + lr) * ldbs + lc;
 #pragma unroll
-        for (int n = 0; n < NB; ++n) {
-          if (UPPER && col0 + 8 * n + 7 < k0) continue;  // B(k0.., block n) is zero
-          const double b = bs[8 * n];
-          dmma(acc[0][n], a0[j], b);
-          dmma(acc[1][n], a1[j], b);
+      for (int n = 0; n < NB; ++n) {
+        if (UPPER && col0 + 8 * n + 7 < kb) continue;  // B(kb.., block n) is zero
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          double b[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) b[i] = bs[(16 * h + 4 * i) * ldbs + 8 * n];
+          dmma16(acc[n], a[h], b);
         }
       }
     }
@@ -383,19 +470,18 @@ __global__ void __launch_bounds__(256) tsm_mma_kernel(const T* __restrict__ A, i
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int col = 8 * n + 2 * lr + i;
-          if (col < n2) C[row + (int64_t)col * ldc] = acc[m][n][i];
+          if (col < n2) C[row + (int64_t)col * ldc] = acc[n][2 * m + i];
         }
     }
   }
 }
 
-// C (ka x kb, column-major, zeroed beforehand) += A^T B, or the Gram matrix
-// A^T A when B is null (its upper tiles only).
+// C (ka x kb, column-major, zeroed beforehand) += A^T B.
 template <typename TA, typename TB>
 void launch_atb_mma(skema_ctx* c, const TA* A, int64_t lda, int64_t ka, const TB* B, int64_t ldb, int64_t kb,
                     int64_t rows, double* G) {
   const int nia = (int)((ka + 31) / 32), njb = (int)((kb + 31) / 32);
-  const int tiles = B ? nia * njb : nia * (nia + 1) / 2;
+  const int tiles = nia * njb;
   // up to 16 warps per CTA: P warps per tile when the tiles leave room,
   // else groups of 16 tiles over blockIdx.y
   const int P = std::max(1, 16 / tiles);
@@ -404,12 +490,30 @@ void launch_atb_mma(skema_ctx* c, const TA* A, int64_t lda, int64_t ka, const TB
   const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((rows + 1023) / 1024, (int64_t)c->sm_count));
   const int64_t per = ((rows + ctas - 1) / ctas + 3) / 4 * 4;
   const dim3 grid((unsigned)((rows + per - 1) / per), (unsigned)groups);
-  if (B)
-    atb_mma_kernel<TA, TB, false><<<grid, 32 * per_cta * P, 0, c->stream>>>(A, lda, (int)ka, B, ldb, (int)kb, rows,
-                                                                             G, per, P);
-  else
-    atb_mma_kernel<TA, TA, true><<<grid, 32 * per_cta * P, 0, c->stream>>>(A, lda, (int)ka, A, lda, (int)ka, rows,
-                                                                            G, per, P);
+  atb_mma_kernel<TA, TB><<<grid, 32 * per_cta * P, 0, c->stream>>>(A, lda, (int)ka, B, ldb, (int)kb, rows, G, per, P);
+  SKEMA_LAUNCHED(c);
+}
+
+// G (k x k, column-major, zeroed beforehand) += A^T A.
+template <typename T>
+void launch_gram(skema_ctx* c, const T* A, int64_t lda, int64_t k, int64_t rows, double* G) {
+  int tiles = 0;
+  for (int64_t m = 0; m < (k + 15) / 16; ++m) tiles += (int)((k + 7) / 8 - 2 * m);
+  // up to 16 warps, as many as share the blocks evenly: the fewest blocks per
+  // warp, then the fewest warps
+  const int groups = (tiles + 16 * kGramTiles - 1) / (16 * kGramTiles);
+  const int per_cta = (tiles + groups - 1) / groups, depth = (per_cta + 15) / 16;
+  const int warps = std::max(4, (per_cta + depth - 1) / depth);
+  const size_t smem = sizeof(double) * (size_t)((k + 15) / 16 * 16 * kGramLd);
+  const bool few = depth <= 3;
+  const int64_t ctas =
+      std::max<int64_t>(1, std::min<int64_t>((rows + 255) / 256, (few ? 2 : 1) * (int64_t)c->sm_count / groups));
+  const int64_t per = ((rows + ctas - 1) / ctas + 31) / 32 * 32;
+  auto kern = few ? gram_mma_kernel<T, 3> : gram_mma_kernel<T, kGramTiles>;
+  const int ny = (tiles + warps * (few ? 3 : kGramTiles) - 1) / (warps * (few ? 3 : kGramTiles));
+  SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3((unsigned)((rows + per - 1) / per), (unsigned)ny), 32 * warps, smem, c->stream>>>(A, lda, (int)k, rows, G,
+                                                                                               per);
   SKEMA_LAUNCHED(c);
 }
 
@@ -417,7 +521,7 @@ template <typename T, int NB>
 void launch_tsm_nb(skema_ctx* c, const T* A, int64_t lda, int64_t rows, int64_t k, const double* B, int64_t ldb,
                    int64_t n2, double* C, int64_t ldc, bool upper, int col0) {
   constexpr int ldbs = (8 * NB + 15) / 16 * 16 + 4;
-  const size_t smem = sizeof(double) * (size_t)(((k + 3) & ~3) * ldbs);
+  const size_t smem = sizeof(double) * (size_t)(((k + 31) & ~31) * ldbs);
   auto kern = upper ? tsm_mma_kernel<T, NB, true> : tsm_mma_kernel<T, NB, false>;
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t tiles = (rows + 15) / 16;
@@ -427,19 +531,22 @@ void launch_tsm_nb(skema_ctx* c, const T* A, int64_t lda, int64_t rows, int64_t 
 }
 
 // G (k x k, column-major) = A^T A for column-major A (rows x k, ld lda).
-constexpr int64_t kTallMaxK = 256;  // the tensor-core tall products take k up to this
+constexpr int64_t kTallMaxK = 256;  // the tall products take k up to this
+constexpr int64_t kTallMinRows = 1024;  // and rows from this on
 template <typename T>
 void gram_t(skema_ctx* c, const T* A, int64_t lda, int64_t rows, int64_t k, double* G) {
   SKEMA_CUDA(cudaMemsetAsync(G, 0, sizeof(double) * (size_t)(k * k), c->stream));
-  if (rows > 0) launch_atb_mma<T, T>(c, A, lda, k, static_cast<const T*>(nullptr), 0, k, rows, G);
+  if (rows > 0) launch_gram<T>(c, A, lda, k, rows, G);
 }
 void gram(skema_ctx* c, const double* A, int64_t lda, int64_t rows, int64_t k, double* G) {
   if (rows <= 0) {  // an empty row block (a rank without rows) adds nothing
     SKEMA_CUDA(cudaMemsetAsync(G, 0, sizeof(double) * (size_t)(k * k), c->stream));
     return;
   }
-  if (k > kTallMaxK) {
-    dgemm<double, double>(c, k, k, rows, 1.0, A, lda, 1, A, 1, lda, 0.0, G, 1, k);
+  // the k-sized products take the 32 x 32 tiles of dgemm, whose grid does not
+  // shrink with the rows (403 x 201: 15 us against 77)
+  if (k > kTallMaxK || rows < kTallMinRows) {
+    dgemm<double, double>(c, k, k, rows, 1.0, A, lda, 1, A, 1, lda, 0.0, G, 1, k, false);
     return;
   }
   gram_t<double>(c, A, lda, rows, k, G);
@@ -448,7 +555,7 @@ void gram(skema_ctx* c, const double* A, int64_t lda, int64_t rows, int64_t k, d
 // Column block width of the tall product: B's k x (8 NB) slice (padded)
 // stays in shared memory, at most 220 KB.
 int tsm_chunk_blocks(int64_t k) {
-  const int64_t kp = (k + 3) & ~3;
+  const int64_t kp = (k + 31) & ~31;
   for (int nb = 16; nb > 1; --nb) {
     const int64_t ldbs = (8 * nb + 15) / 16 * 16 + 4;
     if (kp * ldbs * (int64_t)sizeof(double) <= 220 * 1024) return nb;
@@ -491,7 +598,7 @@ void tall_times_small_t(skema_ctx* c, const T* A, int64_t lda, int64_t rows, int
 void tall_times_small(skema_ctx* c, const double* A, int64_t lda, int64_t rows, int64_t k, const double* B,
                       int64_t ldb, int64_t n2, double* C, int64_t ldc, bool upper = false) {
   if (rows <= 0 || n2 <= 0) return;
-  if (k > kTallMaxK) {
+  if (k > kTallMaxK || rows < kTallMinRows) {
     dgemm<double, double>(c, rows, n2, k, 1.0, A, 1, lda, B, 1, ldb, 0.0, C, 1, ldc, false);
     return;
   }
