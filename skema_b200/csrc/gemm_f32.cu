@@ -30,7 +30,8 @@ __global__ void __launch_bounds__(256, 1)
     sgemm_kernel(int64_t M, int64_t N, int64_t K, float alpha, const float* __restrict__ A,
                  int64_t a_rs, int64_t a_cs, const float* __restrict__ B, int64_t b_rs,
                  int64_t b_cs, float beta, float* __restrict__ C, int64_t c_rs, int64_t c_cs,
-                 int64_t kchunk, int64_t c_zs) {
+                 int64_t kchunk, int64_t c_zs, const uint32_t* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;
   __shared__ __align__(16) float As[2][BK][BM + PAD];
   __shared__ __align__(16) float Bs[2][BK][BN + PAD];
   const int tid = threadIdx.x;
@@ -144,13 +145,14 @@ void launch_sgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, float alpha, Ma
     dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((nn + BN - 1) / BN), (unsigned)gz);
     sgemm_kernel<AM, BN_, AT><<<grid, 256, 0, c->stream>>>(
         M, nn, K, alpha, A.p, A.rs, A.cs, B.p + nb * B.cs, B.rs, B.cs, beta, C.p + nb * C.cs, C.rs,
-        C.cs, kchunk, c_zs);
+        C.cs, kchunk, c_zs, c->run_if);
     SKEMA_LAUNCHED(c);
   }
 }
 
 __global__ void scale_kernel(float* __restrict__ C, int64_t rs, int64_t cs, int64_t M, int64_t N,
-                             float beta) {
+                             float beta, const uint32_t* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;
   const int64_t total = M * N;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
        q += (int64_t)gridDim.x * blockDim.x) {
@@ -227,7 +229,8 @@ __global__ void copy_kernel(const float* __restrict__ S, int64_t srs, int64_t sc
 // depend on scheduling. Consecutive threads follow C's unit stride.
 __global__ void splitk_reduce_kernel(const float* __restrict__ P, int64_t p_rs, int64_t p_cs, int64_t p_zs, int nz,
                                      int64_t M, int64_t N, float alpha, float beta, float* __restrict__ C,
-                                     int64_t c_rs, int64_t c_cs) {
+                                     int64_t c_rs, int64_t c_cs, const uint32_t* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;
   const int64_t total = M * N;
   const bool cm = c_rs == 1;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -298,13 +301,14 @@ void sgemm_split(skema_ctx* c, int64_t M, int64_t N, int64_t K, float alpha, Mat
   else if (bn) launch_sgemm<false, true, false>(c, M, N, K, 1.f, A, B, 0.f, P, (int)sk, pz);
   else launch_sgemm<false, false, false>(c, M, N, K, 1.f, A, B, 0.f, P, (int)sk, pz);
   splitk_reduce_kernel<<<grid1d(c, pz, 256), 256, 0, c->stream>>>(part, P.rs, P.cs, pz, nz, M, N, alpha, beta, C.p,
-                                                                   C.rs, C.cs);
+                                                                   C.rs, C.cs, c->run_if);
   SKEMA_LAUNCHED(c);
 }
 
 void scale_block(skema_ctx* c, MatOut C, int64_t M, int64_t N, float beta, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || beta == 1.f) return;
-  scale_kernel<<<grid1d(c, M * N, 256), 256, 0, stream ? stream : c->stream>>>(C.p, C.rs, C.cs, M, N, beta);
+  scale_kernel<<<grid1d(c, M * N, 256), 256, 0, stream ? stream : c->stream>>>(C.p, C.rs, C.cs, M, N, beta,
+                                                                                      c->run_if);
   SKEMA_LAUNCHED(c);
 }
 

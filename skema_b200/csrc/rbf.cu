@@ -38,7 +38,9 @@ template <int MODE>
 __global__ void __launch_bounds__(256)
     rbf_tile_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N, int64_t d,
                     float gamma, int64_t R0, int64_t wr, float* __restrict__ out, int64_t ldo,
-                    double* __restrict__ dgamma, float* __restrict__ rsum, float* __restrict__ csum) {
+                    double* __restrict__ dgamma, float* __restrict__ rsum, float* __restrict__ csum,
+                    const uint32_t* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;
   __shared__ float xi[TD][TT + 1];
   __shared__ float xj[TD][TT + 1];
   __shared__ float red[256];
@@ -135,68 +137,171 @@ __global__ void __launch_bounds__(256)
 // (x3.h): K is split where it is made, so it is written once (6 bytes) and
 // never as FP32. 64 rows x 128 points per CTA, 4 x 8 per thread: a thread's
 // four rows are adjacent, so 16 lanes write one 128-byte line of a plane, and
-// three 16-byte shared loads feed 32 differences. FCONTIG: a point's features
-// are contiguous (pcs = 1).
-template <bool FCONTIG>
+// three 16-byte shared loads feed 32 differences. Features go 16 at a time
+// through two buffers, the next ones loaded during the current ones' sums; the
+// last chunk stops at a multiple of four. FCONTIG: a point's features are
+// contiguous (pcs = 1). Bound by the two FP32 instructions per difference:
+// 40,000^2 kernel entries of d = 100 take RBN ms (8.8 at one instruction per
+// cycle and scheduler; RBO with one buffer and whole chunks).
+//
+// GRAD: the planes hold E = M o K for the block's M, given by columns (M(i, j)
+// at Mt[j * ldm + i]), E_ii = 0 (the diagonal's terms of the gradient cancel),
+// with the sums -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them;
+// *big is set when a value is out of the planes' range.
+struct RbfGrad {
+  const float* Mt;
+  int64_t ldm;
+  double* dgamma;
+  float* rsum;
+  float* csum;
+  uint32_t* big;
+};
+// s += (a + b)^2 on two packed FP32 values, each rounded as FADD and FFMA do.
+__device__ __forceinline__ void add_sq(unsigned long long& s, unsigned long long a, unsigned long long b) {
+  unsigned long long t;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(a), "l"(b));
+  asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(s) : "l"(t));
+}
+
+__device__ __forceinline__ unsigned long long twice(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+
+template <bool FCONTIG, bool GRAD>
 __global__ void __launch_bounds__(256, 2)
     rbf_planes_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N, int64_t d, float gamma,
-                      int64_t R0, int64_t wr, __nv_bfloat16* __restrict__ out, int64_t pstride) {
-  constexpr int TI = 64, TJ = 128, F = 16;
-  __shared__ __align__(16) float xi[F][TI + 4];
-  __shared__ __align__(16) float xj[F][TJ + 4];
+                      int64_t R0, int64_t wr, __nv_bfloat16* __restrict__ out, int64_t pstride, RbfGrad g) {
+  constexpr int TI = 64, TJ = 128, F = 16, NI = F * TI / 256, NJ = F * TJ / 256;
+  __shared__ __align__(16) float xi[2][F][TI + 4];
+  __shared__ __align__(16) float xj[2][F][TJ + 4];  // -x
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int64_t tiles_j = (N + TJ - 1) / TJ, tiles_i = (wr + TI - 1) / TI;
+  // what a thread stages: feature fi + q sfi of point ri + q sri (i side), and
+  // the same with j; the offsets of the q are constants
+  const int fi = FCONTIG ? tx : threadIdx.x >> 6, ri = FCONTIG ? ty : threadIdx.x & 63;
+  const int fj = FCONTIG ? tx : threadIdx.x >> 7, rj = FCONTIG ? ty : threadIdx.x & 127;
+  const int64_t qi = FCONTIG ? 16 * prs : 4 * pcs, qj = FCONTIG ? 16 * prs : 2 * pcs;
+  bool big = false;
+  double gsum = 0.0;
   for (int64_t tile = blockIdx.x; tile < tiles_i * tiles_j; tile += gridDim.x) {
     const int64_t ib = tile / tiles_j, i0 = ib * TI, j0 = (tile - ib * tiles_j) * TJ;
-    float acc[4][8];
+    const float* pi = P + (R0 + i0 + ri) * prs + fi * pcs;
+    const float* pj = P + (j0 + rj) * prs + fj * pcs;
+    const int ni = (int)min((int64_t)TI, wr - i0), nj = (int)min((int64_t)TJ, N - j0);
+    float li4[NI], lj8[NJ];
+    auto load = [&](int64_t f0) {
+      const int left = (int)min((int64_t)F, d - f0);
+      const float* a = pi + f0 * pcs;
+      const float* b = pj + f0 * pcs;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int q = 0; q < NI; ++q, a += qi)
+        li4[q] = (fi + (FCONTIG ? 0 : 4 * q) < left && ri + (FCONTIG ? 16 * q : 0) < ni) ? __ldg(a) : 0.f;
 #pragma unroll
-      for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
-    for (int64_t f0 = 0; f0 < d; f0 += F) {
+      for (int q = 0; q < NJ; ++q, b += qj)
+        lj8[q] = (fj + (FCONTIG ? 0 : 2 * q) < left && rj + (FCONTIG ? 16 * q : 0) < nj) ? __ldg(b) : 0.f;
+    };
+    auto store = [&](int b) {
 #pragma unroll
-      for (int q = 0; q < F * (TI + TJ) / 256; ++q) {
-        const int e = threadIdx.x + 256 * q;
-        const int ff = FCONTIG ? e % F : e / (TI + TJ), rr = FCONTIG ? e / F : e % (TI + TJ);
-        const int64_t f = f0 + ff;
-        if (rr < TI)
-          xi[ff][rr] = (f < d && i0 + rr < wr) ? P[(R0 + i0 + rr) * prs + f * pcs] : 0.f;
-        else
-          xj[ff][rr - TI] = (f < d && j0 + rr - TI < N) ? P[(j0 + rr - TI) * prs + f * pcs] : 0.f;
-      }
-      __syncthreads();
+      for (int q = 0; q < NI; ++q) xi[b][fi + (FCONTIG ? 0 : 4 * q)][ri + (FCONTIG ? 16 * q : 0)] = li4[q];
 #pragma unroll
-      for (int ff = 0; ff < F; ++ff) {
-        const float4 a4 = *reinterpret_cast<const float4*>(&xi[ff][4 * tx]);
-        const float4 b4 = *reinterpret_cast<const float4*>(&xj[ff][8 * ty]);
-        const float4 c4 = *reinterpret_cast<const float4*>(&xj[ff][8 * ty + 4]);
-        const float a[4] = {a4.x, a4.y, a4.z, a4.w};
-        const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
+      for (int q = 0; q < NJ; ++q)
+        xj[b][fj + (FCONTIG ? 0 : 2 * q)][rj + (FCONTIG ? 16 * q : 0)] = -lj8[q];
+    };
+    // sums of two adjacent rows per 64-bit register: packed FP32 has the rate
+    // of the scalar instructions at half their issue slots, which the loads
+    // and the exponentials need
+    unsigned long long acc2[2][8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) acc2[a][b] = 0ull;
+    load(0);
+    store(0);
+    __syncthreads();
+    int buf = 0;
+    for (int64_t f0 = 0; f0 < d; f0 += F, buf ^= 1) {
+      if (f0 + F < d) load(f0 + F);
+      const int nf = (int)min((int64_t)F, d - f0);
+      for (int f4 = 0; f4 < nf; f4 += 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(&xi[buf][f4 + q][4 * tx]);
+          const float4 b4 = *reinterpret_cast<const float4*>(&xj[buf][f4 + q][8 * ty]);
+          const float4 c4 = *reinterpret_cast<const float4*>(&xj[buf][f4 + q][8 * ty + 4]);
+          const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
           for (int v = 0; v < 8; ++v) {
-            const float df = a[u] - b[v];
-            acc[u][v] = fmaf(df, df, acc[u][v]);
+            const unsigned long long bb = twice(b[v]);
+            add_sq(acc2[0][v], a2.x, bb);
+            add_sq(acc2[1][v], a2.y, bb);
           }
+        }
       }
+      if (f0 + F < d) store(buf ^ 1);  // read last a chunk ago, before the barrier
       __syncthreads();
     }
+    float acc[4][8];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        acc[u][v] = __uint_as_float((uint32_t)(acc2[u >> 1][v] >> (32 * (u & 1))));
+    float rpart[4] = {0.f, 0.f, 0.f, 0.f}, gpart = 0.f;
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const int64_t gj = j0 + 8 * ty + v;
-      if (gj >= N) break;
+      const bool in = gj < N;
+      float cpart = 0.f;
       __nv_bfloat16 q[3][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int64_t li = i0 + 4 * tx + u;
-        const float kv = li >= wr ? 0.f : (gj == R0 + li) ? 1.f : expf(-gamma * acc[u][v]);
+        const bool diag = gj == R0 + li;
+        float kv = li >= wr ? 0.f : diag ? 1.f : expf(-gamma * acc[u][v]);
+        if (GRAD) {
+          kv = (in && li < wr && !diag) ? g.Mt[gj * g.ldm + li] * kv : 0.f;
+          const uint32_t bits = __float_as_uint(kv) & 0x7fffffffu;
+          big |= bits >= 0x71800000u && bits <= 0x7f800000u;
+          gpart = fmaf(kv, acc[u][v], gpart);
+          rpart[u] += kv;
+          cpart += kv;
+        }
         tc::split3(kv, q[0][u], q[1][u], q[2][u]);
       }
-      __nv_bfloat16* dp = out + (ib * N + gj) * 64 + 4 * tx;
+      if (in) {
+        __nv_bfloat16* dp = out + (ib * N + gj) * 64 + 4 * tx;
 #pragma unroll
-      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dp + p * pstride) = *reinterpret_cast<const uint2*>(q[p]);
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dp + p * pstride) = *reinterpret_cast<const uint2*>(q[p]);
+      }
+      if (GRAD) {  // the 16 lanes of a half-warp hold the column's 64 rows
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) cpart += __shfl_xor_sync(0xffffffffu, cpart, o);
+        if (tx == 0 && in) atomicAdd(g.csum + gj, cpart);
+      }
     }
+    if (GRAD) {
+      gsum += (double)gpart;
+      // row sums over the 16 groups of columns, in the first feature buffer
+      // (the last reads of it are behind the barrier above)
+      float* red = &xj[0][0][0];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) red[ty * TI + 4 * tx + u] = rpart[u];
+      __syncthreads();
+      if (threadIdx.x < TI && i0 + threadIdx.x < wr) {
+        float r = 0.f;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) r += red[q * TI + threadIdx.x];
+        atomicAdd(g.rsum + R0 + i0 + threadIdx.x, r);
+      }
+      __syncthreads();
+    }
+  }
+  if (GRAD) {
+    if (big) atomicOr(g.big, 1u);
+    for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(g.dgamma, -gsum);
   }
 }
 
@@ -224,10 +329,10 @@ void launch_tile(skema_ctx* c, int mode, Mat P, int64_t N, int64_t d, float gamm
   const int grid = grid_cap(c, tiles, 8);
   if (mode == 0)
     rbf_tile_kernel<0><<<grid, 256, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr, out, ldo,
-                                                    dg, rs, cs);
+                                                    dg, rs, cs, c->run_if);
   else
     rbf_tile_kernel<1><<<grid, 256, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr, out, ldo,
-                                                    dg, rs, cs);
+                                                    dg, rs, cs, c->run_if);
   SKEMA_LAUNCHED(c);
 }
 
@@ -260,9 +365,9 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
   if (c->p.precision == SKEMA_PREC_FP32 && c->p.dim_redux == SKEMA_MAP_GAUSS && gamma >= 0.f) {
     X3Input in{Mat{nullptr, 0, 0}, [&](int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride) {
                  const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
-                 auto kern = P.cs == 1 ? rbf_planes_kernel<true> : rbf_planes_kernel<false>;
+                 auto kern = P.cs == 1 ? rbf_planes_kernel<true, false> : rbf_planes_kernel<false, false>;
                  kern<<<grid_cap(c, tiles, 8), 256, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr, planes,
-                                                                    pstride);
+                                                                    pstride, RbfGrad{});
                  SKEMA_LAUNCHED(c);
                }};
     if (x3_update(c, in, row0, nrows)) return;
@@ -287,25 +392,166 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
 // (a window's rows times k or d, at most 16 splits).
 constexpr int64_t kRbfPartFloats = (int64_t)4 << 20;
 
+size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+// Y = K Omega~^T by kernel blocks of wb rows in Kw and SIMT products.
+static void rbf_fwd_plain(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega,
+                          int64_t k, float* Y, int64_t wb, float* Kw, float* part) {
+  for (int64_t r = 0; r < N; r += wb) {
+    const int64_t wr = std::min(wb, N - r);
+    launch_tile(c, 0, Mat{pts, d, 1}, N, d, gamma, r, wr, Kw, N, nullptr, nullptr, nullptr);
+    // Y(r:r+wr, :) = K_w Omega~^T ; B(kk=j, col=q) = omega[q*N + j]
+    sgemm_split(c, wr, k, N, 1.f, Mat{Kw, N, 1}, Mat{omega, 1, N}, 0.f, MatOut{Y + r * k, k, 1}, part,
+                kRbfPartFloats);
+  }
+}
+
+// The adjoint's sums (rs, cs, S, *dgamma, zeroed beforehand) by blocks of wb
+// rows of M and E in one buffer.
+static void rbf_vjp_plain(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega,
+                          int64_t k, const float* Ybar, double* dgamma, float* rs, float* cs, float* S, int64_t wb,
+                          float* E, float* part) {
+  const Mat P{pts, d, 1};
+  for (int64_t r = 0; r < N; r += wb) {
+    const int64_t wr = std::min(wb, N - r);
+    // M_w = Ybar_w Omega~   (wr x N)
+    sgemm(c, wr, N, k, 1.f, Mat{Ybar + r * k, k, 1}, Mat{omega, N, 1}, 0.f, MatOut{E, N, 1});
+    // E_w = M_w o K_w, with the gamma / row / column partial sums
+    launch_tile(c, 1, P, N, d, gamma, r, wr, E, N, dgamma, rs, cs);
+    // S(r:r+wr, :) += E_w X ;  S += E_w^T X_w
+    sgemm_split(c, wr, d, N, 1.f, Mat{E, N, 1}, Mat{pts, d, 1}, 1.f, MatOut{S + r * d, d, 1}, part, kRbfPartFloats);
+    sgemm(c, N, d, wr, 1.f, Mat{E, 1, N}, Mat{pts + r * d, d, 1}, 1.f, MatOut{S, d, 1});
+  }
+}
+
+// Below this many kernel entries times columns the conversions and launches of
+// the tensor-core form cost more than its products save.
+static bool rbf_pair_small(int64_t N, int64_t d, int64_t k) { return (double)N * N * (double)(k + d) < 2e8; }
+
+// Rows per block of the tensor-core forms, `bytes` per kernel entry: equal
+// blocks, a multiple of 64, within about 1 GB.
+static int64_t rbf_rows_x3(int64_t N, int64_t bytes) {
+  const int64_t cap = std::max<int64_t>(64, ((int64_t)1 << 30) / (bytes * N) / 64 * 64);
+  const int64_t nb = (N + cap - 1) / cap;
+  return ((N + nb - 1) / nb + 63) / 64 * 64;
+}
+
+struct RunIf {  // the SIMT kernels launched in this scope run when *flag != 0
+  skema_ctx* c;
+  RunIf(skema_ctx* ctx, const uint32_t* flag) : c(ctx) { c->run_if = flag; }
+  ~RunIf() { c->run_if = nullptr; }
+};
+
+static void launch_planes(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, int64_t r, int64_t wr,
+                          __nv_bfloat16* planes, int64_t pstride, const RbfGrad* g) {
+  const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
+  const int grid = grid_cap(c, tiles, 8);
+  if (g)
+    rbf_planes_kernel<true, true><<<grid, 256, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr, planes, pstride, *g);
+  else
+    rbf_planes_kernel<true, false><<<grid, 256, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr, planes, pstride,
+                                                                RbfGrad{});
+  SKEMA_LAUNCHED(c);
+}
+
+// The forward product on the tensor cores: kernel planes a block of rows at a
+// time, Y_w = K_w Omega~^T. Values that the planes cannot carry set the flag,
+// and the SIMT form behind it runs. False when the workspace is not to be had.
+static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega, int64_t k,
+                       float* Y) {
+  if (rbf_pair_small(N, 0, k)) return false;
+  const int64_t ldN = (N + 7) / 8 * 8, rb = rbf_rows_x3(N, 6);
+  const size_t b_o = up256(2 * (size_t)(3 * k * ldN)), b_k = up256(2 * (size_t)(3 * rb * N)),
+               b_p = up256(std::max(x3_part_bytes(c), sizeof(float) * (size_t)kRbfPartFloats));
+  char* ws = static_cast<char*>(try_workspace(c, b_o + b_k + b_p + 256));
+  if (!ws) return false;
+  __nv_bfloat16* Op = reinterpret_cast<__nv_bfloat16*>(ws);
+  __nv_bfloat16* Kp = reinterpret_cast<__nv_bfloat16*>(ws + b_o);
+  float* part = reinterpret_cast<float*>(ws + b_o + b_k);
+  uint32_t* flag = reinterpret_cast<uint32_t*>(ws + b_o + b_k + b_p);
+  SKEMA_CUDA(cudaMemsetAsync(flag, 0, sizeof(uint32_t), c->stream));
+  x3_row_planes(c, omega, N, k, N, Op, ldN, k * ldN, flag);
+  for (int64_t r = 0; r < N; r += rb) {
+    const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
+    launch_planes(c, pts, N, d, gamma, r, wr, Kp, nrb * 64 * N, nullptr);
+    x3_gemm(c, X3A{Kp, true, true, N, nrb, 0, 0}, X3B{Op, ldN, k * ldN}, wr, k, N,
+            tc::X3Out{Y + r * k, k, 1, 1.f, 0.f, nullptr, 0, 0, wr, k, k}, part, flag);
+  }
+  RunIf second(c, flag);
+  rbf_fwd_plain(c, pts, N, d, gamma, omega, k, Y, std::max<int64_t>(1, (int64_t)(b_k / 4) / N),
+                reinterpret_cast<float*>(Kp), part);
+  return true;
+}
+
+// The adjoint's sums on the tensor cores, a block of rows at a time: M_w by
+// columns (FP32), E_w = M_w o K_w as planes with the sums, then E_w X and
+// E_w^T X_w from the same planes. As for the forward, the SIMT form follows for
+// values that the planes cannot carry, over zeroed sums.
+static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega, int64_t k,
+                       const float* Ybar, float* dpts, double* dgamma) {
+  if (rbf_pair_small(N, d, k)) return false;
+  const int64_t ldN = (N + 7) / 8 * 8, ldk = (k + 7) / 8 * 8, rb = rbf_rows_x3(N, 10);
+  const size_t b_k = up256(2 * (size_t)(3 * N * ldk)), b_x = up256(2 * (size_t)(3 * d * ldN)),
+               b_e = up256(2 * (size_t)(3 * rb * N)), b_m = up256(4 * (size_t)(rb * N)),
+               b_p = up256(std::max(x3_part_bytes(c), sizeof(float) * (size_t)kRbfPartFloats)),
+               b_v = up256(4 * (size_t)N), b_s = up256(4 * (size_t)(N * d));
+  char* ws = static_cast<char*>(try_workspace(c, 2 * b_k + b_x + b_e + b_m + b_p + 2 * b_v + b_s + 256));
+  if (!ws) return false;
+  auto take = [&](size_t b) {
+    char* q = ws;
+    ws += b;
+    return q;
+  };
+  __nv_bfloat16* Yp = reinterpret_cast<__nv_bfloat16*>(take(b_k));
+  __nv_bfloat16* Op = reinterpret_cast<__nv_bfloat16*>(take(b_k));
+  __nv_bfloat16* Xp = reinterpret_cast<__nv_bfloat16*>(take(b_x));
+  __nv_bfloat16* Ep = reinterpret_cast<__nv_bfloat16*>(take(b_e));
+  float* Mt = reinterpret_cast<float*>(take(b_m));
+  float* part = reinterpret_cast<float*>(take(b_p));
+  float* rs = reinterpret_cast<float*>(take(b_v));
+  float* cs = reinterpret_cast<float*>(take(b_v));
+  float* S = reinterpret_cast<float*>(take(b_s));
+  uint32_t* flag = reinterpret_cast<uint32_t*>(take(256));
+  // the sums and the flag behind them
+  SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + 256, c->stream));
+  SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
+  x3_row_planes(c, Ybar, k, N, k, Yp, ldk, N * ldk, flag);
+  x3_transposed_planes(c, omega, N, k, N, Op, ldk, N * ldk, 1.f, 1, 1, 0, flag);
+  x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, flag);
+  for (int64_t r = 0; r < N; r += rb) {
+    const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64, ldm = nrb * 64;
+    x3_gemm(c, X3A{Yp + r * ldk, false, false, 0, 0, ldk, N * ldk}, X3B{Op, ldk, N * ldk}, wr, N, k,
+            tc::X3Out{Mt, 1, ldm, 1.f, 0.f, nullptr, 0, 0, wr, N, N}, part, flag);
+    const RbfGrad g{Mt, ldm, dgamma, rs, cs, flag};
+    launch_planes(c, pts, N, d, gamma, r, wr, Ep, nrb * 64 * N, &g);
+    x3_gemm(c, X3A{Ep, true, true, N, nrb, 0, 0}, X3B{Xp, ldN, d * ldN}, wr, d, N,
+            tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, flag);
+    x3_gemm(c, X3A{Ep, true, false, N, nrb, 0, 0}, X3B{Xp + r, ldN, d * ldN}, N, d, wr,
+            tc::X3Out{S, d, 1, 1.f, 1.f, nullptr, 0, 0, N, d, d}, part, flag);
+  }
+  {
+    RunIf second(c, flag);
+    scale_block(c, MatOut{rs, (int64_t)(2 * b_v + b_s) / 4, 1}, 1, (int64_t)(2 * b_v + b_s) / 4, 0.f);
+    scale_block(c, MatOut{reinterpret_cast<float*>(dgamma), 2, 1}, 1, 2, 0.f);
+    rbf_vjp_plain(c, pts, N, d, gamma, omega, k, Ybar, dgamma, rs, cs, S, std::max<int64_t>(1, (int64_t)(b_e / 4) / N),
+                  reinterpret_cast<float*>(Ep), part);
+  }
+  rbf_dx_kernel<<<grid_cap(c, (N * d + 255) / 256, 16), 256, 0, c->stream>>>(pts, d, 1, N, d, gamma, rs, cs, S, dpts);
+  SKEMA_LAUNCHED(c);
+  return true;
+}
+
 void rbf_fwd(skema_ctx* c, const float* pts, int64_t N, int64_t d, double gamma,
              const float* omega, int64_t k, float* Y) {
   if (rbf_pair_tc_supported(c, d, k, gamma)) {
     rbf_fwd_tc(c, pts, N, d, gamma, omega, k, Y);
     return;
   }
-  const Mat P{pts, d, 1};
+  if (rbf_fwd_x3(c, pts, N, d, (float)gamma, omega, k, Y)) return;
   const int64_t wb = rows_per_block(N, N);
-  const size_t kb = (sizeof(float) * (size_t)(wb * N) + 255) / 256 * 256;
+  const size_t kb = up256(sizeof(float) * (size_t)(wb * N));
   char* ws = (char*)workspace(c, kb + sizeof(float) * (size_t)kRbfPartFloats);
-  float* Kw = (float*)ws;
-  float* part = (float*)(ws + kb);  // K-split partial products
-  for (int64_t r = 0; r < N; r += wb) {
-    const int64_t wr = std::min(wb, N - r);
-    launch_tile(c, 0, P, N, d, (float)gamma, r, wr, Kw, N, nullptr, nullptr, nullptr);
-    // Y(r:r+wr, :) = K_w Omega~^T ; B(kk=j, col=q) = omega[q*N + j]
-    sgemm_split(c, wr, k, N, 1.f, Mat{Kw, N, 1}, Mat{omega, 1, N}, 0.f, MatOut{Y + r * k, k, 1}, part,
-                kRbfPartFloats);
-  }
+  rbf_fwd_plain(c, pts, N, d, (float)gamma, omega, k, Y, wb, (float*)ws, (float*)(ws + kb));
 }
 
 void rbf_vjp(skema_ctx* c, const float* pts, int64_t N, int64_t d, double gamma,
@@ -314,29 +560,18 @@ void rbf_vjp(skema_ctx* c, const float* pts, int64_t N, int64_t d, double gamma,
     rbf_vjp_tc(c, pts, N, d, gamma, omega, k, Ybar, dpts, dgamma);
     return;
   }
-  const Mat P{pts, d, 1};
+  if (rbf_vjp_x3(c, pts, N, d, (float)gamma, omega, k, Ybar, dpts, dgamma)) return;
   const int64_t wb = rows_per_block(N, N);
-  const size_t eb = (sizeof(float) * (size_t)(wb * N) + 255) / 256 * 256;
-  const size_t vb = (sizeof(float) * (size_t)N + 255) / 256 * 256;
-  const size_t sb = (sizeof(float) * (size_t)(N * d) + 255) / 256 * 256;
+  const size_t eb = up256(sizeof(float) * (size_t)(wb * N)), vb = up256(sizeof(float) * (size_t)N),
+               sb = up256(sizeof(float) * (size_t)(N * d));
   char* ws = (char*)workspace(c, eb + 2 * vb + sb + sizeof(float) * (size_t)kRbfPartFloats);
-  float* E = (float*)ws;
   float* rs = (float*)(ws + eb);
   float* cs = (float*)(ws + eb + vb);
   float* S = (float*)(ws + eb + 2 * vb);
   float* part = (float*)(ws + eb + 2 * vb + sb);  // K-split partial products
   SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * vb + sb, c->stream));
   SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
-  for (int64_t r = 0; r < N; r += wb) {
-    const int64_t wr = std::min(wb, N - r);
-    // M_w = Ybar_w Omega~   (wr x N)
-    sgemm(c, wr, N, k, 1.f, Mat{Ybar + r * k, k, 1}, Mat{omega, N, 1}, 0.f, MatOut{E, N, 1});
-    // E_w = M_w o K_w, with the gamma / row / column partial sums
-    launch_tile(c, 1, P, N, d, (float)gamma, r, wr, E, N, dgamma, rs, cs);
-    // S(r:r+wr, :) += E_w X ;  S += E_w^T X_w
-    sgemm_split(c, wr, d, N, 1.f, Mat{E, N, 1}, Mat{pts, d, 1}, 1.f, MatOut{S + r * d, d, 1}, part, kRbfPartFloats);
-    sgemm(c, N, d, wr, 1.f, Mat{E, 1, N}, Mat{pts + r * d, d, 1}, 1.f, MatOut{S, d, 1});
-  }
+  rbf_vjp_plain(c, pts, N, d, (float)gamma, omega, k, Ybar, dgamma, rs, cs, S, wb, (float*)ws, part);
   rbf_dx_kernel<<<grid_cap(c, (N * d + 255) / 256, 16), 256, 0, c->stream>>>(
       pts, d, 1, N, d, (float)gamma, rs, cs, S, dpts);
   SKEMA_LAUNCHED(c);

@@ -765,7 +765,7 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
     StageScope st(c, ST_PHI);
     const float* F = c->phi.f32 + (row0 + r) * s;
     const float zb = i == 0 ? wn : 1.f;
-    x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r);
+    x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r, nullptr);
     x3_gemm(c, X3A{Tp, false, false, 0, 0, ldt, ps}, X3B{Fp, ldt, ps}, s, s, wr,
             tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, flags + i);
     q.Y = nullptr, q.T32 = T32;

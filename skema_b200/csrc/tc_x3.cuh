@@ -54,18 +54,6 @@ struct X3Grid {
   int full;  // tiles [0, full) go whole; the rest is cut into gridDim.x runs
 };
 
-struct X3Out {
-  // columns [0, split): FP32, p0[row * rs0 + col * cs0] = beta p0 + alpha acc
-  float* p0;
-  int64_t rs0, cs0;
-  float alpha, beta;
-  // columns [split, ncols): the three planes of acc, plane q of column c at
-  // pl[q * pstride + (c - split) * ld + row]
-  __nv_bfloat16* pl;
-  int64_t ld, pstride;
-  int64_t rows, split, ncols;
-};
-
 // K-major operand descriptor, 64-byte swizzle: lines of 32 K-elements, 512
 // bytes per 8 lines.
 __device__ __forceinline__ uint64_t sdesc64(uint32_t saddr) {

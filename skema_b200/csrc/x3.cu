@@ -116,8 +116,9 @@ struct X3Src {
 };
 __global__ void __launch_bounds__(256)
     x3_maps_kernel(X3Src a, X3Src b, int64_t cols, __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu,
-                   int64_t W, int64_t nwin, int64_t j0) {
+                   int64_t W, int64_t nwin, int64_t j0, uint32_t* __restrict__ flag) {
   const int64_t c8 = ld / 8, total = (a.rows + b.rows) * c8;
+  bool big = false;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = q / c8, j = (q - r * c8) * 8;
     const float* sp = (r < a.rows ? a.p + r * a.rs : b.p + (r - a.rows) * b.rs) + j;
@@ -134,8 +135,13 @@ __global__ void __launch_bounds__(256)
         v[t] *= s;
       }
     }
+    if (flag) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t) big |= too_big(v[t]);
+    }
     store_planes8(v, D + r * ld + j, pstride);
   }
+  if (big) atomicOr(flag, 1u);
 }
 
 // The products of X3Plain3 for the rare block that too_big() refuses (returns
@@ -188,8 +194,9 @@ __global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_
 __global__ void __launch_bounds__(256)
     x3_transposed_kernel(const float* __restrict__ S, int64_t rs, int64_t rows, int64_t cols,
                          __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin,
-                         int64_t j0) {
+                         int64_t j0, uint32_t* __restrict__ flag) {
   __shared__ float tile[32][65];
+  bool big = false;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t ti = (ld + 63) / 64, tj = (cols + 31) / 32;
   for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
@@ -199,6 +206,7 @@ __global__ void __launch_bounds__(256)
       const int r = ty + 8 * q;
       float v = (i0 + r < rows && c0 + tx < cols) ? S[(i0 + r) * rs + c0 + tx] : 0.f;
       if (nu != 1.f && i0 + r < rows) v *= (float)pow((double)nu, (double)(nwin - 1 - (j0 + i0 + r) / W));
+      big |= too_big(v);
       tile[tx][r] = v;
     }
     __syncthreads();
@@ -211,6 +219,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
+  if (flag && big) atomicOr(flag, 1u);
 }
 
 int grid_1d(const skema_ctx* c, int64_t items, int per_sm) {
@@ -244,9 +253,10 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   const size_t stage = tc::kX3ABytes + (size_t)3 * g.nt * tc::kX3BK * 2;
   g.stages = (int)std::min<size_t>(tc::kX3MaxStages, (kX3Smem - 2048) / stage);
   const int64_t tiles = (int64_t)g.mtiles * g.ntiles;
-  // a run of at least four K steps per CTA (so that none is empty)
+  // runs of at least four K steps (so that none is empty)
   const int G = (int)std::max<int64_t>(1, std::min<int64_t>(c->sm_count, tiles * g.ksteps / 4));
   g.full = (int)(tiles / G * G);
+  if ((tiles - g.full) * g.ksteps < 4 * (int64_t)G) g.full = (int)tiles;  // too little to cut
   CUtensorMap ta;
   if (a.blocked)
     ta = tmap_3d(CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.p, 64, (uint64_t)a.cols, (uint64_t)(3 * a.nrb), 128,
@@ -280,10 +290,17 @@ void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfl
 }
 
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
-                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0) {
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag) {
   const int64_t tiles = ((ld + 63) / 64) * ((cols + 31) / 32);
   x3_transposed_kernel<<<grid_1d(c, tiles * 256, 16), 256, 0, c->stream>>>(S, rs, rows, cols, D, ld, pstride, nu, W,
-                                                                          nwin, j0);
+                                                                          nwin, j0, flag);
+  SKEMA_LAUNCHED(c);
+}
+
+void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t ld,
+                   int64_t pstride, uint32_t* flag) {
+  x3_maps_kernel<<<grid_1d(c, rows * ld / 8, 16), 256, 0, c->stream>>>(X3Src{S, rs, rows}, X3Src{S, rs, 0}, cols, D, ld,
+                                                                      pstride, 1.f, 1, 1, 0, flag);
   SKEMA_LAUNCHED(c);
 }
 
@@ -341,7 +358,7 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
     StageScope st(c, ST_WINDOW);
     const X3Src so{c->omg.f32, c->omg.rs, k}, sp{c->psi.f32, c->psi.rs, s};
     x3_maps_kernel<<<grid_1d(c, (k + s) * ldn / 8, 16), 256, 0, c->stream>>>(so, sp, n, op, ldn, (k + s) * ldn, 1.f, 1,
-                                                                            1, 0);
+                                                                            1, 0, nullptr);
     SKEMA_LAUNCHED(c);
   }
   for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
@@ -358,7 +375,7 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
       if (s > 0) {
         const X3Src su{c->ups.f32 + R0, c->ups.rs, k}, sf{c->phi.f32 + R0, c->phi.rs, s};  // cs = 1
         x3_maps_kernel<<<grid_1d(c, (k + s) * ldw / 8, 16), 256, 0, c->stream>>>(su, sf, wr, uf, ldw, (k + s) * ldw, nu,
-                                                                                W, nwin, r);
+                                                                                W, nwin, r, nullptr);
         SKEMA_LAUNCHED(c);
       }
     }

@@ -10,7 +10,18 @@
 namespace skema {
 
 namespace tc {
-struct X3Out;
+// Where an x3_gemm product goes.
+struct X3Out {
+  // columns [0, split): FP32, p0[row * rs0 + col * cs0] = beta p0 + alpha acc
+  float* p0;
+  int64_t rs0, cs0;
+  float alpha, beta;
+  // columns [split, ncols): the three planes of acc, plane q of column c at
+  // pl[q * pstride + (c - split) * ld + row]
+  __nv_bfloat16* pl;
+  int64_t ld, pstride;
+  int64_t rows, split, ncols;
+};
 
 // x as the sum of three BF16 values
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
@@ -48,9 +59,14 @@ void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfl
 
 // K-major planes of a row-major source's transpose: row i of S (rows x cols,
 // rs apart), scaled by nu^(nwin - 1 - (j0 + i) / W), is K index i; D holds
-// cols rows of ld (a multiple of 8) per plane.
+// cols rows of ld (a multiple of 8) per plane. *flag (may be null) is set when
+// a value is out of the planes' range.
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
-                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0);
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag);
+// K-major planes of a row-major source (rows x cols, rs apart): D holds rows of
+// ld (a multiple of 8) per plane.
+void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t ld,
+                   int64_t pstride, uint32_t* flag);
 
 // Up to three FP32 products C = alpha A B + beta C by plain FMA, run when
 // *flag is set: the form of a block whose values the planes cannot carry.

@@ -146,3 +146,65 @@ def test_values_outside_the_planes_range(sk, value):
         for part in (fine & ~hit, fine & hit):
             if part.any() and (not big or part is not None and not (part & hit).any()):
                 assert rel_fro(g[part], w[part]) < 1e-5, q
+
+
+def _pair64(P, gamma, Om, Yb):
+    """Y = K Omega^T and the adjoint in FP64 by explicit differences."""
+    P, Om, Yb = (np.asarray(t, np.float64) for t in (P, Om, Yb))
+    d2 = np.maximum(((P[:, None, :] - P[None]) ** 2).sum(-1), 0.0)
+    K = np.exp(-gamma * d2)
+    np.fill_diagonal(K, 1.0)
+    E = (Yb @ Om) * K
+    np.fill_diagonal(E, 0.0)
+    S = E + E.T
+    return K @ Om.T, -2.0 * gamma * (S.sum(1)[:, None] * P - S @ P), -(E * d2).sum(), (np.abs(E) * d2).sum()
+
+
+@pytest.mark.parametrize("N,d,k", [(1999, 3, 20), (1024, 24, 65), (1500, 70, 190), (1337, 129, 257)])
+def test_pair(sk, oracle, N, d, k):
+    """Forward and adjoint of the kernel sketch; dgamma is held against the sum
+    of its terms' magnitudes, which it is a small difference of. Bar: 4e-6, the
+    sketch's plus the FP32 distances and exponentials (a few 2^-24 of gamma d^2,
+    of order one)."""
+    import torch
+
+    P = oracle.mixture_points(N, d, seed=N)
+    gamma = oracle.median_gamma(P)
+    rng = np.random.default_rng(N)
+    Om, Yb = rng.normal(size=(k, N)).astype(np.float32), rng.normal(size=(N, k)).astype(np.float32)
+    Yw, Xw, gw, gabs = _pair64(P, gamma, Om, Yb)
+    t = [torch.from_numpy(a).cuda() for a in (P, Om, Yb)]
+    Y = sk.rbf_sketch_fwd(t[0], gamma, t[1])
+    dX, dg = sk.rbf_sketch_vjp(t[0], gamma, t[1], t[2])
+    assert rel_fro(Y.cpu().numpy(), Yw) < 4e-6
+    assert rel_fro(dX.cpu().numpy(), Xw) < 4e-6
+    assert abs(dg - gw) < 4e-6 * gabs
+
+
+@pytest.mark.parametrize("where,value", [("Om", np.inf), ("Yb", 2.0**105), ("Yb", np.nan), ("P", np.inf)])
+def test_pair_values_outside_the_planes_range(sk, oracle, where, value):
+    """What the SIMT form gives: the same calls under a workspace limit that
+    leaves no room for the planes."""
+    import torch
+
+    from skema_b200.sketchy import _ctx_for_standalone
+
+    N, d, k = 1600, 9, 70
+    P = oracle.mixture_points(N, d, seed=2)
+    gamma = oracle.median_gamma(P)
+    rng = np.random.default_rng(5)
+    a = {"P": P, "Om": rng.normal(size=(k, N)).astype(np.float32), "Yb": rng.normal(size=(N, k)).astype(np.float32)}
+    a[where][3, 2] = value
+    t = {q: torch.from_numpy(v).cuda() for q, v in a.items()}
+    out = []
+    for limit in (0, 32 << 20):
+        with _ctx_for_standalone(0) as c:
+            assert c.lib.skema_set_workspace_limit(c.h, limit) == 0
+            Y = sk.rbf_sketch_fwd(t["P"], gamma, t["Om"], ctx=c).cpu().numpy()
+            dX, dg = sk.rbf_sketch_vjp(t["P"], gamma, t["Om"], t["Yb"], ctx=c)
+            out.append((Y, dX.cpu().numpy(), np.array([dg])))
+    for g, w in zip(*out):
+        assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(np.isinf(g), np.isinf(w))
+        f = np.isfinite(w)
+        if f.any():
+            assert rel_fro(g[f], w[f]) < 1e-5
