@@ -141,113 +141,135 @@ __global__ void __launch_bounds__(256)
 // through two buffers, the next ones loaded during the current ones' sums; the
 // last chunk stops at a multiple of four. FCONTIG: a point's features are
 // contiguous (pcs = 1). Bound by the two FP32 instructions per difference:
-// 40,000^2 kernel entries of d = 100 take RBN ms (8.8 at one instruction per
-// cycle and scheduler; RBO with one buffer and whole chunks).
+// 40,000^2 kernel entries of d = 100 take 13.3 ms (8.8 at the FP32 rate; 17.5
+// with scalar instructions, one buffer and whole chunks, 14.9 with the packed
+// pairs of J kept in shared memory, whose reads then bound it).
 //
-// GRAD: the planes hold E = M o K for the block's M, given by columns (M(i, j)
-// at Mt[j * ldm + i]), E_ii = 0 (the diagonal's terms of the gradient cancel),
-// with the sums -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them;
-// *big is set when a value is out of the planes' range.
+// GRAD: the planes hold E = M o K with M = Ybar Omega~ formed beside the
+// distances (k more FP32 instructions per entry; as a product of its own it
+// cost an FP32 block written and read back: forward and adjoint at N = 20,000,
+// d = 24, k = 65 took 8.0 ms, now 6.4, this kernel 3.3 of them), E_ii = 0 (the diagonal's terms of the gradient cancel), and the sums
+// -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them; *big is set
+// when a value is out of the planes' range.
 struct RbfGrad {
-  const float* Mt;
-  int64_t ldm;
+  const float* Ybar;   // N x k row-major
+  const float* omega;  // k x N row-major
+  int64_t k;
   double* dgamma;
   float* rsum;
   float* csum;
   uint32_t* big;
 };
-// s += (a + b)^2 on two packed FP32 values, each rounded as FADD and FFMA do.
+// s += (a + b)^2, and s += a b, on two packed FP32 values, each rounded as FADD
+// and FFMA do.
 __device__ __forceinline__ void add_sq(unsigned long long& s, unsigned long long a, unsigned long long b) {
   unsigned long long t;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(a), "l"(b));
   asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(s) : "l"(t));
 }
-
+__device__ __forceinline__ void add_mul(unsigned long long& s, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s) : "l"(a), "l"(b));
+}
 __device__ __forceinline__ unsigned long long twice(float x) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
 }
 
+constexpr int kTI = 64, kTJ = 128, kTF = 16;
+struct RbfTile {
+  float xi[2][kTF][kTI + 4];
+  float xj[2][kTF][kTJ + 4];
+};
+// Over f < d: acc += (I(f, i) - J(f, j))^2 (DIST) or I(f, i) J(f, j) for this
+// thread's 4 x 8 entries, packed by two rows. I(f, i) = Ip[i * irs + f * ics] for
+// i < ni, else 0; J alike. FI, FJ: the f run is the contiguous one. What a thread
+// stages: feature f + q (step) of point r + q (step), the offsets of the q
+// constants. All threads are past the tile's last use when it returns.
+template <bool FI, bool FJ, bool DIST>
+__device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[2][8], const float* __restrict__ Ip,
+                                         int64_t irs, int64_t ics, int ni, const float* __restrict__ Jp, int64_t jrs,
+                                         int64_t jcs, int nj, int64_t d) {
+  constexpr int NI = kTF * kTI / 256, NJ = kTF * kTJ / 256;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int fi = FI ? tx : threadIdx.x >> 6, ri = FI ? ty : threadIdx.x & 63;
+  const int fj = FJ ? tx : threadIdx.x >> 7, rj = FJ ? ty : threadIdx.x & 127;
+  const int64_t qi = FI ? 16 * irs : 4 * ics, qj = FJ ? 16 * jrs : 2 * jcs;
+  const float* pi = Ip + ri * irs + fi * ics;
+  const float* pj = Jp + rj * jrs + fj * jcs;
+  float vi[NI], vj[NJ];
+  auto load = [&](int64_t f0) {
+    const int left = (int)min((int64_t)kTF, d - f0);
+    const float* a = pi + f0 * ics;
+    const float* b = pj + f0 * jcs;
+#pragma unroll
+    for (int q = 0; q < NI; ++q, a += qi)
+      vi[q] = (fi + (FI ? 0 : 4 * q) < left && ri + (FI ? 16 * q : 0) < ni) ? __ldg(a) : 0.f;
+#pragma unroll
+    for (int q = 0; q < NJ; ++q, b += qj)
+      vj[q] = (fj + (FJ ? 0 : 2 * q) < left && rj + (FJ ? 16 * q : 0) < nj) ? __ldg(b) : 0.f;
+  };
+  auto store = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < NI; ++q) t.xi[b][fi + (FI ? 0 : 4 * q)][ri + (FI ? 16 * q : 0)] = vi[q];
+#pragma unroll
+    for (int q = 0; q < NJ; ++q) t.xj[b][fj + (FJ ? 0 : 2 * q)][rj + (FJ ? 16 * q : 0)] = DIST ? -vj[q] : vj[q];
+  };
+  load(0);
+  store(0);
+  __syncthreads();
+  int buf = 0;
+  for (int64_t f0 = 0; f0 < d; f0 += kTF, buf ^= 1) {
+    if (f0 + kTF < d) load(f0 + kTF);
+    const int nf = (int)min((int64_t)kTF, d - f0);
+    for (int f4 = 0; f4 < nf; f4 += 4) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(&t.xi[buf][f4 + q][4 * tx]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&t.xj[buf][f4 + q][8 * ty]);
+        const float4 c4 = *reinterpret_cast<const float4*>(&t.xj[buf][f4 + q][8 * ty + 4]);
+        const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const unsigned long long bb = twice(b[v]);
+          if (DIST) {
+            add_sq(acc[0][v], a2.x, bb);
+            add_sq(acc[1][v], a2.y, bb);
+          } else {
+            add_mul(acc[0][v], a2.x, bb);
+            add_mul(acc[1][v], a2.y, bb);
+          }
+        }
+      }
+    }
+    if (f0 + kTF < d) store(buf ^ 1);  // read last a chunk ago, before the barrier
+    __syncthreads();
+  }
+}
+
 template <bool FCONTIG, bool GRAD>
 __global__ void __launch_bounds__(256, 2)
     rbf_planes_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N, int64_t d, float gamma,
                       int64_t R0, int64_t wr, __nv_bfloat16* __restrict__ out, int64_t pstride, RbfGrad g) {
-  constexpr int TI = 64, TJ = 128, F = 16, NI = F * TI / 256, NJ = F * TJ / 256;
-  __shared__ __align__(16) float xi[2][F][TI + 4];
-  __shared__ __align__(16) float xj[2][F][TJ + 4];  // -x
+  __shared__ __align__(16) RbfTile t;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t tiles_j = (N + TJ - 1) / TJ, tiles_i = (wr + TI - 1) / TI;
-  // what a thread stages: feature fi + q sfi of point ri + q sri (i side), and
-  // the same with j; the offsets of the q are constants
-  const int fi = FCONTIG ? tx : threadIdx.x >> 6, ri = FCONTIG ? ty : threadIdx.x & 63;
-  const int fj = FCONTIG ? tx : threadIdx.x >> 7, rj = FCONTIG ? ty : threadIdx.x & 127;
-  const int64_t qi = FCONTIG ? 16 * prs : 4 * pcs, qj = FCONTIG ? 16 * prs : 2 * pcs;
+  const int64_t tiles_j = (N + kTJ - 1) / kTJ, tiles_i = (wr + kTI - 1) / kTI;
   bool big = false;
   double gsum = 0.0;
   for (int64_t tile = blockIdx.x; tile < tiles_i * tiles_j; tile += gridDim.x) {
-    const int64_t ib = tile / tiles_j, i0 = ib * TI, j0 = (tile - ib * tiles_j) * TJ;
-    const float* pi = P + (R0 + i0 + ri) * prs + fi * pcs;
-    const float* pj = P + (j0 + rj) * prs + fj * pcs;
-    const int ni = (int)min((int64_t)TI, wr - i0), nj = (int)min((int64_t)TJ, N - j0);
-    float li4[NI], lj8[NJ];
-    auto load = [&](int64_t f0) {
-      const int left = (int)min((int64_t)F, d - f0);
-      const float* a = pi + f0 * pcs;
-      const float* b = pj + f0 * pcs;
-#pragma unroll
-      for (int q = 0; q < NI; ++q, a += qi)
-        li4[q] = (fi + (FCONTIG ? 0 : 4 * q) < left && ri + (FCONTIG ? 16 * q : 0) < ni) ? __ldg(a) : 0.f;
-#pragma unroll
-      for (int q = 0; q < NJ; ++q, b += qj)
-        lj8[q] = (fj + (FCONTIG ? 0 : 2 * q) < left && rj + (FCONTIG ? 16 * q : 0) < nj) ? __ldg(b) : 0.f;
-    };
-    auto store = [&](int b) {
-#pragma unroll
-      for (int q = 0; q < NI; ++q) xi[b][fi + (FCONTIG ? 0 : 4 * q)][ri + (FCONTIG ? 16 * q : 0)] = li4[q];
-#pragma unroll
-      for (int q = 0; q < NJ; ++q)
-        xj[b][fj + (FCONTIG ? 0 : 2 * q)][rj + (FCONTIG ? 16 * q : 0)] = -lj8[q];
-    };
-    // sums of two adjacent rows per 64-bit register: packed FP32 has the rate
-    // of the scalar instructions at half their issue slots, which the loads
-    // and the exponentials need
-    unsigned long long acc2[2][8];
+    const int64_t ib = tile / tiles_j, i0 = ib * kTI, j0 = (tile - ib * tiles_j) * kTJ;
+    const int ni = (int)min((int64_t)kTI, wr - i0), nj = (int)min((int64_t)kTJ, N - j0);
+    // two adjacent rows per 64-bit register: packed FP32 has the rate of the
+    // scalar instructions at half their issue slots, which the loads and the
+    // exponentials need
+    unsigned long long acc[2][8], mac[2][8];
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 8; ++b) acc2[a][b] = 0ull;
-    load(0);
-    store(0);
-    __syncthreads();
-    int buf = 0;
-    for (int64_t f0 = 0; f0 < d; f0 += F, buf ^= 1) {
-      if (f0 + F < d) load(f0 + F);
-      const int nf = (int)min((int64_t)F, d - f0);
-      for (int f4 = 0; f4 < nf; f4 += 4) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(&xi[buf][f4 + q][4 * tx]);
-          const float4 b4 = *reinterpret_cast<const float4*>(&xj[buf][f4 + q][8 * ty]);
-          const float4 c4 = *reinterpret_cast<const float4*>(&xj[buf][f4 + q][8 * ty + 4]);
-          const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            const unsigned long long bb = twice(b[v]);
-            add_sq(acc2[0][v], a2.x, bb);
-            add_sq(acc2[1][v], a2.y, bb);
-          }
-        }
-      }
-      if (f0 + F < d) store(buf ^ 1);  // read last a chunk ago, before the barrier
-      __syncthreads();
-    }
-    float acc[4][8];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 8; ++v)
-        acc[u][v] = __uint_as_float((uint32_t)(acc2[u >> 1][v] >> (32 * (u & 1))));
+      for (int b = 0; b < 8; ++b) acc[a][b] = mac[a][b] = 0ull;
+    rbf_pass<FCONTIG, FCONTIG, true>(t, acc, P + (R0 + i0) * prs, prs, pcs, ni, P + j0 * prs, prs, pcs, nj, d);
+    if (GRAD)
+      rbf_pass<true, false, false>(t, mac, g.Ybar + (R0 + i0) * g.k, g.k, 1, ni, g.omega + j0, 1, N, nj, g.k);
     float rpart[4] = {0.f, 0.f, 0.f, 0.f}, gpart = 0.f;
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
@@ -259,12 +281,14 @@ __global__ void __launch_bounds__(256, 2)
       for (int u = 0; u < 4; ++u) {
         const int64_t li = i0 + 4 * tx + u;
         const bool diag = gj == R0 + li;
-        float kv = li >= wr ? 0.f : diag ? 1.f : expf(-gamma * acc[u][v]);
+        const float d2 = __uint_as_float((uint32_t)(acc[u >> 1][v] >> (32 * (u & 1))));
+        float kv = li >= wr ? 0.f : diag ? 1.f : expf(-gamma * d2);
         if (GRAD) {
-          kv = (in && li < wr && !diag) ? g.Mt[gj * g.ldm + li] * kv : 0.f;
+          const float m = __uint_as_float((uint32_t)(mac[u >> 1][v] >> (32 * (u & 1))));
+          kv = (in && li < wr && !diag) ? m * kv : 0.f;
           const uint32_t bits = __float_as_uint(kv) & 0x7fffffffu;
           big |= bits >= 0x71800000u && bits <= 0x7f800000u;
-          gpart = fmaf(kv, acc[u][v], gpart);
+          gpart = fmaf(kv, d2, gpart);
           rpart[u] += kv;
           cpart += kv;
         }
@@ -283,16 +307,15 @@ __global__ void __launch_bounds__(256, 2)
     }
     if (GRAD) {
       gsum += (double)gpart;
-      // row sums over the 16 groups of columns, in the first feature buffer
-      // (the last reads of it are behind the barrier above)
-      float* red = &xj[0][0][0];
+      // row sums over the 16 groups of columns
+      float* red = &t.xj[0][0][0];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) red[ty * TI + 4 * tx + u] = rpart[u];
+      for (int u = 0; u < 4; ++u) red[ty * kTI + 4 * tx + u] = rpart[u];
       __syncthreads();
-      if (threadIdx.x < TI && i0 + threadIdx.x < wr) {
+      if (threadIdx.x < kTI && i0 + threadIdx.x < wr) {
         float r = 0.f;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) r += red[q * TI + threadIdx.x];
+        for (int q = 0; q < 16; ++q) r += red[q * kTI + threadIdx.x];
         atomicAdd(g.rsum + R0 + i0 + threadIdx.x, r);
       }
       __syncthreads();
@@ -483,30 +506,25 @@ static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   return true;
 }
 
-// The adjoint's sums on the tensor cores, a block of rows at a time: M_w by
-// columns (FP32), E_w = M_w o K_w as planes with the sums, then E_w X and
-// E_w^T X_w from the same planes. As for the forward, the SIMT form follows for
+// The adjoint's sums on the tensor cores, a block of rows at a time: E_w = M_w o
+// K_w as planes with the sums, then E_w X and E_w^T X_w from the same planes. As for the forward, the SIMT form follows for
 // values that the planes cannot carry, over zeroed sums.
 static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega, int64_t k,
                        const float* Ybar, float* dpts, double* dgamma) {
   if (rbf_pair_small(N, d, k)) return false;
-  const int64_t ldN = (N + 7) / 8 * 8, ldk = (k + 7) / 8 * 8, rb = rbf_rows_x3(N, 10);
-  const size_t b_k = up256(2 * (size_t)(3 * N * ldk)), b_x = up256(2 * (size_t)(3 * d * ldN)),
-               b_e = up256(2 * (size_t)(3 * rb * N)), b_m = up256(4 * (size_t)(rb * N)),
+  const int64_t ldN = (N + 7) / 8 * 8, rb = rbf_rows_x3(N, 6);
+  const size_t b_x = up256(2 * (size_t)(3 * d * ldN)), b_e = up256(2 * (size_t)(3 * rb * N)),
                b_p = up256(std::max(x3_part_bytes(c), sizeof(float) * (size_t)kRbfPartFloats)),
                b_v = up256(4 * (size_t)N), b_s = up256(4 * (size_t)(N * d));
-  char* ws = static_cast<char*>(try_workspace(c, 2 * b_k + b_x + b_e + b_m + b_p + 2 * b_v + b_s + 256));
+  char* ws = static_cast<char*>(try_workspace(c, b_x + b_e + b_p + 2 * b_v + b_s + 256));
   if (!ws) return false;
   auto take = [&](size_t b) {
     char* q = ws;
     ws += b;
     return q;
   };
-  __nv_bfloat16* Yp = reinterpret_cast<__nv_bfloat16*>(take(b_k));
-  __nv_bfloat16* Op = reinterpret_cast<__nv_bfloat16*>(take(b_k));
   __nv_bfloat16* Xp = reinterpret_cast<__nv_bfloat16*>(take(b_x));
   __nv_bfloat16* Ep = reinterpret_cast<__nv_bfloat16*>(take(b_e));
-  float* Mt = reinterpret_cast<float*>(take(b_m));
   float* part = reinterpret_cast<float*>(take(b_p));
   float* rs = reinterpret_cast<float*>(take(b_v));
   float* cs = reinterpret_cast<float*>(take(b_v));
@@ -515,14 +533,10 @@ static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   // the sums and the flag behind them
   SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + 256, c->stream));
   SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
-  x3_row_planes(c, Ybar, k, N, k, Yp, ldk, N * ldk, flag);
-  x3_transposed_planes(c, omega, N, k, N, Op, ldk, N * ldk, 1.f, 1, 1, 0, flag);
   x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, flag);
   for (int64_t r = 0; r < N; r += rb) {
-    const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64, ldm = nrb * 64;
-    x3_gemm(c, X3A{Yp + r * ldk, false, false, 0, 0, ldk, N * ldk}, X3B{Op, ldk, N * ldk}, wr, N, k,
-            tc::X3Out{Mt, 1, ldm, 1.f, 0.f, nullptr, 0, 0, wr, N, N}, part, flag);
-    const RbfGrad g{Mt, ldm, dgamma, rs, cs, flag};
+    const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
+    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, flag};
     launch_planes(c, pts, N, d, gamma, r, wr, Ep, nrb * 64 * N, &g);
     x3_gemm(c, X3A{Ep, true, true, N, nrb, 0, 0}, X3B{Xp, ldN, d * ldN}, wr, d, N,
             tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, flag);
