@@ -148,7 +148,13 @@ __device__ __forceinline__ void ssign_apply8(uint32_t base, uint4 wv, float a) {
 
 // (A form with one red.shared.add per map entry instead of the load and
 // store measured 30 % slower: 0.170 against 0.131 ms on the 1e6 x 1e5 case.)
-template <int U>
+//
+// S = 4: a row is cut into four equal runs of nonzeros in four adjacent lanes,
+// whose bins are added at the write-out, (0 + 1) + (2 + 3). For calls of few
+// rows, whose time is the walk along the longest row: 2,000 rows of 0 to 200
+// entries take 16 us against 35, 10 against 12 with 10 entries in each. (A warp
+// per row with the bins in its lanes took 42 to 62.)
+template <int U, int S>
 __global__ void __launch_bounds__(128)
     csr_ssign_y16_kernel(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                          const float* __restrict__ val, int64_t col_offset, int64_t nrows,
@@ -162,14 +168,20 @@ __global__ void __launch_bounds__(128)
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int q = lane; q < k * 8; q += 32) bins4[q] = z4;
   __syncwarp();
-  const int64_t ntiles = (nrows + 31) / 32;
+  constexpr int R = 32 / S;  // rows per tile
+  const int64_t ntiles = (nrows + R - 1) / R;
   const int64_t tstride = (int64_t)gridDim.x * nw;
   const bool vec = (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && ldy % 4 == 0;
   int64_t tile = (int64_t)blockIdx.x * nw + warp;
   auto row_range = [&](int64_t t, int64_t& b, int64_t& e) {
-    const int64_t i = t * 32 + lane;
+    const int64_t i = t * R + lane / S;
     b = 0, e = 0;
     if (t < ntiles && i < nrows) b = __ldg(rowptr + i) - col_offset, e = __ldg(rowptr + i + 1) - col_offset;
+    if (S > 1) {
+      const int64_t len = (e - b + S - 1) / S;
+      b = min(e, b + (lane % S) * len);
+      e = min(e, b + len);
+    }
   };
   auto load_batch = [&](int64_t q0, int64_t q1, int32_t* jj, float* aa) {
 #pragma unroll
@@ -204,8 +216,21 @@ __global__ void __launch_bounds__(128)
       if (!more) break;
     }
     __syncwarp();
-    const int64_t r0 = tile * 32;
-    if (vec && r0 + 32 <= nrows) {
+    const int64_t r0 = tile * R;
+    if (S == 4) {
+      // row lane % 8, bins lane / 8, + 4, ..: four lanes' bins lie side by side
+      const int64_t i = r0 + (lane & 7);
+      for (int r = lane >> 3; r < k; r += 4) {
+        float4* bp = bins4 + r * 8 + (lane & 7);
+        const float4 q = *bp;
+        *bp = z4;
+        if (i < nrows) {
+          float* yp = Y + i + r * ldy;
+          const float v = (q.x + q.y) + (q.z + q.w);
+          *yp = beta == 0.f ? v : fmaf(beta, *yp, v);
+        }
+      }
+    } else if (vec && r0 + 32 <= nrows) {
       const int sub = lane >> 3, q4 = lane & 7;
       float* yp = Y + r0 + 4 * q4 + (int64_t)sub * ldy;
       for (int r = sub; r < k; r += 4, yp += 4 * ldy) {
@@ -241,7 +266,9 @@ __global__ void __launch_bounds__(128)
 }
 
 // X and Z contributions of the Upsilon / Phi entries whose input row lies
-// in the call's rows. One warp per entry.
+// in the call's rows. One warp per entry. (Z: the zeta_s = 8 entries of a
+// nonzero's Psi row lie along the lanes; with a 64-bit division per pair the
+// longest rows took 17 us.)
 __global__ void csr_ssign_entries_kernel(
     const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
     const float* __restrict__ val, int64_t col_offset, int64_t row0, int64_t W, int64_t nwin,
@@ -267,14 +294,25 @@ __global__ void csr_ssign_entries_kernel(
       for (int64_t q = b + lane; q < en; q += 32)
         if ((uint64_t)col[q] < (uint64_t)n) atomicAdd(X + r * n + col[q], wgt * val[q]);
     } else {
-      const int64_t pairs = (en - b) * zeta_s;
-      for (int64_t q = lane; q < pairs; q += 32) {
-        const int64_t p = b + q / zeta_s;
-        const int t = (int)(q % zeta_s);
-        if ((uint64_t)col[p] >= (uint64_t)n) continue;
-        const uint32_t w = psi[(int64_t)col[p] * zeta_s + t];
-        const float v = wgt * val[p];
-        atomicAdd(Z + r * s + (w & 0x7fffffffu), (w >> 31) ? -v : v);
+      // zeta_s <= 8: 32 / 8 nonzeros at a time, lane t of eight the entry t
+      const int t = lane & 7;
+      for (int64_t p = b + (lane >> 3); p < en; p += 16) {
+        int32_t j[4];
+        float v[4];
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const bool in = p + 4 * q < en && t < zeta_s;
+          j[q] = in ? col[p + 4 * q] : -1;
+          v[q] = in ? wgt * val[p + 4 * q] : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if ((uint64_t)(int64_t)j[q] < (uint64_t)n) w[q] = psi[(int64_t)j[q] * zeta_s + t];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if ((uint64_t)(int64_t)j[q] < (uint64_t)n)
+            atomicAdd(Z + r * s + (w[q] & 0x7fffffffu), (w[q] >> 31) ? -v[q] : v[q]);
       }
     }
   }
@@ -647,7 +685,7 @@ void launch_csr_ssign_y_variant(skema_ctx* c, int warps_per_block, const int64_t
   SKEMA_LAUNCHED(c);
 }
 
-template <int U>
+template <int U, int S>
 static void launch_csr_ssign_y16(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const float* val,
                                  int64_t col_offset, int64_t nrows, const Map& O, float* Y, int64_t ldy, float alpha,
                                  float beta) {
@@ -666,7 +704,7 @@ static void launch_csr_ssign_y16(skema_ctx* c, const int64_t* rowptr, const int3
     }
   }
   const size_t smem = sizeof(float) * 32 * (size_t)k * wpb;
-  auto kern = csr_ssign_y16_kernel<U>;
+  auto kern = csr_ssign_y16_kernel<U, S>;
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // the bin budget per SM; the carve-out leaves the rest of the unified
   // L1 / shared memory to L1
@@ -675,7 +713,7 @@ static void launch_csr_ssign_y16(skema_ctx* c, const int64_t* rowptr, const int3
   const int per_sm = (int)std::max<size_t>(1, budget / smem);
   const int carve = (int)std::min<size_t>(100, (per_sm * (smem + 1024) * 100 + smem_sm - 1) / std::max(1, smem_sm) + 2);
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-  const int64_t tiles = (nrows + 31) / 32;
+  const int64_t tiles = (nrows + 32 / S - 1) / (32 / S);
   const int grid = grid_cap(c, (tiles + wpb - 1) / wpb, per_sm);
   kern<<<grid, 32 * wpb, smem, c->stream>>>(rowptr, col, val, col_offset, nrows,
                                             static_cast<const uint4*>(O.packed16), k, (int)c->n, Y, ldy, alpha,
@@ -686,12 +724,18 @@ static void launch_csr_ssign_y16(skema_ctx* c, const int64_t* rowptr, const int3
 static void launch_csr_ssign_y(skema_ctx* c, const int64_t* rowptr, const int32_t* col,
                                const float* val, int64_t col_offset, int64_t nrows, const Map& O,
                                float* Y, int64_t ldy, float alpha, float beta) {
+  // four lanes per row while the eight-row tiles of the call all fit on the chip
+  // at once (1024 / k warps of bins per SM within 128 KB)
+  if (O.packed16 && nrows <= 8 * c->sm_count * std::max<int64_t>(1, 1024 / c->k)) {
+    launch_csr_ssign_y16<4, 4>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta);
+    return;
+  }
   if (O.packed16) {  // zeta = 8, k <= 256: at most 32 KB of bins per warp
     switch (c->ssign_batch) {
-      case 2: launch_csr_ssign_y16<2>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      case 6: launch_csr_ssign_y16<6>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      case 8: launch_csr_ssign_y16<8>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      default: launch_csr_ssign_y16<4>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
+      case 2: launch_csr_ssign_y16<2, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
+      case 6: launch_csr_ssign_y16<6, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
+      case 8: launch_csr_ssign_y16<8, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
+      default: launch_csr_ssign_y16<4, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
     }
     return;
   }
