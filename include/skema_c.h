@@ -444,6 +444,14 @@ int skema_set_workspace_limit(skema_ctx* ctx, int64_t bytes);
  * stream. */
 int skema_get_stream(const skema_ctx* ctx, void** stream);
 
+/* Orders ctx's stream and another stream of the context's device against each
+ * other on the device, without a host synchronisation: before != 0 makes what
+ * ctx launches next wait for the work queued on `other` so far (inputs that
+ * another library is still writing, output buffers it is still reading), 0
+ * makes `other` wait for the work ctx has queued so far. Nothing happens when
+ * the two are the same stream. No reference counterpart. */
+int skema_order_streams(skema_ctx* ctx, void* other, int32_t before);
+
 /* Number of this library's kernels launched on ctx so far (for accounting). */
 int64_t skema_launch_count(const skema_ctx* ctx);
 

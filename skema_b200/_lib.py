@@ -127,6 +127,7 @@ SIGNATURES = {
     "skema_rbf_sketch_fwd_noalloc": (C.c_int, [_P, _P, _I64, _I64, _D, _P, _I64, _P]),
     "skema_synchronize": (C.c_int, [_P]),
     "skema_set_stream": (C.c_int, [_P, _P]),
+    "skema_order_streams": (C.c_int, [_P, _P, _I32]),
     "skema_get_stream": (C.c_int, [_P, C.POINTER(_P)]),
     "skema_set_wait_limit": (C.c_int, [_P, _I64]),
     "skema_set_workspace_limit": (C.c_int, [_P, _I64]),

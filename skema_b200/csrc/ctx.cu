@@ -264,6 +264,7 @@ static void free_all(skema_ctx* c) {
   if (c->side) cudaStreamDestroy(c->side);
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
+  if (c->order_ev) cudaEventDestroy(c->order_ev);
   for (cudaEvent_t& e : c->pipe_ev) {
     if (e) cudaEventDestroy(e);
     e = nullptr;
@@ -273,7 +274,7 @@ static void free_all(skema_ctx* c) {
     e = nullptr;
   }
   c->side = nullptr;
-  c->fork_ev = c->join_ev = nullptr;
+  c->fork_ev = c->join_ev = c->order_ev = nullptr;
 }
 
 // Runs f, converting library errors into a status and remembering the message.
@@ -423,6 +424,7 @@ int skema_create(const skema_params* p, skema_ctx** out) {
     SKEMA_CUDA(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     SKEMA_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
     SKEMA_CUDA(cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming));
+    SKEMA_CUDA(cudaEventCreateWithFlags(&c->order_ev, cudaEventDisableTiming));
     for (cudaEvent_t& e : c->pipe_ev) SKEMA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (cudaEvent_t& e : c->stage_ev) SKEMA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     c->pipe_xt_sms = 0;
@@ -1021,6 +1023,28 @@ int skema_set_workspace_limit(skema_ctx* c, int64_t bytes) {
     if (bytes < 0) fail(SKEMA_EINVAL, "workspace limit must be >= 0");
     c->ws_limit = (size_t)bytes;
   });
+}
+
+int skema_order_streams(skema_ctx* c, void* other, int32_t before) {
+  if (!c) return SKEMA_EINVAL;
+  // not guarded(): a pending reset stays pending, so that a CSR update can
+  // still zero X and Z beside its Y kernel
+  const cudaStream_t o = static_cast<cudaStream_t>(other);
+  if (o == c->stream) return SKEMA_OK;
+  try {
+    SKEMA_CUDA(cudaSetDevice(c->dev));
+    // the wait takes the event's state as of the call, so one event serves
+    // every call
+    SKEMA_CUDA(cudaEventRecord(c->order_ev, before ? o : c->stream));
+    SKEMA_CUDA(cudaStreamWaitEvent(before ? c->stream : o, c->order_ev, 0));
+    return SKEMA_OK;
+  } catch (const Error& e) {
+    c->err = e.msg;
+    return e.status;
+  } catch (...) {
+    c->err = "unexpected C++ exception";
+    return SKEMA_ECUDA;
+  }
 }
 
 int64_t skema_launch_count(const skema_ctx* c) { return c ? c->launches : -1; }

@@ -106,6 +106,7 @@ struct skema_ctx {
   // call (forked from and joined back to `stream` before the call returns).
   cudaStream_t side = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+  cudaEvent_t order_ev = nullptr;  // skema_order_streams
   // Hand-offs between the two streams of the BF16 dense pipeline (window
   // copies ready / released, one pair per copy buffer).
   cudaEvent_t pipe_ev[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -595,6 +595,10 @@ class _Context:
     # stream the context creates for itself dies with it, so before the
     # first call on torch tensors the context is moved onto a stream from
     # torch's pool, which lives as long as the process.
+    #
+    # The waits go through skema_order_streams: torch's wait_stream builds an
+    # event and a stream object on every call, which was two thirds of the time
+    # of a small update (seven waits).
     def _lib_stream(self, device):
         import torch
 
@@ -609,34 +613,29 @@ class _Context:
         self._check(self.lib.skema_get_stream(self.h, C.byref(h)))
         return torch.cuda.ExternalStream(h.value or 0, device=device)
 
-    def _cuda_tensors(self, tensors):
-        return [t for t in tensors if _is_torch(t) and t.is_cuda]
+    def _order(self, tensors, before):
+        """Order the library's stream against torch's current one around a
+        call on the CUDA tensors among `tensors`, and record them on it."""
+        lib_s = cur = None
+        for t in tensors:
+            if not (_is_torch(t) and t.is_cuda):
+                continue
+            if lib_s is None:
+                import torch
+
+                device = t.device
+                lib_s = self._lib_stream(device)
+                cur = torch._C._cuda_getCurrentRawStream(device.index)
+                if lib_s.cuda_stream == cur:
+                    return
+                self._check(self.lib.skema_order_streams(self.h, cur, before))
+            t.record_stream(lib_s)
 
     def _torch_inputs_ready(self, *tensors):
-        import torch
-
-        ts = self._cuda_tensors(tensors)
-        if not ts:
-            return
-        lib_s, cur = self._lib_stream(ts[0].device), torch.cuda.current_stream(ts[0].device)
-        if lib_s.cuda_stream == cur.cuda_stream:
-            return
-        lib_s.wait_stream(cur)
-        for t in ts:
-            t.record_stream(lib_s)
+        self._order(tensors, 1)
 
     def _torch_outputs_ready(self, *tensors):
-        import torch
-
-        ts = self._cuda_tensors(tensors)
-        if not ts:
-            return
-        lib_s, cur = self._lib_stream(ts[0].device), torch.cuda.current_stream(ts[0].device)
-        if lib_s.cuda_stream == cur.cuda_stream:
-            return
-        cur.wait_stream(lib_s)
-        for t in ts:
-            t.record_stream(lib_s)
+        self._order(tensors, 0)
 
     # -- sketches ---------------------------------------------------------
     def _sketch_shape(self, which):
