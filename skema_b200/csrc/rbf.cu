@@ -135,20 +135,21 @@ __global__ void __launch_bounds__(256)
 
 // Kernel rows as the row-blocked BF16 planes of the tensor-core FP32 form
 // (x3.h): K is split where it is made, so it is written once (6 bytes) and
-// never as FP32. 64 rows x 128 points per CTA, 4 x 8 per thread: a thread's
-// four rows are adjacent, so 16 lanes write one 128-byte line of a plane, and
-// three 16-byte shared loads feed 32 differences. Features go 16 at a time
+// never as FP32. 64 rows x 128 points per CTA of 128 threads, 8 x 8 per thread
+// (rows 4 t .. 4 t + 3 and 32 more on: eight lanes write 64 bytes of a plane's
+// line), so four 16-byte shared loads feed 64 differences. Features go 16 at a time
 // through two buffers, the next ones loaded during the current ones' sums; the
 // last chunk stops at a multiple of four. FCONTIG: a point's features are
 // contiguous (pcs = 1). Bound by the two FP32 instructions per difference:
-// 40,000^2 kernel entries of d = 100 take 13.3 ms (8.8 at the FP32 rate; 17.5
+// 40,000^2 kernel entries of d = 100 take 12.7 ms (8.8 at the FP32 rate; 17.5
 // with scalar instructions, one buffer and whole chunks, 14.9 with the packed
-// pairs of J kept in shared memory, whose reads then bound it).
+// pairs of J kept in shared memory, whose reads then bound it, 13.3 with 4 x 8
+// entries per thread).
 //
 // GRAD: the planes hold E = M o K with M = Ybar Omega~ formed beside the
 // distances (k more FP32 instructions per entry; as a product of its own it
 // cost an FP32 block written and read back: forward and adjoint at N = 20,000,
-// d = 24, k = 65 took 8.0 ms, now 6.4, this kernel 3.3 of them), E_ii = 0 (the diagonal's terms of the gradient cancel), and the sums
+// d = 24, k = 65 took 8.0 ms, now 6.1, this kernel 3.1 of them), E_ii = 0 (the diagonal's terms of the gradient cancel), and the sums
 // -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them; *big is set
 // when a value is out of the planes' range.
 struct RbfGrad {
@@ -176,25 +177,25 @@ __device__ __forceinline__ unsigned long long twice(float x) {
   return r;
 }
 
-constexpr int kTI = 64, kTJ = 128, kTF = 16;
+constexpr int kTI = 64, kTJ = 128, kTF = 16, kPlThreads = 128;
 struct RbfTile {
   float xi[2][kTF][kTI + 4];
   float xj[2][kTF][kTJ + 4];
 };
 // Over f < d: acc += (I(f, i) - J(f, j))^2 (DIST) or I(f, i) J(f, j) for this
-// thread's 4 x 8 entries, packed by two rows. I(f, i) = Ip[i * irs + f * ics] for
+// thread's 8 x 8 entries, packed by two rows. I(f, i) = Ip[i * irs + f * ics] for
 // i < ni, else 0; J alike. FI, FJ: the f run is the contiguous one. What a thread
 // stages: feature f + q (step) of point r + q (step), the offsets of the q
 // constants. All threads are past the tile's last use when it returns.
 template <bool FI, bool FJ, bool DIST>
-__device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[2][8], const float* __restrict__ Ip,
+__device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[4][8], const float* __restrict__ Ip,
                                          int64_t irs, int64_t ics, int ni, const float* __restrict__ Jp, int64_t jrs,
                                          int64_t jcs, int nj, int64_t d) {
-  constexpr int NI = kTF * kTI / 256, NJ = kTF * kTJ / 256;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int fi = FI ? tx : threadIdx.x >> 6, ri = FI ? ty : threadIdx.x & 63;
-  const int fj = FJ ? tx : threadIdx.x >> 7, rj = FJ ? ty : threadIdx.x & 127;
-  const int64_t qi = FI ? 16 * irs : 4 * ics, qj = FJ ? 16 * jrs : 2 * jcs;
+  constexpr int NI = kTF * kTI / kPlThreads, NJ = kTF * kTJ / kPlThreads;
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+  const int fi = FI ? tid & 15 : tid >> 6, ri = FI ? tid >> 4 : tid & 63;
+  const int fj = FJ ? tid & 15 : 0, rj = FJ ? tid >> 4 : tid;
+  const int64_t qi = FI ? 8 * irs : 2 * ics, qj = FJ ? 8 * jrs : jcs;
   const float* pi = Ip + ri * irs + fi * ics;
   const float* pj = Jp + rj * jrs + fj * jcs;
   float vi[NI], vj[NJ];
@@ -204,16 +205,16 @@ __device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[2
     const float* b = pj + f0 * jcs;
 #pragma unroll
     for (int q = 0; q < NI; ++q, a += qi)
-      vi[q] = (fi + (FI ? 0 : 4 * q) < left && ri + (FI ? 16 * q : 0) < ni) ? __ldg(a) : 0.f;
+      vi[q] = (fi + (FI ? 0 : 2 * q) < left && ri + (FI ? 8 * q : 0) < ni) ? __ldg(a) : 0.f;
 #pragma unroll
     for (int q = 0; q < NJ; ++q, b += qj)
-      vj[q] = (fj + (FJ ? 0 : 2 * q) < left && rj + (FJ ? 16 * q : 0) < nj) ? __ldg(b) : 0.f;
+      vj[q] = (fj + (FJ ? 0 : q) < left && rj + (FJ ? 8 * q : 0) < nj) ? __ldg(b) : 0.f;
   };
   auto store = [&](int b) {
 #pragma unroll
-    for (int q = 0; q < NI; ++q) t.xi[b][fi + (FI ? 0 : 4 * q)][ri + (FI ? 16 * q : 0)] = vi[q];
+    for (int q = 0; q < NI; ++q) t.xi[b][fi + (FI ? 0 : 2 * q)][ri + (FI ? 8 * q : 0)] = vi[q];
 #pragma unroll
-    for (int q = 0; q < NJ; ++q) t.xj[b][fj + (FJ ? 0 : 2 * q)][rj + (FJ ? 16 * q : 0)] = DIST ? -vj[q] : vj[q];
+    for (int q = 0; q < NJ; ++q) t.xj[b][fj + (FJ ? 0 : q)][rj + (FJ ? 8 * q : 0)] = DIST ? -vj[q] : vj[q];
   };
   load(0);
   store(0);
@@ -226,18 +227,20 @@ __device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[2
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(&t.xi[buf][f4 + q][4 * tx]);
+        const ulonglong2 h2 = *reinterpret_cast<const ulonglong2*>(&t.xi[buf][f4 + q][32 + 4 * tx]);
         const float4 b4 = *reinterpret_cast<const float4*>(&t.xj[buf][f4 + q][8 * ty]);
         const float4 c4 = *reinterpret_cast<const float4*>(&t.xj[buf][f4 + q][8 * ty + 4]);
+        const unsigned long long a[4] = {a2.x, a2.y, h2.x, h2.y};
         const float b[8] = {b4.x, b4.y, b4.z, b4.w, c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
           const unsigned long long bb = twice(b[v]);
-          if (DIST) {
-            add_sq(acc[0][v], a2.x, bb);
-            add_sq(acc[1][v], a2.y, bb);
-          } else {
-            add_mul(acc[0][v], a2.x, bb);
-            add_mul(acc[1][v], a2.y, bb);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (DIST)
+              add_sq(acc[u][v], a[u], bb);
+            else
+              add_mul(acc[u][v], a[u], bb);
           }
         }
       }
@@ -246,13 +249,16 @@ __device__ __forceinline__ void rbf_pass(RbfTile& t, unsigned long long (&acc)[2
     __syncthreads();
   }
 }
+__device__ __forceinline__ float half_of(unsigned long long x, int h) {
+  return __uint_as_float((uint32_t)(x >> (32 * h)));
+}
 
 template <bool FCONTIG, bool GRAD>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
     rbf_planes_kernel(const float* __restrict__ P, int64_t prs, int64_t pcs, int64_t N, int64_t d, float gamma,
                       int64_t R0, int64_t wr, __nv_bfloat16* __restrict__ out, int64_t pstride, RbfGrad g) {
   __shared__ __align__(16) RbfTile t;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   const int64_t tiles_j = (N + kTJ - 1) / kTJ, tiles_i = (wr + kTI - 1) / kTI;
   bool big = false;
   double gsum = 0.0;
@@ -262,47 +268,60 @@ __global__ void __launch_bounds__(256, 2)
     // two adjacent rows per 64-bit register: packed FP32 has the rate of the
     // scalar instructions at half their issue slots, which the loads and the
     // exponentials need
-    unsigned long long acc[2][8], mac[2][8];
+    unsigned long long acc[4][8], mac[GRAD ? 4 : 1][8];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 8; ++b) acc[a][b] = mac[a][b] = 0ull;
+      for (int b = 0; b < 8; ++b) {
+        acc[a][b] = 0ull;
+        if (GRAD) mac[GRAD ? a : 0][b] = 0ull;
+      }
     rbf_pass<FCONTIG, FCONTIG, true>(t, acc, P + (R0 + i0) * prs, prs, pcs, ni, P + j0 * prs, prs, pcs, nj, d);
-    if (GRAD)
+    if constexpr (GRAD)
       rbf_pass<true, false, false>(t, mac, g.Ybar + (R0 + i0) * g.k, g.k, 1, ni, g.omega + j0, 1, N, nj, g.k);
-    float rpart[4] = {0.f, 0.f, 0.f, 0.f}, gpart = 0.f;
+    float rpart[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, gpart = 0.f;
+    const int64_t dg = R0 + i0 - j0;  // the diagonal: j = i + dg within the tile
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
-      const int64_t gj = j0 + 8 * ty + v;
-      const bool in = gj < N;
+      const int lj = 8 * ty + v;
+      const bool in = lj < nj;
       float cpart = 0.f;
-      __nv_bfloat16 q[3][4];
+      __nv_bfloat162 q[3][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int64_t li = i0 + 4 * tx + u;
-        const bool diag = gj == R0 + li;
-        const float d2 = __uint_as_float((uint32_t)(acc[u >> 1][v] >> (32 * (u & 1))));
-        float kv = li >= wr ? 0.f : diag ? 1.f : expf(-gamma * d2);
-        if (GRAD) {
-          const float m = __uint_as_float((uint32_t)(mac[u >> 1][v] >> (32 * (u & 1))));
-          kv = (in && li < wr && !diag) ? m * kv : 0.f;
-          const uint32_t bits = __float_as_uint(kv) & 0x7fffffffu;
-          big |= bits >= 0x71800000u && bits <= 0x7f800000u;
-          gpart = fmaf(kv, d2, gpart);
-          rpart[u] += kv;
-          cpart += kv;
+        float kk[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int li = 4 * tx + 32 * (u >> 1) + 2 * (u & 1) + h;
+          const bool diag = (int64_t)lj == li + dg;
+          const float d2 = half_of(acc[u][v], h);
+          float kv = expf(-gamma * d2);
+          if (GRAD) {
+            kv = (in && li < ni && !diag) ? half_of(mac[GRAD ? u : 0][v], h) * kv : 0.f;
+            const uint32_t bits = __float_as_uint(kv) & 0x7fffffffu;
+            big |= bits >= 0x71800000u && bits <= 0x7f800000u;
+            gpart = fmaf(kv, d2, gpart);
+            rpart[2 * u + h] += kv;
+            cpart += kv;
+          } else {
+            kv = li >= ni ? 0.f : diag ? 1.f : kv;
+          }
+          kk[h] = kv;
         }
-        tc::split3(kv, q[0][u], q[1][u], q[2][u]);
+        tc::split3x2(kk[0], kk[1], q[0][u], q[1][u], q[2][u]);
       }
       if (in) {
-        __nv_bfloat16* dp = out + (ib * N + gj) * 64 + 4 * tx;
+        __nv_bfloat16* dp = out + (ib * N + j0 + lj) * 64 + 4 * tx;
 #pragma unroll
-        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dp + p * pstride) = *reinterpret_cast<const uint2*>(q[p]);
+        for (int p = 0; p < 3; ++p) {
+          *reinterpret_cast<uint2*>(dp + p * pstride) = *reinterpret_cast<const uint2*>(&q[p][0]);
+          *reinterpret_cast<uint2*>(dp + p * pstride + 32) = *reinterpret_cast<const uint2*>(&q[p][2]);
+        }
       }
-      if (GRAD) {  // the 16 lanes of a half-warp hold the column's 64 rows
+      if (GRAD) {  // eight lanes hold the column's 64 rows
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) cpart += __shfl_xor_sync(0xffffffffu, cpart, o);
-        if (tx == 0 && in) atomicAdd(g.csum + gj, cpart);
+        for (int o = 4; o > 0; o >>= 1) cpart += __shfl_xor_sync(0xffffffffu, cpart, o);
+        if (tx == 0 && in) atomicAdd(g.csum + j0 + lj, cpart);
       }
     }
     if (GRAD) {
@@ -310,9 +329,9 @@ __global__ void __launch_bounds__(256, 2)
       // row sums over the 16 groups of columns
       float* red = &t.xj[0][0][0];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) red[ty * kTI + 4 * tx + u] = rpart[u];
+      for (int e = 0; e < 8; ++e) red[ty * kTI + 4 * tx + 32 * (e >> 2) + (e & 3)] = rpart[e];
       __syncthreads();
-      if (threadIdx.x < kTI && i0 + threadIdx.x < wr) {
+      if (threadIdx.x < kTI && (int)threadIdx.x < ni) {
         float r = 0.f;
 #pragma unroll
         for (int q = 0; q < 16; ++q) r += red[q * kTI + threadIdx.x];
@@ -389,8 +408,8 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
     X3Input in{Mat{nullptr, 0, 0}, [&](int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride) {
                  const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
                  auto kern = P.cs == 1 ? rbf_planes_kernel<true, false> : rbf_planes_kernel<false, false>;
-                 kern<<<grid_cap(c, tiles, 8), 256, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr, planes,
-                                                                    pstride, RbfGrad{});
+                 kern<<<grid_cap(c, tiles, 3), kPlThreads, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr,
+                                                                           planes, pstride, RbfGrad{});
                  SKEMA_LAUNCHED(c);
                }};
     if (x3_update(c, in, row0, nrows)) return;
@@ -468,12 +487,12 @@ struct RunIf {  // the SIMT kernels launched in this scope run when *flag != 0
 static void launch_planes(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, int64_t r, int64_t wr,
                           __nv_bfloat16* planes, int64_t pstride, const RbfGrad* g) {
   const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
-  const int grid = grid_cap(c, tiles, 8);
   if (g)
-    rbf_planes_kernel<true, true><<<grid, 256, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr, planes, pstride, *g);
+    rbf_planes_kernel<true, true><<<grid_cap(c, tiles, 2), kPlThreads, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr,
+                                                                                       planes, pstride, *g);
   else
-    rbf_planes_kernel<true, false><<<grid, 256, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr, planes, pstride,
-                                                                RbfGrad{});
+    rbf_planes_kernel<true, false><<<grid_cap(c, tiles, 3), kPlThreads, 0, c->stream>>>(pts, d, 1, N, d, gamma, r, wr,
+                                                                                        planes, pstride, RbfGrad{});
   SKEMA_LAUNCHED(c);
 }
 

@@ -37,9 +37,9 @@ __device__ __forceinline__ bool too_big(float x) {
 }
 
 __device__ __forceinline__ void store_planes8(const float* v, __nv_bfloat16* d, int64_t pstride) {
-  __nv_bfloat16 q[3][8];
+  __nv_bfloat162 q[3][4];
 #pragma unroll
-  for (int t = 0; t < 8; ++t) tc::split3(v[t], q[0][t], q[1][t], q[2][t]);
+  for (int t = 0; t < 4; ++t) tc::split3x2(v[2 * t], v[2 * t + 1], q[0][t], q[1][t], q[2][t]);
 #pragma unroll
   for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(d + p * pstride) = *reinterpret_cast<const uint4*>(q[p]);
 }

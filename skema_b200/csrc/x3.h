@@ -10,6 +10,13 @@
 namespace skema {
 
 namespace tc {
+// The same for two values, whose BF16 parts lie side by side.
+__device__ __forceinline__ void split3x2(float x, float y, __nv_bfloat162& h, __nv_bfloat162& m, __nv_bfloat162& l) {
+  h = __floats2bfloat162_rn(x, y);
+  const float rx = x - __low2float(h), ry = y - __high2float(h);
+  m = __floats2bfloat162_rn(rx, ry);
+  l = __floats2bfloat162_rn(rx - __low2float(m), ry - __high2float(m));
+}
 // Where an x3_gemm product goes.
 struct X3Out {
   // columns [0, split): FP32, p0[row * rs0 + col * cs0] = beta p0 + alpha acc
