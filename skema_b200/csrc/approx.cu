@@ -233,14 +233,15 @@ void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA
 // 32 rows are 36 doubles apart, so fragment reads hit distinct banks) and its
 // warps form the 16 x 8 blocks on or above the diagonal with m16n8k16, up to
 // NT each, in registers over all of the CTA's rows; blockIdx.y takes a group of
-// blocks when they do not all fit. Up to three blocks a warp, two CTAs per SM
-// run, one staging while the other multiplies. The parts go to G (column-major k x k, zeroed
+// blocks when they do not all fit. Up to three blocks a warp (k <= 96), two CTAs
+// per SM run and each loads its next rows while it multiplies (502 and 490 us
+// without). The parts go to G (column-major k x k, zeroed
 // beforehand) with atomics, mirrored below the diagonal. Bound by the FP64
-// pipe: 1e6 x 81 takes 502 us from FP32 and 490 from FP64 (793 and 734 with
+// pipe: 1e6 x 81 takes 358 us from FP32 and 386 from FP64 (793 and 734 with
 // fragments read from global memory by every warp that needs them).
 constexpr int kGramTiles = 6, kGramLd = 36;
 template <typename T, int NT>
-__global__ void __launch_bounds__(512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T* __restrict__ A, int64_t lda, int k, int64_t rows,
+__global__ void __launch_bounds__(NT <= 3 ? 384 : 512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T* __restrict__ A, int64_t lda, int k, int64_t rows,
                                                           double* __restrict__ G, int64_t rows_per_cta) {
   extern __shared__ __align__(16) double gr_smem[];  // (k up to 16) x kGramLd
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, lr = lane & 3, lc = lane >> 2;
@@ -273,9 +274,24 @@ __global__ void __launch_bounds__(512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T*
   for (int q = 0; q < NT; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0;
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
   const int kpad = nm * 16;
+  // NT <= 3 (k up to 96, eight columns a warp): the next rows are loaded while
+  // the current ones multiply
+  constexpr int PF = NT <= 3 ? 8 : 0;
+  T nx[PF > 0 ? PF : 1];
+  auto prefetch = [&](int64_t r) {
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int cc = warp + u * nw;
+      nx[u] = (r + lane < r1 && cc < k) ? A[(int64_t)cc * lda + r + lane] : T(0);
+    }
+  };
+  prefetch(r0);
   for (int64_t r = r0; r < r1; r += 32) {
     const bool rv = r + lane < r1;
-    for (int c = warp; c < kpad; c += 4 * nw) {
+#pragma unroll
+    for (int u = 0; u < PF; ++u)
+      if (warp + u * nw < kpad) gr_smem[(warp + u * nw) * kGramLd + lane] = (double)nx[u];
+    for (int c = warp + PF * nw; c < kpad; c += 4 * nw) {
       T v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -287,6 +303,7 @@ __global__ void __launch_bounds__(512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T*
         if (c + u * nw < kpad) gr_smem[(c + u * nw) * kGramLd + lane] = (double)v[u];
     }
     __syncthreads();
+    prefetch(r + 32);
 #pragma unroll
     for (int h = 0; h < 32; h += 16) {
       double a[8];
@@ -502,8 +519,9 @@ void launch_gram(skema_ctx* c, const T* A, int64_t lda, int64_t k, int64_t rows,
   // up to 16 warps, as many as share the blocks evenly: the fewest blocks per
   // warp, then the fewest warps
   const int groups = (tiles + 16 * kGramTiles - 1) / (16 * kGramTiles);
-  const int per_cta = (tiles + groups - 1) / groups, depth = (per_cta + 15) / 16;
-  const int warps = std::max(4, (per_cta + depth - 1) / depth);
+  const int per_cta = (tiles + groups - 1) / groups;
+  int depth = (per_cta + 15) / 16, warps = std::max(4, (per_cta + depth - 1) / depth);
+  if (depth <= 3 && warps > 12) depth = (per_cta + 11) / 12, warps = (per_cta + depth - 1) / depth;
   const size_t smem = sizeof(double) * (size_t)((k + 15) / 16 * 16 * kGramLd);
   const bool few = depth <= 3;
   const int64_t ctas =
