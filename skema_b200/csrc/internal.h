@@ -242,6 +242,14 @@ void y_materialize(skema_ctx* c);
 // no row of the range was written since the reset (the kernel then writes
 // without reading), else nu, after the range's unwritten rows were zeroed.
 float y_beta(skema_ctx* c, int64_t a, int64_t b, float nu);
+// Windows whose weights nu^(G-1-w) may be folded into one pass: nu^G stays
+// within 2^+-40, far from where FP32 (or the low plane of a BF16 split)
+// overflows or loses bits; one for nu = 0.
+inline int64_t weight_windows(float nu) {
+  if (!(nu > 0.f)) return 1;
+  const double l = std::fabs(std::log2((double)nu));
+  return l > 0 ? std::max<int64_t>(1, (int64_t)std::min(40.0 / l, 1e9)) : (int64_t)1 << 40;
+}
 // Zero X and Z on `stream` if a reset left them pending.
 void xz_materialize(skema_ctx* c, cudaStream_t stream);
 

@@ -879,13 +879,19 @@ void csr_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const f
   }
 
   xz_materialize(c, c->stream);
-  if (csr_gauss_update(c, rowptr, col, val, col_offset, row0, nrows, ybeta)) return;
+  int64_t done = 0;
+  const int64_t L = c->spd ? nwin : std::min(nwin, weight_windows(nu));
+  while (done < nrows) {
+    const int64_t wr = std::min(L * W, nrows - done);
+    if (!csr_gauss_update(c, rowptr + done, col, val, col_offset, row0 + done, wr, ybeta)) break;
+    done += wr;
+  }
   // The same window by window, for a workspace limit that has no room for
   // the call's T and X^T.
   // Gauss maps, all stored transposed (src/Skema_SketchySVD.cpp:296-316):
   // stored rows contiguous, logical (r, j) at f32[r + j*lrows].
   const int threads = 256;
-  for (int64_t r = 0; r < nrows; r += W) {
+  for (int64_t r = done; r < nrows; r += W) {
     const int64_t wr = std::min(W, nrows - r);
     const int64_t R0 = row0 + r;
     const float yb = y_beta(c, R0, R0 + wr, nu);

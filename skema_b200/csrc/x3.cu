@@ -309,14 +309,10 @@ void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag) {
   SKEMA_LAUNCHED(c);
 }
 
-bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
+// nrows <= wsrows, which sizes the blocks and the workspace.
+static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows, int64_t wsrows) {
   const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w;
   const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
-  if (nrows <= 0 || !(nu > 0.f)) return false;
-  for (const Map* mp : {&c->ups, &c->omg, &c->phi, &c->psi})
-    if (mp->big) return false;
-  // below this the launches and conversions cost more than the products
-  if ((double)nrows * (double)n * (double)(2 * k + s) < 2e7) return false;
   const int64_t ldn = pad8(n);
   const size_t b_op = up256(sizeof(__nv_bfloat16) * (size_t)(3 * (k + s) * ldn));
   const size_t b_part = up256(x3_part_bytes(c));
@@ -326,13 +322,13 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
   size_t b_a = 0, b_uf = 0, b_t = 0, b_t32 = 0, b_flag = 0;
   for (size_t budget = (size_t)2 << 30; budget >= ((size_t)64 << 20) && !ws; budget >>= 2) {
     const int64_t cap = std::max<int64_t>(64, (int64_t)(budget / (size_t)(6 * n)) / 64 * 64);
-    const int64_t nb = (nrows + cap - 1) / cap;
-    rb = ((nrows + nb - 1) / nb + 63) / 64 * 64;
+    const int64_t nb = (wsrows + cap - 1) / cap;
+    rb = ((wsrows + nb - 1) / nb + 63) / 64 * 64;
     b_a = up256(sizeof(__nv_bfloat16) * (size_t)(3 * rb * n));
     b_uf = up256(sizeof(__nv_bfloat16) * (size_t)(3 * (k + s) * rb));
     b_t = up256(sizeof(__nv_bfloat16) * (size_t)(3 * s * rb));
     b_t32 = in.A.p ? up256(sizeof(float) * (size_t)(s * rb)) : 0;
-    b_flag = up256(sizeof(uint32_t) * (size_t)((nrows + rb - 1) / rb));
+    b_flag = up256(sizeof(uint32_t) * (size_t)((wsrows + rb - 1) / rb));
     ws = static_cast<char*>(try_workspace(c, b_op + b_part + b_a + b_uf + b_t + b_t32 + b_flag));
     if (cap == 64) break;
   }
@@ -421,6 +417,23 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
     }
   }
   y_rows_mark(c, row0, row0 + nrows);
+  return true;
+}
+
+bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
+  const float nu = (float)c->p.sketch_nu;
+  if (nrows <= 0 || !(nu > 0.f)) return false;
+  for (const Map* mp : {&c->ups, &c->omg, &c->phi, &c->psi})
+    if (mp->big) return false;
+  // below this the launches and conversions cost more than the products
+  if ((double)nrows * (double)c->n * (double)(2 * c->k + (c->spd ? 0 : c->s)) < 2e7) return false;
+  const int64_t W = c->w, step = std::min((nrows + W - 1) / W, weight_windows(nu)) * W;
+  for (int64_t r = 0; r < nrows; r += step) {
+    X3Input part = in;
+    if (part.A.p) part.A.p += r * part.A.rs;
+    // false at r = 0 only: every run asks for the same workspace
+    if (!x3_windows(c, part, row0 + r, std::min(step, nrows - r), std::min(step, nrows))) return false;
+  }
   return true;
 }
 
