@@ -287,7 +287,7 @@ __global__ void f32_to_bf16_cm_kernel(const float* __restrict__ S, int64_t lds, 
 // takes 211 KB of shared memory).
 // Tiles, K-steps and schedule of one launch; *grid gets the CTA count.
 tc::Grid3 grid_of(const skema_ctx* c, int64_t M, int64_t N, int64_t K, int nt, int bk, const Plan& pl, int m_fast,
-                  int* grid) {
+                  int* grid, int nwin = 1) {
   tc::Grid3 g;
   g.mtiles = (int)((M + tc::BM - 1) / tc::BM);
   g.ntiles = (int)((N + nt - 1) / nt);
@@ -296,8 +296,10 @@ tc::Grid3 grid_of(const skema_ctx* c, int64_t M, int64_t N, int64_t K, int nt, i
   g.ksteps = (K + bk - 1) / bk;
   g.kcsteps = pl.kchunk > 0 ? (int)(pl.kchunk / bk) : (int)g.ksteps;
   g.streamk = pl.streamk > 0 ? 1 : 0;
-  const int64_t units = (int64_t)g.mtiles * g.ntiles * (g.streamk ? g.ksteps : g.ksplit);
+  g.wtiles = g.mtiles, g.wk = 0, g.wlog2 = 0.f;
+  const int64_t units = (int64_t)nwin * g.mtiles * g.ntiles * (g.streamk ? g.ksteps : g.ksplit);
   if (units > 0x7fffffff) fail(SKEMA_EINVAL, "tensor-core grid too large");
+  g.mtiles *= nwin;
   *grid = (int)std::min<int64_t>(units, g.streamk ? pl.streamk : c->sm_count);
   if (c->tc_cta_cap > 0) *grid = std::min(*grid, c->tc_cta_cap);
   if (M <= 0 || N <= 0 || K <= 0) *grid = 0;
@@ -323,15 +325,17 @@ void launch_gemm(skema_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int
 // X^T product straight from the FP32 window (converts it and writes A16).
 template <bool AROW, int S1, int S2, bool STT>
 void launch_gemm_a32_s(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& ta16,
-                       int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax) {
+                       int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax, int nwin,
+                       float wlog2) {
   constexpr uint32_t STAGE = ((tc::BM * tc::BK * 2 + kNT * tc::BK * 2 + 1023) / 1024) * 1024;
   const size_t smem = (size_t)S1 * tc::BM * tc::BK * 4 + (size_t)S2 * STAGE + 1024 + 256;
   auto kern = amax ? tc::gemm_a32_kernel<kNT, S1, S2, AROW, true, STT>
                    : tc::gemm_a32_kernel<kNT, S1, S2, AROW, false, STT>;
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int grid = 0;
-  const tc::Grid3 g = grid_of(c, M, N, K, kNT, tc::BK, pl, 1, &grid);
+  tc::Grid3 g = grid_of(c, M, N, K, kNT, tc::BK, pl, 1, &grid, nwin);
   if (grid <= 0) return;
+  g.wk = K, g.wlog2 = wlog2;
   kern<<<grid, STT ? tc::kThreadsA32St : tc::kThreadsA32, smem, c->stream>>>(ta32, tb, ta16, g, o, amax,
                                                                             c->dev_err);
   SKEMA_LAUNCHED(c);
@@ -344,11 +348,12 @@ void launch_gemm_a32_s(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap&
 // of the two.
 template <bool AROW>
 void launch_gemm_a32(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& ta16,
-                     int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax) {
+                     int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax, int nwin,
+                     float wlog2) {
   if (c->xt_store_thread)
-    launch_gemm_a32_s<AROW, 3, 3, true>(c, ta32, tb, ta16, M, N, K, pl, o, amax);
+    launch_gemm_a32_s<AROW, 3, 3, true>(c, ta32, tb, ta16, M, N, K, pl, o, amax, nwin, wlog2);
   else
-    launch_gemm_a32_s<AROW, 3, 3, false>(c, ta32, tb, ta16, M, N, K, pl, o, amax);
+    launch_gemm_a32_s<AROW, 3, 3, false>(c, ta32, tb, ta16, M, N, K, pl, o, amax, nwin, wlog2);
 }
 
 // ---- FP8 form -------------------------------------------------------------
@@ -688,16 +693,48 @@ TcSlices xt_window(skema_ctx* c, Mat Aw, int64_t R0, int64_t wr, __nv_bfloat16* 
   const CUtensorMap ta16 = tmap_bf16_blocked(A16, (uint64_t)n, (uint64_t)nrb, 128);
   if (a32_cm) {
     const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)wr, (uint64_t)n, (uint64_t)Aw.cs * 4, 32, 128);
-    launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, amax);
+    launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.f);
   } else if (a32_rm) {
     const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)n, (uint64_t)wr, (uint64_t)Aw.rs * 4, 32, 64);
-    launch_gemm_a32<true>(c, ta32, tb, ta16, n, k, wr, pl, o, amax);
+    launch_gemm_a32<true>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.f);
   } else {
     launch_gemm<tc::A_KMAJ_BLK>(c, ta16, tb, n, k, wr, pl, 1, o);
   }
   return sl;
 }
 
+// xt_window for nwin whole windows of wr rows (a multiple of 64) that TMA can
+// address, in one launch: X = nu^nwin X + eta sum_w nu^(nwin-1-w) x_w, every x_w
+// summed by itself. Each launch per window waited for the last tiles of the one
+// before and then for its own first loads, which a window of a few MB never
+// made up for: 33,228 x 931 in windows of 3,136 rows (k = 65, s = 131) went
+// from 835 to 377 us, 60,000 x 9,000 in 4,096s (k = 101) from 2.21 to 1.70 ms, 200,000 x
+// 20,000 in 8,192s from 10.2 to 9.7 ms.
+bool xt_batchable(Mat Aw, int64_t R0) {
+  const bool al = reinterpret_cast<uintptr_t>(Aw.p) % 16 == 0;
+  return al && R0 % 8 == 0 && ((Aw.rs == 1 && Aw.cs % 4 == 0) || (Aw.cs == 1 && Aw.rs % 4 == 0));
+}
+void xt_batch(skema_ctx* c, Mat Aw, int64_t R0, int64_t wr, int nwin, __nv_bfloat16* A16) {
+  const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
+  const int64_t k = c->k, n = c->n, rows = wr * nwin;
+  StageScope st(c, ST_UPSILON);
+  const CUtensorMap tb = tmap_bf16(static_cast<const __nv_bfloat16*>(c->ups.lowp) + R0, (uint64_t)rows, (uint64_t)k,
+                                   (uint64_t)c->ld_maps16 * 2, 64, kNT);
+  const Plan pl = plan_streamk(c, c->sm_count);
+  tc::OutSpec o = out_spec();
+  o.p0 = c->X, o.rs0 = 1, o.cs0 = n, o.alpha0 = eta, o.beta0 = 0.f, o.atomic0 = 1;
+  o.rows = n, o.split = k, o.ncols = k;
+  scale_block(c, MatOut{c->X, n, 1}, k, n, (float)std::pow((double)nu, (double)nwin));
+  const CUtensorMap ta16 = tmap_bf16_blocked(A16, (uint64_t)n, (uint64_t)(rows / 64), 128);
+  const float wlog2 = nu == 1.f ? 0.f : std::log2(nu);
+  if (Aw.rs == 1) {
+    const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)rows, (uint64_t)n, (uint64_t)Aw.cs * 4, 32, 128);
+    launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, nullptr, nwin, wlog2);
+  } else {
+    const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)n, (uint64_t)rows, (uint64_t)Aw.rs * 4, 32, 64);
+    launch_gemm_a32<true>(c, ta32, tb, ta16, n, k, wr, pl, o, nullptr, nwin, wlog2);
+  }
+}
 // A8 = e4m3(scale_A A16) row-major for rows rows, from the window's amax.
 void to_a8(skema_ctx* c, const __nv_bfloat16* A16, int64_t rows, uint8_t* A8, int64_t ld8, const uint32_t* amax,
            float* scale_out) {
@@ -918,7 +955,15 @@ void tc_dense_update(skema_ctx* c, Mat A, int64_t row0, int64_t nrows) {
       // the buffer's previous group must have been read by its [Y | T]
       if (pipe && gi >= nbuf) SKEMA_CUDA(cudaStreamWaitEvent(main_st, c->pipe_ev[2 + b], 0));
       if (fp8) SKEMA_CUDA(cudaMemsetAsync(amaxb[b], 0, sizeof(uint32_t) * (size_t)(2 * gwin_max), main_st));
-      for (int64_t w = 0; w < G; ++w) {
+      // whole windows together, a last partial one (or FP8's, each with its
+      // amax) by itself
+      const Mat Ag{A.p + g0 * A.rs, A.rs, A.cs};
+      const int64_t whole = !fp8 && xt_batchable(Ag, R0) ? gr / W : 0;
+      for (int64_t w = 0, nw; w < whole; w += nw) {
+        nw = std::min(whole - w, weight_windows(nu));
+        xt_batch(c, Mat{Ag.p + w * W * A.rs, A.rs, A.cs}, R0 + w * W, W, (int)nw, A16 + w * W * n);
+      }
+      for (int64_t w = whole; w < G; ++w) {
         const int64_t r = g0 + w * W, wr = std::min(W, nrows - r);
         __nv_bfloat16* A16w = A16 + (w * W / 64) * 64 * n;
         char* sp = wslice_sp;

@@ -290,6 +290,13 @@ struct Grid3 {
   int64_t ksteps;
   int kcsteps;
   int streamk;
+  // gemm_a32_kernel over several windows at once: wtiles M tiles per window
+  // (mtiles = windows * wtiles), whose rows of A and B start wk K-elements
+  // after the window before's, all adding into one output; the parts of window
+  // w carry 2^((windows - 1 - w) wlog2). wtiles = mtiles: one window.
+  int wtiles;
+  int64_t wk;
+  float wlog2;
 };
 __device__ __forceinline__ void decode_unit(const Grid3& g, int t, int& mt, int& nt, int& ks) {
   if (g.m_fast) {
@@ -735,6 +742,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tbase;
+  auto k_of = [&](int mt) { return (int)(mt / g.wtiles * g.wk); };  // the window's first row
 
   if (warp == 4 && lane == 0) {
     // ---------------- TMA producer: FP32 tiles ----------------
@@ -748,7 +756,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s1 = it % S1;
         const uint32_t ph1 = (it / S1) & 1;
-        const int kc = (kt0 + kt) * BK;
+        const int kc = (kt0 + kt) * BK + k_of(mt), m0 = (mt % g.wtiles) * BM;
         if (!mbar_wait(f32empty + s1, ph1 ^ 1, err)) {
           ok = false;
           break;
@@ -756,11 +764,11 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
         unsigned char* a32 = st32 + s1 * A32_BYTES;
         mbar_expect_tx(f32full + s1, A32_BYTES);
         if (!AROW) {
-          tma_load_2d(&tmA32, f32full + s1, a32, kc, mt * BM);
-          tma_load_2d(&tmA32, f32full + s1, a32 + 16384, kc + 32, mt * BM);
+          tma_load_2d(&tmA32, f32full + s1, a32, kc, m0);
+          tma_load_2d(&tmA32, f32full + s1, a32 + 16384, kc + 32, m0);
         } else {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) tma_load_2d(&tmA32, f32full + s1, a32 + q * 8192, mt * BM + 32 * q, kc);
+          for (int q = 0; q < 4; ++q) tma_load_2d(&tmA32, f32full + s1, a32 + q * 8192, m0 + 32 * q, kc);
         }
       }
     }
@@ -776,7 +784,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s2 = it % S2;
         const uint32_t ph2 = (it / S2) & 1;
-        const int kc = (kt0 + kt) * BK;
+        const int kc = (kt0 + kt) * BK + k_of(mt);
         if (!mbar_wait(empty + s2, ph2 ^ 1, err)) {
           ok = false;
           break;
@@ -885,8 +893,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
             break;
           }
           fence_proxy_async();
-          const int kc = (kt0 + kt) * BK;
-          tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, mt * BM, kc / BK);
+          tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, (mt % g.wtiles) * BM, kt0 + kt + k_of(mt) / BK);
           bulk_commit();
           if (pend >= 0) {
             asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -925,7 +932,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
           break;
         }
         fence_proxy_async();
-        tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, mt * BM, kt0 + kt);
+        tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, (mt % g.wtiles) * BM, kt0 + kt + k_of(mt) / BK);
         bulk_commit();
         bulk_wait_read_all();
         mbar_arrive(empty + s2);
@@ -940,7 +947,9 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     int mt, nt, kt0, kt1;
     for (; next_seg(g, sc, mt, nt, kt0, kt1); ++tcount) {
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
-      if (!epilogue_unit<NT, TCOLS>(o, tmem, acc, aph, tfull, tempty, mt, nt, warp, lane, err)) break;
+      OutSpec ow = o;
+      if (g.wlog2 != 0.f) ow.alpha0 *= exp2f((float)(g.mtiles / g.wtiles - 1 - mt / g.wtiles) * g.wlog2);
+      if (!epilogue_unit<NT, TCOLS>(ow, tmem, acc, aph, tfull, tempty, mt % g.wtiles, nt, warp, lane, err)) break;
     }
   }
   drain_on_error(err);

@@ -1,4 +1,5 @@
-"""Several windows of a call in one pass: their weights nu^(G-1-w)."""
+"""Several windows of a call in one pass: their weights nu^(G-1-w), and the
+BF16 form's X product over whole windows against one launch per window."""
 import numpy as np
 import pytest
 
@@ -42,3 +43,33 @@ def test_weights_far_from_one(lib_built, oracle, form, nu, nwin, lo, hi):
         X, Y, Z = s.get_sketches()
     for got, want, bar in ((X, o.X, 1e-5 if form == "csr" else 4e-6), (Y, o.Y, 4e-6), (Z, o.Z, 4e-6)):
         assert rel_fro(np.asarray(got, np.float64), want) < bar
+
+
+@pytest.mark.parametrize("m,n,order,window,nu", [
+    (1000, 200, "F", 64, 0.9),     # 15 whole windows of one K step and a partial one
+    (4133, 1132, "C", 512, 0.95),  # nine M tiles, the last of 108 columns
+    (3072, 130, "F", 1024, 1.0),   # whole windows only, a last tile of two columns
+    (640, 128, "C", 320, 0.5),
+])
+def test_bf16_windows_together(lib_built, m, n, order, window, nu):
+    # The same BF16 operands and products; X's FP32 sums over at most 1024 rows
+    # (64 tensor-core steps, each off by at most 2^-23 of the sum) are cut
+    # differently: 64 x 2^-23 = 8e-6.
+    import torch
+    import skema_b200 as sk
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    buf = torch.randn(m * n + 4, device="cuda", generator=g)
+    out = []
+    for off in (0, 1):  # a base that TMA cannot address takes window after window
+        v = torch.empty(m * n + 4, device="cuda")[off:off + m * n]
+        v.copy_(buf[: m * n])
+        A = v.view(n, m).t() if order == "F" else v.view(m, n)
+        with sk.SketchySVD(sk.AlgParams(matrix_m=m, matrix_n=n, rank=10, window=window, sketch_nu=nu,
+                                        precision=sk._lib.PREC_BF16)) as s:
+            s.reset()
+            s.update_rows(A, 0)
+            s.update_rows(A, 0)  # X not empty
+            out.append([np.array(q, np.float64) for q in s.get_sketches()])
+    for a, b in zip(*out):
+        assert rel_fro(a, b) < 8e-6
