@@ -344,18 +344,19 @@ __device__ __forceinline__ bool next_seg(const Grid3& g, Sched& s, int& mt, int&
 
 // Stores one finished 128 x NT accumulator (warps 0-3, warp w on TMEM lanes
 // 32w..32w+31): waits for it, reads it 16 columns at a time, hands it back
-// to the MMA issuer after the last read, and writes the columns per OutSpec.
+// to the MMA issuer after the last read, and writes the columns per OutSpec
+// (the first part times w0).
 // False when the wait failed (the warp then stops).
 template <int NT, uint32_t TCOLS>
 __device__ __forceinline__ bool epilogue_unit(const OutSpec& o, uint32_t tmem, uint32_t acc, uint32_t aph,
                                               uint64_t* tfull, uint64_t* tempty, int mt, int nt, int warp,
-                                              int lane, int* err) {
+                                              int lane, int* err, float w0 = 1.f) {
   // tcgen05.ld is warp-collective: the whole warp reads TMEM or none of it
   if (!__all_sync(0xffffffffu, mbar_wait(tfull + acc, aph, err))) return false;
   tc_fence_after();
   const int64_t row = (int64_t)mt * BM + warp * 32 + lane;
   const uint32_t taddr = tmem + acc * TCOLS + ((uint32_t)(warp * 32) << 16);
-  float alpha0 = o.alpha0, alpha1 = o.alpha1;
+  float alpha0 = o.alpha0 * w0, alpha1 = o.alpha1;
   if (o.scale && row < o.rows) {
     const float sc = o.scale[row / o.scale_wlen];
     alpha0 *= sc;
@@ -742,7 +743,9 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tbase;
-  auto k_of = [&](int mt) { return (int)(mt / g.wtiles * g.wk); };  // the window's first row
+  // a segment's first K element (its window's first row added) and M row
+  auto k_of = [&](int mt, int kt0) { return kt0 * BK + (int)(mt / g.wtiles * g.wk); };
+  auto m_of = [&](int mt) { return mt % g.wtiles * BM; };
 
   if (warp == 4 && lane == 0) {
     // ---------------- TMA producer: FP32 tiles ----------------
@@ -752,11 +755,11 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     sched_init(g, sc);
     int mt, nt, kt0, kt1;
     while (ok && next_seg(g, sc, mt, nt, kt0, kt1)) {
-      const int KT = kt1 - kt0;
+      const int KT = kt1 - kt0, k0 = k_of(mt, kt0), m0 = m_of(mt);
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s1 = it % S1;
         const uint32_t ph1 = (it / S1) & 1;
-        const int kc = (kt0 + kt) * BK + k_of(mt), m0 = (mt % g.wtiles) * BM;
+        const int kc = k0 + kt * BK;
         if (!mbar_wait(f32empty + s1, ph1 ^ 1, err)) {
           ok = false;
           break;
@@ -780,11 +783,11 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     sched_init(g, sc);
     int mt, nt, kt0, kt1;
     while (ok && next_seg(g, sc, mt, nt, kt0, kt1)) {
-      const int KT = kt1 - kt0;
+      const int KT = kt1 - kt0, k0 = k_of(mt, kt0);
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s2 = it % S2;
         const uint32_t ph2 = (it / S2) & 1;
-        const int kc = (kt0 + kt) * BK + k_of(mt);
+        const int kc = k0 + kt * BK;
         if (!mbar_wait(empty + s2, ph2 ^ 1, err)) {
           ok = false;
           break;
@@ -837,6 +840,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     int mt, nt, kt0, kt1;
     while (ok && next_seg(g, sc, mt, nt, kt0, kt1)) {
       const int KT = kt1 - kt0;
+      const int kb = STT ? 0 : k_of(mt, kt0) / BK, m0 = STT ? 0 : m_of(mt);
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s1 = it % S1, s2 = it % S2;
         const uint32_t ph1 = (it / S1) & 1, ph2 = (it / S2) & 1;
@@ -893,7 +897,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
             break;
           }
           fence_proxy_async();
-          tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, (mt % g.wtiles) * BM, kt0 + kt + k_of(mt) / BK);
+          tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, m0, kb + kt);
           bulk_commit();
           if (pend >= 0) {
             asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -923,7 +927,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     sched_init(g, sc);
     int mt, nt, kt0, kt1;
     while (ok && next_seg(g, sc, mt, nt, kt0, kt1)) {
-      const int KT = kt1 - kt0;
+      const int KT = kt1 - kt0, kb = k_of(mt, kt0) / BK, m0 = m_of(mt);
       for (int kt = 0; kt < KT; ++kt, ++it) {
         const int s2 = it % S2;
         const uint32_t ph2 = (it / S2) & 1;
@@ -932,7 +936,7 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
           break;
         }
         fence_proxy_async();
-        tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, (mt % g.wtiles) * BM, kt0 + kt + k_of(mt) / BK);
+        tma_store_3d(&tmA16, stbf + s2 * STAGE, 0, m0, kb + kt);
         bulk_commit();
         bulk_wait_read_all();
         mbar_arrive(empty + s2);
@@ -947,9 +951,9 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     int mt, nt, kt0, kt1;
     for (; next_seg(g, sc, mt, nt, kt0, kt1); ++tcount) {
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
-      OutSpec ow = o;
-      if (g.wlog2 != 0.f) ow.alpha0 *= exp2f((float)(g.mtiles / g.wtiles - 1 - mt / g.wtiles) * g.wlog2);
-      if (!epilogue_unit<NT, TCOLS>(ow, tmem, acc, aph, tfull, tempty, mt % g.wtiles, nt, warp, lane, err)) break;
+      float w = 1.f;
+      if (g.wlog2 != 0.f) w = exp2f((float)(g.mtiles / g.wtiles - 1 - mt / g.wtiles) * g.wlog2);
+      if (!epilogue_unit<NT, TCOLS>(o, tmem, acc, aph, tfull, tempty, mt % g.wtiles, nt, warp, lane, err, w)) break;
     }
   }
   drain_on_error(err);
