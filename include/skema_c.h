@@ -466,8 +466,10 @@ int64_t skema_launch_count(const skema_ctx* ctx);
  *   "update.upsilon" X += Upsilon_w A_w
  *   "update.phi"     Z += Phi_w T
  *   "update.entries" the sparse-sign X/Z entry kernel
- *   "update.window"  kernel-window generation
- *   "update.fused"   the fused tensor-core window kernel
+ *   "update.window"  kernel-window generation; conversion of the input and
+ *                    the maps for the tensor cores
+ *   "update.fused"   [Y | T] in one tensor-core product (BF16, FP8, and the
+ *                    FP32 form of larger calls)
  *   "update.daxpy"   sketch scaling by nu
  *   "approx.orth"    orthonormal bases of Y and X^T (skema_low_rank_approx)
  *   "approx.core"    the core matrix: Phi Q, Psi P, their QR and the solves

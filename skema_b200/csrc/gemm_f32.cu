@@ -1,9 +1,11 @@
-// gemm_f32.cu -- the plain FP32 contraction used by the FP32 form of the
-// sketch (the drop-in for KokkosBlas::gemm in Impl::mm,
-// src/Skema_Common.hpp:32-40) plus small strided elementwise kernels.
+// gemm_f32.cu -- the plain FP32 contraction (the drop-in for KokkosBlas::gemm
+// in Impl::mm, src/Skema_Common.hpp:32-40) plus small strided elementwise
+// kernels. The FP32 sketch takes it for small calls, nu = 0, imported maps
+// beyond the range of the three-plane form (x3.cu) and workspace caps below
+// that form's need.
 //
 // SIMT GEMM: 128x128 output tile per 256-thread CTA, 8x8 outputs per thread,
-// K staged through double-buffered shared memory 8 deep. Operands are
+// K staged through double-buffered shared memory 16 deep. Operands are
 // addressed by (row stride, col stride) so that column-major A windows,
 // row-major maps and transposed views need no copies; the template picks the
 // coalesced load pattern from which stride is 1. Optional split-K over

@@ -887,7 +887,7 @@ void csr_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const f
     done += wr;
   }
   // The same window by window, for a workspace limit that has no room for
-  // the call's T and X^T.
+  // the call's T and X^T (SPD calls need none).
   // Gauss maps, all stored transposed (src/Skema_SketchySVD.cpp:296-316):
   // stored rows contiguous, logical (r, j) at f32[r + j*lrows].
   const int threads = 256;
@@ -902,7 +902,6 @@ void csr_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const f
       SKEMA_LAUNCHED(c);
     }
     y_rows_mark(c, R0, R0 + wr);
-    if (c->spd) continue;
     {  // X = nu X + eta (A_w^T Upsilon_stored(R0:R0+wr, :))^T
       StageScope st(c, ST_UPSILON);
       scale_block(c, MatOut{c->X, c->n, 1}, c->k, c->n, nu);

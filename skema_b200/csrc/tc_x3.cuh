@@ -12,8 +12,8 @@
 // (about 230 TFLOP/s of FP32 work at the measured sustained 1400) against 74
 // nominal and 31-37 measured for the SIMT kernel. Whole sketch updates: 50,000
 // x 20,000 at k = 201, s = 403 in 52.2 -> 11.2 ms; the RBF kernel of 40,000
-// points (d = 100, k = 129, s = 259) in 102.6 -> 28.5 ms; 3001 x 1003 in six
-// windows in 2.43 -> 0.21 ms.
+// points (d = 100, k = 129, s = 259) in 102.6 -> 25.0 ms; 3001 x 1003 in six
+// windows in 2.42 -> 0.15 ms.
 //
 // Accuracy. tcgen05 accumulates in FP32 without round-to-nearest, so a long
 // run of MMAs on one accumulator drifts towards zero. Each K step of 32 is
