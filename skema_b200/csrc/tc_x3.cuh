@@ -290,10 +290,13 @@ __global__ void __launch_bounds__(kX3Threads, 1)
 }
 
 // Adds the parts of the tiles that were cut, in K order, and stores them.
-// blockIdx.x: tile, blockIdx.y: two columns; G: the product's grid; a thread
-// per row and column. A product of few tiles cuts each into as many as G
-// parts, so eight parts are loaded at a time (one after another took 79
-// us, this way 22, for two tiles of 74 parts).
+// blockIdx.x: tile, blockIdx.y: 2 COLS columns; G: the product's grid; a
+// thread per row and COLS columns. A product of few tiles cuts each into as
+// many as G parts: COLS = 1, eight parts loaded at a time (one after another took 79
+// us, this way 22, for two tiles of 74 parts). One of many tiles has two or
+// three parts per tile, and finding them (64-bit divisions) cost more than
+// adding them: COLS = 4, 60 -> 17 us for 97 tiles of 208 columns.
+template <int COLS>
 static __global__ void __launch_bounds__(256) x3_reduce_kernel(X3Grid g, X3Out o, int G, const float* __restrict__ part,
                                                         const uint32_t* __restrict__ flag) {
   if (flag && *flag) return;
@@ -308,22 +311,32 @@ static __global__ void __launch_bounds__(256) x3_reduce_kernel(X3Grid g, X3Out o
   while (x3_run(g, e, G) > ke - 1) --e;
   while (x3_run(g, e + 1, G) <= ke - 1) ++e;
   const int tile = g.full + (int)q;
-  const int r = threadIdx.x & 127, cl = blockIdx.y * 2 + (threadIdx.x >> 7);
+  const int r = threadIdx.x & 127, cl = (blockIdx.y * 2 + (threadIdx.x >> 7)) * COLS;
   const int64_t row = (int64_t)(tile / g.ntiles) * BM + r;
   const float* pp = part + (int64_t)cl * BM + r;
   const int64_t slot = (int64_t)g.nt * BM;
   // the first run may begin in the tile before: its part of this tile is its
   // second; every other run begins inside the tile (runs are never empty)
-  float sum = pp[(2 * b + (x3_run(g, b, G) < kb ? 1 : 0)) * slot];
+  float sum[COLS];
+  const float* p0 = pp + (2 * b + (x3_run(g, b, G) < kb ? 1 : 0)) * slot;
+#pragma unroll
+  for (int q = 0; q < COLS; ++q) sum[q] = p0[q * BM];
   pp += 2 * slot;
-  for (int64_t i = b; i < e; i += 8) {
-    float v[8];
+  constexpr int U = 8 / COLS;
+  for (int64_t i = b; i < e; i += U) {
+    float v[U][COLS];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = i + u < e ? pp[2 * (i + u) * slot] : 0.f;
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) sum += v[u];
+      for (int q = 0; q < COLS; ++q) v[u][q] = i + u < e ? pp[2 * (i + u) * slot + q * BM] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < COLS; ++q) sum[q] += v[u][q];
   }
-  if (row < o.rows) x3_store(o, row, (int64_t)(tile % g.ntiles) * g.nt + cl, sum);
+  if (row >= o.rows) return;
+#pragma unroll
+  for (int q = 0; q < COLS; ++q) x3_store(o, row, (int64_t)(tile % g.ntiles) * g.nt + cl + q, sum[q]);
 }
 
 }  // namespace tc

@@ -272,7 +272,10 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   c->dev_err_armed = true;
   const int rem = (int)(tiles - g.full);
   if (rem > 0) {
-    tc::x3_reduce_kernel<<<dim3(rem, g.nt / 2), 256, 0, c->stream>>>(g, o, G, part, flag);
+    if (rem * (g.nt / 8) >= 2 * c->sm_count)
+      tc::x3_reduce_kernel<4><<<dim3(rem, g.nt / 8), 256, 0, c->stream>>>(g, o, G, part, flag);
+    else
+      tc::x3_reduce_kernel<1><<<dim3(rem, g.nt / 2), 256, 0, c->stream>>>(g, o, G, part, flag);
     SKEMA_LAUNCHED(c);
   }
 }
