@@ -751,7 +751,7 @@ static void launch_csr_ssign_y(skema_ctx* c, const int64_t* rowptr, const int32_
 // CSR x Gauss over all windows of a call (src/Skema_SketchySVD.cpp:296-316):
 // Z = nu^G Z + eta sum_i w_i Phi(i, :)^T T(i, :) with T = A Psi, the
 // association of the dense form, instead of an n x s scatter and an n-deep
-// product per window: 3.64 -> 0.52 ms for 100,000 x 20,000, 1e6 nonzeros, ten
+// product per window: 3.64 -> 0.46 ms for 100,000 x 20,000, 1e6 nonzeros, ten
 // windows, k = 81, s = 163. False when the workspace is not to be had.
 static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const float* val,
                              int64_t col_offset, int64_t row0, int64_t nrows, float ybeta) {

@@ -189,33 +189,48 @@ __global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_
 }
 
 // K-major planes D[q * pstride + c * ld + i] of a row-major source (rows i of
-// `cols` values, rs apart), turned by 64 x 32 tiles; columns i past `rows` up
-// to ld are zeros. Row i is scaled by nu^(nwin - 1 - (j0 + i) / W).
+// `cols` values, rs apart), turned by kTrRows x 32 tiles; columns i past `rows`
+// up to ld are zeros. Row i is scaled by nu^(nwin - 1 - (j0 + i) / W), which a
+// lane forms for each of its warp's rows (a pow in FP64 by every lane took 110 us
+// longer). Bound by memory: 100,000 x 163 in 68 us with 64 rows per tile, 34
+// with 128, whose stores are runs of 256 bytes.
+constexpr int kTrRows = 128;
 __global__ void __launch_bounds__(256)
     x3_transposed_kernel(const float* __restrict__ S, int64_t rs, int64_t rows, int64_t cols,
                          __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin,
                          int64_t j0, uint32_t* __restrict__ flag) {
-  __shared__ float tile[32][65];
+  constexpr int NR = kTrRows / 8;  // rows per warp
+  __shared__ float tile[32][kTrRows + 1];
   bool big = false;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t ti = (ld + 63) / 64, tj = (cols + 31) / 32;
+  const int64_t ti = (ld + kTrRows - 1) / kTrRows, tj = (cols + 31) / 32;
   for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
-    const int64_t i0 = (t / tj) * 64, c0 = (t % tj) * 32;
+    const int64_t i0 = (t / tj) * kTrRows, c0 = (t % tj) * 32;
+    float v[NR];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < NR; ++q) {
       const int r = ty + 8 * q;
-      float v = (i0 + r < rows && c0 + tx < cols) ? S[(i0 + r) * rs + c0 + tx] : 0.f;
-      if (nu != 1.f && i0 + r < rows) v *= (float)pow((double)nu, (double)(nwin - 1 - (j0 + i0 + r) / W));
-      big |= too_big(v);
-      tile[tx][r] = v;
+      v[q] = (i0 + r < rows && c0 + tx < cols) ? S[(i0 + r) * rs + c0 + tx] : 0.f;
+    }
+    float w = 1.f;
+    if (nu != 1.f && tx < NR && i0 + ty + 8 * tx < rows)
+      w = (float)pow((double)nu, (double)(nwin - 1 - (j0 + i0 + ty + 8 * tx) / W));
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      if (nu != 1.f) v[q] *= __shfl_sync(0xffffffffu, w, q);
+      big |= too_big(v[q]);
+      tile[tx][ty + 8 * q] = v[q];
     }
     __syncthreads();
-    const int j = threadIdx.x >> 3, g8 = (threadIdx.x & 7) * 8;
-    if (c0 + j < cols && i0 + g8 < ld) {
-      float v[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = tile[j][g8 + e];
-      store_planes8(v, D + (c0 + j) * ld + i0 + g8, pstride);
+    for (int h = 0; h < kTrRows / 64; ++h) {
+      const int item = threadIdx.x + 256 * h, j = item / NR, g8 = (item % NR) * 8;
+      if (c0 + j < cols && i0 + g8 < ld) {
+        float x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = tile[j][g8 + e];
+        store_planes8(x, D + (c0 + j) * ld + i0 + g8, pstride);
+      }
     }
     __syncthreads();
   }
@@ -294,7 +309,7 @@ void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfl
 
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
                           int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag) {
-  const int64_t tiles = ((ld + 63) / 64) * ((cols + 31) / 32);
+  const int64_t tiles = ((ld + kTrRows - 1) / kTrRows) * ((cols + 31) / 32);
   x3_transposed_kernel<<<grid_1d(c, tiles * 256, 16), 256, 0, c->stream>>>(S, rs, rows, cols, D, ld, pstride, nu, W,
                                                                           nwin, j0, flag);
   SKEMA_LAUNCHED(c);
