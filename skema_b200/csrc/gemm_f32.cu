@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "x3.h"
 
 namespace skema {
 
@@ -33,7 +34,7 @@ __global__ void __launch_bounds__(256, 1)
                  int64_t a_rs, int64_t a_cs, const float* __restrict__ B, int64_t b_rs,
                  int64_t b_cs, float beta, float* __restrict__ C, int64_t c_rs, int64_t c_cs,
                  int64_t kchunk, int64_t c_zs, const uint32_t* __restrict__ run_if) {
-  if (run_if && *run_if == 0) return;
+  if (run_if && !x3_refused(*run_if)) return;
   __shared__ __align__(16) float As[2][BK][BM + PAD];
   __shared__ __align__(16) float Bs[2][BK][BN + PAD];
   const int tid = threadIdx.x;
@@ -154,7 +155,7 @@ void launch_sgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, float alpha, Ma
 
 __global__ void scale_kernel(float* __restrict__ C, int64_t rs, int64_t cs, int64_t M, int64_t N,
                              float beta, const uint32_t* __restrict__ run_if) {
-  if (run_if && *run_if == 0) return;
+  if (run_if && !x3_refused(*run_if)) return;
   const int64_t total = M * N;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
        q += (int64_t)gridDim.x * blockDim.x) {
@@ -232,7 +233,7 @@ __global__ void copy_kernel(const float* __restrict__ S, int64_t srs, int64_t sc
 __global__ void splitk_reduce_kernel(const float* __restrict__ P, int64_t p_rs, int64_t p_cs, int64_t p_zs, int nz,
                                      int64_t M, int64_t N, float alpha, float beta, float* __restrict__ C,
                                      int64_t c_rs, int64_t c_cs, const uint32_t* __restrict__ run_if) {
-  if (run_if && *run_if == 0) return;
+  if (run_if && !x3_refused(*run_if)) return;
   const int64_t total = M * N;
   const bool cm = c_rs == 1;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {

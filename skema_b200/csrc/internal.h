@@ -193,9 +193,9 @@ struct skema_ctx {
   // dev_err[0] non-zero when a wait timed out (checked at the next
   // synchronising call); dev_err[2..3] the wait limit in ns (64-bit).
   int* dev_err = nullptr;
-  // While set, the FP32 SIMT kernels (gemm_f32.cu, rbf.cu) return at once when
-  // the device word is 0: the second form of a call whose first, on the tensor
-  // cores, may have refused its values (x3.h). Null: they run.
+  // While set, the FP32 SIMT kernels (gemm_f32.cu, rbf.cu) return at once unless
+  // the device word is refused (x3.h): the second form of a call whose first is
+  // on the tensor cores. Null: they run.
   const uint32_t* run_if = nullptr;
   // The rotations that the Jacobi SVD's two CTAs exchange (approx.cu), in the
   // allocation of dev_err.

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256)
                     float gamma, int64_t R0, int64_t wr, float* __restrict__ out, int64_t ldo,
                     double* __restrict__ dgamma, float* __restrict__ rsum, float* __restrict__ csum,
                     const uint32_t* __restrict__ run_if) {
-  if (run_if && *run_if == 0) return;
+  if (run_if && !x3_refused(*run_if)) return;
   __shared__ float xi[TD][TT + 1];
   __shared__ float xj[TD][TT + 1];
   __shared__ float red[256];
@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(256)
 // distances (k more FP32 instructions per entry; as a product of its own it
 // cost an FP32 block written and read back: forward and adjoint at N = 20,000,
 // d = 24, k = 65 took 8.0 ms, now 6.1, this kernel 3.1 of them), E_ii = 0 (the diagonal's terms of the gradient cancel), and the sums
-// -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them; *big is set
-// when a value is out of the planes' range.
+// -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them; E's magnitudes
+// are noted in *word.
 struct RbfGrad {
   const float* Ybar;   // N x k row-major
   const float* omega;  // k x N row-major
@@ -159,7 +159,7 @@ struct RbfGrad {
   double* dgamma;
   float* rsum;
   float* csum;
-  uint32_t* big;
+  uint32_t* word;
 };
 // s += (a + b)^2, and s += a b, on two packed FP32 values, each rounded as FADD
 // and FFMA do.
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
   __shared__ __align__(16) RbfTile t;
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   const int64_t tiles_j = (N + kTJ - 1) / kTJ, tiles_i = (wr + kTI - 1) / kTI;
-  bool big = false;
+  uint32_t top = 0;
   double gsum = 0.0;
   for (int64_t tile = blockIdx.x; tile < tiles_i * tiles_j; tile += gridDim.x) {
     const int64_t ib = tile / tiles_j, i0 = ib * kTI, j0 = (tile - ib * tiles_j) * kTJ;
@@ -298,8 +298,7 @@ __global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
           float kv = expf(-gamma * d2);
           if (GRAD) {
             kv = (in && li < ni && !diag) ? half_of(mac[GRAD ? u : 0][v], h) * kv : 0.f;
-            const uint32_t bits = __float_as_uint(kv) & 0x7fffffffu;
-            big |= bits >= 0x71800000u && bits <= 0x7f800000u;
+            x3_note(top, kv);
             gpart = fmaf(kv, d2, gpart);
             rpart[2 * u + h] += kv;
             cpart += kv;
@@ -341,7 +340,7 @@ __global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
     }
   }
   if (GRAD) {
-    if (big) atomicOr(g.big, 1u);
+    x3_report(top, g.word);
     for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(g.dgamma, -gsum);
   }
@@ -478,7 +477,7 @@ static int64_t rbf_rows_x3(int64_t N, int64_t bytes) {
   return ((N + nb - 1) / nb + 63) / 64 * 64;
 }
 
-struct RunIf {  // the SIMT kernels launched in this scope run when *flag != 0
+struct RunIf {  // the SIMT kernels launched in this scope run when *flag is refused
   skema_ctx* c;
   RunIf(skema_ctx* ctx, const uint32_t* flag) : c(ctx) { c->run_if = flag; }
   ~RunIf() { c->run_if = nullptr; }
@@ -497,8 +496,8 @@ static void launch_planes(skema_ctx* c, const float* pts, int64_t N, int64_t d, 
 }
 
 // The forward product on the tensor cores: kernel planes a block of rows at a
-// time, Y_w = K_w Omega~^T. Values that the planes cannot carry set the flag,
-// and the SIMT form behind it runs. False when the workspace is not to be had.
+// time, Y_w = K_w Omega~^T. When Omega~ is refused (x3.h), the SIMT form behind it
+// runs (K has ones on its diagonal). False when the workspace is not to be had.
 static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega, int64_t k,
                        float* Y) {
   if (rbf_pair_small(N, 0, k)) return false;
@@ -511,13 +510,14 @@ static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   __nv_bfloat16* Kp = reinterpret_cast<__nv_bfloat16*>(ws + b_o);
   float* part = reinterpret_cast<float*>(ws + b_o + b_k);
   uint32_t* flag = reinterpret_cast<uint32_t*>(ws + b_o + b_k + b_p);
+  const X3Words words{flag, nullptr};
   SKEMA_CUDA(cudaMemsetAsync(flag, 0, sizeof(uint32_t), c->stream));
   x3_row_planes(c, omega, N, k, N, Op, ldN, k * ldN, flag);
   for (int64_t r = 0; r < N; r += rb) {
     const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
     launch_planes(c, pts, N, d, gamma, r, wr, Kp, nrb * 64 * N, nullptr);
     x3_gemm(c, X3A{Kp, true, true, N, nrb, 0, 0}, X3B{Op, ldN, k * ldN}, wr, k, N,
-            tc::X3Out{Y + r * k, k, 1, 1.f, 0.f, nullptr, 0, 0, wr, k, k}, part, flag);
+            tc::X3Out{Y + r * k, k, 1, 1.f, 0.f, nullptr, 0, 0, wr, k, k}, part, words);
   }
   RunIf second(c, flag);
   rbf_fwd_plain(c, pts, N, d, gamma, omega, k, Y, std::max<int64_t>(1, (int64_t)(b_k / 4) / N),
@@ -526,16 +526,18 @@ static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
 }
 
 // The adjoint's sums on the tensor cores, a block of rows at a time: E_w = M_w o
-// K_w as planes with the sums, then E_w X and E_w^T X_w from the same planes. As for the forward, the SIMT form follows for
-// values that the planes cannot carry, over zeroed sums.
+// K_w as planes with the sums, then E_w X and E_w^T X_w from the same planes. As
+// for the forward, the SIMT form follows when X or a block's E is refused, over
+// zeroed sums.
 static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, float gamma, const float* omega, int64_t k,
                        const float* Ybar, float* dpts, double* dgamma) {
   if (rbf_pair_small(N, d, k)) return false;
   const int64_t ldN = (N + 7) / 8 * 8, rb = rbf_rows_x3(N, 6);
   const size_t b_x = up256(2 * (size_t)(3 * d * ldN)), b_e = up256(2 * (size_t)(3 * rb * N)),
                b_p = up256(std::max(x3_part_bytes(c), sizeof(float) * (size_t)kRbfPartFloats)),
-               b_v = up256(4 * (size_t)N), b_s = up256(4 * (size_t)(N * d));
-  char* ws = static_cast<char*>(try_workspace(c, b_x + b_e + b_p + 2 * b_v + b_s + 256));
+               b_v = up256(4 * (size_t)N), b_s = up256(4 * (size_t)(N * d)),
+               b_w = up256(4 * (size_t)(1 + (N + rb - 1) / rb));
+  char* ws = static_cast<char*>(try_workspace(c, b_x + b_e + b_p + 2 * b_v + b_s + b_w));
   if (!ws) return false;
   auto take = [&](size_t b) {
     char* q = ws;
@@ -548,19 +550,20 @@ static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   float* rs = reinterpret_cast<float*>(take(b_v));
   float* cs = reinterpret_cast<float*>(take(b_v));
   float* S = reinterpret_cast<float*>(take(b_s));
-  uint32_t* flag = reinterpret_cast<uint32_t*>(take(256));
-  // the sums and the flag behind them
-  SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + 256, c->stream));
+  uint32_t* flag = reinterpret_cast<uint32_t*>(take(b_w));  // X's and the call's word, then one per block
+  // the sums and the words behind them
+  SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + b_w, c->stream));
   SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
   x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, flag);
-  for (int64_t r = 0; r < N; r += rb) {
+  for (int64_t r = 0, i = 1; r < N; r += rb, ++i) {
     const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
-    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, flag};
+    const X3Words words{flag + i, flag};
+    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, flag + i};
     launch_planes(c, pts, N, d, gamma, r, wr, Ep, nrb * 64 * N, &g);
     x3_gemm(c, X3A{Ep, true, true, N, nrb, 0, 0}, X3B{Xp, ldN, d * ldN}, wr, d, N,
-            tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, flag);
+            tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, words);
     x3_gemm(c, X3A{Ep, true, false, N, nrb, 0, 0}, X3B{Xp + r, ldN, d * ldN}, N, d, wr,
-            tc::X3Out{S, d, 1, 1.f, 1.f, nullptr, 0, 0, N, d, d}, part, flag);
+            tc::X3Out{S, d, 1, 1.f, 1.f, nullptr, 0, 0, N, d, d}, part, words);
   }
   {
     RunIf second(c, flag);

@@ -386,7 +386,7 @@ __global__ void csr_gauss_scatter_kernel(const int64_t* __restrict__ rowptr,
 // columns, six each. The tile is turned in shared memory, so that Y (column
 // major) and T leave as lines of 32 rows. T goes out as the three BF16 planes
 // of the tensor-core product Z += Phi^T T (T32 null), or as FP32 columns of
-// ldt when a value left the planes' range (run again under *cond).
+// ldt when T is refused (x3.h; run again under *cond).
 // Bound by the gathered bytes, 4 (k + s) per nonzero out of L2: 100,000 x
 // 20,000 with 1e6 nonzeros at k = 81, s = 163 takes 178 us, 5.4 TB/s. With all
 // 244 columns in one pass of eight slots it took 338 (the loads of a group not
@@ -406,7 +406,7 @@ struct GaussGather {
   __nv_bfloat16* T;
   float* T32;
   int64_t ldt, pstride;
-  uint32_t* big;  // set when |T| >= 2^100 or infinite
+  uint32_t* word;  // T's magnitudes are noted here
 };
 // One row against NU x 32 columns of a map: acc[u] = sum_p a_p map(j_p, c0 +
 // lane + 32 u), cols columns left from c0 on. 32 entries are loaded at once,
@@ -462,14 +462,14 @@ __device__ __forceinline__ void gauss_tile(const GaussGather& g, int64_t r0, int
 }
 
 __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g, const uint32_t* __restrict__ cond) {
-  if (cond && *cond == 0) return;
+  if (cond && !x3_refused(*cond)) return;
   constexpr int CH = 192;  // columns per pass
   extern __shared__ float gg_tile[];  // CH x 33
   __shared__ int next;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * 32;
   const int nr = (int)min((int64_t)32, g.nrows - r0);
-  bool big = false;
+  uint32_t top = 0;
   // the columns of Omega, then those of Psi
   for (int64_t c = g.Y ? 0 : g.k; c < g.k + g.s;) {
     const bool om = c < g.k;
@@ -496,8 +496,7 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
       } else if (g.T32) {
         g.T32[(c0 + cl) * g.ldt + r0 + lane] = v;
       } else {
-        const uint32_t bits = __float_as_uint(v) & 0x7fffffffu;
-        big |= bits >= 0x71800000u && bits <= 0x7f800000u;
+        x3_note(top, v);
         __nv_bfloat16 h, m, l;
         tc::split3(v, h, m, l);
         __nv_bfloat16* tp = g.T + (c0 + cl) * g.ldt + r0 + lane;
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
     __syncthreads();
     c += cols;
   }
-  if (big) atomicOr(g.big, 1u);
+  if (g.word) x3_report(top, g.word);
 }
 
 // X^T(j, :) += w_i a_ij Upsilon(i, :) into a zeroed n x kp scratch (kp a
@@ -801,7 +800,7 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
     const int64_t wr = std::min(rb, nrows - r), ps = s * ldt;
     GaussGather q = g;
-    q.rowptr += r, q.nrows = wr, q.Y += r, q.T = Tp, q.ldt = ldt, q.pstride = ps, q.big = flags + i;
+    q.rowptr += r, q.nrows = wr, q.Y += r, q.T = Tp, q.ldt = ldt, q.pstride = ps, q.word = flags + i;
     {
       StageScope st(c, ST_OMEGA);
       gather(q, nullptr);
@@ -811,8 +810,8 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
     const float zb = i == 0 ? wn : 1.f;
     x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r, nullptr);
     x3_gemm(c, X3A{Tp, false, false, 0, 0, ldt, ps}, X3B{Fp, ldt, ps}, s, s, wr,
-            tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, flags + i);
-    q.Y = nullptr, q.T32 = T32;
+            tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, X3Words{flags + i, nullptr});
+    q.Y = nullptr, q.T32 = T32, q.word = nullptr;
     gather(q, flags + i);
     X3Plain3 z;
     z.n = 1;

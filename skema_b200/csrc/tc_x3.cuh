@@ -2,7 +2,8 @@
 //
 // An FP32 value is the sum of three BF16 values (8 + 8 + 8 significant bits):
 //   x0 = bf16(x), x1 = bf16(x - x0), x2 = bf16(x - x0 - x1),
-// exact up to 2^-24 |x|, over the whole FP32 exponent range. A product of two
+// exact up to 2^-24 |x| down to |x| = 2^-109 and to half of BF16's smallest step,
+// 2^-134, below (x3.h says what becomes of such values). A product of two
 // such sums keeps six of its nine BF16 products,
 //   a b = a0 b0 + (a0 b1 + a1 b0) + (a1 b1 + a0 b2 + a2 b0) + O(2^-24 |a b|),
 // each of which the tensor core forms exactly and adds in FP32. The split is
@@ -122,13 +123,16 @@ __device__ __forceinline__ void x3_store(const X3Out& o, int64_t row, int64_t co
 //              the output are the block's contiguous rows);
 // AMN = false: the same layout {64, M, 3 nrb}, read K-major (K runs along the
 //              contiguous rows), or any 3-D map {K, M, 3} with a_blk = 0.
-// *flag != 0: an operand is not representable (see x3.cu); nothing is written.
+// words: nothing is written when an operand is refused (x3.h).
 template <bool AMN>
 __global__ void __launch_bounds__(kX3Threads, 1)
     gemm_x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, X3Grid g, X3Out o,
-                   int a_blk, int nrb, float* __restrict__ part, const uint32_t* __restrict__ flag, int* err) {
+                   int a_blk, int nrb, float* __restrict__ part, X3Words words, int* err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  if (flag && *flag) return;
+  if (x3_skip(words)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && words.all) atomicOr(words.all, kX3Big);
+    return;
+  }
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t bplane = (uint32_t)g.nt * kX3BK * 2;
@@ -298,8 +302,8 @@ __global__ void __launch_bounds__(kX3Threads, 1)
 // adding them: COLS = 4, 60 -> 17 us for 97 tiles of 208 columns.
 template <int COLS>
 static __global__ void __launch_bounds__(256) x3_reduce_kernel(X3Grid g, X3Out o, int G, const float* __restrict__ part,
-                                                        const uint32_t* __restrict__ flag) {
-  if (flag && *flag) return;
+                                                        X3Words words) {
+  if (x3_skip(words)) return;
   const int64_t q = blockIdx.x;
   const int64_t kb = q * g.ksteps, ke = kb + g.ksteps;
   const int64_t T = (int64_t)(g.mtiles * g.ntiles - g.full) * g.ksteps;

@@ -27,15 +27,6 @@ namespace skema {
 
 namespace {
 
-// |x| at or above this (2^100) leaves the range in which planes and sums are
-// certain to stay finite (infinities included; a NaN is a NaN in its planes
-// too and passes): the block is then formed by x3_plain_kernel instead.
-constexpr uint32_t kBigBits = 0x71800000u;  // 2^100
-__device__ __forceinline__ bool too_big(float x) {
-  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
-  return b >= kBigBits && b <= 0x7f800000u;
-}
-
 __device__ __forceinline__ void store_planes8(const float* v, __nv_bfloat16* d, int64_t pstride) {
   __nv_bfloat162 q[3][4];
 #pragma unroll
@@ -52,7 +43,7 @@ __global__ void __launch_bounds__(256)
     x3_block_vec_kernel(const float* __restrict__ S, int64_t scs, int64_t rows, int64_t cols,
                         __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t* __restrict__ flag) {
   const int64_t total = nrb * 8 * cols;
-  bool big = false;
+  uint32_t top = 0;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     // 64-row block outermost, then columns, then the 8 groups of a line: a
     // warp's stores are 512 contiguous bytes per plane
@@ -68,10 +59,10 @@ __global__ void __launch_bounds__(256)
       for (int t = 0; t < 8; ++t) v[t] = (i + t < rows) ? sp[t] : 0.f;
     }
 #pragma unroll
-    for (int t = 0; t < 8; ++t) big |= too_big(v[t]);
+    for (int t = 0; t < 8; ++t) x3_note(top, v[t]);
     store_planes8(v, D + (rb * cols + j) * 64 + (w & 7) * 8, pstride);
   }
-  if (big) atomicOr(flag, 1u);
+  x3_report(top, flag);
 }
 
 // The same from any strides, by 64 x 32 tiles through shared memory.
@@ -82,7 +73,7 @@ __global__ void __launch_bounds__(256)
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t tj = (cols + 31) / 32;
   const bool rowfast = srs <= scs;
-  bool big = false;
+  uint32_t top = 0;
   for (int64_t t = blockIdx.x; t < nrb * tj; t += gridDim.x) {
     const int64_t rb = t / tj, j0 = (t - rb * tj) * 32;
 #pragma unroll
@@ -91,7 +82,7 @@ __global__ void __launch_bounds__(256)
       const int r = rowfast ? tx + 32 * (e >> 5) : e, j = rowfast ? (e & 31) : tx;
       const int64_t gi = rb * 64 + r, gj = j0 + j;
       const float v = (gi < rows && gj < cols) ? S[gi * srs + gj * scs] : 0.f;
-      big |= too_big(v);
+      x3_note(top, v);
       tile[j][r] = v;
     }
     __syncthreads();
@@ -104,7 +95,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
-  if (big) atomicOr(flag, 1u);
+  x3_report(top, flag);
 }
 
 // Map columns [0, cols) of up to two row-contiguous FP32 sources into one
@@ -118,7 +109,7 @@ __global__ void __launch_bounds__(256)
     x3_maps_kernel(X3Src a, X3Src b, int64_t cols, __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu,
                    int64_t W, int64_t nwin, int64_t j0, uint32_t* __restrict__ flag) {
   const int64_t c8 = ld / 8, total = (a.rows + b.rows) * c8;
-  bool big = false;
+  uint32_t top = 0;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = q / c8, j = (q - r * c8) * 8;
     const float* sp = (r < a.rows ? a.p + r * a.rs : b.p + (r - a.rows) * b.rs) + j;
@@ -137,17 +128,17 @@ __global__ void __launch_bounds__(256)
     }
     if (flag) {
 #pragma unroll
-      for (int t = 0; t < 8; ++t) big |= too_big(v[t]);
+      for (int t = 0; t < 8; ++t) x3_note(top, v[t]);
     }
     store_planes8(v, D + r * ld + j, pstride);
   }
-  if (big) atomicOr(flag, 1u);
+  if (flag) x3_report(top, flag);
 }
 
-// The products of X3Plain3 for the rare block that too_big() refuses (returns
-// at once otherwise), by 64 x 64 tiles.
+// The products of X3Plain3 for the rare block that is refused (returns at once
+// otherwise), by 64 x 64 tiles.
 __global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_t* __restrict__ flag) {
-  if (*flag == 0) return;
+  if (!x3_refused(*flag)) return;
   __shared__ float As[16][65], Bs[16][65];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   for (int w = 0; w < a.n; ++w) {
@@ -201,7 +192,7 @@ __global__ void __launch_bounds__(256)
                          int64_t j0, uint32_t* __restrict__ flag) {
   constexpr int NR = kTrRows / 8;  // rows per warp
   __shared__ float tile[32][kTrRows + 1];
-  bool big = false;
+  uint32_t top = 0;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t ti = (ld + kTrRows - 1) / kTrRows, tj = (cols + 31) / 32;
   for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
@@ -218,7 +209,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
       if (nu != 1.f) v[q] *= __shfl_sync(0xffffffffu, w, q);
-      big |= too_big(v[q]);
+      x3_note(top, v[q]);
       tile[tx][ty + 8 * q] = v[q];
     }
     __syncthreads();
@@ -234,7 +225,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
-  if (flag && big) atomicOr(flag, 1u);
+  if (flag) x3_report(top, flag);
 }
 
 int grid_1d(const skema_ctx* c, int64_t items, int per_sm) {
@@ -258,7 +249,7 @@ size_t x3_part_bytes(const skema_ctx* c) {
 }
 
 void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int64_t K, const tc::X3Out& o, float* part,
-             const uint32_t* flag) {
+             X3Words words) {
   if (M <= 0 || N <= 0 || K <= 0) return;
   tc::X3Grid g;
   g.mtiles = (int)((M + tc::BM - 1) / tc::BM);
@@ -282,15 +273,15 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   const CUtensorMap tb = tmap_planes_k(b.p, K, N, b.ld, b.pstride, (uint32_t)g.nt, 3);
   auto kern = a.mn ? tc::gemm_x3_kernel<true> : tc::gemm_x3_kernel<false>;
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kX3Smem));
-  kern<<<G, tc::kX3Threads, kX3Smem, c->stream>>>(ta, tb, g, o, a.blocked ? 1 : 0, (int)a.nrb, part, flag, c->dev_err);
+  kern<<<G, tc::kX3Threads, kX3Smem, c->stream>>>(ta, tb, g, o, a.blocked ? 1 : 0, (int)a.nrb, part, words, c->dev_err);
   SKEMA_LAUNCHED(c);
   c->dev_err_armed = true;
   const int rem = (int)(tiles - g.full);
   if (rem > 0) {
     if (rem * (g.nt / 8) >= 2 * c->sm_count)
-      tc::x3_reduce_kernel<4><<<dim3(rem, g.nt / 8), 256, 0, c->stream>>>(g, o, G, part, flag);
+      tc::x3_reduce_kernel<4><<<dim3(rem, g.nt / 8), 256, 0, c->stream>>>(g, o, G, part, words);
     else
-      tc::x3_reduce_kernel<1><<<dim3(rem, g.nt / 2), 256, 0, c->stream>>>(g, o, G, part, flag);
+      tc::x3_reduce_kernel<1><<<dim3(rem, g.nt / 2), 256, 0, c->stream>>>(g, o, G, part, words);
     SKEMA_LAUNCHED(c);
   }
 }
@@ -379,6 +370,7 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     const int64_t wr = std::min(rb, nrows - r), R0 = row0 + r;
     const int64_t nrb = (wr + 63) / 64, ldw = pad8(wr), ps = nrb * 64 * n;
     uint32_t* flag = flags ? flags + i : nullptr;
+    const X3Words words{flag, nullptr};
     const Mat Aw{in.A.p ? in.A.p + r * in.A.rs : nullptr, in.A.rs, in.A.cs};
     {
       StageScope st(c, ST_WINDOW);
@@ -397,18 +389,18 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     {
       StageScope st(c, s > 0 ? ST_FUSED : ST_OMEGA);
       x3_gemm(c, an, X3B{op, ldn, (k + s) * ldn}, wr, k + s, n,
-              tc::X3Out{c->Y + R0, 1, c->m, eta, ybeta, Tp, ldw, s * ldw, wr, k, k + s}, part, flag);
+              tc::X3Out{c->Y + R0, 1, c->m, eta, ybeta, Tp, ldw, s * ldw, wr, k, k + s}, part, words);
     }
     if (s > 0) {
       const float xb = i == 0 ? xbeta : 1.f;
       {
         StageScope st(c, ST_UPSILON);
         x3_gemm(c, at, X3B{uf, ldw, (k + s) * ldw}, n, k, wr, tc::X3Out{c->X, 1, n, eta, xb, nullptr, 0, 0, n, k, k},
-                part, flag);
+                part, words);
       }
       StageScope st(c, ST_PHI);
       x3_gemm(c, X3A{Tp, false, false, 0, 0, ldw, s * ldw}, X3B{uf + k * ldw, ldw, (k + s) * ldw}, s, s, wr,
-              tc::X3Out{c->Z, 1, s, eta, xb, nullptr, 0, 0, s, s, s}, part, flag);
+              tc::X3Out{c->Z, 1, s, eta, xb, nullptr, 0, 0, s, s, s}, part, words);
     }
     if (flag) {
       const int64_t j0 = r;

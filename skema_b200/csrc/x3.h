@@ -9,8 +9,39 @@
 
 namespace skema {
 
+// The range of the planes. The low planes of a value below about 2^-109 reach
+// BF16's smallest step (2^-133) and lose bits, so what counts is the largest
+// magnitude of a block of values: from 2^-90 on, what the smaller ones lose is
+// below 2^-44 of it. At 2^100 and above, planes and sums may leave FP32's range.
+// A kernel that makes planes notes in a device word which kinds it met; a block
+// that is all tiny, or holds a big value, is refused, and FP32 arithmetic forms
+// its products. A NaN is a NaN in its planes too and counts for nothing here.
+constexpr uint32_t kX3Normal = 1, kX3Tiny = 2, kX3Big = 4;
+constexpr uint32_t kX3SmallBits = (uint32_t)(127 - 90) << 23, kX3BigBits = (uint32_t)(127 + 100) << 23;
+__host__ __device__ __forceinline__ bool x3_refused(uint32_t w) {
+  return (w & kX3Big) || (w & (kX3Normal | kX3Tiny)) == kX3Tiny;
+}
+// m: the largest of this thread's magnitudes, as bits
+__device__ __forceinline__ void x3_note(uint32_t& m, float x) {
+  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+  m = max(m, b <= 0x7f800000u ? b : 0u);
+}
+// Notes the block's largest magnitude in *word; called by all its threads.
+__device__ __forceinline__ void x3_report(uint32_t m, uint32_t* word) {
+  uint32_t kind = 0;
+  if (__syncthreads_or(m >= kX3BigBits))
+    kind = kX3Big;
+  else if (__syncthreads_or(m >= kX3SmallBits))
+    kind = kX3Normal;
+  else if (__syncthreads_or(m > 0))
+    kind = kX3Tiny;
+  // most blocks find their kind noted
+  if (threadIdx.x == 0 && kind && !(*(volatile uint32_t*)word & kind)) atomicOr(word, kind);
+}
+
 namespace tc {
-// The same for two values, whose BF16 parts lie side by side.
+// Two values as sums of three BF16 values each (split3), whose parts lie side
+// by side.
 __device__ __forceinline__ void split3x2(float x, float y, __nv_bfloat162& h, __nv_bfloat162& m, __nv_bfloat162& l) {
   h = __floats2bfloat162_rn(x, y);
   const float rx = x - __low2float(h), ry = y - __high2float(h);
@@ -55,19 +86,26 @@ struct X3B {
 };
 // Room for the parts of cut tiles.
 size_t x3_part_bytes(const skema_ctx* c);
-// acc(i, j) = sum_kk A(i, kk) B(j, kk) into o; nothing when *flag (may be
-// null) is set.
+// The words that decide a product: word, of its own operands (null: no check),
+// and all (may be null), of the call, which a refused word marks as refused.
+struct X3Words {
+  const uint32_t* word;
+  uint32_t* all;
+};
+__device__ __forceinline__ bool x3_skip(const X3Words& w) {
+  return (w.word && x3_refused(*w.word)) || (w.all && x3_refused(*w.all));
+}
+// acc(i, j) = sum_kk A(i, kk) B(j, kk) into o; nothing when refused.
 void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int64_t K, const tc::X3Out& o, float* part,
-             const uint32_t* flag);
+             X3Words words);
 // A strided FP32 block into row-blocked planes (zero rows up to a multiple of
-// 64); sets *flag when a value is out of the planes' range.
+// 64); its magnitudes are noted in *flag, here and below (null: not).
 void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
                      uint32_t* flag);
 
 // K-major planes of a row-major source's transpose: row i of S (rows x cols,
 // rs apart), scaled by nu^(nwin - 1 - (j0 + i) / W), is K index i; D holds
-// cols rows of ld (a multiple of 8) per plane. *flag (may be null) is set when
-// a value is out of the planes' range.
+// cols rows of ld (a multiple of 8) per plane.
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
                           int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag);
 // K-major planes of a row-major source (rows x cols, rs apart): D holds rows of
@@ -76,7 +114,7 @@ void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64
                    int64_t pstride, uint32_t* flag);
 
 // Up to three FP32 products C = alpha A B + beta C by plain FMA, run when
-// *flag is set: the form of a block whose values the planes cannot carry.
+// *flag is refused: the form of a block whose values the planes cannot carry.
 // A(i, kk) is scaled by nu^(nwin - 1 - (j0 + kk) / W).
 struct X3Plain {
   const float* A;
