@@ -47,9 +47,8 @@ struct Map {
   // Gauss: FP32 values; logical (r, c) at f32[r*rs + c*cs].
   float* f32 = nullptr;
   int64_t rs = 0, cs = 0;
-  // Imported values of 2^100 or more, or infinite: the products of this map
-  // stay on the SIMT kernels.
-  bool big = false;
+  // Gauss: no value's magnitude is above this (an imported NaN left out).
+  float amax = 0.f;
   // Gauss, tensor-core forms: logical rows in row-major BF16 / FP8 copies.
   void* lowp = nullptr;
   // SparseSign: stored rows, zeta packed entries each: column | sign << 31.

@@ -123,6 +123,7 @@ void map_generate(skema_ctx* c, Map& mp, int precision) {
   (void)precision;
   if (mp.kind == SKEMA_MAP_GAUSS) {
     mp.maxval = std::sqrt(2.0 * std::log((double)((uint64_t)mp.nrow * (uint64_t)mp.ncol)));
+    mp.amax = (float)mp.maxval;
     gauss_layout(c, mp);
     SKEMA_CUDA(cudaMalloc(&mp.f32, sizeof(float) * (size_t)(mp.lrows * mp.lcols)));
     const int threads = 256;
@@ -236,7 +237,9 @@ void map_import(skema_ctx* c, Map& mp, const double* values, const int32_t* indi
     gauss_import_kernel<<<grid_for(total, threads, c->sm_count), threads, 0, c->stream>>>(
         mp.f32, d, mp.lrows, mp.lcols, mp.rs, mp.cs, mp.nrow, mp.transposed ? 1 : 0);
     SKEMA_LAUNCHED(c);
-    mp.big = std::any_of(values, values + total, [](double v) { return std::fabs(v) >= 0x1p100; });
+    double top = 0.0;
+    for (int64_t q = 0; q < total; ++q) top = std::max(top, std::fabs(values[q]));  // a NaN compares false
+    mp.amax = (float)top;
     SKEMA_CUDA(cudaStreamSynchronize(c->stream));
     return;
   }

@@ -159,6 +159,7 @@ struct RbfGrad {
   double* dgamma;
   float* rsum;
   float* csum;
+  uint32_t big;  // x3_report's
   uint32_t* word;
 };
 // s += (a + b)^2, and s += a b, on two packed FP32 values, each rounded as FADD
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
     }
   }
   if (GRAD) {
-    x3_report(top, g.word);
+    x3_report(top, g.big, g.word);
     for (int o = 16; o > 0; o >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(g.dgamma, -gsum);
   }
@@ -512,7 +513,8 @@ static bool rbf_fwd_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   uint32_t* flag = reinterpret_cast<uint32_t*>(ws + b_o + b_k + b_p);
   const X3Words words{flag, nullptr};
   SKEMA_CUDA(cudaMemsetAsync(flag, 0, sizeof(uint32_t), c->stream));
-  x3_row_planes(c, omega, N, k, N, Op, ldN, k * ldN, flag);
+  // sums of N products with values of K, at most one
+  x3_row_planes(c, omega, N, k, N, Op, ldN, k * ldN, std::min(100, 126 - x3_log2(N)), flag);
   for (int64_t r = 0; r < N; r += rb) {
     const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
     launch_planes(c, pts, N, d, gamma, r, wr, Kp, nrb * 64 * N, nullptr);
@@ -554,11 +556,12 @@ static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   // the sums and the words behind them
   SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + b_w, c->stream));
   SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
-  x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, flag);
+  const int top = (126 - x3_log2(N)) / 2;  // of E and of X: sums of N products
+  x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, top, flag);
   for (int64_t r = 0, i = 1; r < N; r += rb, ++i) {
     const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
     const X3Words words{flag + i, flag};
-    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, flag + i};
+    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, x3_bits(top), flag + i};
     launch_planes(c, pts, N, d, gamma, r, wr, Ep, nrb * 64 * N, &g);
     x3_gemm(c, X3A{Ep, true, true, N, nrb, 0, 0}, X3B{Xp, ldN, d * ldN}, wr, d, N,
             tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, words);

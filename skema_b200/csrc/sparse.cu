@@ -406,6 +406,7 @@ struct GaussGather {
   __nv_bfloat16* T;
   float* T32;
   int64_t ldt, pstride;
+  uint32_t big;    // x3_report's
   uint32_t* word;  // T's magnitudes are noted here
 };
 // One row against NU x 32 columns of a map: acc[u] = sum_p a_p map(j_p, c0 +
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
     __syncthreads();
     c += cols;
   }
-  if (g.word) x3_report(top, g.word);
+  if (g.word) x3_report(top, g.big, g.word);
 }
 
 // X^T(j, :) += w_i a_ij Upsilon(i, :) into a zeroed n x kp scratch (kp a
@@ -758,7 +759,7 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w, nwin = (nrows + W - 1) / W;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   GaussGather g{rowptr, col, val, col_offset, nrows, n, c->omg.f32, c->psi.f32, k, s, c->Y + row0, c->m,
-                eta, ybeta, nullptr, nullptr, 0, 0, nullptr};
+                eta, ybeta, nullptr, nullptr, 0, 0, 0, nullptr};
   const size_t smem = sizeof(float) * 192 * 33;
   auto gather = [&](const GaussGather& q, const uint32_t* cond) {
     csr_gauss_gather_kernel<<<(unsigned)((q.nrows + 31) / 32), 256, smem, c->stream>>>(q, cond);
@@ -770,11 +771,16 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
     y_rows_mark(c, row0, row0 + nrows);
     return true;
   }
-  if (c->phi.big) return false;  // an imported map beyond the planes' range
+  // imported maps beyond the range of the planes, or of a weight on top
+  const int lw = nu > 1.f ? (int)std::ceil(std::log2((double)nu) * (double)(nwin - 1)) : 0;
+  if (!x3_carries(c->phi) || !x3_carries(c->ups) || x3_exp(c->ups) + lw > 126) return false;
   const int64_t kp = (k + 3) / 4 * 4;
   // rows per block: T, its FP32 form and Phi's planes within 512 MB
   const int64_t rb = std::min<int64_t>(nrows, std::max<int64_t>(32, ((int64_t)512 << 20) / (16 * s) / 32 * 32));
   const int64_t ldt = (rb + 7) / 8 * 8, nblk = (nrows + rb - 1) / rb;
+  // T's bound: sums over a block's rows with Phi's weights stay below 2^126
+  const int top = std::min(100, 126 - x3_log2(rb) - x3_exp(c->phi) - lw);
+  if (top < 40) return false;
   const size_t b_xt = up(sizeof(float) * (size_t)(n * kp)), b_pl = up(sizeof(__nv_bfloat16) * (size_t)(3 * s * ldt)),
                b_t32 = up(sizeof(float) * (size_t)(s * ldt)), b_flag = up(sizeof(uint32_t) * (size_t)nblk);
   char* ws = static_cast<char*>(try_workspace(c, b_xt + 2 * b_pl + b_t32 + x3_part_bytes(c) + b_flag));
@@ -800,7 +806,8 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
     const int64_t wr = std::min(rb, nrows - r), ps = s * ldt;
     GaussGather q = g;
-    q.rowptr += r, q.nrows = wr, q.Y += r, q.T = Tp, q.ldt = ldt, q.pstride = ps, q.word = flags + i;
+    q.rowptr += r, q.nrows = wr, q.Y += r, q.T = Tp, q.ldt = ldt, q.pstride = ps;
+    q.big = x3_bits(top), q.word = flags + i;
     {
       StageScope st(c, ST_OMEGA);
       gather(q, nullptr);
@@ -808,7 +815,7 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
     StageScope st(c, ST_PHI);
     const float* F = c->phi.f32 + (row0 + r) * s;
     const float zb = i == 0 ? wn : 1.f;
-    x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r, nullptr);
+    x3_transposed_planes(c, F, s, wr, s, Fp, ldt, ps, nu, W, nwin, r, 0, nullptr);
     x3_gemm(c, X3A{Tp, false, false, 0, 0, ldt, ps}, X3B{Fp, ldt, ps}, s, s, wr,
             tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, X3Words{flags + i, nullptr});
     q.Y = nullptr, q.T32 = T32, q.word = nullptr;

@@ -41,7 +41,8 @@ __device__ __forceinline__ void store_planes8(const float* v, __nv_bfloat16* d, 
 // bound.
 __global__ void __launch_bounds__(256)
     x3_block_vec_kernel(const float* __restrict__ S, int64_t scs, int64_t rows, int64_t cols,
-                        __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t* __restrict__ flag) {
+                        __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t big,
+                        uint32_t* __restrict__ flag) {
   const int64_t total = nrb * 8 * cols;
   uint32_t top = 0;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -62,13 +63,14 @@ __global__ void __launch_bounds__(256)
     for (int t = 0; t < 8; ++t) x3_note(top, v[t]);
     store_planes8(v, D + (rb * cols + j) * 64 + (w & 7) * 8, pstride);
   }
-  x3_report(top, flag);
+  x3_report(top, big, flag);
 }
 
 // The same from any strides, by 64 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256)
     x3_block_tiled_kernel(const float* __restrict__ S, int64_t srs, int64_t scs, int64_t rows, int64_t cols,
-                          __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t* __restrict__ flag) {
+                          __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t big,
+                          uint32_t* __restrict__ flag) {
   __shared__ float tile[32][65];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t tj = (cols + 31) / 32;
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
-  x3_report(top, flag);
+  x3_report(top, big, flag);
 }
 
 // Map columns [0, cols) of up to two row-contiguous FP32 sources into one
@@ -107,7 +109,7 @@ struct X3Src {
 };
 __global__ void __launch_bounds__(256)
     x3_maps_kernel(X3Src a, X3Src b, int64_t cols, __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu,
-                   int64_t W, int64_t nwin, int64_t j0, uint32_t* __restrict__ flag) {
+                   int64_t W, int64_t nwin, int64_t j0, uint32_t big, uint32_t* __restrict__ flag) {
   const int64_t c8 = ld / 8, total = (a.rows + b.rows) * c8;
   uint32_t top = 0;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(256)
     }
     store_planes8(v, D + r * ld + j, pstride);
   }
-  if (flag) x3_report(top, flag);
+  if (flag) x3_report(top, big, flag);
 }
 
 // The products of X3Plain3 for the rare block that is refused (returns at once
@@ -189,7 +191,7 @@ constexpr int kTrRows = 128;
 __global__ void __launch_bounds__(256)
     x3_transposed_kernel(const float* __restrict__ S, int64_t rs, int64_t rows, int64_t cols,
                          __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin,
-                         int64_t j0, uint32_t* __restrict__ flag) {
+                         int64_t j0, uint32_t big, uint32_t* __restrict__ flag) {
   constexpr int NR = kTrRows / 8;  // rows per warp
   __shared__ float tile[32][kTrRows + 1];
   uint32_t top = 0;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
-  if (flag) x3_report(top, flag);
+  if (flag) x3_report(top, big, flag);
 }
 
 int grid_1d(const skema_ctx* c, int64_t items, int per_sm) {
@@ -286,30 +288,31 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   }
 }
 
-void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
+void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride, int top,
                      uint32_t* flag) {
   const int64_t nrb = (rows + 63) / 64;
   if (src.rs == 1 && src.cs % 4 == 0 && reinterpret_cast<uintptr_t>(src.p) % 16 == 0)
     x3_block_vec_kernel<<<grid_1d(c, nrb * 8 * cols, 16), 256, 0, c->stream>>>(src.p, src.cs, rows, cols, D, nrb,
-                                                                               pstride, flag);
+                                                                               pstride, x3_bits(top), flag);
   else
     x3_block_tiled_kernel<<<grid_1d(c, nrb * ((cols + 31) / 32) * 256, 16), 256, 0, c->stream>>>(
-        src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, flag);
+        src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, x3_bits(top), flag);
   SKEMA_LAUNCHED(c);
 }
 
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
-                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag) {
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, int top,
+                          uint32_t* flag) {
   const int64_t tiles = ((ld + kTrRows - 1) / kTrRows) * ((cols + 31) / 32);
   x3_transposed_kernel<<<grid_1d(c, tiles * 256, 16), 256, 0, c->stream>>>(S, rs, rows, cols, D, ld, pstride, nu, W,
-                                                                          nwin, j0, flag);
+                                                                          nwin, j0, x3_bits(top), flag);
   SKEMA_LAUNCHED(c);
 }
 
 void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t ld,
-                   int64_t pstride, uint32_t* flag) {
+                   int64_t pstride, int top, uint32_t* flag) {
   x3_maps_kernel<<<grid_1d(c, rows * ld / 8, 16), 256, 0, c->stream>>>(X3Src{S, rs, rows}, X3Src{S, rs, 0}, cols, D, ld,
-                                                                      pstride, 1.f, 1, 1, 0, flag);
+                                                                      pstride, 1.f, 1, 1, 0, x3_bits(top), flag);
   SKEMA_LAUNCHED(c);
 }
 
@@ -318,8 +321,22 @@ void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag) {
   SKEMA_LAUNCHED(c);
 }
 
-// nrows <= wsrows, which sizes the blocks and the workspace.
-static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows, int64_t wsrows) {
+// The exponent of the bound on A's values for sums over n columns and up to
+// `rows` rows of nwin windows: T = A Psi, and the three sketches' sums over the
+// block with the window weights (of nu > 1: 2^40 at most) in the maps, stay below
+// 2^126.
+static int x3_top(const skema_ctx* c, int64_t rows, int64_t nwin) {
+  const int ln = x3_log2(c->n), lr = x3_log2(rows);
+  int top = std::min(100, 126 - ln - x3_exp(c->omg));
+  if (c->spd) return top;
+  const double nu = c->p.sketch_nu;
+  const int lw = nu > 1.0 ? (int)std::ceil(std::log2(nu) * (double)(nwin - 1)) : 0;
+  const int t = ln + x3_exp(c->psi);
+  return std::min({top, 126 - t, 126 - lr - x3_exp(c->ups) - lw, 126 - t - lr - x3_exp(c->phi) - lw});
+}
+
+// nrows <= wsrows, which sizes the blocks and the workspace. top: x3_top.
+static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows, int64_t wsrows, int top) {
   const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w;
   const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
   const int64_t ldn = pad8(n);
@@ -363,7 +380,7 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     StageScope st(c, ST_WINDOW);
     const X3Src so{c->omg.f32, c->omg.rs, k}, sp{c->psi.f32, c->psi.rs, s};
     x3_maps_kernel<<<grid_1d(c, (k + s) * ldn / 8, 16), 256, 0, c->stream>>>(so, sp, n, op, ldn, (k + s) * ldn, 1.f, 1,
-                                                                            1, 0, nullptr);
+                                                                            1, 0, 0, nullptr);
     SKEMA_LAUNCHED(c);
   }
   for (int64_t r = 0, i = 0; r < nrows; r += rb, ++i) {
@@ -375,13 +392,13 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     {
       StageScope st(c, ST_WINDOW);
       if (in.A.p)
-        x3_block_planes(c, Aw, wr, n, Ap, ps, flag);
+        x3_block_planes(c, Aw, wr, n, Ap, ps, top, flag);
       else
         in.fill(R0, wr, Ap, ps);
       if (s > 0) {
         const X3Src su{c->ups.f32 + R0, c->ups.rs, k}, sf{c->phi.f32 + R0, c->phi.rs, s};  // cs = 1
         x3_maps_kernel<<<grid_1d(c, (k + s) * ldw / 8, 16), 256, 0, c->stream>>>(su, sf, wr, uf, ldw, (k + s) * ldw, nu,
-                                                                                W, nwin, r, nullptr);
+                                                                                W, nwin, r, 0, nullptr);
         SKEMA_LAUNCHED(c);
       }
     }
@@ -434,15 +451,19 @@ bool x3_update(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nrows) {
   const float nu = (float)c->p.sketch_nu;
   if (nrows <= 0 || !(nu > 0.f)) return false;
   for (const Map* mp : {&c->ups, &c->omg, &c->phi, &c->psi})
-    if (mp->big) return false;
+    if (!x3_carries(*mp)) return false;
   // below this the launches and conversions cost more than the products
   if ((double)nrows * (double)c->n * (double)(2 * c->k + (c->spd ? 0 : c->s)) < 2e7) return false;
-  const int64_t W = c->w, step = std::min((nrows + W - 1) / W, weight_windows(nu)) * W;
+  const int64_t W = c->w, nwin = std::min((nrows + W - 1) / W, weight_windows(nu)), step = nwin * W;
+  // maps so large that ordinary values (2^40) would be refused; kernel values are
+  // at most one
+  const int top = x3_top(c, std::min(step, nrows), nwin);
+  if (top < (in.A.p ? 40 : 1)) return false;
   for (int64_t r = 0; r < nrows; r += step) {
     X3Input part = in;
     if (part.A.p) part.A.p += r * part.A.rs;
     // false at r = 0 only: every run asks for the same workspace
-    if (!x3_windows(c, part, row0 + r, std::min(step, nrows - r), std::min(step, nrows))) return false;
+    if (!x3_windows(c, part, row0 + r, std::min(step, nrows - r), std::min(step, nrows), top)) return false;
   }
   return true;
 }

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <functional>
 
 #include "internal.h"
@@ -12,12 +14,28 @@ namespace skema {
 // The range of the planes. The low planes of a value below about 2^-109 reach
 // BF16's smallest step (2^-133) and lose bits, so what counts is the largest
 // magnitude of a block of values: from 2^-90 on, what the smaller ones lose is
-// below 2^-44 of it. At 2^100 and above, planes and sums may leave FP32's range.
+// below 2^-44 of it. Upwards, what counts is that the sums stay within FP32's
+// range: an infinity, or one in a plane, turns into a NaN where FP32 arithmetic
+// has an infinity. The bound, 2^100 at most, follows from the length of the sums
+// and the other operand's largest value (x3_top).
 // A kernel that makes planes notes in a device word which kinds it met; a block
-// that is all tiny, or holds a big value, is refused, and FP32 arithmetic forms
-// its products. A NaN is a NaN in its planes too and counts for nothing here.
+// that is all tiny, or holds a value from the bound on, is refused, and FP32
+// arithmetic forms its products. A NaN is a NaN in its planes too and counts for
+// nothing here.
 constexpr uint32_t kX3Normal = 1, kX3Tiny = 2, kX3Big = 4;
-constexpr uint32_t kX3SmallBits = (uint32_t)(127 - 90) << 23, kX3BigBits = (uint32_t)(127 + 100) << 23;
+constexpr uint32_t kX3SmallBits = (uint32_t)(127 - 90) << 23;
+inline uint32_t x3_bits(int e) { return (uint32_t)(127 + e) << 23; }  // 2^e
+// Least e with 2^e >= n
+inline int x3_log2(int64_t n) {
+  int e = 0;
+  while (((int64_t)1 << e) < n) ++e;
+  return e;
+}
+// A bound 2^e on a map's magnitudes, and whether planes carry the map: its
+// largest value is finite, and far enough up that T = A Psi is no smaller than
+// 2^-102 where A reaches 2^-90.
+inline int x3_exp(const Map& mp) { return mp.amax > 0.f ? std::max(-12, std::ilogb(mp.amax) + 1) : -12; }
+inline bool x3_carries(const Map& mp) { return mp.amax == 0.f || (mp.amax >= 0x1p-12f && mp.amax <= 0x1p100f); }
 __host__ __device__ __forceinline__ bool x3_refused(uint32_t w) {
   return (w & kX3Big) || (w & (kX3Normal | kX3Tiny)) == kX3Tiny;
 }
@@ -26,10 +44,11 @@ __device__ __forceinline__ void x3_note(uint32_t& m, float x) {
   const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
   m = max(m, b <= 0x7f800000u ? b : 0u);
 }
-// Notes the block's largest magnitude in *word; called by all its threads.
-__device__ __forceinline__ void x3_report(uint32_t m, uint32_t* word) {
+// Notes the block's largest magnitude in *word, big from the bits `big` on;
+// called by all its threads.
+__device__ __forceinline__ void x3_report(uint32_t m, uint32_t big, uint32_t* word) {
   uint32_t kind = 0;
-  if (__syncthreads_or(m >= kX3BigBits))
+  if (__syncthreads_or(m >= big))
     kind = kX3Big;
   else if (__syncthreads_or(m >= kX3SmallBits))
     kind = kX3Normal;
@@ -99,19 +118,21 @@ __device__ __forceinline__ bool x3_skip(const X3Words& w) {
 void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int64_t K, const tc::X3Out& o, float* part,
              X3Words words);
 // A strided FP32 block into row-blocked planes (zero rows up to a multiple of
-// 64); its magnitudes are noted in *flag, here and below (null: not).
-void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride,
+// 64); its magnitudes are noted in *flag, 2^top and above as big, here and below
+// (null: not).
+void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride, int top,
                      uint32_t* flag);
 
 // K-major planes of a row-major source's transpose: row i of S (rows x cols,
 // rs apart), scaled by nu^(nwin - 1 - (j0 + i) / W), is K index i; D holds
 // cols rows of ld (a multiple of 8) per plane.
 void x3_transposed_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D,
-                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, uint32_t* flag);
+                          int64_t ld, int64_t pstride, float nu, int64_t W, int64_t nwin, int64_t j0, int top,
+                          uint32_t* flag);
 // K-major planes of a row-major source (rows x cols, rs apart): D holds rows of
 // ld (a multiple of 8) per plane.
 void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t ld,
-                   int64_t pstride, uint32_t* flag);
+                   int64_t pstride, int top, uint32_t* flag);
 
 // Up to three FP32 products C = alpha A B + beta C by plain FMA, run when
 // *flag is refused: the form of a block whose values the planes cannot carry.
