@@ -408,6 +408,9 @@ struct GaussGather {
   int64_t ldt, pstride;
   uint32_t big;    // x3_report's
   uint32_t* word;  // T's magnitudes are noted here
+  float* scale;    // nscale values to be scaled by `by`: Z before a split product
+  int64_t nscale;
+  float by;
 };
 // One row against NU x 32 columns of a map: acc[u] = sum_p a_p map(j_p, c0 +
 // lane + 32 u), cols columns left from c0 on. 32 entries are loaded at once,
@@ -470,6 +473,8 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * 32;
   const int nr = (int)min((int64_t)32, g.nrows - r0);
+  for (int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x; q < g.nscale; q += (int64_t)gridDim.x * 256)
+    g.scale[q] = g.by == 0.f ? 0.f : g.by * g.scale[q];
   uint32_t top = 0;
   // the columns of Omega, then those of Psi
   for (int64_t c = g.Y ? 0 : g.k; c < g.k + g.s;) {
@@ -759,7 +764,7 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w, nwin = (nrows + W - 1) / W;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   GaussGather g{rowptr, col, val, col_offset, nrows, n, c->omg.f32, c->psi.f32, k, s, c->Y + row0, c->m,
-                eta, ybeta, nullptr, nullptr, 0, 0, 0, nullptr};
+                eta, ybeta, nullptr, nullptr, 0, 0, 0, nullptr, nullptr, 0, 0.f};
   const size_t smem = sizeof(float) * 192 * 33;
   auto gather = [&](const GaussGather& q, const uint32_t* cond) {
     csr_gauss_gather_kernel<<<(unsigned)((q.nrows + 31) / 32), 256, smem, c->stream>>>(q, cond);
@@ -819,10 +824,12 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
     x3_gemm(c, X3A{Tp, false, false, 0, 0, ldt, ps}, X3B{Fp, ldt, ps}, s, s, wr,
             tc::X3Out{c->Z, 1, s, eta, zb, nullptr, 0, 0, s, s, s}, part, X3Words{flags + i, nullptr});
     q.Y = nullptr, q.T32 = T32, q.word = nullptr;
+    q.scale = c->Z, q.nscale = s * s, q.by = zb;
     gather(q, flags + i);
-    X3Plain3 z;
+    X3Plain3 z{};
     z.n = 1;
-    z.g[0] = X3Plain{F, 1, s, T32, 1, ldt, c->Z, s, 1, s, s, wr, eta, zb, nu, W, nwin, r};
+    z.g[0] = X3Plain{nullptr, 0, 0, Fp, ldt, ps, T32, 1, ldt, c->Z, s, 1, s, s, wr, eta, 1.f,
+                     x3_plain_split(c, s, wr)};
     x3_plain(c, z, flags + i);
   }
   y_rows_mark(c, row0, row0 + nrows);

@@ -138,46 +138,121 @@ __global__ void __launch_bounds__(256)
 }
 
 // The products of X3Plain3 for the rare block that is refused (returns at once
-// otherwise), by 64 x 64 tiles.
-__global__ void __launch_bounds__(256) x3_plain_kernel(X3Plain3 a, const uint32_t* __restrict__ flag) {
+// otherwise): 128 x 128 tiles, 8 x 8 per thread, K steps of 16 through two
+// buffers, and K cut into g.split parts that are added to C with atomics when
+// the tiles alone would leave the chip idle. Bound by FP32 issue, as
+// sgemm_kernel is (36 TFLOP/s): 50,000 x 20,000 (k = 201, s = 403) with an
+// infinity in every block takes 59.5 ms in all, 12,000 x 5,000 (k = 81, s = 163)
+// 3.1; SIMT calls take 52.3 and 5.5 (64 x 64 tiles with 4 x 4 per thread and a pow
+// per weighted value took 174 and 7.8, 228 and 11.6 for nu = 0.95).
+constexpr int kPlBM = 128, kPlBK = 16, kPlLd = kPlBM + 4;
+// What a thread stages of one operand, element (r, k) with r < R: value q < 8 is
+// (r, k + 2 q) where the rows are the contiguous ones, else (r + 16 q, k).
+struct PlainSrc {
+  const float* p;
+  const __nv_bfloat16* pl;  // or the sum of three planes, ps apart, k along the rows
+  int64_t ps, dq, adv;      // from value to value, from K step to K step
+  int r, k, left, R;        // in the tile; K left from this thread's k on; rows of the tile
+  bool rfast;
+  __device__ __forceinline__ void init(const float* P, int64_t rs, int64_t ks, const __nv_bfloat16* Pl, int64_t ld,
+                                       int64_t planes, int64_t r0, int64_t rows, int64_t k0, int64_t k1) {
+    rfast = !Pl && rs <= ks;
+    r = rfast ? threadIdx.x & 127 : threadIdx.x >> 4;
+    k = rfast ? threadIdx.x >> 7 : threadIdx.x & 15;
+    R = (int)min((int64_t)kPlBM, rows - r0);
+    left = (int)min((int64_t)0x7fffffff, k1 - k0 - k);
+    p = P + (r0 + r) * rs + (k0 + k) * ks;
+    pl = Pl ? Pl + (r0 + r) * ld + k0 + k : nullptr;
+    ps = planes;
+    dq = Pl ? 16 * ld : rfast ? 2 * ks : 16 * rs;
+    adv = Pl ? kPlBK : kPlBK * ks;
+  }
+  __device__ __forceinline__ void load(float (&v)[8]) {
+    const int n = rfast ? (r < R ? (left + 1) / 2 : 0) : (left > 0 ? (R - r + 15) / 16 : 0);
+    if (pl) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const __nv_bfloat16* t = pl + q * dq;
+        v[q] = q < n ? (__bfloat162float(t[0]) + __bfloat162float(t[ps])) + __bfloat162float(t[2 * ps]) : 0.f;
+      }
+      pl += adv;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = q < n ? p[q * dq] : 0.f;
+      p += adv;
+    }
+    left -= kPlBK;
+  }
+  __device__ __forceinline__ void store(const float (&v)[8], float (*sm)[kPlLd]) const {
+    float* s = &sm[k][r];
+    const int d = rfast ? 2 * kPlLd : 16;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s[q * d] = v[q];
+  }
+};
+__global__ void __launch_bounds__(256, 1) x3_plain_kernel(X3Plain3 a, const uint32_t* __restrict__ flag) {
   if (!x3_refused(*flag)) return;
-  __shared__ float As[16][65], Bs[16][65];
+  __shared__ __align__(16) float As[2][kPlBK][kPlLd], Bs[2][kPlBK][kPlLd];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  for (int64_t q = blockIdx.x * 256 + threadIdx.x; q < a.nscale; q += (int64_t)gridDim.x * 256)
+    a.scale[q] = a.by == 0.f ? 0.f : a.by * a.scale[q];
+  int64_t t = blockIdx.x;  // tiles of all the products, one after another
   for (int w = 0; w < a.n; ++w) {
     const X3Plain& g = a.g[w];
-    const int64_t tm = (g.M + 63) / 64, tn = (g.N + 63) / 64;
-    for (int64_t t = blockIdx.x; t < tm * tn; t += gridDim.x) {
-      const int64_t m0 = (t / tn) * 64, n0 = (t % tn) * 64;
-      float acc[4][4] = {};
-      for (int64_t k0 = 0; k0 < g.K; k0 += 16) {
-        for (int q = threadIdx.x; q < 1024; q += 256) {
-          const int r = q & 63, kk = q >> 6;
-          const int64_t k = k0 + kk;
-          float av = (m0 + r < g.M && k < g.K) ? g.A[(m0 + r) * g.ars + k * g.acs] : 0.f;
-          if (g.nu != 1.f && k < g.K)
-            av *= (float)pow((double)g.nu, (double)(g.nwin - 1 - (g.j0 + k) / g.W));
-          As[kk][r] = av;
-          Bs[kk][r] = (n0 + r < g.N && k < g.K) ? g.B[k * g.brs + (n0 + r) * g.bcs] : 0.f;
+    const int64_t tn = (g.N + kPlBM - 1) / kPlBM, tiles = (g.M + kPlBM - 1) / kPlBM * tn;
+    const int64_t kc = (g.K + g.split - 1) / g.split;
+    for (; t < tiles * g.split; t += gridDim.x) {
+      const int64_t part = t / tiles, q = t - part * tiles;
+      const int64_t m0 = (q / tn) * kPlBM, n0 = (q % tn) * kPlBM, kb = part * kc, ke = min(g.K, kb + kc);
+      float acc[8][8] = {}, ra[8], rb[8];
+      PlainSrc sa, sb;
+      sa.init(g.A, g.ars, g.acs, g.Apl, g.ald, g.aps, m0, g.M, kb, ke);
+      sb.init(g.B, g.bcs, g.brs, nullptr, 0, 0, n0, g.N, kb, ke);
+      sa.load(ra);
+      sb.load(rb);
+      sa.store(ra, As[0]);
+      sb.store(rb, Bs[0]);
+      __syncthreads();
+      int buf = 0;
+      for (int64_t k0 = kb; k0 < ke; k0 += kPlBK, buf ^= 1) {
+        const bool more = k0 + kPlBK < ke;
+        if (more) {
+          sa.load(ra);
+          sb.load(rb);
         }
-        __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk)
+        for (int kk = 0; kk < kPlBK; ++kk) {
+          float x[8], y[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+          for (int h = 0; h < 2; ++h) {
+            *reinterpret_cast<float4*>(x + 4 * h) = *reinterpret_cast<const float4*>(&As[buf][kk][4 * tx + 64 * h]);
+            *reinterpret_cast<float4*>(y + 4 * h) = *reinterpret_cast<const float4*>(&Bs[buf][kk][4 * ty + 64 * h]);
+          }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(As[kk][ty + 16 * i], Bs[kk][tx + 16 * j], acc[i][j]);
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+        }
+        if (more) {  // the other buffer was read last a step ago, before the barrier
+          sa.store(ra, As[buf ^ 1]);
+          sb.store(rb, Bs[buf ^ 1]);
+        }
         __syncthreads();
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int64_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+        for (int j = 0; j < 8; ++j) {
+          const int64_t m = m0 + 4 * tx + 64 * (i >> 2) + (i & 3), n = n0 + 4 * ty + 64 * (j >> 2) + (j & 3);
           if (m >= g.M || n >= g.N) continue;
           float* p = g.C + m * g.crs + n * g.ccs;
-          *p = g.beta == 0.f ? g.alpha * acc[i][j] : fmaf(g.beta, *p, g.alpha * acc[i][j]);
+          if (g.split > 1)
+            atomicAdd(p, g.alpha * acc[i][j]);
+          else
+            *p = g.beta == 0.f ? g.alpha * acc[i][j] : fmaf(g.beta, *p, g.alpha * acc[i][j]);
         }
     }
+    t -= tiles * g.split;
   }
 }
 
@@ -316,8 +391,14 @@ void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64
   SKEMA_LAUNCHED(c);
 }
 
+// K parts of an s x s product, of 256 or more, that fill the chip.
+int x3_plain_split(const skema_ctx* c, int64_t s, int64_t K) {
+  const int64_t tiles = ((s + kPlBM - 1) / kPlBM) * ((s + kPlBM - 1) / kPlBM);
+  return (int)std::max<int64_t>(2, std::min<int64_t>(c->sm_count / tiles, K / 256));
+}
+
 void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag) {
-  x3_plain_kernel<<<2 * c->sm_count, 256, 0, c->stream>>>(p, flag);
+  x3_plain_kernel<<<c->sm_count, 256, 0, c->stream>>>(p, flag);
   SKEMA_LAUNCHED(c);
 }
 
@@ -420,24 +501,23 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
               tc::X3Out{c->Z, 1, s, eta, xb, nullptr, 0, 0, s, s, s}, part, words);
     }
     if (flag) {
-      const int64_t j0 = r;
       const float xb = i == 0 ? xbeta : 1.f;
-      X3Plain3 p;
-      p.g[0] = X3Plain{Aw.p, Aw.rs, Aw.cs, c->omg.f32, c->omg.cs, c->omg.rs, c->Y + R0, 1, c->m,
-                       wr, k, n, eta, ybeta, 1.f, 1, 1, 0};
+      X3Plain3 p{};
+      p.g[0] = X3Plain{Aw.p, Aw.rs, Aw.cs, nullptr, 0, 0, c->omg.f32, c->omg.cs, c->omg.rs, c->Y + R0, 1, c->m,
+                       wr, k, n, eta, ybeta, 1};
       p.n = 1;
       if (s > 0) {
-        p.g[1] = X3Plain{Aw.p, Aw.rs, Aw.cs, c->psi.f32, c->psi.cs, c->psi.rs, T32, 1, wr,
-                         wr, s, n, 1.f, 0.f, 1.f, 1, 1, 0};
-        p.g[2] = X3Plain{c->ups.f32 + R0, c->ups.rs, 1, Aw.p, Aw.rs, Aw.cs, c->X, n, 1,
-                         k, n, wr, eta, xb, nu, W, nwin, j0};
+        p.g[1] = X3Plain{Aw.p, Aw.rs, Aw.cs, nullptr, 0, 0, c->psi.f32, c->psi.cs, c->psi.rs, T32, 1, wr,
+                         wr, s, n, 1.f, 0.f, 1};
+        p.g[2] = X3Plain{nullptr, 0, 0, uf, ldw, (k + s) * ldw, Aw.p, Aw.rs, Aw.cs, c->X, n, 1, k, n, wr, eta, xb, 1};
         p.n = 3;
+        p.scale = c->Z, p.nscale = s * s, p.by = xb;
       }
       x3_plain(c, p, flag);
       if (s > 0) {
-        X3Plain3 z;
-        z.g[0] = X3Plain{c->phi.f32 + R0, c->phi.rs, 1, T32, 1, wr, c->Z, s, 1,
-                         s, s, wr, eta, xb, nu, W, nwin, j0};
+        X3Plain3 z{};
+        z.g[0] = X3Plain{nullptr, 0, 0, uf + k * ldw, ldw, (k + s) * ldw, T32, 1, wr, c->Z, s, 1, s, s, wr, eta, 1.f,
+                         x3_plain_split(c, s, wr)};
         z.n = 1;
         x3_plain(c, z, flag);
       }

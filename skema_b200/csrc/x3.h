@@ -136,22 +136,27 @@ void x3_row_planes(skema_ctx* c, const float* S, int64_t rs, int64_t rows, int64
 
 // Up to three FP32 products C = alpha A B + beta C by plain FMA, run when
 // *flag is refused: the form of a block whose values the planes cannot carry.
-// A(i, kk) is scaled by nu^(nwin - 1 - (j0 + kk) / W).
 struct X3Plain {
   const float* A;
   int64_t ars, acs;
+  const __nv_bfloat16* Apl;  // A null: the sum of its planes (aps apart), rows of ald with K along them
+  int64_t ald, aps;
   const float* B;
   int64_t brs, bcs;
   float* C;
   int64_t crs, ccs;
   int64_t M, N, K;
-  float alpha, beta, nu;
-  int64_t W, nwin, j0;
+  float alpha, beta;
+  int split;  // above 1: K in so many parts, added to C (beta not applied)
 };
 struct X3Plain3 {
   X3Plain g[3];
   int n;
+  float* scale;  // nscale values are scaled by `by`: the C of a split product to follow
+  int64_t nscale;
+  float by;
 };
+int x3_plain_split(const skema_ctx* c, int64_t s, int64_t K);
 void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag);
 
 // One call's input: a dense matrix, or a filler of window planes (A.p null)
