@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kPlThreads, GRAD ? 2 : 3)
   __shared__ __align__(16) RbfTile t;
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
   const int64_t tiles_j = (N + kTJ - 1) / kTJ, tiles_i = (wr + kTI - 1) / kTI;
-  uint32_t top = 0;
+  float top = 0.f;
   double gsum = 0.0;
   for (int64_t tile = blockIdx.x; tile < tiles_i * tiles_j; tile += gridDim.x) {
     const int64_t ib = tile / tiles_j, i0 = ib * kTI, j0 = (tile - ib * tiles_j) * kTJ;

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
   const int nr = (int)min((int64_t)32, g.nrows - r0);
   for (int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x; q < g.nscale; q += (int64_t)gridDim.x * 256)
     g.scale[q] = g.by == 0.f ? 0.f : g.by * g.scale[q];
-  uint32_t top = 0;
+  float top = 0.f;
   // the columns of Omega, then those of Psi
   for (int64_t c = g.Y ? 0 : g.k; c < g.k + g.s;) {
     const bool om = c < g.k;

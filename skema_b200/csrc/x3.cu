@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256)
                         __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t big,
                         uint32_t* __restrict__ flag) {
   const int64_t total = nrb * 8 * cols;
-  uint32_t top = 0;
+  float top = 0.f;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     // 64-row block outermost, then columns, then the 8 groups of a line: a
     // warp's stores are 512 contiguous bytes per plane
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256)
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t tj = (cols + 31) / 32;
   const bool rowfast = srs <= scs;
-  uint32_t top = 0;
+  float top = 0.f;
   for (int64_t t = blockIdx.x; t < nrb * tj; t += gridDim.x) {
     const int64_t rb = t / tj, j0 = (t - rb * tj) * 32;
 #pragma unroll
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256)
     x3_maps_kernel(X3Src a, X3Src b, int64_t cols, __nv_bfloat16* __restrict__ D, int64_t ld, int64_t pstride, float nu,
                    int64_t W, int64_t nwin, int64_t j0, uint32_t big, uint32_t* __restrict__ flag) {
   const int64_t c8 = ld / 8, total = (a.rows + b.rows) * c8;
-  uint32_t top = 0;
+  float top = 0.f;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = q / c8, j = (q - r * c8) * 8;
     const float* sp = (r < a.rows ? a.p + r * a.rs : b.p + (r - a.rows) * b.rs) + j;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256)
                          int64_t j0, uint32_t big, uint32_t* __restrict__ flag) {
   constexpr int NR = kTrRows / 8;  // rows per warp
   __shared__ float tile[32][kTrRows + 1];
-  uint32_t top = 0;
+  float top = 0.f;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t ti = (ld + kTrRows - 1) / kTrRows, tj = (cols + 31) / 32;
   for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
@@ -336,8 +336,9 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   const size_t stage = tc::kX3ABytes + (size_t)3 * g.nt * tc::kX3BK * 2;
   g.stages = (int)std::min<size_t>(tc::kX3MaxStages, (kX3Smem - 2048) / stage);
   const int64_t tiles = (int64_t)g.mtiles * g.ntiles;
-  // runs of at least four K steps (so that none is empty)
-  const int G = (int)std::max<int64_t>(1, std::min<int64_t>(c->sm_count, tiles * g.ksteps / 4));
+  // runs of at least four K steps (so that none is empty), or a tile: a K of one
+  // to three steps leaves nothing to cut
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>(c->sm_count, std::max(tiles, tiles * g.ksteps / 4)));
   g.full = (int)(tiles / G * G);
   if ((tiles - g.full) * g.ksteps < 4 * (int64_t)G) g.full = (int)tiles;  // too little to cut
   CUtensorMap ta;

@@ -39,14 +39,12 @@ inline bool x3_carries(const Map& mp) { return mp.amax == 0.f || (mp.amax >= 0x1
 __host__ __device__ __forceinline__ bool x3_refused(uint32_t w) {
   return (w & kX3Big) || (w & (kX3Normal | kX3Tiny)) == kX3Tiny;
 }
-// m: the largest of this thread's magnitudes, as bits
-__device__ __forceinline__ void x3_note(uint32_t& m, float x) {
-  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
-  m = max(m, b <= 0x7f800000u ? b : 0u);
-}
+// m: the largest of this thread's magnitudes (fmaxf passes a NaN over)
+__device__ __forceinline__ void x3_note(float& m, float x) { m = fmaxf(m, fabsf(x)); }
 // Notes the block's largest magnitude in *word, big from the bits `big` on;
 // called by all its threads.
-__device__ __forceinline__ void x3_report(uint32_t m, uint32_t big, uint32_t* word) {
+__device__ __forceinline__ void x3_report(float top, uint32_t big, uint32_t* word) {
+  const uint32_t m = __float_as_uint(top);
   uint32_t kind = 0;
   if (__syncthreads_or(m >= big))
     kind = kX3Big;
