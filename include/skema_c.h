@@ -242,7 +242,9 @@ int skema_residuals_finish(skema_ctx* ctx, double* rnorms, int32_t mem);
 
 /* Copy one sketch out of / into the context (the reference only exposes them
  * through its debug dumps, src/Skema_SketchySVD.cpp:192-206, 235-245).
- * X is k x n, Y is m x k, Z is s x s; `layout` is the layout of buf. */
+ * X is k x n, Y is m x k, Z is s x s; `layout` is the layout of buf. A copy to
+ * device memory is asynchronous on ctx's stream, except after BF16 or FP8
+ * updates, whose status it reads first (skema_set_wait_limit). */
 int skema_get_sketch(skema_ctx* ctx, int32_t which, float* buf, int64_t ld,
                      int32_t layout, int32_t mem);
 int skema_set_sketch(skema_ctx* ctx, int32_t which, const float* buf,

@@ -50,7 +50,7 @@ void check_device_error(skema_ctx* c) {
   int h = 0;
   SKEMA_CUDA(cudaMemcpyAsync(&h, c->dev_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   SKEMA_CUDA(cudaStreamSynchronize(c->stream));
-  c->dev_err_armed = false;
+  c->dev_err_armed = 0;
   if (h != 0) {
     SKEMA_CUDA(cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream));
     SKEMA_CUDA(cudaStreamSynchronize(c->stream));
@@ -835,7 +835,9 @@ int skema_get_sketch(skema_ctx* c, int32_t which, float* buf, int64_t ld, int32_
     int64_t rows, cols;
     sketch_shape(c, which, &src, &rows, &cols);
     check_dense_args(buf, ld, layout, rows, cols, mem);
-    check_device_error(c);
+    // reading the word waits for the stream: an FP32 fetch to device memory stays
+    // asynchronous, one to host memory reads it when it has waited anyway
+    if (c->dev_err_armed > 1) check_device_error(c);
     if (which == SKEMA_SKETCH_Y) y_materialize(c);
     const bool irow = sketch_row_major(which);
     const int64_t inner = irow ? cols : rows, outer = irow ? rows : cols;
@@ -881,7 +883,10 @@ int skema_get_sketch(skema_ctx* c, int32_t which, float* buf, int64_t ld, int32_
         SKEMA_CUDA(cudaEventRecord(out_done[sl], c->stream));
       }
     }
-    if (mem == SKEMA_MEM_HOST) SKEMA_CUDA(cudaStreamSynchronize(c->stream));
+    if (mem == SKEMA_MEM_HOST) {
+      SKEMA_CUDA(cudaStreamSynchronize(c->stream));
+      check_device_error(c);
+    }
   });
 }
 

@@ -319,7 +319,7 @@ void launch_gemm(skema_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int
   if (grid <= 0) return;
   kern<<<grid, tc::kThreads, smem, c->stream>>>(ta, tb, g, o, c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = 2;
 }
 
 // X^T product straight from the FP32 window (converts it and writes A16).
@@ -339,7 +339,7 @@ void launch_gemm_a32_s(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap&
   kern<<<grid, STT ? tc::kThreadsA32St : tc::kThreadsA32, smem, c->stream>>>(ta32, tb, ta16, g, o, amax,
                                                                             c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = 2;
 }
 
 // 3 FP32 + 3 BF16 stages (228 KB of shared memory). With separate FP32 and
@@ -516,7 +516,7 @@ void launch_gemm_fp8(skema_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb,
   if (grid <= 0) return;
   kern<<<grid, tc::kThreads, smem, c->stream>>>(ta, tb, g, o, c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = 2;
 }
 
 }  // namespace

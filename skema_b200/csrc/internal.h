@@ -199,7 +199,9 @@ struct skema_ctx {
   // The rotations that the Jacobi SVD's two CTAs exchange (approx.cu), in the
   // allocation of dev_err.
   void* jac_rot = nullptr;
-  bool dev_err_armed = false;
+  // What may have set it since it was last read: 0 nothing, 1 the FP32 form
+  // (x3.cu), 2 a BF16 or FP8 kernel.
+  int dev_err_armed = 0;
   // stage timers
   bool timing = false;
   std::vector<skema::PendingTimer> pending;

@@ -86,7 +86,7 @@ void launch_rbf(skema_ctx* c, const CUtensorMap& tq, const CUtensorMap& tk, cons
   const int grid = (int)std::min<int64_t>(units, c->sm_count);
   kern<<<grid, tc::kThreads, smem, c->stream>>>(tq, tk, tv1, tv2, a, o, c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = 2;
 }
 
 // Output-column chunks of one pass: (NC1, NC2) = (256, 144) with two key /
@@ -289,7 +289,7 @@ void launch_vjp(skema_ctx* c, const CUtensorMap& tqx, const CUtensorMap& tkx, co
   const int grid = (int)std::min<int64_t>(units, c->sm_count);
   kern<<<grid, tc::kThreads, smem, c->stream>>>(tqx, tkx, tqa, tkb, txt, a, c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = 2;
 }
 
 }  // namespace

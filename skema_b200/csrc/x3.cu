@@ -353,7 +353,7 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
   SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kX3Smem));
   kern<<<G, tc::kX3Threads, kX3Smem, c->stream>>>(ta, tb, g, o, a.blocked ? 1 : 0, (int)a.nrb, part, words, c->dev_err);
   SKEMA_LAUNCHED(c);
-  c->dev_err_armed = true;
+  c->dev_err_armed = std::max(c->dev_err_armed, 1);
   const int rem = (int)(tiles - g.full);
   if (rem > 0) {
     if (rem * (g.nt / 8) >= 2 * c->sm_count)
