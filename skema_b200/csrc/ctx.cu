@@ -84,14 +84,25 @@ void* workspace(skema_ctx* c, size_t bytes) {
   return c->ws;
 }
 
-void* try_workspace(skema_ctx* c, size_t bytes) {
+void* try_workspace(skema_ctx* c, size_t bytes, size_t otherwise) {
   if (bytes <= c->ws_bytes) return c->ws;
-  try {
-    return workspace(c, bytes);
-  } catch (const Error& e) {
-    if (e.status != SKEMA_ENOMEM) throw;
-    return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  SKEMA_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone || bytes >= c->ws_refused) return nullptr;
+  const size_t had = c->ws_bytes;
+  for (size_t b : {std::max(bytes, otherwise), bytes}) {
+    try {
+      return workspace(c, b);
+    } catch (const Error& e) {
+      if (e.status != SKEMA_ENOMEM) throw;
+    }
+    if (b == bytes) break;
   }
+  if (c->ws_bytes < had) {  // the device refused it, after the old one was freed
+    c->ws_refused = bytes;
+    workspace(c, had);
+  }
+  return nullptr;
 }
 
 // A pitched copy whose rows lie back to back on both sides goes as one
@@ -1027,6 +1038,7 @@ int skema_set_workspace_limit(skema_ctx* c, int64_t bytes) {
   return guarded(c, [&] {
     if (bytes < 0) fail(SKEMA_EINVAL, "workspace limit must be >= 0");
     c->ws_limit = (size_t)bytes;
+    c->ws_refused = (size_t)-1;
   });
 }
 

@@ -114,7 +114,7 @@ void dense_update(skema_ctx* c, Mat A, int64_t row0, int64_t nrows) {
     return;
   }
   if (c->p.precision == SKEMA_PREC_FP32 && c->p.dim_redux == SKEMA_MAP_GAUSS &&
-      x3_update(c, X3Input{A, nullptr}, row0, nrows))
+      x3_update(c, X3Input{A, nullptr, dense_scratch_bytes(c, std::min(c->w, nrows))}, row0, nrows))
     return;
   const int64_t W = c->w;
   float* T = (float*)workspace(c, dense_scratch_bytes(c, std::min(W, nrows)));

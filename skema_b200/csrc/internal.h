@@ -133,6 +133,7 @@ struct skema_ctx {
   void* stage = nullptr;  // host-input staging
   size_t stage_bytes = 0;
   size_t ws_limit = 0;    // cap on ws_bytes + stage_bytes (0: none)
+  size_t ws_refused = (size_t)-1;  // try_workspace
   int sm_count = 148;
   // Upper bound on the CTAs of one tensor-core launch (0: one per SM); set
   // while the dense pipeline splits the SMs between its two streams.
@@ -231,9 +232,12 @@ class StageScope {
 };
 
 void* workspace(skema_ctx* c, size_t bytes);
-// The same, or nullptr when the limit or the device does not allow it (what
-// the context holds may have been given back by then).
-void* try_workspace(skema_ctx* c, size_t bytes);
+// The same, or nullptr when the limit or the device does not allow it, or the
+// stream is being captured. `otherwise`: what the caller's other form takes from
+// workspace(), had along when there is room, so that a capture after a warm-up
+// call finds it. A size that the device refused is not asked for again until
+// skema_set_workspace_limit is called.
+void* try_workspace(skema_ctx* c, size_t bytes, size_t otherwise = 0);
 void* staging(skema_ctx* c, size_t bytes);
 bool y_rows_clean(const skema_ctx* c, int64_t a, int64_t b);
 void y_rows_mark(skema_ctx* c, int64_t a, int64_t b);

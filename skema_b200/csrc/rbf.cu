@@ -404,6 +404,8 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
   const int64_t W = c->w;
   const int64_t N = npts;
   const float gamma = (float)c->p.kernel_gamma;
+  const int64_t wmax = std::min(W, nrows);
+  const size_t kbytes = (sizeof(float) * (size_t)(wmax * N) + 255) / 256 * 256;
   if (c->p.precision == SKEMA_PREC_FP32 && c->p.dim_redux == SKEMA_MAP_GAUSS && gamma >= 0.f) {
     X3Input in{Mat{nullptr, 0, 0}, [&](int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride) {
                  const int64_t tiles = ((wr + 63) / 64) * ((N + 127) / 128);
@@ -411,11 +413,10 @@ void rbf_update(skema_ctx* c, Mat P, int64_t npts, int64_t d, int64_t row0, int6
                  kern<<<grid_cap(c, tiles, 3), kPlThreads, 0, c->stream>>>(P.p, P.rs, P.cs, N, d, gamma, R0, wr,
                                                                            planes, pstride, RbfGrad{});
                  SKEMA_LAUNCHED(c);
-               }};
+               },
+               kbytes + dense_scratch_bytes(c, wmax)};
     if (x3_update(c, in, row0, nrows)) return;
   }
-  const int64_t wmax = std::min(W, nrows);
-  const size_t kbytes = (sizeof(float) * (size_t)(wmax * N) + 255) / 256 * 256;
   char* ws = (char*)workspace(c, kbytes + dense_scratch_bytes(c, wmax));
   float* Kw = (float*)ws;
   float* T = (float*)(ws + kbytes);

@@ -788,7 +788,8 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   if (top < 40) return false;
   const size_t b_xt = up(sizeof(float) * (size_t)(n * kp)), b_pl = up(sizeof(__nv_bfloat16) * (size_t)(3 * s * ldt)),
                b_t32 = up(sizeof(float) * (size_t)(s * ldt)), b_flag = up(sizeof(uint32_t) * (size_t)nblk);
-  char* ws = static_cast<char*>(try_workspace(c, b_xt + 2 * b_pl + b_t32 + x3_part_bytes(c) + b_flag));
+  char* ws = static_cast<char*>(try_workspace(c, b_xt + 2 * b_pl + b_t32 + x3_part_bytes(c) + b_flag,
+                                             sizeof(float) * (size_t)(n * s)));
   if (!ws) return false;
   float* XT = reinterpret_cast<float*>(ws);
   __nv_bfloat16* Tp = reinterpret_cast<__nv_bfloat16*>(ws + b_xt);

@@ -437,7 +437,7 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     b_t = up256(sizeof(__nv_bfloat16) * (size_t)(3 * s * rb));
     b_t32 = in.A.p ? up256(sizeof(float) * (size_t)(s * rb)) : 0;
     b_flag = up256(sizeof(uint32_t) * (size_t)((wsrows + rb - 1) / rb));
-    ws = static_cast<char*>(try_workspace(c, b_op + b_part + b_a + b_uf + b_t + b_t32 + b_flag));
+    ws = static_cast<char*>(try_workspace(c, b_op + b_part + b_a + b_uf + b_t + b_t32 + b_flag, in.otherwise));
     if (cap == 64) break;
   }
   if (!ws) return false;

@@ -162,6 +162,7 @@ void x3_plain(skema_ctx* c, const X3Plain3& p, const uint32_t* flag);
 struct X3Input {
   Mat A;
   std::function<void(int64_t R0, int64_t wr, __nv_bfloat16* planes, int64_t pstride)> fill;
+  size_t otherwise;  // the SIMT form's workspace (try_workspace)
 };
 // All windows of one call of a Gauss-map FP32 context. False (and nothing
 // done) when the call is small, its workspace is not to be had, or nu or the
