@@ -296,7 +296,7 @@ tc::Grid3 grid_of(const skema_ctx* c, int64_t M, int64_t N, int64_t K, int nt, i
   g.ksteps = (K + bk - 1) / bk;
   g.kcsteps = pl.kchunk > 0 ? (int)(pl.kchunk / bk) : (int)g.ksteps;
   g.streamk = pl.streamk > 0 ? 1 : 0;
-  g.wtiles = g.mtiles, g.wk = 0, g.wlog2 = 0.f;
+  g.wtiles = g.mtiles, g.wk = 0, g.wlog2 = 0.0;
   const int64_t units = (int64_t)nwin * g.mtiles * g.ntiles * (g.streamk ? g.ksteps : g.ksplit);
   if (units > 0x7fffffff) fail(SKEMA_EINVAL, "tensor-core grid too large");
   g.mtiles *= nwin;
@@ -326,7 +326,7 @@ void launch_gemm(skema_ctx* c, const CUtensorMap& ta, const CUtensorMap& tb, int
 template <bool AROW, int S1, int S2, bool STT>
 void launch_gemm_a32_s(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& ta16,
                        int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax, int nwin,
-                       float wlog2) {
+                       double wlog2) {
   constexpr uint32_t STAGE = ((tc::BM * tc::BK * 2 + kNT * tc::BK * 2 + 1023) / 1024) * 1024;
   const size_t smem = (size_t)S1 * tc::BM * tc::BK * 4 + (size_t)S2 * STAGE + 1024 + 256;
   auto kern = amax ? tc::gemm_a32_kernel<kNT, S1, S2, AROW, true, STT>
@@ -349,7 +349,7 @@ void launch_gemm_a32_s(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap&
 template <bool AROW>
 void launch_gemm_a32(skema_ctx* c, const CUtensorMap& ta32, const CUtensorMap& tb, const CUtensorMap& ta16,
                      int64_t M, int64_t N, int64_t K, Plan pl, const tc::OutSpec& o, uint32_t* amax, int nwin,
-                     float wlog2) {
+                     double wlog2) {
   if (c->xt_store_thread)
     launch_gemm_a32_s<AROW, 3, 3, true>(c, ta32, tb, ta16, M, N, K, pl, o, amax, nwin, wlog2);
   else
@@ -693,10 +693,10 @@ TcSlices xt_window(skema_ctx* c, Mat Aw, int64_t R0, int64_t wr, __nv_bfloat16* 
   const CUtensorMap ta16 = tmap_bf16_blocked(A16, (uint64_t)n, (uint64_t)nrb, 128);
   if (a32_cm) {
     const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)wr, (uint64_t)n, (uint64_t)Aw.cs * 4, 32, 128);
-    launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.f);
+    launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.0);
   } else if (a32_rm) {
     const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)n, (uint64_t)wr, (uint64_t)Aw.rs * 4, 32, 64);
-    launch_gemm_a32<true>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.f);
+    launch_gemm_a32<true>(c, ta32, tb, ta16, n, k, wr, pl, o, amax, 1, 0.0);
   } else {
     launch_gemm<tc::A_KMAJ_BLK>(c, ta16, tb, n, k, wr, pl, 1, o);
   }
@@ -726,7 +726,7 @@ void xt_batch(skema_ctx* c, Mat Aw, int64_t R0, int64_t wr, int nwin, __nv_bfloa
   o.rows = n, o.split = k, o.ncols = k;
   scale_block(c, MatOut{c->X, n, 1}, k, n, (float)std::pow((double)nu, (double)nwin));
   const CUtensorMap ta16 = tmap_bf16_blocked(A16, (uint64_t)n, (uint64_t)(rows / 64), 128);
-  const float wlog2 = nu == 1.f ? 0.f : std::log2(nu);
+  const double wlog2 = nu == 1.f ? 0.0 : std::log2((double)nu);
   if (Aw.rs == 1) {
     const CUtensorMap ta32 = tmap_f32(Aw.p, (uint64_t)rows, (uint64_t)n, (uint64_t)Aw.cs * 4, 32, 128);
     launch_gemm_a32<false>(c, ta32, tb, ta16, n, k, wr, pl, o, nullptr, nwin, wlog2);

@@ -296,7 +296,7 @@ struct Grid3 {
   // w carry 2^((windows - 1 - w) wlog2). wtiles = mtiles: one window.
   int wtiles;
   int64_t wk;
-  float wlog2;
+  double wlog2;
 };
 __device__ __forceinline__ void decode_unit(const Grid3& g, int t, int& mt, int& nt, int& ks) {
   if (g.m_fast) {
@@ -952,7 +952,8 @@ __global__ void __launch_bounds__(kThreadsA32St, 1)
     for (; next_seg(g, sc, mt, nt, kt0, kt1); ++tcount) {
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
       float w = 1.f;
-      if (g.wlog2 != 0.f) w = exp2f((float)(g.mtiles / g.wtiles - 1 - mt / g.wtiles) * g.wlog2);
+      // in FP64: exponents of up to 40 would cost an FP32 weight 1e-6
+      if (g.wlog2 != 0.0) w = (float)exp2((double)(g.mtiles / g.wtiles - 1 - mt / g.wtiles) * g.wlog2);
       if (!epilogue_unit<NT, TCOLS>(o, tmem, acc, aph, tfull, tempty, mt % g.wtiles, nt, warp, lane, err, w)) break;
     }
   }
