@@ -152,8 +152,8 @@ __device__ __forceinline__ void ssign_apply8(uint32_t base, uint4 wv, float a) {
 // S = 4: a row is cut into four equal runs of nonzeros in four adjacent lanes,
 // whose bins are added at the write-out, (0 + 1) + (2 + 3). For calls of few
 // rows, whose time is the walk along the longest row: 2,000 rows of 0 to 200
-// entries take 16 us against 35, 10 against 12 with 10 entries in each. (A warp
-// per row with the bins in its lanes took 42 to 62.)
+// entries take 16 us against 35. (A warp per row with the bins in its lanes took
+// 42 to 62.) The line between the two is at launch_csr_ssign_y.
 template <int U, int S>
 __global__ void __launch_bounds__(128)
     csr_ssign_y16_kernel(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ col,
@@ -219,15 +219,25 @@ __global__ void __launch_bounds__(128)
     const int64_t r0 = tile * R;
     if (S == 4) {
       // row lane % 8, bins lane / 8, + 4, ..: four lanes' bins lie side by side
+      // (four at a time: what beta scales is loaded ahead of the stores)
       const int64_t i = r0 + (lane & 7);
-      for (int r = lane >> 3; r < k; r += 4) {
+      const bool in = i < nrows, last = tile + tstride >= ntiles;
+      float* yp = Y + i + (lane >> 3) * ldy;
+      for (int r = lane >> 3; r < k; r += 16, yp += 16 * ldy) {
         float4* bp = bins4 + r * 8 + (lane & 7);
-        const float4 q = *bp;
-        *bp = z4;
-        if (i < nrows) {
-          float* yp = Y + i + r * ldy;
-          const float v = (q.x + q.y) + (q.z + q.w);
-          *yp = beta == 0.f ? v : fmaf(beta, *yp, v);
+        float4 q[4];
+        float o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          q[u] = r + 4 * u < k ? bp[32 * u] : z4;
+          o[u] = beta != 0.f && in && r + 4 * u < k ? yp[4 * u * ldy] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (r + 4 * u >= k) continue;
+          if (!last) bp[32 * u] = z4;
+          const float v = (q[u].x + q[u].y) + (q[u].z + q[u].w);
+          if (in) yp[4 * u * ldy] = beta == 0.f ? v : fmaf(beta, o[u], v);
         }
       }
     } else if (vec && r0 + 32 <= nrows) {
@@ -729,18 +739,25 @@ static void launch_csr_ssign_y16(skema_ctx* c, const int64_t* rowptr, const int3
 static void launch_csr_ssign_y(skema_ctx* c, const int64_t* rowptr, const int32_t* col,
                                const float* val, int64_t col_offset, int64_t nrows, const Map& O,
                                float* Y, int64_t ldy, float alpha, float beta) {
-  // four lanes per row while the eight-row tiles of the call all fit on the chip
-  // at once (1024 / k warps of bins per SM within 128 KB)
-  if (O.packed16 && nrows <= 8 * c->sm_count * std::max<int64_t>(1, 1024 / c->k)) {
-    launch_csr_ssign_y16<4, 4>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta);
-    return;
-  }
+  // Four lanes per row while the eight-row tiles of the call all fit on the chip
+  // at once (1024 / k warps of bins per SM within 128 KB, and no more than 48).
+  // Measured from 32 rows to the line, k = 9 to 253, after a reset: log-normal
+  // row lengths (mean 10) take 0.40 to 0.62 of the time of a lane per row, rows
+  // of 10 entries 0.74 to 1.05 (k = 201: 1.0 to 1.13), rows of 2 or 4 0.8 to
+  // 1.3, which is 8 to 10 us +- 2 either way, and at 49,152 rows and k = 21 10
+  // against 11 to 16 us, where log-normal ones take 40 against 23. Past the cap,
+  // at k = 9 and 131,072 rows, short rows would take 12 to 17 against 17 to 20.
+  // (Added to a Y that is not empty: 0.26 to 1.1.)
   if (O.packed16) {  // zeta = 8, k <= 256: at most 32 KB of bins per warp
+    const bool few = nrows <= 8 * c->sm_count * std::min<int64_t>(48, std::max<int64_t>(1, 1024 / c->k));
+    auto go = [&](auto one, auto four) {
+      (few ? four : one)(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta);
+    };
     switch (c->ssign_batch) {
-      case 2: launch_csr_ssign_y16<2, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      case 6: launch_csr_ssign_y16<6, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      case 8: launch_csr_ssign_y16<8, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
-      default: launch_csr_ssign_y16<4, 1>(c, rowptr, col, val, col_offset, nrows, O, Y, ldy, alpha, beta); break;
+      case 2: go(launch_csr_ssign_y16<2, 1>, launch_csr_ssign_y16<2, 4>); break;
+      case 6: go(launch_csr_ssign_y16<6, 1>, launch_csr_ssign_y16<6, 4>); break;
+      case 8: go(launch_csr_ssign_y16<8, 1>, launch_csr_ssign_y16<8, 4>); break;
+      default: go(launch_csr_ssign_y16<4, 1>, launch_csr_ssign_y16<4, 4>); break;
     }
     return;
   }
