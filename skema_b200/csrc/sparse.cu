@@ -407,6 +407,7 @@ struct GaussGather {
   const int32_t* col;
   const float* val;
   int64_t col_offset, nrows, ncol;
+  int tile;          // rows per CTA, up to 32
   const float* omg;  // ncol x k
   const float* psi;  // ncol x s
   int64_t k, s;
@@ -481,8 +482,8 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
   extern __shared__ float gg_tile[];  // CH x 33
   __shared__ int next;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t r0 = (int64_t)blockIdx.x * 32;
-  const int nr = (int)min((int64_t)32, g.nrows - r0);
+  const int64_t r0 = (int64_t)blockIdx.x * g.tile;
+  const int nr = (int)min((int64_t)g.tile, g.nrows - r0);
   for (int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x; q < g.nscale; q += (int64_t)gridDim.x * 256)
     g.scale[q] = g.by == 0.f ? 0.f : g.by * g.scale[q];
   float top = 0.f;
@@ -503,13 +504,23 @@ __global__ void __launch_bounds__(256, 4) csr_gauss_gather_kernel(GaussGather g,
       default: gauss_tile<6>(g, r0, nr, map, width, cols, lane, &next, gg_tile); break;
     }
     __syncthreads();
-    for (int cl = warp; cl < cols; cl += 8) {
+    // what beta scales is loaded ahead of the stores
+    for (int cl = warp; om && cl < cols && lane < nr; cl += 32) {
+      float* yp = g.Y + r0 + lane + (c0 + cl) * g.ldy;
+      float o[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) o[u] = g.beta != 0.f && cl + 8 * u < cols ? yp[8 * u * g.ldy] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (cl + 8 * u >= cols) continue;
+        const float v = g.alpha * gg_tile[(cl + 8 * u) * 33 + lane];
+        yp[8 * u * g.ldy] = g.beta == 0.f ? v : fmaf(g.beta, o[u], v);
+      }
+    }
+    for (int cl = warp; !om && cl < cols; cl += 8) {
       const float v = gg_tile[cl * 33 + lane];
       if (lane >= nr) continue;
-      if (om) {
-        float* yp = g.Y + r0 + lane + (c0 + cl) * g.ldy;
-        *yp = (g.beta == 0.f) ? g.alpha * v : fmaf(g.beta, *yp, g.alpha * v);
-      } else if (g.T32) {
+      if (g.T32) {
         g.T32[(c0 + cl) * g.ldt + r0 + lane] = v;
       } else {
         x3_note(top, v);
@@ -780,11 +791,15 @@ static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t*
   const float eta = (float)c->p.sketch_eta, nu = (float)c->p.sketch_nu;
   const int64_t n = c->n, k = c->k, s = c->spd ? 0 : c->s, W = c->w, nwin = (nrows + W - 1) / W;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  GaussGather g{rowptr, col, val, col_offset, nrows, n, c->omg.f32, c->psi.f32, k, s, c->Y + row0, c->m,
+  // a row per warp where 32 rows per CTA would leave SMs idle: 20 rows of 20
+  // entries (k = 201) 246 -> 78 us a call, 500 of 300 (k = 281) 817 -> 328, 3,000
+  // of 10 (k = 81) 81 -> 76; 9,000 (k = 41) 85 against 90
+  const int tile = nrows < (int64_t)32 * c->sm_count ? 8 : 32;
+  GaussGather g{rowptr, col, val, col_offset, nrows, n, tile, c->omg.f32, c->psi.f32, k, s, c->Y + row0, c->m,
                 eta, ybeta, nullptr, nullptr, 0, 0, 0, nullptr, nullptr, 0, 0.f};
   const size_t smem = sizeof(float) * 192 * 33;
   auto gather = [&](const GaussGather& q, const uint32_t* cond) {
-    csr_gauss_gather_kernel<<<(unsigned)((q.nrows + 31) / 32), 256, smem, c->stream>>>(q, cond);
+    csr_gauss_gather_kernel<<<(unsigned)((q.nrows + q.tile - 1) / q.tile), 256, smem, c->stream>>>(q, cond);
     SKEMA_LAUNCHED(c);
   };
   if (c->spd) {
