@@ -525,7 +525,7 @@ void launch_gram(skema_ctx* c, const T* A, int64_t lda, int64_t k, int64_t rows,
   const size_t smem = sizeof(double) * (size_t)((k + 15) / 16 * 16 * kGramLd);
   const bool few = depth <= 3;
   const int64_t ctas =
-      std::max<int64_t>(1, std::min<int64_t>((rows + 255) / 256, (few ? 2 : 1) * (int64_t)c->sm_count / groups));
+      std::max<int64_t>(1, std::min<int64_t>((rows + 63) / 64, (few ? 2 : 1) * (int64_t)c->sm_count / groups));
   const int64_t per = ((rows + ctas - 1) / ctas + 31) / 32 * 32;
   auto kern = few ? gram_mma_kernel<T, 3> : gram_mma_kernel<T, kGramTiles>;
   const int ny = (tiles + warps * (few ? 3 : kGramTiles) - 1) / (warps * (few ? 3 : kGramTiles));
@@ -561,10 +561,11 @@ void gram(skema_ctx* c, const double* A, int64_t lda, int64_t rows, int64_t k, d
     SKEMA_CUDA(cudaMemsetAsync(G, 0, sizeof(double) * (size_t)(k * k), c->stream));
     return;
   }
-  // the k-sized products take the 32 x 32 tiles of dgemm, whose grid does not
-  // shrink with the rows (403 x 201: 15 us against 77)
-  if (k > kTallMaxK || rows < kTallMinRows) {
-    dgemm<double, double>(c, k, k, rows, 1.0, A, lda, 1, A, 1, lda, 0.0, G, 1, k, false);
+  // the k-sized products of a larger k take the 32 x 32 tiles of dgemm, whose
+  // grid does not shrink with the rows (403 x 201: 15 us against 77; 300 x 81 the
+  // same within 2 us; 1,000 x 9 36 against 10)
+  if (k > kTallMaxK || (rows < kTallMinRows && k > 40)) {
+    dgemm<double, double>(c, k, k, rows, 1.0, A, lda, 1, A, 1, lda, 0.0, G, 1, k);
     return;
   }
   gram_t<double>(c, A, lda, rows, k, G);
@@ -805,10 +806,14 @@ __global__ void __launch_bounds__(kTriThreads)
 // registers. Two barriers per panel; bound by the chain of 8 reciprocal square
 // roots per panel and the FP64 FMAs of the update (k = 201: 128 us, and
 // 35 us for the inverse by tri_solve_kernel; one column at a time with a barrier
-// each, and the inverse column by column in the same CTA, took 690). status[0] = 0, or j + 1 when the j-th pivot is not positive
-// (R is then not written).
-constexpr int kCholThreads = 512;
-__global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double* __restrict__ G, int k, double* R,
+// each, and the inverse column by column in the same CTA, took 690). Rinv (null:
+// not; k up to kCholInvMaxK): the inverse of R from the first warp, lane c column c
+// of L^-1 by forward substitution in registers, which for a small k is shorter
+// than a launch of tri_solve_kernel (k = 9, 300 x 300: the approximation's
+// eight factorisations took 30 us longer). Rinv may be G. status[0] = 0, or j + 1
+// when the j-th pivot is not positive (R and Rinv are then not written).
+constexpr int kCholThreads = 512, kCholInvMaxK = 32;
+__global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double* G, int k, double* R, double* Rinv,
                                                                    int* status) {
   extern __shared__ double cf_smem[];
   double* L = cf_smem;
@@ -918,6 +923,24 @@ __global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double*
       if (i < k) R[i + j * k] = (i <= j) ? L[lo_off(i, k) + j - i] : 0.0;
     }
   if (threadIdx.x == 0) status[0] = 0;
+  if (!Rinv || warp != 0) return;
+  const double inv = lane < k ? 1.0 / L[lo_off(lane, k)] : 0.0;
+  double x[kCholInvMaxK];
+#pragma unroll
+  for (int i = 0; i < kCholInvMaxK; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+  for (int l = 0; l < kCholInvMaxK; ++l) {
+    if (l >= k) break;
+    x[l] *= __shfl_sync(0xffffffffu, inv, l);
+    const double* c = L + lo_off(l, k) - l;
+#pragma unroll
+    for (int i = l + 1; i < kCholInvMaxK; ++i)
+      if (i < k) x[i] = fma(-c[i], x[l], x[i]);
+  }
+  if (lane < k)
+#pragma unroll
+    for (int i = 0; i < kCholInvMaxK; ++i)
+      if (i < k) Rinv[lane + i * k] = x[i];
 }
 
 // D = S^T for column-major k x k matrices.
@@ -1654,9 +1677,10 @@ void chol_inverse(skema_ctx* c, double* G, int64_t k, double* R, double* Rinv, i
   if (k <= kPackedMaxK) {
     const size_t smem = packed_smem_bytes(k);
     SKEMA_CUDA(cudaFuncSetAttribute(chol_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    chol_factor_kernel<<<1, kCholThreads, smem, c->stream>>>(G, (int)k, R, st);
+    const bool small = k <= kCholInvMaxK;
+    chol_factor_kernel<<<1, kCholThreads, smem, c->stream>>>(G, (int)k, R, small ? Rinv : nullptr, st);
     SKEMA_LAUNCHED(c);
-    tri_solve(c, R, k, Rinv, k, k, true, st);
+    if (!small) tri_solve(c, R, k, Rinv, k, k, true, st);
     return;
   }
   cholesky_kernel<<<1, 1024, 0, c->stream>>>(G, k, st);
