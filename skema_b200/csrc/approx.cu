@@ -1567,12 +1567,17 @@ bool launch_one_cluster(skema_ctx* c, Kern kern, int ctas, int threads, size_t s
 // The SVD kernel for a k x k problem: one pair of CTAs while A and V fit their
 // shared memory, block sweeps in one cluster up to k = 256, else block sweeps
 // driven from the host.
-void jacobi_svd(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, double tol, int* sweeps_out) {
+// st: the caller's status block of kStatusBytes; st[1] gets the sweeps, st[3] is
+// the host-driven form's flag, and the rotations that the pair of CTAs exchanges
+// follow at st + 64.
+constexpr size_t kStatusBytes = 64 * sizeof(int) + kJacRotBytes;
+void jacobi_svd(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, double tol, int* st) {
+  int* sweeps_out = st + 1;
+  double2* rot = reinterpret_cast<double2*>(st + 64);
   if (k <= kJacMaxK) {
     const int kp = (int)((k + 1) & ~1);
     const size_t smem = sizeof(double) * ((size_t)(k * k + 1) / 2 * 2) + sizeof(double2) * (size_t)(kp - 1) * (kp / 2);
     const int threads = std::max(128, (kp / 2 * 16 + 31) / 32 * 32);
-    double2* rot = static_cast<double2*>(c->jac_rot);
     auto go = [&](auto kern) {
       return launch_one_cluster(c, kern, 2, threads, smem, A, V, (int)k, max_sweeps, tol, rot, sweeps_out);
     };
@@ -1802,7 +1807,7 @@ void orth(skema_ctx* c, double* Qm, int64_t rows, int64_t k, double* Rscratch, d
   double* Sv = Vs + k * k;                       // k
   double* sig = Sv + k;                          // k
   dgemm<double, double>(c, k, k, rows, 1.0, Qm, rows, 1, Qm, 1, rows, 0.0, G, 1, k);
-  jacobi_svd(c, G, V, k, 60, 1e-15, dstatus + 1);
+  jacobi_svd(c, G, V, k, 60, 1e-15, dstatus);
   // G V = U diag(lambda) with U = V for the symmetric positive semidefinite G
   svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(G, V, k, Rscratch /*U, unused*/, Vs, Sv, sig);
   SKEMA_LAUNCHED(c);
@@ -2019,7 +2024,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   const size_t b_mk = sizeof(double) * (size_t)(m * k), b_nk = sizeof(double) * (size_t)(n * k);
   const size_t b_w = sizeof(double) * cholqr_work_doubles(m, k);
   const size_t b_small = sizeof(double) * (size_t)(8 * k * k + 4 * k + 64);
-  Carve cv(c, {b_mk, b_mk, b_nk, b_w, b_small, 16});
+  Carve cv(c, {b_mk, b_mk, b_nk, b_w, b_small, kStatusBytes});
   double* Yd = cv.take(b_mk);
   double* Ye = cv.take(b_mk);
   double* Od = cv.take(b_nk);
@@ -2034,7 +2039,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   double* RE = Vt + k * k;      // k x k
   double* Sv = RE + k * k;      // k
   double* sig = Sv + k;         // k
-  int* st = reinterpret_cast<int*>(cv.take(16));
+  int* st = reinterpret_cast<int*>(cv.take(kStatusBytes));
 
   f2d_kernel<<<g1(c, m * k), 256, 0, c->stream>>>(c->Y, 1, m, Yd, 1, m, m, k);
   SKEMA_LAUNCHED(c);
@@ -2049,7 +2054,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
 
   // nu = ||Y||_2 = sqrt(lambda_max(Y^T Y))
   dgemm<double, double>(c, k, k, m, 1.0, Yd, m, 1, Yd, 1, m, 0.0, G, 1, k);
-  jacobi_svd(c, G, Vc, k, 60, 1e-15, st + 1);
+  jacobi_svd(c, G, Vc, k, 60, 1e-15, st);
   svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(G, Vc, k, Uc, Vt, Sv, sig);
   SKEMA_LAUNCHED(c);
   double lmax = 0.0;
@@ -2085,7 +2090,7 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   // svd(E) = Q svd(R_E)
   cholqr(c, E, m, k, RE, W, st);
   SKEMA_CUDA(cudaMemcpyAsync(Cw, RE, sizeof(double) * (size_t)(k * k), cudaMemcpyDeviceToDevice, c->stream));
-  jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st + 1);
+  jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st);
   svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(Cw, Vc, k, Uc, Vt, Sv, sig);
   SKEMA_LAUNCHED(c);
   if (Uout) dgemm<double, double>(c, m, r, k, 1.0, E, 1, m, Uc, 1, k, 0.0, Uout, 1, m, false);
@@ -2095,8 +2100,6 @@ void spd_low_rank_approx(skema_ctx* c, double* Uout, double* Sout) {
   }
   SKEMA_CUDA(cudaStreamSynchronize(c->stream));
 }
-
-size_t jacobi_rot_bytes() { return kJacRotBytes; }
 
 void dgemm_f32_f64(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const float* A, int64_t ars,
                    int64_t acs, const double* B, int64_t brs, int64_t bcs, double beta, double* C, int64_t crs,
@@ -2116,7 +2119,7 @@ void low_rank_approx_rows(skema_ctx* c, int64_t row0, int64_t nrows, const RankS
   const size_t b_w = sizeof(double) * cholqr_work_doubles(std::max(m, std::max(n, s)), k);
   const size_t b_u = sizeof(double) * (size_t)(s * k);
   const size_t b_small = sizeof(double) * (size_t)(12 * k * k + s * s + k * s + 4 * k + 64);
-  Carve cv(c, {b_q, b_p, b_w, b_u, b_u, b_small, 16});
+  Carve cv(c, {b_q, b_p, b_w, b_u, b_u, b_small, kStatusBytes});
   double* Q = cv.take(b_q);
   double* P = cv.take(b_p);
   double* W = cv.take(b_w);
@@ -2136,7 +2139,7 @@ void low_rank_approx_rows(skema_ctx* c, int64_t row0, int64_t nrows, const RankS
   double* TP = TQ + k * k;         // k x k: the basis of X^T is P TP
   double* WU = TP + k * k;         // k x r
   double* WV = WU + k * k;         // k x r
-  int* st = reinterpret_cast<int*>(cv.take(16));
+  int* st = reinterpret_cast<int*>(cv.take(kStatusBytes));
 
   auto orth_scope = std::make_unique<StageScope>(c, ST_A_ORTH);
   f2d_kernel<<<g1(c, s * s), 256, 0, c->stream>>>(c->Z, s, 1, Zd, 1, s, s, s);
@@ -2172,7 +2175,7 @@ void low_rank_approx_rows(skema_ctx* c, int64_t row0, int64_t nrows, const RankS
     double* Cw = W;  // k x k working copy
     dtranspose_kernel<<<g1(c, k * k), 256, 0, c->stream>>>(Z2t, Cw, k);
     SKEMA_LAUNCHED(c);
-    jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st + 1);
+    jacobi_svd(c, Cw, Vc, k, 60, 1e-15, st);
     svd_finish_kernel<<<1, kFinishThreads, 0, c->stream>>>(Cw, Vc, k, C, Z2 /*Vout*/, Sv, sig);
     SKEMA_LAUNCHED(c);
   }

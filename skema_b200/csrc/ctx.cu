@@ -464,9 +464,7 @@ int skema_create(const skema_params* p, skema_ctx** out) {
       tc_prepare_maps(c);
     }
     // device status block: int status at [0], the wait limit (ns) at [2..3]
-    // (16 bytes), then the Jacobi SVD's exchange buffer
-    SKEMA_CUDA(cudaMalloc(&c->dev_err, 256 + jacobi_rot_bytes()));
-    c->jac_rot = reinterpret_cast<char*>(c->dev_err) + 256;
+    SKEMA_CUDA(cudaMalloc(&c->dev_err, 4 * sizeof(int)));
     SKEMA_CUDA(cudaMemsetAsync(c->dev_err, 0, 4 * sizeof(int), c->stream));
     set_wait_limit(c, 0);
     if (!c->spd) {

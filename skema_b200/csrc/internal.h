@@ -197,9 +197,6 @@ struct skema_ctx {
   // the device word is refused (x3.h): the second form of a call whose first is
   // on the tensor cores. Null: they run.
   const uint32_t* run_if = nullptr;
-  // The rotations that the Jacobi SVD's two CTAs exchange (approx.cu), in the
-  // allocation of dev_err.
-  void* jac_rot = nullptr;
   // What may have set it since it was last read: 0 nothing, 1 the FP32 form
   // (x3.cu), 2 a BF16 or FP8 kernel.
   int dev_err_armed = 0;
@@ -345,7 +342,6 @@ void rbf_vjp(skema_ctx* c, const float* pts, int64_t N, int64_t d,
              float* dpts, double* dgamma);
 
 // ---- FP64 approximation (approx.cu) ----
-size_t jacobi_rot_bytes();
 void low_rank_approx(skema_ctx* c, double* U, double* S, double* V);
 // Rows [row0, row0 + nrows) of a row-block sharded sketch, sums over the
 // ranks through fn (skema_low_rank_approx_rows).
