@@ -241,8 +241,9 @@ void dgemm(skema_ctx* c, int64_t M, int64_t N, int64_t K, double alpha, const TA
 // fragments read from global memory by every warp that needs them).
 constexpr int kGramTiles = 6, kGramLd = 36;
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT <= 3 ? 384 : 512, NT <= 3 ? 2 : 1) gram_mma_kernel(const T* __restrict__ A, int64_t lda, int k, int64_t rows,
-                                                          double* __restrict__ G, int64_t rows_per_cta) {
+__global__ void __launch_bounds__(NT <= 3 ? 384 : 512, NT <= 3 ? 2 : 1)
+    gram_mma_kernel(const T* __restrict__ A, int64_t lda, int k, int64_t rows, double* __restrict__ G,
+                    int64_t rows_per_cta) {
   extern __shared__ __align__(16) double gr_smem[];  // (k up to 16) x kGramLd
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, lr = lane & 3, lc = lane >> 2;
   const int nm = (k + 15) >> 4, nn = (k + 7) >> 3;
@@ -1102,19 +1103,19 @@ __device__ __forceinline__ void robin_pair(int np, int round, int pr, int& p, in
 // per lane), writing every (cs, sn) of the sweep to rot; CTA 1 holds V and
 // applies the sweep before, rows along the threads and the round's pairs over
 // groups of threads. So a round is one read and one write of A, its dot products
-// and one angle; V's traffic and FP64 work (as much again) are off that chain. A sweep without a rotation
-// (every pair within tol of orthogonal) ends the loop.
+// and one angle; V's traffic and FP64 work (as much again) are off that chain. A
+// sweep without a rotation (every pair within tol of orthogonal) ends the loop.
 // rot: two buffers of (kp - 1) (kp / 2) double2, kp = k rounded up to even, and
-// two flags after them. k = 81, 11 sweeps: 1.18 ms (2,500 cycles a round: the chain of
-// dependent FP64 operations and 1,000 cycles of shared memory); one CTA with A
-// and V took 1.80.
+// two flags after them. k = 81, 11 sweeps: 1.18 ms (2,500 cycles a round: the
+// chain of dependent FP64 operations and 1,000 cycles of shared memory); one CTA
+// with A and V took 1.80.
 constexpr int kJacMaxK = 114;
 constexpr size_t kJacRotBytes = sizeof(double2) * 2 * (kJacMaxK - 1) * (kJacMaxK / 2) + 16;
 
 template <int EPL>
-__global__ void __launch_bounds__(EPL == 8 ? 960 : 128 * EPL) jacobi_svd_kernel(double* __restrict__ Ag, double* __restrict__ Vg, int k,
-                                                            int max_sweeps, double tol, double2* rot,
-                                                            int* sweeps_out) {
+__global__ void __launch_bounds__(EPL == 8 ? 960 : 128 * EPL)
+    jacobi_svd_kernel(double* __restrict__ Ag, double* __restrict__ Vg, int k, int max_sweeps, double tol, double2* rot,
+                      int* sweeps_out) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) double jac_smem[];
@@ -1404,11 +1405,11 @@ __global__ void __launch_bounds__(256, 1) jacobi_cluster_kernel(double* Ag, doub
 }
 
 // Block one-sided Jacobi for k above the cluster form, or where the device has
-// no room for its cluster: one launch per outer round. The columns are cut into nb blocks of bs (the last ones short or
-// empty). An outer round pairs the blocks round-robin; each CTA takes one
+// no room for its cluster: one launch per outer round. The columns are cut into
+// nb blocks of bs (the last ones short or empty). An outer round pairs the blocks round-robin; each CTA takes one
 // pair (I, J), copies the up to 2 bs columns of A and V into shared memory,
 // runs one inner sweep of the one-sided Jacobi rotations over all pairs of
-// those columns (a half-warp per pair, as in the single-CTA kernel), and
+// those columns (a half-warp per pair, as in jacobi_svd_kernel), and
 // writes them back. rotated[0] is set when any rotation was made. nb - 1
 // outer rounds make an outer sweep, after which every pair of columns has
 // met; sweeps continue until one makes no rotation.
@@ -1504,7 +1505,7 @@ __global__ void __launch_bounds__(1024) jacobi_block_kernel(double* __restrict__
 
 __global__ void store_int_kernel(int* dst, int v) { *dst = v; }
 
-// One-sided Jacobi for k above the single-CTA size: block sweeps driven
+// One-sided Jacobi by jacobi_block_kernel: block sweeps driven
 // from the host, each outer sweep's rotation flag read back once.
 void jacobi_svd_blocked(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, double tol,
                         int* sweeps_out) {
@@ -1581,7 +1582,11 @@ void jacobi_svd(skema_ctx* c, double* A, double* V, int64_t k, int max_sweeps, d
     auto go = [&](auto kern) {
       return launch_one_cluster(c, kern, 2, threads, smem, A, V, (int)k, max_sweeps, tol, rot, sweeps_out);
     };
-    if (k <= 32 ? go(jacobi_svd_kernel<2>) : k <= 64 ? go(jacobi_svd_kernel<4>) : k <= 96 ? go(jacobi_svd_kernel<6>) : go(jacobi_svd_kernel<8>)) return;
+    if (k <= 32   ? go(jacobi_svd_kernel<2>)
+        : k <= 64 ? go(jacobi_svd_kernel<4>)
+        : k <= 96 ? go(jacobi_svd_kernel<6>)
+                  : go(jacobi_svd_kernel<8>))
+      return;
   } else if (k <= kJacClusterMaxK) {
     const int nb = (int)((k + 15) / 16 * 2);
     const size_t smem = sizeof(double) * 2 * 16 * (size_t)tri_ld((int)k);
@@ -1656,8 +1661,8 @@ void tri_solve(skema_ctx* c, const double* R, int64_t k, double* B, int64_t ldb,
                const int* status) {
   // up to four warps a CTA, as many as have room for their right-hand sides
   const size_t warp_bytes = sizeof(double) * 8 * (size_t)tri_ld((int)k);
-  const int warps =
-      (int)std::max<size_t>(1, std::min<size_t>({4, (size_t)(nrhs + 7) / 8, (226 * 1024 - packed_smem_bytes(k)) / warp_bytes}));
+  const size_t room = (226 * 1024 - packed_smem_bytes(k)) / warp_bytes;
+  const int warps = (int)std::max<size_t>(1, std::min<size_t>({4, (size_t)(nrhs + 7) / 8, room}));
   const size_t smem = packed_smem_bytes(k) + warps * warp_bytes;
   SKEMA_CUDA(cudaFuncSetAttribute(tri_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (int)((nrhs + 8 * warps - 1) / (8 * warps));

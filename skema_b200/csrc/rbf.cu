@@ -4,9 +4,11 @@
 //
 // K(i, j) = exp(-gamma * sum_f (x_if - x_jf)^2) with explicit differences
 // (the reference's formula, src/Skema_Kernel.cpp:37-44), and K(i, i) = 1
-// (src/Skema_Kernel.cpp:62-74). Kernel rows are produced a window at a time
-// into a scratch block and consumed by the dense sketch of the same window;
-// the window is reused for the next one, so K never exists as a whole.
+// (src/Skema_Kernel.cpp:62-74). Kernel rows are made a block at a time and
+// consumed by the sketch products of the same block, so K never exists as a
+// whole: as BF16 planes for the tensor-core FP32 form (rbf_planes_kernel, blocks
+// of up to 2 GB that need not follow the windows), or as FP32 rows, a window at
+// a time, for the SIMT form (rbf_tile_kernel).
 //
 // VJP of Y = K Omega~^T with respect to gamma and the points, given
 // Ybar = dL/dY:  M = Ybar Omega~,  E = M o K,
@@ -149,9 +151,9 @@ __global__ void __launch_bounds__(256)
 // GRAD: the planes hold E = M o K with M = Ybar Omega~ formed beside the
 // distances (k more FP32 instructions per entry; as a product of its own it
 // cost an FP32 block written and read back: forward and adjoint at N = 20,000,
-// d = 24, k = 65 took 8.0 ms, now 6.1, this kernel 3.1 of them), E_ii = 0 (the diagonal's terms of the gradient cancel), and the sums
-// -E d^2, rowsum(E) and colsum(E) as rbf_tile_kernel<1> adds them; E's magnitudes
-// are noted in *word.
+// d = 24, k = 65 took 8.0 ms, now 6.1, this kernel 3.1 of them), E_ii = 0 (the
+// diagonal's terms of the gradient cancel), and the sums -E d^2, rowsum(E) and
+// colsum(E) as rbf_tile_kernel<1> adds them; E's magnitudes are noted in *word.
 struct RbfGrad {
   const float* Ybar;   // N x k row-major
   const float* omega;  // k x N row-major
@@ -557,12 +559,13 @@ static bool rbf_vjp_x3(skema_ctx* c, const float* pts, int64_t N, int64_t d, flo
   // the sums and the words behind them
   SKEMA_CUDA(cudaMemsetAsync(rs, 0, 2 * b_v + b_s + b_w, c->stream));
   SKEMA_CUDA(cudaMemsetAsync(dgamma, 0, sizeof(double), c->stream));
-  const int top = (126 - x3_log2(N)) / 2;  // of E and of X: sums of N products
-  x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, top, flag);
+  // sums of N products of E and X: points far below 2^36, cotangents anywhere
+  const int top_x = 36, top_e = std::min(100, 126 - x3_log2(N) - top_x);
+  x3_transposed_planes(c, pts, d, N, d, Xp, ldN, d * ldN, 1.f, 1, 1, 0, top_x, flag);
   for (int64_t r = 0, i = 1; r < N; r += rb, ++i) {
     const int64_t wr = std::min(rb, N - r), nrb = (wr + 63) / 64;
     const X3Words words{flag + i, flag};
-    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, x3_bits(top), flag + i};
+    const RbfGrad g{Ybar, omega, k, dgamma, rs, cs, x3_bits(top_e), flag + i};
     launch_planes(c, pts, N, d, gamma, r, wr, Ep, nrb * 64 * N, &g);
     x3_gemm(c, X3A{Ep, true, true, N, nrb, 0, 0}, X3B{Xp, ldN, d * ldN}, wr, d, N,
             tc::X3Out{S + r * d, d, 1, 1.f, 1.f, nullptr, 0, 0, wr, d, d}, part, words);
