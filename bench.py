@@ -290,10 +290,15 @@ def run_vjp(args, cfg, peaks, peak_kind):
                 "kernel": "rbf_sketch_kernel (forward) + 2 x rbf_vjp_kernel (adjoint)", "kernel_ms": ms,
                 "algorithmic_flops_per_step": flops, "traffic": None}
     else:
-        roof = {"bound": "fp32-simt", "achieved": flops / (ms / 1e3) / 1e12, "peak": 74.4, "unit": "TFLOP/s",
-                "frac": flops / (ms / 1e3) / 1e12 / 74.4,
+        # rbf_planes_kernel makes the kernel entries twice by explicit differences
+        # (two FP32 instructions each per feature) and M beside the second (one per
+        # column of Omega): its issue slots, counted as two flops, bound the step.
+        # The products of the planes are tensor-core work.
+        slots = 2.0 * N * N * (4 * d + k)
+        roof = {"bound": "fp32-simt", "achieved": slots / (ms / 1e3) / 1e12, "peak": 74.4, "unit": "TFLOP/s",
+                "frac": slots / (ms / 1e3) / 1e12 / 74.4,
                 "peak_source": "nominal FP32 SIMT (148 SMs x 128 FMA/clk x 2 x 1.965 GHz)",
-                "kernel": "sgemm_kernel + rbf_tile_kernel (forward and adjoint)", "kernel_ms": ms,
+                "kernel": "rbf_planes_kernel (forward and adjoint), beside gemm_x3_kernel", "kernel_ms": ms,
                 "algorithmic_flops_per_step": flops, "traffic": None}
     acc = None
     if rank == 0 and world == 1 and not args.no_accuracy:

@@ -1051,13 +1051,16 @@ __global__ void colsparse_apply_smem_kernel(const uint32_t* __restrict__ mp, int
 // tan of the angle is the smaller root of t^2 + 2 zeta t - 1 with zeta = d / h,
 // d = beta - alpha, h = 2 gamma, t = sign(d) h / (|d| + sqrt(d^2 + h^2)). It is
 // on the chain that every round waits for, and a dependent FP64 operation takes
-// about 30 cycles, so (c0, s0) comes from FP32 (d and h scaled by a power of
-// two) and one Newton step corrects it in FP64: the rotated product is
+// 9 cycles with up to four warps on the SM, 13 with 16 and 25 with 32 (a square
+// root or a division many of them), so (c0, s0) comes from FP32 (d and h scaled by
+// a power of two) and one Newton step corrects it in FP64: the rotated product is
 //   F = (c0^2 - s0^2) h / 2 - c0 s0 d,  delta = F / (sign(d) sqrt(d^2 + h^2)),
 // the angle moves by delta (1e-7, so its square is FP64 rounding) and the pair
 // is normalised by 1 - e / 2 + 3 e^2 / 8 - delta^2 / 2, e = c0^2 + s0^2 - 1, which
-// needs neither the corrected values nor a square root. False: the pair is
-// orthogonal to tol and stays.
+// needs neither the corrected values nor a square root. cs^2 + sn^2 is one to
+// 4e-16, as by FP64 square roots; the product falls to 1e-12 of itself or less
+// (3e-15 by them), and the next sweep, which there is unless every pair is within
+// tol, sees the rest. False: the pair is orthogonal to tol and stays.
 __device__ __forceinline__ bool jacobi_angle(double al, double be, double ga, double tol2, double& cs, double& sn) {
   cs = 1.0, sn = 0.0;
   if (ga == 0.0 || ga * ga <= tol2 * (al * be)) return false;

@@ -709,8 +709,7 @@ TcSlices xt_window(skema_ctx* c, Mat Aw, int64_t R0, int64_t wr, __nv_bfloat16* 
 // before and then for its own first loads, which a window of a few MB never
 // made up for: 33,228 x 931 in windows of 3,136 rows (k = 129, s = 259) went
 // from 835 to 351 us, 60,000 x 9,000 in 4,096s (k = 201) from 2.21 to 1.66 ms.
-// 200,000 x 20,000 in 8,192s, 10.6 before and BF16NOW now, differ by no more than its
-// runs do.
+// 200,000 x 20,000 in 8,192s, 10.6 ms before and 10.1 now, differs by what its runs do.
 bool xt_batchable(Mat Aw, int64_t R0) {
   const bool al = reinterpret_cast<uintptr_t>(Aw.p) % 16 == 0;
   return al && R0 % 8 == 0 && ((Aw.rs == 1 && Aw.cs % 4 == 0) || (Aw.cs == 1 && Aw.rs % 4 == 0));

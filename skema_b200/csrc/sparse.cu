@@ -398,7 +398,8 @@ __global__ void csr_gauss_scatter_kernel(const int64_t* __restrict__ rowptr,
 // of the tensor-core product Z += Phi^T T (T32 null), or as FP32 columns of
 // ldt when T is refused (x3.h; run again under *cond).
 // Bound by the gathered bytes, 4 (k + s) per nonzero out of L2: 100,000 x
-// 20,000 with 1e6 nonzeros at k = 81, s = 163 takes 178 us, 5.4 TB/s. With all
+// 20,000 with 1e6 nonzeros at k = 81, s = 163 takes 178 us, 5.4 TB/s, with rows of
+// log-normal lengths, and 135 with rows of ten entries. With all
 // 244 columns in one pass of eight slots it took 338 (the loads of a group not
 // all in flight) and 588 us (144 registers, one CTA per SM); 64 registers and
 // four CTAs per SM are what pays.
@@ -470,7 +471,8 @@ __device__ __forceinline__ void gauss_tile(const GaussGather& g, int64_t r0, int
     i = __shfl_sync(0xffffffffu, i, 0);
     if (i >= nr) return;
     float acc[NU];
-    gauss_row<NU>(g, g.rowptr[r0 + i] - g.col_offset, g.rowptr[r0 + i + 1] - g.col_offset, map, stride, cols, lane, acc);
+    gauss_row<NU>(g, g.rowptr[r0 + i] - g.col_offset, g.rowptr[r0 + i + 1] - g.col_offset, map, stride, cols, lane,
+                  acc);
 #pragma unroll
     for (int u = 0; u < NU; ++u) tile[(lane + 32 * u) * 33 + i] = acc[u];
   }
@@ -784,7 +786,7 @@ static void launch_csr_ssign_y(skema_ctx* c, const int64_t* rowptr, const int32_
 // CSR x Gauss over all windows of a call (src/Skema_SketchySVD.cpp:296-316):
 // Z = nu^G Z + eta sum_i w_i Phi(i, :)^T T(i, :) with T = A Psi, the
 // association of the dense form, instead of an n x s scatter and an n-deep
-// product per window: 3.64 -> 0.46 ms for 100,000 x 20,000, 1e6 nonzeros, ten
+// product per window: 3.64 -> 0.44 ms for 100,000 x 20,000, 1e6 nonzeros, ten
 // windows, k = 81, s = 163. False when the workspace is not to be had.
 static bool csr_gauss_update(skema_ctx* c, const int64_t* rowptr, const int32_t* col, const float* val,
                              int64_t col_offset, int64_t row0, int64_t nrows, float ybeta) {

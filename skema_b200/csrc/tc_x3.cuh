@@ -12,9 +12,9 @@
 // What bounds it: six BF16 MMAs per FP32 one, so 1/6 of the BF16 tensor rate
 // (about 230 TFLOP/s of FP32 work at the measured sustained 1400) against 74
 // nominal and 31-37 measured for the SIMT kernel. Whole sketch updates: 50,000
-// x 20,000 at k = 201, s = 403 in 52.2 -> 11.2 ms; the RBF kernel of 40,000
-// points (d = 100, k = 129, s = 259) in 102.6 -> 25.0 ms; 3001 x 1003 in six
-// windows in 2.42 -> 0.15 ms.
+// x 20,000 at k = 201, s = 403 in 52.4 -> 11.1 ms; the RBF kernel of 40,000
+// points (d = 100, k = 129, s = 259) in 102.5 -> 24.6 ms; 3001 x 1003 in six
+// windows in 2.42 -> 0.12 ms.
 //
 // Accuracy. tcgen05 accumulates in FP32 without round-to-nearest, so a long
 // run of MMAs on one accumulator drifts towards zero. Each K step of 32 is
