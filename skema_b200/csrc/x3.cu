@@ -42,7 +42,7 @@ __device__ __forceinline__ void store_planes8(const float* v, __nv_bfloat16* d, 
 __global__ void __launch_bounds__(256)
     x3_block_vec_kernel(const float* __restrict__ S, int64_t scs, int64_t rows, int64_t cols,
                         __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t big,
-                        uint32_t* __restrict__ flag) {
+                        uint32_t small, uint32_t* __restrict__ flag) {
   const int64_t total = nrb * 8 * cols;
   float top = 0.f;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -63,14 +63,14 @@ __global__ void __launch_bounds__(256)
     for (int t = 0; t < 8; ++t) x3_note(top, v[t]);
     store_planes8(v, D + (rb * cols + j) * 64 + (w & 7) * 8, pstride);
   }
-  x3_report(top, big, flag);
+  x3_report(top, big, flag, small);
 }
 
 // The same from any strides, by 64 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256)
     x3_block_tiled_kernel(const float* __restrict__ S, int64_t srs, int64_t scs, int64_t rows, int64_t cols,
                           __nv_bfloat16* __restrict__ D, int64_t nrb, int64_t pstride, uint32_t big,
-                          uint32_t* __restrict__ flag) {
+                          uint32_t small, uint32_t* __restrict__ flag) {
   __shared__ float tile[32][65];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t tj = (cols + 31) / 32;
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256)
     }
     __syncthreads();
   }
-  x3_report(top, big, flag);
+  x3_report(top, big, flag, small);
 }
 
 // Map columns [0, cols) of up to two row-contiguous FP32 sources into one
@@ -365,14 +365,15 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
 }
 
 void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride, int top,
-                     uint32_t* flag) {
+                     int bottom, uint32_t* flag) {
   const int64_t nrb = (rows + 63) / 64;
   if (src.rs == 1 && src.cs % 4 == 0 && reinterpret_cast<uintptr_t>(src.p) % 16 == 0)
     x3_block_vec_kernel<<<grid_1d(c, nrb * 8 * cols, 16), 256, 0, c->stream>>>(src.p, src.cs, rows, cols, D, nrb,
-                                                                               pstride, x3_bits(top), flag);
+                                                                               pstride, x3_bits(top), x3_bits(bottom),
+                                                                               flag);
   else
     x3_block_tiled_kernel<<<grid_1d(c, nrb * ((cols + 31) / 32) * 256, 16), 256, 0, c->stream>>>(
-        src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, x3_bits(top), flag);
+        src.p, src.rs, src.cs, rows, cols, D, nrb, pstride, x3_bits(top), x3_bits(bottom), flag);
   SKEMA_LAUNCHED(c);
 }
 
@@ -474,7 +475,7 @@ static bool x3_windows(skema_ctx* c, const X3Input& in, int64_t row0, int64_t nr
     {
       StageScope st(c, ST_WINDOW);
       if (in.A.p)
-        x3_block_planes(c, Aw, wr, n, Ap, ps, top, flag);
+        x3_block_planes(c, Aw, wr, n, Ap, ps, top, s > 0 ? std::max(-90, -102 - x3_exp(c->psi)) : -90, flag);
       else
         in.fill(R0, wr, Ap, ps);
       if (s > 0) {

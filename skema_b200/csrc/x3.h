@@ -14,7 +14,8 @@ namespace skema {
 // The range of the planes. The low planes of a value below about 2^-109 reach
 // BF16's smallest step (2^-133) and lose bits, so what counts is the largest
 // magnitude of a block of values: from 2^-90 on, what the smaller ones lose is
-// below 2^-44 of it. Upwards, what counts is that the sums stay within FP32's
+// below 2^-44 of it. (A block of A that meets a map of small values needs as much
+// more as leaves T = A Psi at 2^-102.) Upwards, what counts is that the sums stay within FP32's
 // range: an infinity, or one in a plane, turns into a NaN where FP32 arithmetic
 // has an infinity. The bound, 2^100 at most, follows from the length of the sums
 // and the other operand's largest value (x3_top).
@@ -32,23 +33,23 @@ inline int x3_log2(int64_t n) {
   return e;
 }
 // A bound 2^e on a map's magnitudes, and whether planes carry the map: its
-// largest value is finite, and far enough up that T = A Psi is no smaller than
-// 2^-102 where A reaches 2^-90.
-inline int x3_exp(const Map& mp) { return mp.amax > 0.f ? std::max(-12, std::ilogb(mp.amax) + 1) : -12; }
-inline bool x3_carries(const Map& mp) { return mp.amax == 0.f || (mp.amax >= 0x1p-12f && mp.amax <= 0x1p100f); }
+// largest value is finite, and far enough up that a weight of 2^-40 leaves it
+// all its bits.
+inline int x3_exp(const Map& mp) { return mp.amax > 0.f ? std::max(-50, std::ilogb(mp.amax) + 1) : -50; }
+inline bool x3_carries(const Map& mp) { return mp.amax == 0.f || (mp.amax >= 0x1p-50f && mp.amax <= 0x1p100f); }
 __host__ __device__ __forceinline__ bool x3_refused(uint32_t w) {
   return (w & kX3Big) || (w & (kX3Normal | kX3Tiny)) == kX3Tiny;
 }
 // m: the largest of this thread's magnitudes (fmaxf passes a NaN over)
 __device__ __forceinline__ void x3_note(float& m, float x) { m = fmaxf(m, fabsf(x)); }
-// Notes the block's largest magnitude in *word, big from the bits `big` on;
-// called by all its threads.
-__device__ __forceinline__ void x3_report(float top, uint32_t big, uint32_t* word) {
+// Notes the block's largest magnitude in *word, big from the bits `big` on, tiny
+// below the bits `small`; called by all its threads.
+__device__ __forceinline__ void x3_report(float top, uint32_t big, uint32_t* word, uint32_t small = kX3SmallBits) {
   const uint32_t m = __float_as_uint(top);
   uint32_t kind = 0;
   if (__syncthreads_or(m >= big))
     kind = kX3Big;
-  else if (__syncthreads_or(m >= kX3SmallBits))
+  else if (__syncthreads_or(m >= small))
     kind = kX3Normal;
   else if (__syncthreads_or(m > 0))
     kind = kX3Tiny;
@@ -117,9 +118,9 @@ void x3_gemm(skema_ctx* c, const X3A& a, const X3B& b, int64_t M, int64_t N, int
              X3Words words);
 // A strided FP32 block into row-blocked planes (zero rows up to a multiple of
 // 64); its magnitudes are noted in *flag, 2^top and above as big, here and below
-// (null: not).
+// (null: not), those below 2^bottom (-90 elsewhere) as tiny.
 void x3_block_planes(skema_ctx* c, Mat src, int64_t rows, int64_t cols, __nv_bfloat16* D, int64_t pstride, int top,
-                     uint32_t* flag);
+                     int bottom, uint32_t* flag);
 
 // K-major planes of a row-major source's transpose: row i of S (rows x cols,
 // rs apart), scaled by nu^(nwin - 1 - (j0 + i) / W), is K index i; D holds

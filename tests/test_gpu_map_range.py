@@ -79,3 +79,14 @@ def test_overflow_is_an_infinity(lib_built, form, scales, ascale, A):
         assert not np.isnan(g).any(), q
         if fine.any():
             assert rel_fro(np.asarray(g, np.float64)[fine], w[fine]) < 1e-5, q
+
+
+@pytest.mark.parametrize("form", ["dense", "csr"])
+@pytest.mark.parametrize("scales,ascale", [((-40, -40, -40, -40), 0), ((0, 0, 0, -30), -70), ((-49, -30, -20, -45), -60)])
+def test_small_maps(lib_built, form, scales, ascale, A):
+    """Maps that planes carry although their values are small, with A on either side
+    of the bound that goes with Psi."""
+    got, want = _run(form, A * np.float32(2.0**ascale), scales, 0.5)
+    for q, g, w in zip("XYZ", got, want):
+        if np.abs(w).max() > 2.0**-100:  # else FP32 atomics and accumulators round at 2^-149
+            assert rel_fro(np.asarray(g, np.float64), w) < 1e-5, q
