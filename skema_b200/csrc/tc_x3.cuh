@@ -120,8 +120,8 @@ __device__ __forceinline__ void x3_store(const X3Out& o, int64_t row, int64_t co
 }
 
 // Eight columns. What beta scales is loaded ahead of the stores, which the
-// compiler cannot move it past: one after another, a tile of 208 columns and
-// one K step took 55 us, and a call of 16 x 20,000 (k = 201, s = 403) 605; 146 now.
+// compiler cannot move it past: one after another, a tile of 208 columns and one K
+// step took 55 us, and a call of 16 x 20,000 (k = 201, s = 403) 605; 146 now.
 __device__ __forceinline__ void x3_store8(const X3Out& o, int64_t row, int64_t col, const float* v) {
   if (o.beta != 0.f && col + 8 <= o.split) {
     float* p = o.p0 + row * o.rs0 + col * o.cs0;

@@ -15,10 +15,10 @@ namespace skema {
 // BF16's smallest step (2^-133) and lose bits, so what counts is the largest
 // magnitude of a block of values: from 2^-90 on, what the smaller ones lose is
 // below 2^-44 of it. (A block of A that meets a map of small values needs as much
-// more as leaves T = A Psi at 2^-102.) Upwards, what counts is that the sums stay within FP32's
-// range: an infinity, or one in a plane, turns into a NaN where FP32 arithmetic
-// has an infinity. The bound, 2^100 at most, follows from the length of the sums
-// and the other operand's largest value (x3_top).
+// more as leaves T = A Psi at 2^-102.) Upwards, what counts is that the sums stay
+// within FP32's range: an infinity, or one in a plane, turns into a NaN where FP32
+// arithmetic has an infinity. The bound, 2^100 at most, follows from the length of
+// the sums and the other operand's largest value (x3_top).
 // A kernel that makes planes notes in a device word which kinds it met; a block
 // that is all tiny, or holds a value from the bound on, is refused, and FP32
 // arithmetic forms its products. A NaN is a NaN in its planes too and counts for

@@ -82,9 +82,17 @@ def test_exactly_rank_deficient_sketches(lib_built, k, p):
         l0 = c.launch_count()
         Uo, So, Vo = c.low_rank_approx()
         launches = c.launch_count() - l0
+        # the same call on sketches of full rank
+        for which, t in ((L.SKETCH_X, X), (L.SKETCH_Y, Y), (L.SKETCH_Z, Z)):
+            c.set_sketch(which, rng.normal(size=t.shape).astype(np.float32))
+        l0 = c.launch_count()
+        c.low_rank_approx()
+        plain = c.launch_count() - l0
     A = a @ b.T
     Ua, Sa, Va = np.linalg.svd(A, full_matrices=False)
     best = (Ua[:, :r] * Sa[:r]) @ Va[:r]
     assert np.abs(Uo.T @ Uo - np.eye(r)).max() < 1e-9 and np.abs(Vo.T @ Vo - np.eye(r)).max() < 1e-9
     assert rel_fro((Uo * So) @ Vo.T, best) < 1e-5
-    assert launches > 80, launches  # a basis by way of the eigenvectors takes more than twice the 47 of a plain one
+    # a basis by way of the eigenvectors takes launches that a plain one does not;
+    # how many depends on which Cholesky fails first, and so on rounding
+    assert launches > plain, (launches, plain)
