@@ -807,13 +807,14 @@ __global__ void __launch_bounds__(kTriThreads)
 // registers. Two barriers per panel; bound by the chain of 8 reciprocal square
 // roots per panel and the FP64 FMAs of the update (k = 201: 128 us, and
 // 35 us for the inverse by tri_solve_kernel; one column at a time with a barrier
-// each, and the inverse column by column in the same CTA, took 690). Rinv (null:
-// not; k up to kCholInvMaxK): the inverse of R from the first warp, lane c column c
+// each, and the inverse column by column in the same CTA, took 690). INV (k up to
+// kCholInvMaxK): Rinv, the inverse of R, from the first warp, lane c column c
 // of L^-1 by forward substitution in registers, which for a small k is shorter
 // than a launch of tri_solve_kernel (k = 9, 300 x 300: the approximation's
 // eight factorisations took 30 us longer). Rinv may be G. status[0] = 0, or j + 1
 // when the j-th pivot is not positive (R and Rinv are then not written).
 constexpr int kCholThreads = 512, kCholInvMaxK = 32;
+template <bool INV>
 __global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double* G, int k, double* R, double* Rinv,
                                                                    int* status) {
   extern __shared__ double cf_smem[];
@@ -924,7 +925,7 @@ __global__ void __launch_bounds__(kCholThreads) chol_factor_kernel(const double*
       if (i < k) R[i + j * k] = (i <= j) ? L[lo_off(i, k) + j - i] : 0.0;
     }
   if (threadIdx.x == 0) status[0] = 0;
-  if (!Rinv || warp != 0) return;
+  if (!INV || warp != 0) return;
   const double inv = lane < k ? 1.0 / L[lo_off(lane, k)] : 0.0;
   double x[kCholInvMaxK];
 #pragma unroll
@@ -1689,9 +1690,10 @@ void trsm_upper(skema_ctx* c, const double* R, int64_t k, double* B, int64_t ldb
 void chol_inverse(skema_ctx* c, double* G, int64_t k, double* R, double* Rinv, int* st) {
   if (k <= kPackedMaxK) {
     const size_t smem = packed_smem_bytes(k);
-    SKEMA_CUDA(cudaFuncSetAttribute(chol_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const bool small = k <= kCholInvMaxK;
-    chol_factor_kernel<<<1, kCholThreads, smem, c->stream>>>(G, (int)k, R, small ? Rinv : nullptr, st);
+    auto kern = small ? chol_factor_kernel<true> : chol_factor_kernel<false>;
+    SKEMA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<1, kCholThreads, smem, c->stream>>>(G, (int)k, R, Rinv, st);
     SKEMA_LAUNCHED(c);
     if (!small) tri_solve(c, R, k, Rinv, k, k, true, st);
     return;
